@@ -209,11 +209,32 @@ static int32_t check_block(int body, const unsigned char* blk, size_t bytes) {
   return ETXB_OK;
 }
 
+// The batched step on the tensor cores: only its own tiles and grouped attention (any group size) -> its kernel.
+static bool batched_plan(const etxb_session* s, const std::vector<unsigned char>& pool) {
+  bool tc = false;
+  for (const etxb_type& ty : s->types) {
+    switch (ty.body) {
+      case ETXB_BODY_NOP: case ETXB_BODY_NORM_COL: case ETXB_BODY_ROUTE: case ETXB_BODY_PROLOGUE_NB: case ETXB_BODY_ARGMAX_NB: break;
+      case ETXB_BODY_GEMV_TC: case ETXB_BODY_MOE_UP_TC: case ETXB_BODY_MOE_DOWN_TC: tc = true; break;
+      case ETXB_BODY_ATTN_FUSED: {
+        etxb_attnf_args a;
+        if (ty.args[0] != 0 || ty.cst[1] != 0 || ty.cst[0] < 0 || (size_t)ty.cst[0] + sizeof a > pool.size()) return false;
+        memcpy(&a, pool.data() + ty.cst[0], sizeof a);
+        if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8)) return false;
+        break;
+      }
+      default: return false;
+    }
+  }
+  return tc;
+}
+
 // Which kernel can run this plan?  The lean decode kernels hold only the tiles of a fused decode step; a plan qualifies
 // when every grid is one of those tiles with its argument block in the pool (one block per grid) and the blocks stay
 // inside what the lean forms cover: norm folds of at most one row (or the flagged rows of a sharded model), top-k folds over at most 128 experts, grouped
 // attention (head_dim 128, cache blocks of 16, partitions of 128) with the same group size everywhere.
 static int select_variant(const etxb_session* s, const std::vector<unsigned char>& pool) {
+  if (batched_plan(s, pool)) return 11;
   int gq = 0;
   bool any_attn = false, any_mla = false;
   for (const etxb_type& ty : s->types) {
@@ -248,11 +269,13 @@ static int select_variant(const etxb_session* s, const std::vector<unsigned char
 // q heads per task (etxb_kernel.cuh, run_body).
 // Entries 5..9: the same five with the exchange code of a sharded session compiled in (launch_kernel adds 5).
 // Entry 10: the lean decode kernel of a latent-attention model (no sharded form: such a session falls back to entry 5).
-static const void* const g_kernels[11] = {(const void*)etxb::etxb_megakernel<0>, (const void*)etxb::etxb_megakernel<1>, (const void*)etxb::etxb_megakernel<2>,
+// Entry 11: the kernel of a batched step on the tensor cores.
+static const void* const g_kernels[12] = {(const void*)etxb::etxb_megakernel<0>, (const void*)etxb::etxb_megakernel<1>, (const void*)etxb::etxb_megakernel<2>,
                                           (const void*)etxb::etxb_megakernel<4>, (const void*)etxb::etxb_megakernel<8>,
                                           (const void*)etxb::etxb_megakernel<0, true>, (const void*)etxb::etxb_megakernel<1, true>,
                                           (const void*)etxb::etxb_megakernel<2, true>, (const void*)etxb::etxb_megakernel<4, true>,
-                                          (const void*)etxb::etxb_megakernel<8, true>, (const void*)etxb::etxb_megakernel<ETXB_VARIANT_MLA>};
+                                          (const void*)etxb::etxb_megakernel<8, true>, (const void*)etxb::etxb_megakernel<ETXB_VARIANT_MLA>,
+                                          (const void*)etxb::etxb_megakernel<ETXB_VARIANT_BATCH>};
 static int kernel_index(const etxb_session* s) {
   const int v = s->force_full ? 0 : s->variant;
   if (s->xbase == nullptr) return v;
@@ -985,7 +1008,7 @@ __global__ void __launch_bounds__(ETXB_CONSUMERS, 1) etxb_attn_static_kernel(con
   Smem sm;
   sm.xs = (float*)st_smem;
   sm.scr = (float*)(st_smem + ETXB_GEN_BYTES);
-  sm.ring = nullptr; sm.full = nullptr; sm.empty = nullptr; sm.prod = nullptr; sm.deadline = nullptr; sm.ctrl = nullptr; sm.stop = nullptr; sm.tr = nullptr; sm.tc = nullptr; sm.epoch = 0; sm.cur = 0;
+  sm.ring = nullptr; sm.full = nullptr; sm.empty = nullptr; sm.prod = nullptr; sm.deadline = nullptr; sm.stop = nullptr; sm.tc = nullptr; sm.geo = nullptr; sm.vars = nullptr;
   tile_attn_fused((const unsigned char*)&d, (int)blockIdx.x, sm, S);
 }
 }  // namespace etxb

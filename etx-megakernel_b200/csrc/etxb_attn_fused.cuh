@@ -16,7 +16,7 @@ namespace etxb {
 // One head row in shared memory (xh, HD floats; d = lane * epl + j held by lane): optional RMSNorm with weight nw, then
 // neox rotary with the cos | sin row cs (both as floats in shared memory).  o[j] = the bf16-rounded results.  One warp.
 template <int HDT>
-__device__ __noinline__ void head_norm_rope_s(const float* xh, const float* nw, const float* cs, int HDr, float eps, float* o) {
+__device__ __forceinline__ void head_norm_rope_s(const float* xh, const float* nw, const float* cs, int HDr, float eps, float* o) {
   const int HD = HDT ? HDT : HDr;                                  // HDT: head_dim as a compile-time constant (0: read it)
   const int lane = tidx() & 31, half = HD >> 1, epl = HD >> 5;
   constexpr int EPL = HDT ? HDT / 32 : 8;

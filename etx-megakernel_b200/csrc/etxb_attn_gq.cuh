@@ -49,9 +49,9 @@ __device__ __forceinline__ float poll_pair(const uint2* p, uint32_t fl, const Sm
     const uint2 v = ld_pair(p);
     if (v.y == fl) return __uint_as_float(v.x);
     if ((++spins & 63u) == 0) {
-      if (ld_relaxed(sm.ctrl) != 0) { *(volatile int*)sm.stop = 1; return 0.f; }
+      if (ld_relaxed(sm.ctrl()) != 0) { *(volatile int*)sm.stop = 1; return 0.f; }
       if ((spins & 1023u) == 0 && globaltimer() > *sm.deadline) {
-        if (atomicOr(sm.ctrl, ETXB_CTRL_TIMEOUT) == 0) { sm.ctrl[1] = sm.cur; sm.ctrl[2] = -3; sm.ctrl[3] = (int32_t)v.y; sm.ctrl[4] = (int32_t)fl; }
+        if (atomicOr(sm.ctrl(), ETXB_CTRL_TIMEOUT) == 0) { sm.ctrl()[1] = sm.cur(); sm.ctrl()[2] = -3; sm.ctrl()[3] = (int32_t)v.y; sm.ctrl()[4] = (int32_t)fl; }
         *(volatile int*)sm.stop = 1;
         return 0.f;
       }
@@ -86,7 +86,7 @@ static_assert(((8 + 2) + 3 + 8 + 2 + 32 + 8 + 32) * 128 * 4 + 128 <= ETXB_GEN_BY
 // The statistics AND the partial outputs are requested in one round (up to ETXB_GQ_NPR partitions out of registers), so the
 // tail of the attention phase is one L2 round trip after the slowest partition has published.
 template <int GQ>
-__device__ __noinline__ void attn_gq_merge(const etxb_attnf_args& d, const Smem& sm, int hq0, int np, uint32_t fl) {
+__device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Smem& sm, int hq0, int np, uint32_t fl) {
 #ifndef ETXB_GQ_NPR
 #define ETXB_GQ_NPR 12               // partitions merged out of registers in one round (a 1.5K context); measured against 16: 0.8 % faster
 #endif
@@ -174,8 +174,10 @@ __device__ __noinline__ void attn_gq_merge(const etxb_attnf_args& d, const Smem&
   mark(sm, 2);
 }
 
+// (inlined into the lean kernels, which hold one of it: a call takes the address of Smem, which then lives on the stack for
+// every tile of the kernel)
 template <int GQ>
-__device__ __noinline__ void attn_gq_impl(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S) {
+__device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S) {
   constexpr int HD = 128, BS = 16, X = 8, PL = ETXB_GQ_PART, HV = HD / 8;
   const int NKV = d.NKV, G = d.NH / NKV, NQG = d.NH / GQ;
   const int part = blk / NQG, qg = blk - part * NQG;
@@ -187,7 +189,7 @@ __device__ __noinline__ void attn_gq_impl(const etxb_attnf_args& d, int blk, con
   const int seq = (const void*)d.seq_lens == (const void*)S.seq_lens ? S.pos + 1 : __ldcg(d.seq_lens);
   const int t0 = part * PL;
   const int tid = tidx(), lane = tid & 31, warp = tid >> 5;
-  const uint32_t fl = pair_flag(sm.epoch, d.part_len);
+  const uint32_t fl = pair_flag(sm.epoch(), d.part_len);
   if (t0 < seq) {
     const GqSmem<GQ> s(sm.xs);
     const bool owner = pos >= t0 && pos < t0 + PL;                // this partition holds the position being written
@@ -380,7 +382,7 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 }
 
 template <int GQ>
-__device__ __noinline__ void attn_gq_seq(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S) {
+__device__ __forceinline__ void attn_gq_seq(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S) {
   constexpr int HD = 128, BS = 16, X = 8, PL = ETXB_GQ_PART, HV = HD / 8;
   const int NKV = d.NKV, G = d.NH / NKV;
   const int hq0 = blk * GQ, h = hq0 / G;
@@ -643,35 +645,6 @@ __device__ __noinline__ void attn_gq_seq(const etxb_attnf_args& d, int blk, cons
   mark(sm, 3);
   cp_async_wait0();
   csync();                                                         // the next task may overwrite the partials
-}
-
-// The grouped forms (gq > 0 in the argument block; head_dim 128, cache blocks of 16, partitions of 128): one task per
-// partition, or (part_len bit 24) one task per sequence and q group.
-__device__ __forceinline__ void tile_attn_gq(const unsigned char* a, int blk, const Smem& sm, const etxb_stepv& S) {
-  const etxb_attnf_args& d = *(const etxb_attnf_args*)a;
-  if (blk >= (int)d.nblocks || d.gq <= 0) return;
-  if (d.part_len & ETXB_GQ_WHOLE) {
-    switch (d.gq) {
-      case 1: attn_gq_seq<1>(d, blk, sm, S); break;
-      case 2: attn_gq_seq<2>(d, blk, sm, S); break;
-      case 4: attn_gq_seq<4>(d, blk, sm, S); break;
-      default: attn_gq_seq<8>(d, blk, sm, S); break;
-    }
-    return;
-  }
-  switch (d.gq) {
-    case 1: attn_gq_impl<1>(d, blk, sm, S); break;
-    case 2: attn_gq_impl<2>(d, blk, sm, S); break;
-    case 4: attn_gq_impl<4>(d, blk, sm, S); break;
-    default: attn_gq_impl<8>(d, blk, sm, S); break;
-  }
-}
-
-// Fused attention, either form: gq > 0 in the argument block selects the grouped forms above, else the general tile.
-__device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, const Smem& sm, const etxb_stepv& S) {
-  const etxb_attnf_args& d = *(const etxb_attnf_args*)a;
-  if (d.gq == 0) { tile_attn_fused(a, blk, sm, S); return; }
-  tile_attn_gq(a, blk, sm, S);
 }
 
 }  // namespace etxb

@@ -40,7 +40,7 @@ __device__ __forceinline__ uint2 ld_volatile8(const void* p) {
   asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
   return v;
 }
-__device__ __noinline__ void argmax_exchange(const etxb_params& p, const Smem& sm, float& bv, int& bi) {
+__device__ __forceinline__ void argmax_exchange(const etxb_params& p, const Smem& sm, float& bv, int& bi) {
   const uint32_t fl = row_flag(p.epoch);
   bi += p.rank * p.step.V;
   const int q_self = p.rank;
@@ -59,9 +59,9 @@ __device__ __noinline__ void argmax_exchange(const etxb_params& p, const Smem& s
       a = ld_volatile8(slot); b = ld_volatile8(slot + 8);
       if (a.y == fl && b.y == fl) break;
       if ((++spins & 63u) == 0) {
-        if (ld_relaxed(sm.ctrl) != 0) { *(volatile int*)sm.stop = 1; return; }
+        if (ld_relaxed(sm.ctrl()) != 0) { *(volatile int*)sm.stop = 1; return; }
         if ((spins & 1023u) == 0 && globaltimer() > *sm.deadline) {
-          if (atomicOr(sm.ctrl, ETXB_CTRL_TIMEOUT) == 0) { sm.ctrl[1] = sm.cur; sm.ctrl[2] = -100 - r; sm.ctrl[3] = (int32_t)(a.y >> 16); sm.ctrl[4] = (int32_t)(fl >> 16); }
+          if (atomicOr(sm.ctrl(), ETXB_CTRL_TIMEOUT) == 0) { sm.ctrl()[1] = sm.cur(); sm.ctrl()[2] = -100 - r; sm.ctrl()[3] = (int32_t)(a.y >> 16); sm.ctrl()[4] = (int32_t)(fl >> 16); }
           *(volatile int*)sm.stop = 1;
           return;
         }
@@ -166,57 +166,128 @@ __device__ __forceinline__ void fetch_ctx(const etxb_params& p, TaskCtx* ctx, in
   }
 }
 
+// The persistent kernel's shared memory beside the dynamic part.  At namespace scope so that the tiles that are calls find
+// it at known addresses too: passed by reference, Smem would live on the stack; passed by value, in registers.
+__shared__ int s_stop;
+__shared__ unsigned long long s_deadline;
+__shared__ GemvGeom s_geo;
+__shared__ CtaVars s_vars;
+__shared__ __align__(8) TcShared s_tc;                             // (used by the kernels of a batched plan only)
+__device__ __forceinline__ Smem smem_view() {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Smem sm;
+  sm.ring = smem_raw;
+  sm.xs = (float*)(smem_raw + ETXB_RING_BYTES);
+  sm.scr = (float*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES);
+  sm.full = (uint64_t*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4);
+  sm.empty = sm.full + ETXB_NSTAGE;
+  sm.prod = (int32_t*)(sm.empty + ETXB_NSTAGE) + 8;                 // (behind the notes of the stages' uses)
+  sm.deadline = &s_deadline; sm.stop = &s_stop; sm.tc = &s_tc; sm.geo = &s_geo; sm.vars = &s_vars;
+  return sm;
+}
+// A tile of the batched step.  These are calls: each tile gets the registers for itself (inlined side by side they spilled
+// into each other's paths).
+template <int B>
+__device__ __noinline__ void batch_call(const unsigned char* args, int c0, int cur, const etxb_stepv& S) {
+  const Smem sm = smem_view();
+  if constexpr (B == 18) tile_prologue_nb(args, c0, S);
+  else if constexpr (B == 13) tile_norm_col(args, c0, sm);
+  else if constexpr (B == 14) tile_gemv_nb(args, c0, sm);
+  else if constexpr (B == 15) tile_route(args, c0, sm);
+  else if constexpr (B == 16) tile_moe_up_g(args, c0, sm);
+  else if constexpr (B == 17) tile_moe_down_g(args, c0, sm);
+  else if constexpr (B == 20) tile_gemv_tc(args, c0, sm, s_tc, cur);
+  else if constexpr (B == 21) tile_moe_up_tc(args, c0, sm, s_tc, cur);
+  else if constexpr (B == 22) tile_moe_down_tc(args, c0, sm, s_tc, cur);
+  else if constexpr (B == 23) tile_mla_attn(args, c0, sm, S);
+  else if constexpr (B == 7) tile_attnprep(args, c0, sm, S);
+  else if constexpr (B == 8) tile_attn(args, c0, sm, S);
+  else if constexpr (B == 9) tile_attn_reduce(args, c0, sm, S);
+  else tile_attn_fused(args, c0, sm, S);
+}
+__device__ __noinline__ void argmax_col_call(const etxb_params& p, const unsigned char* args, int c0) {
+  const int nb = ((const etxb_batch_args*)args)->nb;
+  if (c0 < nb) tile_argmax<false>(p, smem_view(), c0, nb);
+}
+// Attention out of a kernel that holds all its forms, a call each: the grouped forms (gq > 0 in the argument block; head_dim
+// 128, cache blocks of 16, partitions of 128), one task per partition or (part_len bit 24) one per sequence and q group ..
+template <int GQ, bool WHOLE>
+__device__ __noinline__ void attn_call(const etxb_attnf_args& d, int blk, const etxb_stepv& S) {
+  if constexpr (WHOLE) attn_gq_seq<GQ>(d, blk, smem_view(), S);
+  else attn_gq_tile<GQ>(d, blk, smem_view(), S);
+}
+// .. and, in the full kernel, the general tile.
+template <bool GENERAL>
+__device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, int cur, const etxb_stepv& S) {
+  const etxb_attnf_args& d = *(const etxb_attnf_args*)a;
+  if (GENERAL && d.gq == 0) { batch_call<12>(a, blk, cur, S); return; }
+  if (blk >= (int)d.nblocks || d.gq <= 0) return;
+  const int form = (d.gq == 1 ? 0 : d.gq == 2 ? 1 : d.gq == 4 ? 2 : 3) + ((d.part_len & ETXB_GQ_WHOLE) ? 4 : 0);
+  switch (form) {
+    case 0: attn_call<1, false>(d, blk, S); break;
+    case 1: attn_call<2, false>(d, blk, S); break;
+    case 2: attn_call<4, false>(d, blk, S); break;
+    case 3: attn_call<8, false>(d, blk, S); break;
+    case 4: attn_call<1, true>(d, blk, S); break;
+    case 5: attn_call<2, true>(d, blk, S); break;
+    case 6: attn_call<4, true>(d, blk, S); break;
+    default: attn_call<8, true>(d, blk, S); break;
+  }
+}
+
 // Run the body of the task whose context is `c` on the consumer warps.
 // GQV: the kernel variant.  0 = every tile.  1, 2, 4, 8 = the lean decode kernel: only the tiles of a fused decode step
 // (prologue, argmax, the GEMV family with norm folds of at most one row and top-k folds over at most 128 experts, the
 // grouped attention tile with GQV q heads per task); ETXB_VARIANT_MLA = the lean kernel of a latent-attention model (the
-// same GEMV family with the latent-attention tile in place of the grouped one).  The host picks it from the plan (select_variant): the full
+// same GEMV family with the latent-attention tile in place of the grouped one); ETXB_VARIANT_BATCH = the tiles of a batched step
+// on the tensor cores.  The host picks it from the plan (select_variant): the full
 // kernel is 550 KB of code, of which a decode step uses a fraction scattered through it, and the step runs about 10 %
 // faster from the 150 KB kernel (instruction fetch).
 // XCH: the variants a sharded session launches -- the same bodies plus the exchange code (flagged-row folds of R = ranks
 // rows, row publishing after the body, the argmax exchange); compiled out of the others.
 #define ETXB_VARIANT_MLA 16
+#define ETXB_VARIANT_BATCH 32         // the batched step on the tensor cores: its tiles and the attention tiles, nothing else
 template <int GQV, bool XCH>
 __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c, int cur, const Smem& sm, uint32_t& n) {
   const unsigned char* args = c->args;
   const int c0 = c->r.c0, c1 = c->r.c1;
   constexpr bool LEAN = GQV != 0;
   constexpr bool SH = GQV == 0 || GQV == ETXB_VARIANT_MLA;         // always-on (shared) experts: the full kernel and the latent-attention variant
-  constexpr bool BATCH = GQV == 0;                                 // the tiles of a batched step: full kernel only (a lean kernel of just these
-                                                                   // tiles was measured: 1852 against 1873 tok/s at 32 sequences -- a batched task
-                                                                   // runs long enough in one code region for instruction fetch not to matter)
+  constexpr bool FULL = GQV == 0, BATCHED = GQV == ETXB_VARIANT_BATCH;
   // (a body this variant does not hold: the host picks the variant from the plan's bodies, so this is a corrupted record)
 #define ETXB_TILE(cond, call) if constexpr (cond) { call; } else { if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK); } break
   switch (c->r.body) {
     case 0: break;
-    case 1: tile_prologue(p.step); break;
-    case 2: tile_argmax<XCH>(p, sm); break;
-    case 3: tile_gemv<LEAN, XCH>(args, c0, sm, n, cur); break;
-    case 4: tile_moe_up<LEAN, XCH, SH>(args, c0, sm, n, cur); break;
-    case 5: tile_moe_down<LEAN, SH>(args, c0, sm, n, cur); break;
+    case 1: ETXB_TILE(!BATCHED, tile_prologue(p.step));
+    case 2: ETXB_TILE(!BATCHED, tile_argmax<XCH>(p, sm));
+    case 3: case 4: case 5: ETXB_TILE(!BATCHED, (tile_gemv_family<LEAN, XCH, SH>(c->r.body, args, c0, sm, n, cur)));
     case 12:
       if constexpr (GQV == ETXB_VARIANT_MLA) { if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK); }      // (the latent-attention variant has no GQA tile)
-      else if constexpr (LEAN) { if (c0 < (int)((const etxb_attnf_args*)args)->nblocks) attn_gq_impl<GQV ? GQV : 1>(*(const etxb_attnf_args*)args, c0, sm, p.step); }
-      else tile_attn_any(args, c0, sm, p.step);
+      else if constexpr (BATCHED) tile_attn_any<false>(args, c0, cur, p.step);
+      else if constexpr (LEAN) { if (c0 < (int)((const etxb_attnf_args*)args)->nblocks) attn_gq_tile<GQV ? GQV : 1>(*(const etxb_attnf_args*)args, c0, sm, p.step); }
+      else tile_attn_any<true>(args, c0, cur, p.step);
       break;
     case 6: ETXB_TILE(!LEAN, tile_topk(args, c0, sm));
-    case 7: ETXB_TILE(!LEAN, tile_attnprep(args, c0, sm, p.step));
-    case 8: ETXB_TILE(!LEAN, tile_attn(args, c0, sm, p.step));
-    case 9: ETXB_TILE(!LEAN, tile_attn_reduce(args, c0, sm, p.step));
+    case 7: ETXB_TILE(!LEAN, batch_call<7>(args, c0, cur, p.step));
+    case 8: ETXB_TILE(!LEAN, batch_call<8>(args, c0, cur, p.step));
+    case 9: ETXB_TILE(!LEAN, batch_call<9>(args, c0, cur, p.step));
     case 10: ETXB_TILE(!LEAN, tile_splitk_part(args, c0, c1, sm));
     case 11: ETXB_TILE(!LEAN, tile_splitk_sum(args, c0));
-    // batched decode (several columns per step): full kernel only
-    case 13: ETXB_TILE(BATCH, tile_norm_col(args, c0, sm));
-    case 14: ETXB_TILE(!LEAN, tile_gemv_nb(args, c0, sm));
-    case 15: ETXB_TILE(BATCH, tile_route(args, c0, sm));
-    case 16: ETXB_TILE(!LEAN, tile_moe_up_g(args, c0, sm));
-    case 17: ETXB_TILE(!LEAN, tile_moe_down_g(args, c0, sm));
-    case 18: ETXB_TILE(BATCH, tile_prologue_nb(args, c0, p.step));
-    case 19: ETXB_TILE(BATCH, (c0 < ((const etxb_batch_args*)args)->nb ? tile_argmax<false>(p, sm, c0, ((const etxb_batch_args*)args)->nb) : (void)0));
-    case 20: ETXB_TILE(BATCH && !XCH, tile_gemv_tc(args, c0, sm, *sm.tc, cur));
-    case 21: ETXB_TILE(BATCH && !XCH, tile_moe_up_tc(args, c0, sm, *sm.tc, cur));
-    case 22: ETXB_TILE(BATCH && !XCH, tile_moe_down_tc(args, c0, sm, *sm.tc, cur));
-    case 23: ETXB_TILE(!LEAN || GQV == ETXB_VARIANT_MLA, tile_mla_attn(args, c0, sm, p.step));
+    // batched decode (several columns per step)
+    case 13: ETXB_TILE(FULL || BATCHED, batch_call<13>(args, c0, cur, p.step));
+    case 14: ETXB_TILE(!LEAN, batch_call<14>(args, c0, cur, p.step));
+    case 15: ETXB_TILE(FULL || BATCHED, batch_call<15>(args, c0, cur, p.step));
+    case 16: ETXB_TILE(!LEAN, batch_call<16>(args, c0, cur, p.step));
+    case 17: ETXB_TILE(!LEAN, batch_call<17>(args, c0, cur, p.step));
+    case 18: ETXB_TILE(FULL || BATCHED, batch_call<18>(args, c0, cur, p.step));
+    case 19: ETXB_TILE(FULL || BATCHED, argmax_col_call(p, args, c0));
+    case 20: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<20>(args, c0, cur, p.step));
+    case 21: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<21>(args, c0, cur, p.step));
+    case 22: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<22>(args, c0, cur, p.step));
+    case 23:
+      if constexpr (GQV == ETXB_VARIANT_MLA) tile_mla_attn(args, c0, sm, p.step);
+      else { ETXB_TILE(FULL, batch_call<23>(args, c0, cur, p.step)); }
+      break;
     default:
       if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK);
       break;
@@ -240,6 +311,10 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
     etxb_gemv_args* pa = (etxb_gemv_args*)(sm.prod + 32);
     if (lane < 20) ((uint64_t*)pa)[lane] = __ldg((const uint64_t*)t->args + lane);
     __syncwarp();
+    GemvGeom gg;                                                   // (nor does the task's geometry)
+    gg.t = gemv_task(body, *pa, t->c0);
+    gemv_geom(body, gg);
+    const GemvTask gt = gg.t;
     const int sw = t->stream_word;
     if (sw != -1) {
       int good = 1;
@@ -256,9 +331,8 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
     } else if (ld_relaxed(p.ctrl) != 0) {
       break;
     }
-    const GemvTask gt = gemv_task(body, *pa, t->c0);
     if (gt.n > 0 && body != 3) gemv_routing<LEAN, SH>(*pa, sm.prod, (float*)(sm.prod + 16));
-    ok = produce_task<SH>(body, *pa, gt, sm.prod, n, sm, cur, p.trace ? p.trace + 8 * (size_t)t->id : nullptr);
+    ok = produce_task<SH>(body, *pa, gt, gg.rps, sm.prod, n, sm, cur, p.trace ? p.trace + 8 * (size_t)t->id : nullptr);
   }
   // Nothing is left in flight on a normal exit (the consumers waited for every stage).  When the step was abandoned,
   // wait (bounded) for the copies already issued before the CTA's shared memory goes away.
@@ -274,28 +348,13 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
 template <int GQV, bool XCH = false>
 __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_constant__ etxb_params p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_stop;
-  __shared__ unsigned long long s_deadline;
-  __shared__ __align__(8) TcShared s_tc;                           // (used by the full kernel of a batched plan only)
-  constexpr bool TC = GQV == 0 && !XCH;
-  Smem sm;
-  sm.ring = smem_raw;
-  sm.xs = (float*)(smem_raw + ETXB_RING_BYTES);
-  sm.scr = (float*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES);
-  sm.full = (uint64_t*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4);
-  sm.empty = sm.full + ETXB_NSTAGE;
-  sm.prod = (int32_t*)(sm.empty + ETXB_NSTAGE);
-  sm.deadline = &s_deadline;
-  sm.ctrl = p.ctrl;
-  sm.stop = &s_stop;
-  sm.tr = nullptr;
-  sm.tc = &s_tc;
-  sm.epoch = p.epoch;
-  sm.cur = 0;
+  constexpr bool TC = (GQV == 0 || GQV == ETXB_VARIANT_BATCH) && !XCH;
+  const Smem sm = smem_view();
   if (threadIdx.x == 0) {
     s_stop = 0;
+    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.cur = 0;
     s_deadline = globaltimer() + p.timeout_ns;
-    for (int i = 0; i < ETXB_NSTAGE; ++i) { mbar_init(sm.full + i, 1); mbar_init(sm.empty + i, ETXB_CONSUMER_WARPS); }
+    for (int i = 0; i < ETXB_NSTAGE; ++i) { mbar_init(sm.full + i, 1); mbar_init(sm.empty + i, ETXB_EMPTY_COUNT); ((uint32_t*)(sm.empty + ETXB_NSTAGE))[i] = 0xffffffffu; }
     if constexpr (TC) {
       for (int i = 0; i < ETXB_TC_MAXSTAGE; ++i) { mbar_init(s_tc.full + i, 1); mbar_init(s_tc.empty + i, 1); s_tc.lu[i] = 0; s_tc.mu[i] = 0; }
       for (int i = 0; i < 2; ++i) { mbar_init(s_tc.acc_full + i, 1); mbar_init(s_tc.acc_free + i, 4); s_tc.nfull[i] = 0; s_tc.nfree[i] = 0; }
@@ -305,20 +364,22 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
   }
   __syncthreads();
   if ((int)blockIdx.x >= p.n_workers) return;
+  {
   const int q0 = p.qbegin[blockIdx.x], q1 = p.qbegin[blockIdx.x + 1];
   if (threadIdx.x >= ETXB_CONSUMERS) {
-    producer_loop<GQV != 0, GQV == 0 || GQV == ETXB_VARIANT_MLA>(p, sm, q0, q1);
+    if constexpr (GQV != ETXB_VARIANT_BATCH)                        // (nothing is streamed through the ring in a batched plan)
+      producer_loop<GQV != 0, GQV == 0 || GQV == ETXB_VARIANT_MLA>(p, sm, q0, q1);
     return;
   }
-  TaskCtx* ctx = (TaskCtx*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4 + 512);
-  const bool fetcher = threadIdx.x >= ETXB_CONSUMERS - 32;          // the last consumer warp keeps the contexts coming
+  TaskCtx* const ctx = (TaskCtx*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4 + 512);
   if constexpr (TC) {
     // tensor memory for the tensor-core tiles of a batched plan: allocated once per launch by warp 0 (one CTA per SM, so
     // the columns are always there), freed by the same warp after the last task on every path out of the loop below
     if (p.tc_on != 0u && threadIdx.x < 32) tc_alloc(&s_tc.tmem);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
-  if (fetcher && q0 < q1) {
+  if (threadIdx.x == 0) { s_vars.q0 = q0; s_vars.q1 = q1; s_vars.cur = q0; }
+  if (threadIdx.x >= ETXB_CONSUMERS - 32 && q0 < q1) {
     fetch_ctx(p, ctx, q0, q0, -1);
     fetch_ctx(p, ctx, q0, q0 + 1 < q1 ? q0 + 1 : -1, -1);
     cp_async_wait_all();
@@ -326,11 +387,17 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
     fetch_ctx(p, ctx, q0, -1, q0);
     cp_async_wait_all();
   }
+  }
   csync();
+  // What the loop needs after a body it reads again from shared memory: held in registers across the calls (or the widest tiles) it
+  // would go to the stack, and a stack access that follows an event's acquire is a trip to L2 (the acquire empties the
+  // L1) -- the hand-off between two tiles of the batched step took 1 us more.
+  volatile CtaVars* const vars = &s_vars;
+  TaskCtx* const ctx = (TaskCtx*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4 + 512);
   uint32_t n = 0;                                                  // stages consumed so far (same count the producer keeps)
-  for (int cur = q0; cur < q1; ++cur) {
-    const TaskCtx* c = ctx + ((cur - q0) & (ETXB_CTX_SLOTS - 1));
-    if (threadIdx.x == 0) {
+  for (int cur = vars->q0; cur < vars->q1; ++cur) {
+    const TaskCtx* c = ctx + ((cur - vars->q0) & (ETXB_CTX_SLOTS - 1));
+    if (tidx() == 0) {
       const int in_n = c->r.in_n;
       if (p.trace) p.trace[8 * (size_t)c->r.id] = globaltimer();
       bool ok = true;                                              // wait_event polls the abort word itself
@@ -341,15 +408,28 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
         ok = wait_event(p, word, (int32_t)(p.epoch * (uint32_t)cnt), cur, s_deadline);
       }
       if (!ok) s_stop = 1;
+      s_vars.tr = p.trace ? p.trace + 8 * (size_t)c->r.id : nullptr;
+      s_vars.cur = cur;
       if (p.trace) p.trace[8 * (size_t)c->r.id + 1] = globaltimer();
+    } else if (GQV != ETXB_VARIANT_BATCH && tidx() == 32) {   // meanwhile: what the task multiplies and how the warps share it
+      const int body = c->r.body;
+      if (body >= 3 && body <= 5) {
+        GemvGeom g;
+        g.t = gemv_task(body, *(const etxb_gemv_args*)c->args, c->r.c0);
+        gemv_geom(body, g);
+        s_geo = g;
+      }
     }
     csync();
     if (s_stop) break;
-    if (fetcher) fetch_ctx(p, ctx, q0, cur + 2 < q1 ? cur + 2 : -1, cur + 1 < q1 ? cur + 1 : -1);   // asynchronous
-    sm.tr = p.trace ? p.trace + 8 * (size_t)c->r.id : nullptr;
-    if constexpr (XCH) sm.cur = cur;
-    run_body<GQV, XCH>(p, c, cur, sm, n);
-    if (fetcher) cp_async_wait_all();
+    if (tidx() >= ETXB_CONSUMERS - 32) {                            // the last consumer warp keeps the contexts coming (asynchronously)
+      const int q1 = vars->q1;
+      fetch_ctx(p, ctx, vars->q0, cur + 2 < q1 ? cur + 2 : -1, cur + 1 < q1 ? cur + 1 : -1);
+    }
+    run_body<GQV, XCH>(p, c, cur, smem_view(), n);
+    cur = vars->cur;                                               // (before the barrier: thread 0 moves it on behind it)
+    c = ctx + ((cur - vars->q0) & (ETXB_CTX_SLOTS - 1));
+    if (tidx() >= ETXB_CONSUMERS - 32) cp_async_wait_all();
     csync();                                                       // every consumer thread's stores are issued, the next contexts landed
     // Sharded model: warp 1 publishes the bf16 rows this task wrote as flagged words (value | this step's flag) into the
     // grid's block of every rank's exchange region, its own included -- plain 4-byte stores, over NVLink for the peers.
@@ -367,7 +447,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
         st_flagged((uint32_t*)p.xbase + off + i, v);
       }
     }
-    if (threadIdx.x == 0) {
+    if (tidx() == 0) {
       const int out_n = c->r.out_n, id = c->r.id;
       if (s_stop == 0)                                             // (set when a stage wait gave up inside the body: no arrivals then)
         for (int i = 0; i < out_n; ++i) {                          // release: orders the CTA's stores (seen through the barrier) before the count

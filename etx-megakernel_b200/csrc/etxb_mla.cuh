@@ -51,7 +51,7 @@ struct etxb_mla_args {
 __device__ __forceinline__ void mla_finish(const etxb_mla_args& d, const Smem& sm, int h, int f, int np) {
   const int C = d.C, DN = d.DN, DV = d.DV, PW = C + 8;
   const int tid = tidx(), lane = tid & 31, warp = tid >> 5;
-  const uint32_t fl = pair_flag(sm.epoch, d.tag << 16);
+  const uint32_t fl = pair_flag(sm.epoch(), d.tag << 16);
   float* oc = sm.xs;                                               // [C] merged, normalised latent
   float* wl = oc + 512;                                            // [np <= 64] max logits, then weights
   float* es = wl + 64;                                             // [np] exp sums
@@ -133,7 +133,7 @@ __device__ __forceinline__ void mla_finish(const etxb_mla_args& d, const Smem& s
   csync();
 }
 
-__device__ __noinline__ void tile_mla_attn(const unsigned char* a, int blk, const Smem& sm, const etxb_stepv& S) {
+__device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, const Smem& sm, const etxb_stepv& S) {
   const etxb_mla_args& d = *(const etxb_mla_args*)a;
   if (blk >= (int)d.nblocks || blk >= d.NH * (d.max_parts + ETXB_MLA_FIN)) return;
   const int part_i = blk / d.NH, h = blk - part_i * d.NH;            // part_i >= max_parts: finishing task part_i - max_parts of the head
@@ -148,7 +148,7 @@ __device__ __noinline__ void tile_mla_attn(const unsigned char* a, int blk, cons
   const int seq = min(seq_all - tbase, ETXB_MLA_PART);               // its positions: tbase .. tbase + seq - 1
   const bool owner = pos >= tbase && pos < tbase + ETXB_MLA_PART;    // the new position falls into this partition
   const int lpos = owner ? (int)pos - tbase : -1;
-  const uint32_t fl = pair_flag(sm.epoch, d.tag << 16);
+  const uint32_t fl = pair_flag(sm.epoch(), d.tag << 16);
   const int tid = tidx(), lane = tid & 31, warp = tid >> 5;
   float* qf = sm.xs;            // [QH <= 256] this head's q row
   float* kvf = qf + 256;        // [ROW <= 640] the raw kv_a row

@@ -138,7 +138,7 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core's reads
     csync();
-    if (sm.tr != nullptr && tid == 0 && pass == 0) sm.tr[4] = globaltimer();
+    if (sm.tr() != nullptr && tid == 0 && pass == 0) sm.tr()[4] = globaltimer();
     if (warp == 1 && lane == 0 && alive0) {                        // loader: every tile of the pass, chunk by chunk
       bool ok = true;
       int st = 0;
@@ -183,7 +183,7 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
         }
         if (ok) tc_commit(tc.acc_full + bsel);                     // the tile's MMAs (of this window) are complete
       }
-      if (sm.tr != nullptr && pass == npass - 1) sm.tr[5] = globaltimer();
+      if (sm.tr() != nullptr && pass == npass - 1) sm.tr()[5] = globaltimer();
     }
     __syncwarp();                                                  // the role threads' warp-mates wait here, not in a spin beside them
     // epilogue: warps 0, 4, 8, 12 own TMEM lanes 0..31 (one token per lane), a quarter of each box's 128 columns each.  Only

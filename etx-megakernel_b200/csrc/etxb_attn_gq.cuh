@@ -60,6 +60,20 @@ __device__ __forceinline__ float poll_pair(const uint2* p, uint32_t fl, const Sm
   }
 }
 
+// Between two rounds of a poll of several pairs: false when the step is being abandoned (deadline or abort, see poll_pair).
+__device__ __forceinline__ bool poll_again(uint32_t& spins, const Smem& sm) {
+  if ((++spins & 15u) == 0) {
+    if (ld_relaxed(sm.ctrl()) != 0) { *(volatile int*)sm.stop = 1; return false; }
+    if ((spins & 255u) == 0 && globaltimer() > *sm.deadline) {
+      if (atomicOr(sm.ctrl(), ETXB_CTRL_TIMEOUT) == 0) { sm.ctrl()[1] = sm.cur(); sm.ctrl()[2] = -3; sm.ctrl()[3] = 0; sm.ctrl()[4] = 0; }
+      *(volatile int*)sm.stop = 1;
+      return false;
+    }
+    __nanosleep(32);
+  }
+  return true;
+}
+
 template <int GQ>
 struct GqSmem {
   static constexpr int HD = 128, PL = ETXB_GQ_PART;
@@ -106,12 +120,18 @@ __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Sm
       if (idx < GQ * HD) {
         const int g = idx >> 7, dd = idx & (HD - 1);
         const uint2* tp = pw + (size_t)(hq0 + g) * d.max_parts * ETXB_GQ_PW + dd;
-        uint2 first[NPR];
+        // all requests in flight at once, all again while one is missing (a poll per pair, inlined NPR times, is 20 KB of code
+        // that the instruction cache has to hold)
+        bool ok;
+        uint32_t spins = 0;
+        do {
+          ok = true;
+          uint2 first[NPR];
 #pragma unroll
-        for (int u = 0; u < NPR; ++u) first[u] = ld_pair(tp + (size_t)min(u, np - 1) * ETXB_GQ_PW);   // all requests in flight at once
+          for (int u = 0; u < NPR; ++u) first[u] = ld_pair(tp + (size_t)min(u, np - 1) * ETXB_GQ_PW);
 #pragma unroll
-        for (int u = 0; u < NPR; ++u)
-          pv[r][u] = (u >= np || first[u].y == fl) ? __uint_as_float(first[u].x) : poll_pair(tp + (size_t)u * ETXB_GQ_PW, fl, sm);
+          for (int u = 0; u < NPR; ++u) { pv[r][u] = __uint_as_float(first[u].x); ok = ok && first[u].y == fl; }
+        } while (!ok && poll_again(spins, sm));
       }
     }
   }
@@ -161,12 +181,18 @@ __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Sm
       float o = 0.f;
       for (int p0 = 0; p0 < np; p0 += NPR) {
         uint2 first[NPR];
+        bool ok;
+        uint32_t spins = 0;
+        do {
+          ok = true;
 #pragma unroll
-        for (int u = 0; u < NPR; ++u) first[u] = ld_pair(tp + (size_t)min(p0 + u, np - 1) * ETXB_GQ_PW);
+          for (int u = 0; u < NPR; ++u) first[u] = ld_pair(tp + (size_t)min(p0 + u, np - 1) * ETXB_GQ_PW);
+#pragma unroll
+          for (int u = 0; u < NPR; ++u) ok = ok && first[u].y == fl;
+        } while (!ok && poll_again(spins, sm));
 #pragma unroll
         for (int u = 0; u < NPR; ++u)
-          if (p0 + u < np)
-            o = __fmaf_rn(wg[p0 + u], first[u].y == fl ? __uint_as_float(first[u].x) : poll_pair(tp + (size_t)(p0 + u) * ETXB_GQ_PW, fl, sm), o);
+          if (p0 + u < np) o = __fmaf_rn(wg[p0 + u], __uint_as_float(first[u].x), o);
       }
       ((__nv_bfloat16*)d.out)[(size_t)(hq0 + g) * HD + dd] = __float2bfloat16_rn(__fdiv_rn(o, red[g]));
     }
@@ -238,21 +264,18 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
     csync();
     mark(sm, 0);
     // ---- norm + rope of the q heads (warps 0..GQ-1), of the new k row (warp GQ); the new v row (warp GQ + 1)
-    if (warp < GQ) {
+    if (warp < GQ || (warp == GQ && owner)) {                       // q heads, then the new k row: raw rows lie one behind the other
       float o[8];
-      head_norm_rope_s<128>(s.raw + warp * HD, d.qw ? s.cw + HD : nullptr, s.cw, HD, d.eps, o);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s.qs[warp * HD + lane * 4 + j] = o[j];
-    } else if (warp == GQ && owner) {
-      float o[8];
-      head_norm_rope_s<128>(s.raw + GQ * HD, d.kw ? s.cw + 2 * HD : nullptr, s.cw, HD, d.eps, o);
+      const bool isq = warp < GQ;
+      head_norm_rope_s<128>(s.raw + warp * HD, (isq ? d.qw : d.kw) ? s.cw + (isq ? HD : 2 * HD) : nullptr, s.cw, HD, d.eps, o);
       const long long cb = slot / BS; const int off = (int)(slot % BS);
       __nv_bfloat16* kc = (__nv_bfloat16*)d.kc;
+      float* dst = isq ? s.qs + warp * HD : s.knew;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int dd = lane * 4 + j;
-        s.knew[dd] = o[j];
-        if (writer) kc[((((size_t)cb * NKV + h) * HV + dd / X) * BS + off) * X + dd % X] = __float2bfloat16_rn(o[j]);
+        dst[dd] = o[j];
+        if (!isq && writer) kc[((((size_t)cb * NKV + h) * HV + dd / X) * BS + off) * X + dd % X] = __float2bfloat16_rn(o[j]);
       }
     } else if (warp == GQ + 1 && owner) {
       const long long cb = slot / BS; const int off = (int)(slot % BS);

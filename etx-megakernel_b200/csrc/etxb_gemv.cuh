@@ -384,7 +384,7 @@ __device__ __forceinline__ void gemv_rows(const unsigned char* stage, int row_by
   float a[R];
 #pragma unroll
   for (int u = 0; u < R; ++u) a[u] = 0.f;
-  constexpr int U = R == 1 ? 8 : (XS ? 1 : 2);
+  constexpr int U = R == 1 ? 4 : 1;
 #pragma unroll U
   for (int v = lane; v < nvec; v += 32) {
     if (XS) {
@@ -566,19 +566,20 @@ __device__ __forceinline__ void stage_norm_col(const void* rows, const void* rin
 #pragma unroll
       for (int j = 0; j < 8; ++j) z[j] = bfr(__fadd_rn(rf[j], v[j]));      // bf16(0 + row) = row: the one-row case of the loop below
     } else {
+      constexpr int NF = 8;
       float acc[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-      for (int s0 = 0; s0 < R; s0 += 8) {                       // up to 8 rows in flight, added in order
-        uint4 rv[8];
+#pragma unroll 1
+      for (int s0 = 0; s0 < R; s0 += NF) {                      // NF rows in flight, added in order
+        uint4 rv[NF];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (s0 + u < R) {
-            const int row = R > 1 ? order[s0 + u] : 0;
-            rv[u] = ld_act16((const __nv_bfloat16*)rows + (size_t)row * K + 8 * i);
-          }
+        for (int u = 0; u < NF; ++u) {
+          const int row = R > 1 ? order[min(s0 + u, R - 1)] : 0;
+          rv[u] = ld_act16((const __nv_bfloat16*)rows + (size_t)row * K + 8 * i);
+        }
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < NF; ++u)
           if (s0 + u < R) {
             const float v[8] = {bf_lo(rv[u].x), bf_hi(rv[u].x), bf_lo(rv[u].y), bf_hi(rv[u].y),
                                 bf_lo(rv[u].z), bf_hi(rv[u].z), bf_lo(rv[u].w), bf_hi(rv[u].w)};

@@ -81,22 +81,33 @@ __device__ __forceinline__ void tile_argmax(const etxb_params& p, const Smem& sm
   float bv = -INFINITY; int bi = 0x7fffffff;
   const uint4* lg4 = (const uint4*)((const __nv_bfloat16*)S.logits + (size_t)col * S.V);
   const int n4 = S.V / 8;
-  auto scan = [&](const uint4 w, int base) {
+  // One CTA reads the row (300 KB for 151936 logits), so what counts is how much of it is in flight: 12 vectors per thread
+  // (96 KB), compared by their largest element (packed maxima); the element itself is looked up in the one vector that
+  // won.  4 in flight, every element compared: 8.3 us; now 4.1.
+  // (max of bf16 pairs drops NaN like the comparison does; +0 and -0 compare equal, so the lookup takes the first of them)
+  int bj = -1;
+  const int B = ETXB_CONSUMERS;
+  constexpr int NF = 12;
+  for (int j0 = tidx(); j0 < n4; j0 += NF * B) {
+    uint4 w[NF];
+#pragma unroll
+    for (int k = 0; k < NF; ++k) w[k] = ld_act16(lg4 + min(j0 + k * B, n4 - 1));
+#pragma unroll
+    for (int k = 0; k < NF; ++k) {
+      const uint32_t m = max_bf2(max_bf2(w[k].x, w[k].y), max_bf2(w[k].z, w[k].w));
+      const float v = fmaxf(bf_lo(m), bf_hi(m));
+      if (j0 + k * B < n4 && v > bv) { bv = v; bj = j0 + k * B; }
+    }
+  }
+  if (bj >= 0) {
+    const uint4 w = ld_act16(lg4 + bj);
     const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float lo = bf_lo(u[k]), hi = bf_hi(u[k]);
-      if (lo > bv) { bv = lo; bi = base + 2 * k; }
-      if (hi > bv) { bv = hi; bi = base + 2 * k + 1; }
+    for (int k = 3; k >= 0; --k) {
+      if (bf_hi(u[k]) == bv) bi = 8 * bj + 2 * k + 1;
+      if (bf_lo(u[k]) == bv) bi = 8 * bj + 2 * k;
     }
-  };
-  int j = tidx();
-  const int B = ETXB_CONSUMERS;
-  for (; j + 3 * B < n4; j += 4 * B) {
-    const uint4 a0 = ld_act16(lg4 + j), a1 = ld_act16(lg4 + j + B), a2 = ld_act16(lg4 + j + 2 * B), a3 = ld_act16(lg4 + j + 3 * B);
-    scan(a0, 8 * j); scan(a1, 8 * (j + B)); scan(a2, 8 * (j + 2 * B)); scan(a3, 8 * (j + 3 * B));
   }
-  for (; j < n4; j += B) scan(ld_act16(lg4 + j), 8 * j);
   for (int i = 8 * n4 + tidx(); i < S.V; i += B) {
     const float v = ld_bf(lg4, i);
     if (v > bv) { bv = v; bi = i; }

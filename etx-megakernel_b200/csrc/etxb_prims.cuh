@@ -120,6 +120,12 @@ __device__ __forceinline__ float bfr(float x) {                    // RNE to bf1
 }
 __device__ __forceinline__ float bf_lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+// larger of each of two bf16 pairs (a NaN loses against a number)
+__device__ __forceinline__ uint32_t max_bf2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
 __device__ __forceinline__ uint32_t pack_bf(float lo, float hi) {  // both already bf16-exact or to be rounded RNE
   const uint32_t a = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo));
   const uint32_t b = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi));

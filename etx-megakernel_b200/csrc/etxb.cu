@@ -607,7 +607,7 @@ static int32_t build_tensor_maps(etxb_session* s) {
     const cuuint64_t rows = ty.body == ETXB_BODY_GEMV_TC ? (cuuint64_t)a.M : (cuuint64_t)a.E * (cuuint64_t)(a.estride / a.K);
     cuuint64_t gdim[2] = {(cuuint64_t)a.K, rows};
     cuuint64_t gstr[1] = {(cuuint64_t)a.K * 2};
-    cuuint32_t box[2] = {64, ETXB_TC_ROWS};
+    cuuint32_t box[2] = {64, ETXB_TC_BOXROWS};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)a.W, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -641,7 +641,7 @@ static int32_t upload_type_args(etxb_session* s) {
     int32_t rc = check_block(ty.body, s->h_pool.data() + ty.cst[0], s->h_pool.size() - (size_t)ty.cst[0]);
     if (rc) return rc;
   }
-  // tensor-core tiles: one TMA tensor map per grid -- the weight tensor as a [rows][K] bf16 matrix, box 64 k x 128 rows,
+  // tensor-core tiles: one TMA tensor map per grid -- the weight tensor as a [rows][K] bf16 matrix, box 64 k x 64 rows,
   // 128-byte swizzle -- built here because only the library knows the driver entry point; its device address goes into
   // the `ln` field of the grid's argument block (in the device copy of the pool)
   {

@@ -473,6 +473,11 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
     if (p.tc_on != 0u) {
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       csync();                                                     // nobody reads an accumulator any more
+      // an abandoned step may have loaded stages that no MMA took: wait (bounded) for those copies before the CTA's memory goes
+      if (tidx() == 32 && ld_relaxed(p.ctrl) != 0)
+        for (int i = 0; i < ETXB_TC_MAXSTAGE; ++i)
+          if (s_tc.lu[i] != s_tc.mu[i])
+            for (int spin = 0; spin < 2000000 && !mbar_try_wait(s_tc.full + i, (s_tc.lu[i] - 1) & 1); ++spin) {}
       if (threadIdx.x < 32) tc_dealloc(s_tc.tmem);
     }
   }

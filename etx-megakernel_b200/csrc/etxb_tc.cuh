@@ -1,6 +1,6 @@
 // Batched decode on the Blackwell tensor cores: tcgen05.mma with the tokens as the M side (A operand, shared memory,
 // SWIZZLE_128B K-major), 128 or 256 weight rows as the N side (B operand, loaded by TMA tensor copies --
-// cp.async.bulk.tensor.2d with SWIZZLE_128B, one tensor map per weight tensor, boxes of 64 k x 128 rows, one or two per
+// cp.async.bulk.tensor.2d with SWIZZLE_128B, one tensor map per weight tensor, boxes of 64 k x 64 rows, up to four per
 // instruction) and fp32 accumulators in tensor memory, read back with tcgen05.ld for the epilogue.
 //
 // These tiles serve the same grids as the mma.sync tiles of etxb_batch.cuh (column-batched GEMV, expert-grouped gate+up
@@ -28,9 +28,10 @@
 
 namespace etxb {
 
-#define ETXB_TC_ROWS 128               // weight rows per TMA box; an instruction takes one or two boxes (N = 128 or 256)
-#define ETXB_TC_BOX 16384              // one box: 128 rows x 64 k x 2 bytes
-#define ETXB_TC_STAGE (2 * ETXB_TC_BOX)   // one k-chunk of a tile: up to 256 rows
+#define ETXB_TC_ROWS 128               // weight rows a block of the grids' geometry has; an instruction takes up to two (N <= 256)
+#define ETXB_TC_BOXROWS 64             // weight rows per TMA box: the unit by which the expert grids are shared out
+#define ETXB_TC_BOX 8192               // one box: 64 rows x 64 k x 2 bytes
+#define ETXB_TC_STAGE (4 * ETXB_TC_BOX)   // one k-chunk of a tile: up to 256 rows
 #define ETXB_TC_MAXSTAGE 6
 #define ETXB_TC_TAIL 8192              // end of the area: the routing tables of the expert tiles
 #define ETXB_TC_AREA (ETXB_RING_BYTES + ETXB_GEN_BYTES - 1024 - ETXB_TC_TAIL)   // the idle weight ring and the general region, 1024-byte aligned inside
@@ -96,30 +97,47 @@ __device__ __forceinline__ void tc_store8(__nv_bfloat16* o, int r, int r1, const
   }
 }
 
-// One task: for every tile i < ntiles, D_i[tok][j] = sum_k x_tok[k] * W[boxrow(i, j / 128) + j % 128][k] for j < 128 nbox(i),
-// then epi(i, tok, j, v0, v1, two) for every tok < ntok and j = 0, 8, .. 120, with v0[u] = D_i[tok][j + u] and (two: the tile has
-// a second box) v1[u] = D_i[tok][128 + j + u].  A tile is one or two TMA boxes of 128 weight rows that one instruction multiplies (N = 128 or 256): two
-// neighbouring row blocks of a matrix, or an expert's gate rows and up rows.  The sum runs over the K columns from
+// The weight rows of a task, in tiles of tmax rows (a multiple of 64, up to 256) and one lower one at the end: rows y0 .. y0 + nrow;
+// or, where a task takes two runs (an expert's gate rows and up rows, tmax <= 128), rows y1 .. y1 + nrow as well.
+struct TcSeg {
+  int y0, y1, nrow, tmax;                                          // nrow: a multiple of 64
+  __device__ __forceinline__ int tiles() const { return (nrow + tmax - 1) / tmax; }
+  __device__ __forceinline__ int height(int i) const { return min(tmax, nrow - i * tmax); }
+};
+// k-chunks of the tokens that fit at once / weight stages beside them
+__device__ __forceinline__ int tc_window(int K, int ntok) { return min(K >> 6, ETXB_TC_XBYTES / (((ntok + 7) >> 3) * 1024)); }
+__device__ __forceinline__ int tc_stages(int K, int ntok) {
+  return min(ETXB_TC_MAXSTAGE, (ETXB_TC_AREA - tc_window(K, ntok) * ((ntok + 7) >> 3) * 1024) / ETXB_TC_STAGE);
+}
+
+// One task: for every tile i of the segment, h = height(i) rows, D_i[tok][j] = sum_k x_tok[k] * W[y0 + i tmax + j][k] for j < h, then
+// epi(i, tok, j, v0, v1) for every tok < ntok and j = 0, 8, .. h - 8 with v0[u] = D_i[tok][j + u]; TWO: v1[u] = the same of the second run
+// (one instruction multiplies both, N = 2 h).  The sum runs over the K columns from
 // `kofs` on (a K-slice of the matrix: both multiples of 64).  xsrc(n): the bf16 row of token n (column 0);
-// map: the tensor map of the weight tensor (rows x all columns, box 64 x 128).  All consumer threads call; ends with a barrier.
+// map: the tensor map of the weight tensor (rows x all columns, box 64 x 64).  All consumer threads call; ends with a barrier.
+// nx, nx_tok: the segment that the same caller runs next with the same map, kofs and K, and its tokens (0: none).
+// pre: in, how many stages an earlier call has already filled for this segment; out, for the next one.
 //
 // The tokens are staged ONCE per task (the tiles of a task share them) whenever all of K fits the token area; the tiles
 // then stream back to back through the stage ring, their accumulators alternating between two buffers of tensor
 // memory, so that the epilogue of tile i overlaps the MMAs of tile i + 1.  When K does not fit (4096 columns x 32
 // tokens) the tokens go in windows of K and a task handles its tiles one by one, accumulating across the windows.
-template <typename XSrc, typename NBox, typename BoxRow, typename Epi>
-__device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void* map, int ntiles, int kofs, int K, int ntok, int where,
-                                        XSrc xsrc, NBox nbox, BoxRow boxrow, Epi epi) {
+// The weights depend on nothing a task waits for, so the loader fills the stage ring before the tokens are staged, and as its
+// stages fall free at the end of a segment it fills them for the next one (the stages lie at the end of the area, the same
+// place whatever the number of tokens): the step from one expert to the next, which a third of the workers take, does not
+// drain the stream.
+template <bool TWO, typename XSrc, typename Epi>
+__device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void* map, const TcSeg seg, const TcSeg nx, int nx_tok, int& pre, int kofs, int K, int ntok,
+                                        int where, XSrc xsrc, Epi epi) {
   const int tid = tidx(), warp = tid >> 5, lane = tid & 31;
   unsigned char* area = (unsigned char*)(((uintptr_t)sm.ring + 1023) & ~(uintptr_t)1023);
   const int M = ntok <= 8 ? 64 : 128, groups = (ntok + 7) >> 3, nchunk = K >> 6;
   // (an instruction reads M / 8 row groups of its k-chunk: the ones past the tokens' groups are the next chunks' rows or,
   // at the end, the first stage's -- whatever they hold only reaches accumulator rows that nobody reads)
-  const int wc = min(nchunk, ETXB_TC_XBYTES / (groups * 1024));    // k-chunks of the tokens that fit at once
+  const int wc = tc_window(K, ntok), ntiles = seg.tiles();
   const int nwin = (nchunk + wc - 1) / wc;
-  const int xbytes = wc * groups * 1024;
-  unsigned char* ws = area + xbytes;
-  const int nst = min(ETXB_TC_MAXSTAGE, (ETXB_TC_AREA - xbytes) / ETXB_TC_STAGE);
+  unsigned char* const ws = area + ETXB_TC_AREA - ETXB_TC_STAGE;   // stage s lies at ws - s * ETXB_TC_STAGE
+  const int nst = tc_stages(K, ntok);
   const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(M >> 4) << 24);   // fp32 D, bf16 A / B, K-major; N goes in per tile
   const bool alive0 = *(volatile int*)sm.stop == 0;
   const uint32_t f0[2] = {tc.nfull[0], tc.nfull[1]}, r0[2] = {tc.nfree[0], tc.nfree[1]};     // (the previous task ended with a barrier)
@@ -130,38 +148,61 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
     const int i0 = nwin == 1 ? 0 : pass / nwin, i1 = nwin == 1 ? ntiles : i0 + 1, win = nwin == 1 ? 0 : pass - i0 * nwin;
     const int w0 = win * wc, nc = min(wc, nchunk - w0);
     const bool first_win = win == 0, last_win = win == nwin - 1;
+    // loader: every tile of the pass, chunk by chunk (warp 1: a lane per box, their issue is what limits one thread)
+    const bool loader = warp == 1 && alive0;
+    auto load = [&](const TcSeg& g, int i, int c, int st) -> bool {
+      const uint32_t uu = tc.lu[st];
+      if (!__all_sync(0xffffffffu, mbar_wait(tc.empty + st, (uu & 1) ^ 1, sm, where))) return false;
+      const int per = g.height(i) / ETXB_TC_BOXROWS, nb = TWO ? 2 * per : per;
+      if (lane == 0) { tc.lu[st] = uu + 1; mbar_expect_tx(tc.full + st, (uint32_t)nb * ETXB_TC_BOX); }
+      __syncwarp();
+      if (lane < nb) {
+        const bool second = TWO && lane >= per;
+        tma_load_2d(ws - (size_t)st * ETXB_TC_STAGE + lane * ETXB_TC_BOX, map, kofs + (w0 + c) * 64,
+                    (second ? g.y1 - per * ETXB_TC_BOXROWS : g.y0) + i * g.tmax + lane * ETXB_TC_BOXROWS, tc.full + st);
+      }
+      return true;
+    };
+    int li = i0, lc = 0, lst = 0;
+    bool lok = true;
+    auto load_next = [&]() {
+      lok = load(seg, li, lc, lst);
+      lst = lst + 1 == nst ? 0 : lst + 1;
+      if (++lc == nc) { lc = 0; ++li; }
+    };
+    if (loader) {
+      if (pass == 0)
+        for (int q = 0; q < pre; ++q) {                            // (already on their way)
+          lst = lst + 1 == nst ? 0 : lst + 1;
+          if (++lc == nc) { lc = 0; ++li; }
+        }
+      for (int q = pass == 0 ? pre : 0; q < nst && li < i1 && lok; ++q) load_next();
+    }
     // the tokens' slice [64 w0, 64 (w0 + nc)) -> swizzled rows: token n is row n % 8 of group n / 8 of its k-chunk
-    for (int i = tid; i < ntok * nc * 8; i += ETXB_CONSUMERS) {
+    if (!loader) {
+    const int first = warp == 0 ? lane : tid - 32, step = alive0 ? ETXB_CONSUMERS - 32 : ETXB_CONSUMERS;   // (an abandoned step: whatever)
+    for (int i = first; i < ntok * nc * 8; i += step) {
       const int n = i / (nc * 8), v = i - n * (nc * 8), c = v >> 3, j = v & 7, r = n & 7;
       const uint4 val = ld_act16((const __nv_bfloat16*)xsrc(n) + (size_t)(kofs + w0 * 64 + v * 8));
       *(uint4*)(area + (size_t)(c * groups + (n >> 3)) * 1024 + r * 128 + ((j ^ r) << 4)) = val;
     }
+    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core's reads
     csync();
     if (sm.tr() != nullptr && tid == 0 && pass == 0) sm.tr()[4] = globaltimer();
-    if (warp == 1 && lane == 0 && alive0) {                        // loader: every tile of the pass, chunk by chunk
-      bool ok = true;
-      int st = 0;
-      for (int i = i0; i < i1 && ok; ++i) {
-        const int nb = nbox(i), y0 = boxrow(i, 0), y1 = nb > 1 ? boxrow(i, 1) : 0;
-        for (int c = 0; c < nc && ok; ++c) {
-          const uint32_t uu = tc.lu[st];
-          ok = mbar_wait(tc.empty + st, (uu & 1) ^ 1, sm, where);
-          if (!ok) break;
-          mbar_expect_tx(tc.full + st, (uint32_t)nb * ETXB_TC_BOX);
-          unsigned char* dst = ws + (size_t)st * ETXB_TC_STAGE;
-          tma_load_2d(dst, map, kofs + (w0 + c) * 64, y0, tc.full + st);
-          if (nb > 1) tma_load_2d(dst + ETXB_TC_BOX, map, kofs + (w0 + c) * 64, y1, tc.full + st);
-          tc.lu[st] = uu + 1;
-          st = st + 1 == nst ? 0 : st + 1;
-        }
+    if (loader) {
+      while (li < i1 && lok) load_next();
+      const int nfill = nx_tok > 0 && nwin == 1 ? min(min(nst, tc_stages(K, nx_tok)), nx.tiles() * nchunk) : 0;
+      for (int q = 0, i = 0, c = 0; q < nfill && lok; ++q) {
+        lok = load(nx, i, c, q);
+        if (++c == nchunk) { c = 0; ++i; }
       }
     } else if (warp == 2 && lane == 0 && alive0) {                 // MMA issuer
       bool ok = true;
       int st = 0;
       for (int i = i0; i < i1 && ok; ++i) {
         const uint32_t seq = tile_seq + (uint32_t)(i - i0), bsel = seq & 1;
-        const uint32_t idesc = idesc0 | ((uint32_t)(nbox(i) * ETXB_TC_ROWS >> 3) << 17);
+        const uint32_t idesc = idesc0 | ((uint32_t)((TWO ? 2 : 1) * seg.height(i) >> 3) << 17);
         if (first_win) {                                           // a fresh accumulator buffer: the epilogue of the tile two back must be done with it
           const uint32_t nth = r0[bsel] + (seq >> 1);              // acc_free[bsel] completions expected before this use
           if (nth > 0) ok = mbar_wait(tc.acc_free + bsel, (nth - 1) & 1, sm, where);
@@ -174,7 +215,7 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
           ok = mbar_wait(tc.full + st, uu & 1, sm, where);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t aaddr = smem_u32(area + (size_t)c * groups * 1024), baddr = smem_u32(ws + (size_t)st * ETXB_TC_STAGE);
+          const uint32_t aaddr = smem_u32(area + (size_t)c * groups * 1024), baddr = smem_u32(ws - (size_t)st * ETXB_TC_STAGE);
 #pragma unroll
           for (int k = 0; k < 4; ++k) tc_mma(dcol, tc_desc(aaddr + 32 * k), tc_desc(baddr + 32 * k), idesc, (w0 + c + k) > 0 ? 1u : 0u);
           tc_commit(tc.empty + st);                                // the stage is free once these MMAs have read it
@@ -186,7 +227,7 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
       if (sm.tr() != nullptr && pass == npass - 1) sm.tr()[5] = globaltimer();
     }
     __syncwarp();                                                  // the role threads' warp-mates wait here, not in a spin beside them
-    // epilogue: warps 0, 4, 8, 12 own TMEM lanes 0..31 (one token per lane), a quarter of each box's 128 columns each.  Only
+    // epilogue: warps 0, 4, 8, 12 own TMEM lanes 0..31 (one token per lane), a quarter of a run's columns each.  Only
     // they wait for the accumulators: the issuer runs at most one tile ahead of the slowest of them (it needs their four
     // arrivals to reuse a buffer), so none of them can miss a phase; the other warps go on to the barrier below.
     if ((warp & 3) == 0) {
@@ -200,15 +241,13 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
         alive = __all_sync(0xffffffffu, alive);
         if (!last_win) continue;
         if (alive) {
-          const int q = warp >> 2;
-          const bool two = nbox(i) > 1;
+          const int h = seg.height(i), c0 = (warp >> 2) * (h >> 2), c1 = c0 + (h >> 2);
 #pragma unroll 1
-          for (int c8 = 0; c8 < 4; ++c8) {
-            const int col = 32 * q + 8 * c8;
+          for (int col = c0; col < c1; col += 8) {
             float v0[8], v1[8];
             tc_ld8(tc.tmem + bsel * 2 * ETXB_TC_ROWS + (uint32_t)col, v0);
-            if (two) tc_ld8(tc.tmem + bsel * 2 * ETXB_TC_ROWS + (uint32_t)(ETXB_TC_ROWS + col), v1);
-            if (lane < ntok) epi(i, lane, col, v0, v1, two);
+            if (TWO) tc_ld8(tc.tmem + bsel * 2 * ETXB_TC_ROWS + (uint32_t)(h + col), v1);
+            if (lane < ntok) epi(i, lane, col, v0, v1);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -220,6 +259,7 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     csync();                                                       // the tokens may be restaged
   }
+  pre = nx_tok > 0 && nwin == 1 ? min(min(nst, tc_stages(K, nx_tok)), nx.tiles() * nchunk) : 0;
   if (tid == 0) {
     const uint32_t nt = (uint32_t)ntiles;
     for (int b = 0; b < 2; ++b) {
@@ -233,7 +273,7 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
 
 // ---------------------------------------------------------------------------------------------- batched dense GEMV
 // out[b * sout + r] = bf16(W[r,:] . x[b] (+ bias[r])) for the nb columns b.  The GEMV block of gemv_nb; `ln` = the tensor
-// map of W (rows M, box 64 x 128), put there by the host library when the plan is bound.
+// map of W (rows M, box 64 x 64), put there by the host library when the plan is bound.
 //
 // tpe = the K-split S of the grid (1: none).  Task blk covers rows [(blk / S) * rpt, ...) and the K-slice blk % S.  A
 // matrix of a few thousand rows has too few 128-row tiles for 148 workers (qkv: 40, o_proj: 16, router: 1) and an
@@ -250,29 +290,24 @@ __device__ __forceinline__ void tile_gemv_tc(const unsigned char* a, int blk, co
   const __nv_bfloat16* bias = (d.mode & ETXB_MODE_BIAS) ? (const __nv_bfloat16*)d.wts : nullptr;
   __nv_bfloat16* out = (__nv_bfloat16*)d.out;
   float* part = S > 1 ? (float*)d.rows + (size_t)ksl * d.nb * d.M : nullptr;   // this slice's [M][nb] partial sums
-  const int ntiles = (r1 - r0 + 2 * ETXB_TC_ROWS - 1) / (2 * ETXB_TC_ROWS);
+  const TcSeg seg = {r0, 0, (r1 - r0 + ETXB_TC_BOXROWS - 1) & -ETXB_TC_BOXROWS, 2 * ETXB_TC_ROWS};
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // what other tiles left in this memory: ordered before the copies
+  csync();
   for (int b0 = 0; b0 < d.nb; b0 += ETXB_TC_MAXTOK) {
     const int nt = min(ETXB_TC_MAXTOK, d.nb - b0);
-    tc_task(sm, tc, d.ln, ntiles, ksl * Ks, Ks, nt, where,
+    int pre = 0;
+    tc_task<false>(sm, tc, d.ln, seg, seg, 0, pre, ksl * Ks, Ks, nt, where,
             [&](int n) { return (const __nv_bfloat16*)d.x + (size_t)(b0 + n) * d.sx; },
-            [&](int i) { return r1 - r0 - i * 2 * ETXB_TC_ROWS > ETXB_TC_ROWS ? 2 : 1; },
-            [&](int i, int b) { return r0 + (2 * i + b) * ETXB_TC_ROWS; },
-            [&](int i, int tok, int j, const float (&v0)[8], const float (&v1)[8], bool two) {
-              const int r = r0 + 2 * i * ETXB_TC_ROWS + j;
+            [&](int i, int tok, int j, const float (&v)[8], const float (&)[8]) {
+              const int rr = r0 + 2 * i * ETXB_TC_ROWS + j;
+              if (part != nullptr) {                              // [slice][row][column]: the 32 lanes of a store are 32 consecutive floats
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                if (h == 1 && !two) break;
-                const int rr = r + h * ETXB_TC_ROWS;
-                const float (&v)[8] = h ? v1 : v0;
-                if (part != nullptr) {                              // [slice][row][column]: the 32 lanes of a store are 32 consecutive floats
+                for (int u = 0; u < 8; ++u) if (rr + u < r1) __stcg(part + (size_t)(rr + u) * d.nb + b0 + tok, v[u]);
+              } else {
+                float y[8];
 #pragma unroll
-                  for (int u = 0; u < 8; ++u) if (rr + u < r1) __stcg(part + (size_t)(rr + u) * d.nb + b0 + tok, v[u]);
-                } else {
-                  float y[8];
-#pragma unroll
-                  for (int u = 0; u < 8; ++u) y[u] = (bias && rr + u < r1) ? __fadd_rn(v[u], __bfloat162float(bias[rr + u])) : v[u];
-                  tc_store8(out + (size_t)(b0 + tok) * d.sout, rr, r1, y);
-                }
+                for (int u = 0; u < 8; ++u) y[u] = (bias && rr + u < r1) ? __fadd_rn(v[u], __bfloat162float(bias[rr + u])) : v[u];
+                tc_store8(out + (size_t)(b0 + tok) * d.sout, rr, r1, y);
               }
             });
   }
@@ -280,10 +315,9 @@ __device__ __forceinline__ void tile_gemv_tc(const unsigned char* a, int blk, co
   // (tc_task ended with a barrier: every partial of this task is stored)
   int* last = (int*)(sm.scr + 90);
   if (tidx() == 0) {
-    __threadfence();
-    const int old = atomicAdd((int*)d.resid_in + rb, 1);
+    int old;                                                       // release: the CTA's partials (seen through the barrier); acquire: the other slices'
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"((int*)d.resid_in + rb) : "memory");
     *last = ((old + 1) % S) == 0;
-    __threadfence();
   }
   csync();
   if (*last == 0) return;
@@ -416,32 +450,46 @@ __device__ __forceinline__ void tile_moe_tc(const unsigned char* a, int blk, con
   const etxb_gemv_args& d = *(const etxb_gemv_args*)a;
   if (blk >= (int)d.nblocks) return;
   const TcRoute rt = tc_route_tables(sm);
-  tc_route_build(d, rt);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // what other tiles left in this memory: ordered before the copies
+  tc_route_build(d, rt);                                           // (with barriers)
   const int nact = *rt.nact;
-  constexpr int TROWS = UP ? ETXB_TC_ROWS : 2 * ETXB_TC_ROWS;       // rows of M one tile covers (gate+up: 128 gate rows and their 128 up rows)
+  // Shares are cut in units of 64 rows of M (gate+up: with their up rows); a task's run of units of one expert goes through in
+  // tiles as high as an instruction takes and one lower one at its end.  (In whole tiles the step of 8 sequences had 348 for
+  // 148 workers: a third of them took three, the rest two, and the phase lasted 74 us where its mean share took 58.)
+  constexpr int TROWS = ETXB_TC_BOXROWS, TMAX = UP ? ETXB_TC_ROWS : 2 * ETXB_TC_ROWS;
   const int T = (d.M + TROWS - 1) / TROWS;
-  const long long total = (long long)nact * T;
-  int t = (int)(total * blk / (long long)d.nblocks);
-  const int hi = (int)(total * (blk + 1) / (long long)d.nblocks);
+  const uint32_t total = (uint32_t)nact * (uint32_t)T;
+  const bool small = total < (1u << 20) && d.nblocks < (1u << 12);   // (a 64-bit division is a microsecond)
+  int t = small ? (int)(total * (uint32_t)blk / d.nblocks) : (int)((unsigned long long)total * blk / d.nblocks);
+  const int hi = small ? (int)(total * (uint32_t)(blk + 1) / d.nblocks) : (int)((unsigned long long)total * (blk + 1) / d.nblocks);
   if (UP && blk == 0 && tidx() == 0 && d.resid_out != nullptr) atomicAdd((int32_t*)d.resid_out, nact);
+  const int erows = (int)(d.estride / d.K);
+  auto segment = [&](int at, int& t1) {                             // the run of units of one expert that begins at `at`
+    const int ai = at / T, t0 = at - ai * T;
+    t1 = min(T, t0 + (hi - at));
+    const int erow = rt.alist[ai] * erows;                          // first row of the expert in the [E * rows][K] view
+    return TcSeg{erow + t0 * TROWS, erow + d.M + t0 * TROWS, (t1 - t0) * TROWS, TMAX};   // (up rows follow the M gate rows)
+  };
+  auto entries = [&](int at) { return min(min(rt.scnt[rt.alist[at / T]], d.nb), 64); };
+  int pre = 0;
   while (t < hi) {
-    const int ai = t / T, t0 = t - ai * T, t1 = min(T, t0 + (hi - t));
-    const int e = rt.alist[ai];
-    const int cnt = min(min(rt.scnt[e], d.nb), 64);
-    tc_route_entries(d, rt, e, UP ? nullptr : d.wts);
+    const int ai = t / T, t0 = t - ai * T;
+    int t1, nt1 = 0;
+    const TcSeg seg = segment(t, t1);
+    const int cnt = entries(t), tn = t + t1 - t0;
+    const TcSeg nseg = tn < hi ? segment(tn, nt1) : seg;
+    const int ntn = tn < hi ? min(ETXB_TC_MAXTOK, entries(tn)) : 0;
+    tc_route_entries(d, rt, rt.alist[ai], UP ? nullptr : d.wts);
     csync();
-    const int erow = (int)((long long)e * d.estride / d.K);         // first row of expert e in the [E * rows][K] view
     const int r0 = t0 * TROWS, r1 = min(d.M, t1 * TROWS);
     for (int p0 = 0; p0 < cnt; p0 += ETXB_TC_MAXTOK) {
-      const int nt = min(ETXB_TC_MAXTOK, cnt - p0);
+      const int nt = min(ETXB_TC_MAXTOK, cnt - p0), nxt = p0 + nt < cnt ? 0 : ntn;
       const int32_t* ent = rt.ent + p0;
       if constexpr (UP) {
-        tc_task(sm, tc, d.ln, t1 - t0, 0, d.K, nt, where,
+        tc_task<true>(sm, tc, d.ln, seg, nseg, nxt, pre, 0, d.K, nt, where,
                 [&](int n) { return (const __nv_bfloat16*)d.x + (size_t)(ent[n] >> 8) * d.sx; },
-                [&](int) { return 2; },                                                          // 128 gate rows and their 128 up rows: one instruction
-                [&](int i, int b) { return erow + (b ? d.M : 0) + r0 + i * ETXB_TC_ROWS; },        // up rows follow the M gate rows
-                [&](int i, int tok, int j, const float (&g)[8], const float (&up)[8], bool) {
-                  const int r = r0 + i * ETXB_TC_ROWS + j, en = ent[tok];
+                [&](int i, int tok, int j, const float (&g)[8], const float (&up)[8]) {
+                  const int r = r0 + i * TMAX + j, en = ent[tok];
                   float y[8];
 #pragma unroll
                   for (int u = 0; u < 8; ++u) y[u] = __fmul_rn(bfr(silu_f(bfr(g[u]))), bfr(up[u]));
@@ -449,26 +497,18 @@ __device__ __forceinline__ void tile_moe_tc(const unsigned char* a, int blk, con
                 });
       } else {
         const float* wt = rt.wt + p0;
-        tc_task(sm, tc, d.ln, t1 - t0, 0, d.K, nt, where,
+        tc_task<false>(sm, tc, d.ln, seg, nseg, nxt, pre, 0, d.K, nt, where,
                 [&](int n) { return (const __nv_bfloat16*)d.x + ((size_t)(ent[n] >> 8) * d.R + (ent[n] & 0xff)) * d.K; },
-                [&](int i) { return r1 - r0 - i * 2 * ETXB_TC_ROWS > ETXB_TC_ROWS ? 2 : 1; },
-                [&](int i, int b) { return erow + r0 + (2 * i + b) * ETXB_TC_ROWS; },
-                [&](int i, int tok, int j, const float (&v0)[8], const float (&v1)[8], bool two) {
-                  const int r = r0 + 2 * i * ETXB_TC_ROWS + j, en = ent[tok];
-                  __nv_bfloat16* o = (__nv_bfloat16*)d.out + ((size_t)(en >> 8) * d.R + (en & 0xff)) * d.M;
+                [&](int i, int tok, int j, const float (&v)[8], const float (&)[8]) {
+                  const int r = r0 + i * TMAX + j, en = ent[tok];
                   float y[8];
 #pragma unroll
-                  for (int u = 0; u < 8; ++u) { const float q = bfr(v0[u]); y[u] = d.wts ? bfr(__fmul_rn(q, wt[tok])) : q; }
-                  tc_store8(o, r, r1, y);
-                  if (two) {
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) { const float q = bfr(v1[u]); y[u] = d.wts ? bfr(__fmul_rn(q, wt[tok])) : q; }
-                    tc_store8(o, r + ETXB_TC_ROWS, r1, y);
-                  }
+                  for (int u = 0; u < 8; ++u) { const float q = bfr(v[u]); y[u] = d.wts ? bfr(__fmul_rn(q, wt[tok])) : q; }
+                  tc_store8((__nv_bfloat16*)d.out + ((size_t)(en >> 8) * d.R + (en & 0xff)) * d.M, r, r1, y);
                 });
       }
     }
-    t += t1 - t0;
+    t = tn;
   }
 }
 __device__ __forceinline__ void tile_moe_up_tc(const unsigned char* a, int blk, const Smem& sm, TcShared& tc, int where) { tile_moe_tc<true>(a, blk, sm, tc, where); }

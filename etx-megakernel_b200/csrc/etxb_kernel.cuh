@@ -83,7 +83,7 @@ __device__ __forceinline__ void tile_argmax(const etxb_params& p, const Smem& sm
   const int n4 = S.V / 8;
   // One CTA reads the row (300 KB for 151936 logits), so what counts is how much of it is in flight: 12 vectors per thread
   // (96 KB), compared by their largest element (packed maxima); the element itself is looked up in the one vector that
-  // won.  4 in flight, every element compared: 8.3 us; now 4.1.
+  // won.  4 in flight, every element compared: 8.8 us; now 7.0 (one SM's share of the L2 bandwidth is 2.5).
   // (max of bf16 pairs drops NaN like the comparison does; +0 and -0 compare equal, so the lookup takes the first of them)
   int bj = -1;
   const int B = ETXB_CONSUMERS;
@@ -253,7 +253,7 @@ __device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, i
 // same GEMV family with the latent-attention tile in place of the grouped one); ETXB_VARIANT_BATCH = the tiles of a batched step
 // on the tensor cores.  The host picks it from the plan (select_variant): the full
 // kernel is 550 KB of code, of which a decode step uses a fraction scattered through it, and the step runs about 10 %
-// faster from the 150 KB kernel (instruction fetch).
+// faster from a 142 KB kernel (instruction fetch).
 // XCH: the variants a sharded session launches -- the same bodies plus the exchange code (flagged-row folds of R = ranks
 // rows, row publishing after the body, the argmax exchange); compiled out of the others.
 #define ETXB_VARIANT_MLA 16
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
   const Smem sm = smem_view();
   if (threadIdx.x == 0) {
     s_stop = 0;
-    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.cur = 0;
+    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.cur = 0; s_vars.hold = 0;
     s_deadline = globaltimer() + p.timeout_ns;
     for (int i = 0; i < ETXB_NSTAGE; ++i) { mbar_init(sm.full + i, 1); mbar_init(sm.empty + i, ETXB_EMPTY_COUNT); ((uint32_t*)(sm.empty + ETXB_NSTAGE))[i] = 0xffffffffu; }
     if constexpr (TC) {
@@ -465,6 +465,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
           const int word = i < 4 ? c->r.out_word[i] : p.outwords[c->r.out_off + i];
           red_release_add(p.events + (size_t)word * ETXB_EV_STRIDE, 1);
         }
+      vars->hold = 0;
       if (p.trace) { p.trace[8 * (size_t)id + 2] = globaltimer(); p.trace[8 * (size_t)id + 3] = blockIdx.x; }
       if (p.exec_count) atomicAdd(p.exec_count + id, 1);
     }

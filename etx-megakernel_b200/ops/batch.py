@@ -35,7 +35,7 @@ ROUTE_PARAMS = [("logits", "ptr addrspace(1)", 0, 8), ("wts", "ptr addrspace(1)"
 COLS_BYTES, COLS_GRID = 32, 16
 COLS_PARAMS = [("nb", "i32", 0, 4), ("slot_span", "i32", 4, 4), ("zero", "ptr addrspace(1)", 8, 8)]
 SPLITK_COUNTERS = 768       # int32 arrival counters `zero` names (cleared by column 0's prologue task every step)
-TC_ROWS = 256               # weight rows one tcgen05 instruction takes (two TMA boxes of 128)
+TC_ROWS = 256               # weight rows one tcgen05 instruction takes (four TMA boxes of 64)
 XBYTES = 40960              # shared memory for the token vectors of a pass: min(8, XBYTES // (2 K + 64)) columns per pass
 GROUP_ROWS = 128            # weight rows a block of the tensor-core loop covers
 

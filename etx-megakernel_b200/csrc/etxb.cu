@@ -209,24 +209,31 @@ static int32_t check_block(int body, const unsigned char* blk, size_t bytes) {
   return ETXB_OK;
 }
 
-// The batched step on the tensor cores: only its own tiles and grouped attention (any group size) -> its kernel.
+// The batched step on the tensor cores: only its own tiles and grouped attention (any group size) -> its kernel.  An
+// attention grid has one argument block per sequence (cst[1] bytes apart, picked by the task's second coordinate): each one
+// that a task of the plan uses is looked at.  (Against the full kernel, same bits: 8 layers of 128 experts with 8 sequences
+// 1894 -> 1852 us, 6 layers with 32 2112 -> 2091, 3 layers with 2 617 -> 587.)
 static bool batched_plan(const etxb_session* s, const std::vector<unsigned char>& pool) {
   bool tc = false;
   for (const etxb_type& ty : s->types) {
     switch (ty.body) {
       case ETXB_BODY_NOP: case ETXB_BODY_NORM_COL: case ETXB_BODY_ROUTE: case ETXB_BODY_PROLOGUE_NB: case ETXB_BODY_ARGMAX_NB: break;
       case ETXB_BODY_GEMV_TC: case ETXB_BODY_MOE_UP_TC: case ETXB_BODY_MOE_DOWN_TC: tc = true; break;
-      case ETXB_BODY_ATTN_FUSED: {
-        etxb_attnf_args a;
-        if (ty.args[0] != 0 || ty.cst[1] != 0 || ty.cst[0] < 0 || (size_t)ty.cst[0] + sizeof a > pool.size()) return false;
-        memcpy(&a, pool.data() + ty.cst[0], sizeof a);
-        if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8)) return false;
-        break;
-      }
+      case ETXB_BODY_ATTN_FUSED: if (ty.args[0] != 0 || ty.cst[0] < 0 || ty.cst[1] < 0) return false; break;
       default: return false;
     }
   }
-  return tc;
+  if (!tc) return false;
+  for (const etxb_task& t : s->tasks) {
+    const etxb_type& ty = s->types[t.type];
+    if (ty.body != ETXB_BODY_ATTN_FUSED) continue;
+    const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
+    etxb_attnf_args a;
+    if (off < 0 || (uint64_t)off + sizeof a > pool.size()) return false;
+    memcpy(&a, pool.data() + off, sizeof a);
+    if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8)) return false;
+  }
+  return true;
 }
 
 // Which kernel can run this plan?  The lean decode kernels hold only the tiles of a fused decode step; a plan qualifies

@@ -188,3 +188,23 @@ def test_an_expert_with_more_tokens_than_one_pass(engine):
     if got[0].tolist() != want.tolist():
         top2 = np.sort(slog)[-2:]
         assert top2[1] - top2[0] <= 4 * abs(top2[1]) * 2.0 ** -7
+
+
+@pytest.mark.parametrize("B,whole", [(5, False), (20, True), (40, True)])
+def test_the_batched_plan_gets_its_own_kernel_and_matches_the_full_one(B, whole):
+    """A batched step on the tensor cores (one attention argument block per sequence, either attention form, one or two
+    passes of the dense grids) runs on the kernel that holds only its tiles; the full kernel gives the same bits."""
+    W = O.SyntheticWeights(MID, seed=36, gamma="ones")
+    prompts = np.random.default_rng(B).integers(0, MID.V, (B, 7))
+    res = []
+    for full in (0, 1):
+        prog = program(MID, W, B, 192)
+        assert prog.info["attn_whole"] == whole
+        prog.session.set_option("full_kernel", full)
+        assert prog.session.status().kernel_variant == (0 if full else 11)
+        res.append((prog.generate(prompts, 4), *(prog.read(n) for n in ("logits", "kc", "vc", "ti", "tw"))))
+        prog.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*res))
+    mma = program(SMALL_MOE, O.SyntheticWeights(SMALL_MOE, seed=36, gamma="ones"), 2, 64, "mma")
+    assert mma.session.status().kernel_variant == 0                                      # tiles the batched kernel does not hold
+    mma.close()

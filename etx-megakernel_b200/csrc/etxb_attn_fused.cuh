@@ -109,19 +109,17 @@ __device__ __forceinline__ void attn_fused_prep(const etxb_attnf_args& d, const 
   const int lane = tidx() & 31, warp = tidx() >> 5, epl = HD >> 5;
   const long long cb = slot / BS; const int off = (int)(slot % BS);
   const int lb_new = (int)(pos / BS) - part * P / BS, lo_new = (int)(pos % BS);
-  if (warp < G) {
+  if (warp < G || (warp == G && owner)) {                           // q heads, then the new k row: raw rows lie one behind the other
+    // (one copy of the norm for both: with two, the form for any head_dim kept 164 bytes of registers on the stack)
     float o[8];
-    head_norm_rope_s<0>(s.raw + warp * HD, d.qw ? s.cw + HD : nullptr, s.cw, HD, d.eps, o);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) if (j < epl) s.qs[warp * HD + lane * epl + j] = o[j];
-  } else if (warp == G && owner) {
-    float o[8];
-    head_norm_rope_s<0>(s.raw + G * HD, d.kw ? s.cw + 2 * HD : nullptr, s.cw, HD, d.eps, o);
+    const bool isq = warp < G;
+    head_norm_rope_s<0>(s.raw + warp * HD, (isq ? d.qw : d.kw) ? s.cw + (isq ? HD : 2 * HD) : nullptr, s.cw, HD, d.eps, o);
     __nv_bfloat16* kc = (__nv_bfloat16*)d.kc;
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (j < epl) {
         const int dd = lane * epl + j;
+        if (isq) { s.qs[warp * HD + dd] = o[j]; continue; }
         const __nv_bfloat16 kb = __float2bfloat16_rn(o[j]);
         kc[(((size_t)cb * NKV + h) * (HD / X) + dd / X) * BS * X + (size_t)off * X + dd % X] = kb;
         s.ks[(size_t)lb_new * HD * BS + ((size_t)(dd / X) * BS + lo_new) * X + dd % X] = kb;
@@ -200,7 +198,7 @@ __device__ __forceinline__ void attn_fused_core(const etxb_attnf_args& d, const 
 
 // out[hq][:] = bf16(sum_p w_p * tmp[p][:] / sum_p w_p * l_p), w_p = exp(m_p - max m), for the G q heads of kv head h.
 // Run by the last task of the kv head; reads the partials the other CTAs wrote (L2).  G * np <= 8192.
-__device__ __noinline__ void attn_fused_merge(const etxb_attnf_args& d, const Smem& sm, int h, int np, int HD) {
+__device__ __forceinline__ void attn_fused_merge(const etxb_attnf_args& d, const Smem& sm, int h, int np, int HD) {
   const int G = d.NH / d.NKV, lane = tidx() & 31, warp = tidx() >> 5;
   float* wl = sm.xs;                                              // [G][np] max logits, then weights
   float* es = sm.xs + 8192;                                       // [G][np] exp sums
@@ -263,8 +261,11 @@ __device__ __noinline__ void attn_fused_merge(const etxb_attnf_args& d, const Sm
   }
 }
 
+// (inlined with the merge into the call that runs the tile: a call in between takes the address of Smem, which then lives on the
+// stack behind the event's acquire.  6 layers with head_dim 64, 32 q heads on 8 kv heads, a step at 600 positions 393 -> 360 us, at
+// 8000 1296 -> 1178; head_dim 128 with this form 310 -> 295)
 template <int HDT, int BST>
-__device__ __noinline__ void attn_fused_impl(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S) {
+__device__ __forceinline__ void attn_fused_impl(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S) {
   const int HD = HDT ? HDT : d.HD;
   const int NKV = d.NKV, G = d.NH / NKV, P = ETXB_ATTN_PART;
   const int part = blk / NKV, h = blk - part * NKV;
@@ -300,10 +301,11 @@ __device__ __noinline__ void attn_fused_impl(const etxb_attnf_args& d, int blk, 
   if (*flag) attn_fused_merge(d, sm, h, min((seq + P - 1) / P, d.max_parts), HD);
 }
 
+__device__ __forceinline__ bool attn_fused_128(const etxb_attnf_args& d) { return d.HD == 128 && d.BS == 16; }
 __device__ __forceinline__ void tile_attn_fused(const unsigned char* a, int blk, const Smem& sm, const etxb_stepv& S) {
   const etxb_attnf_args& d = *(const etxb_attnf_args*)a;
   if (blk >= (int)d.nblocks) return;
-  if (d.HD == 128 && d.BS == 16) attn_fused_impl<128, 16>(d, blk, sm, S);
+  if (attn_fused_128(d)) attn_fused_impl<128, 16>(d, blk, sm, S);
   else attn_fused_impl<0, 0>(d, blk, sm, S);
 }
 

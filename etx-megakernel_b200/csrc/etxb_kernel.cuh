@@ -196,8 +196,8 @@ __device__ __forceinline__ Smem smem_view() {
   sm.deadline = &s_deadline; sm.stop = &s_stop; sm.tc = &s_tc; sm.geo = &s_geo; sm.vars = &s_vars;
   return sm;
 }
-// A tile of the batched step.  These are calls: each tile gets the registers for itself (inlined side by side they spilled
-// into each other's paths).
+// A tile of the full kernel or of the batched step.  These are calls: each tile gets the registers for itself (inlined side by
+// side they spilled into each other's paths).
 template <int B>
 __device__ __noinline__ void batch_call(const unsigned char* args, int c0, int cur, const etxb_stepv& S) {
   const Smem sm = smem_view();
@@ -214,7 +214,8 @@ __device__ __noinline__ void batch_call(const unsigned char* args, int c0, int c
   else if constexpr (B == 7) tile_attnprep(args, c0, sm, S);
   else if constexpr (B == 8) tile_attn(args, c0, sm, S);
   else if constexpr (B == 9) tile_attn_reduce(args, c0, sm, S);
-  else tile_attn_fused(args, c0, sm, S);
+  else if constexpr (B == 12) attn_fused_impl<0, 0>(*(const etxb_attnf_args*)args, c0, sm, S);
+  else attn_fused_impl<128, 16>(*(const etxb_attnf_args*)args, c0, sm, S);
 }
 __device__ __noinline__ void argmax_col_call(const etxb_params& p, const unsigned char* args, int c0) {
   const int nb = ((const etxb_batch_args*)args)->nb;
@@ -231,8 +232,11 @@ __device__ __noinline__ void attn_call(const etxb_attnf_args& d, int blk, const 
 template <bool GENERAL>
 __device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, int cur, const etxb_stepv& S) {
   const etxb_attnf_args& d = *(const etxb_attnf_args*)a;
-  if (GENERAL && d.gq == 0) { batch_call<12>(a, blk, cur, S); return; }
-  if (blk >= (int)d.nblocks || d.gq <= 0) return;
+  if (blk >= (int)d.nblocks || d.gq < 0) return;
+  if (d.gq == 0) {
+    if constexpr (GENERAL) { if (attn_fused_128(d)) batch_call<12 + 128>(a, blk, cur, S); else batch_call<12>(a, blk, cur, S); }
+    return;
+  }
   const int form = (d.gq == 1 ? 0 : d.gq == 2 ? 1 : d.gq == 4 ? 2 : 3) + ((d.part_len & ETXB_GQ_WHOLE) ? 4 : 0);
   switch (form) {
     case 0: attn_call<1, false>(d, blk, S); break;

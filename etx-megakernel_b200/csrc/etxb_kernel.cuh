@@ -203,10 +203,7 @@ __device__ __noinline__ void batch_call(const unsigned char* args, int c0, int c
   const Smem sm = smem_view();
   if constexpr (B == 18) tile_prologue_nb(args, c0, S);
   else if constexpr (B == 13) tile_norm_col(args, c0, sm);
-  else if constexpr (B == 14) tile_gemv_nb(args, c0, sm);
   else if constexpr (B == 15) tile_route(args, c0, sm);
-  else if constexpr (B == 16) tile_moe_up_g(args, c0, sm);
-  else if constexpr (B == 17) tile_moe_down_g(args, c0, sm);
   else if constexpr (B == 20) tile_gemv_tc(args, c0, sm, s_tc, cur);
   else if constexpr (B == 21) tile_moe_up_tc(args, c0, sm, s_tc, cur);
   else if constexpr (B == 22) tile_moe_down_tc(args, c0, sm, s_tc, cur);
@@ -288,12 +285,14 @@ __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c,
     case 9: ETXB_TILE(!LEAN, batch_call<9>(args, c0, cur, p.step));
     case 10: ETXB_TILE(!LEAN, tile_splitk_part(args, c0, c1, sm));
     case 11: ETXB_TILE(!LEAN, tile_splitk_sum(args, c0));
-    // batched decode (several columns per step)
+    // batched decode (several columns per step).  The mma.sync tiles (14, 16, 17) are inlined: their loops want every register, and
+    // a call saves the caller's on the stack first.  3 layers of 64 experts: 8 sequences at 1000 positions 818 us with calls, 661
+    // inlined; 32 at 300 positions 1416, 1199.
     case 13: ETXB_TILE(FULL || BATCHED, batch_call<13>(args, c0, cur, p.step));
-    case 14: ETXB_TILE(!LEAN, batch_call<14>(args, c0, cur, p.step));
+    case 14: ETXB_TILE(!LEAN, tile_gemv_nb(args, c0, sm));
     case 15: ETXB_TILE(FULL || BATCHED, batch_call<15>(args, c0, cur, p.step));
-    case 16: ETXB_TILE(!LEAN, batch_call<16>(args, c0, cur, p.step));
-    case 17: ETXB_TILE(!LEAN, batch_call<17>(args, c0, cur, p.step));
+    case 16: ETXB_TILE(!LEAN, tile_moe_up_g(args, c0, sm));
+    case 17: ETXB_TILE(!LEAN, tile_moe_down_g(args, c0, sm));
     case 18: ETXB_TILE(FULL || BATCHED, batch_call<18>(args, c0, cur, p.step));
     case 19: ETXB_TILE(FULL || BATCHED, argmax_col_call(p, args, c0));
     case 20: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<20>(args, c0, cur, p.step));

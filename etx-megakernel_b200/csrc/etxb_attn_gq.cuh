@@ -60,12 +60,18 @@ __device__ __forceinline__ float poll_pair(const uint2* p, uint32_t fl, const Sm
   }
 }
 
-// Between two rounds of a poll of several pairs: false when the step is being abandoned (deadline or abort, see poll_pair).
-__device__ __forceinline__ bool poll_again(uint32_t& spins, const Smem& sm) {
+// Between two rounds of a poll of n pairs (from `p` on, a partition apart): false when the step is being abandoned (deadline or
+// abort, see poll_pair).  The flag that is missing is looked up again for the report, so that the poll need not keep it.
+__device__ __forceinline__ bool poll_again(uint32_t& spins, const uint2* p, int n, uint32_t fl, const Smem& sm) {
   if ((++spins & 15u) == 0) {
     if (ld_relaxed(sm.ctrl()) != 0) { *(volatile int*)sm.stop = 1; return false; }
     if ((spins & 255u) == 0 && globaltimer() > *sm.deadline) {
-      if (atomicOr(sm.ctrl(), ETXB_CTRL_TIMEOUT) == 0) { sm.ctrl()[1] = sm.cur(); sm.ctrl()[2] = -3; sm.ctrl()[3] = 0; sm.ctrl()[4] = 0; }
+      if (atomicOr(sm.ctrl(), ETXB_CTRL_TIMEOUT) == 0) {
+        uint32_t seen = fl;
+#pragma unroll 1
+        for (int u = 0; u < n && seen == fl; ++u) seen = ld_pair(p + (size_t)u * ETXB_GQ_PW).y;
+        sm.ctrl()[1] = sm.cur(); sm.ctrl()[2] = -3; sm.ctrl()[3] = (int32_t)seen; sm.ctrl()[4] = (int32_t)fl;
+      }
       *(volatile int*)sm.stop = 1;
       return false;
     }
@@ -131,7 +137,7 @@ __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Sm
           for (int u = 0; u < NPR; ++u) first[u] = ld_pair(tp + (size_t)min(u, np - 1) * ETXB_GQ_PW);
 #pragma unroll
           for (int u = 0; u < NPR; ++u) { pv[r][u] = __uint_as_float(first[u].x); ok = ok && first[u].y == fl; }
-        } while (!ok && poll_again(spins, sm));
+        } while (!ok && poll_again(spins, tp, np, fl, sm));
       }
     }
   }
@@ -189,7 +195,7 @@ __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Sm
           for (int u = 0; u < NPR; ++u) first[u] = ld_pair(tp + (size_t)min(p0 + u, np - 1) * ETXB_GQ_PW);
 #pragma unroll
           for (int u = 0; u < NPR; ++u) ok = ok && first[u].y == fl;
-        } while (!ok && poll_again(spins, sm));
+        } while (!ok && poll_again(spins, tp + (size_t)p0 * ETXB_GQ_PW, min(NPR, np - p0), fl, sm));
 #pragma unroll
         for (int u = 0; u < NPR; ++u)
           if (p0 + u < np) o = __fmaf_rn(wg[p0 + u], __uint_as_float(first[u].x), o);

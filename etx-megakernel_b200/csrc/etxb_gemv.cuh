@@ -48,6 +48,7 @@ struct CtaVars {
   uint32_t epoch;            // the step (sharded sessions: the flag of this step's exchanged words derives from it)
   int cur;                   // the running task's index in the queue order (reported when a wait gives up)
   int q0, q1;                // the CTA's queue
+  int halt;                  // thread 0's word before a task: the step is being abandoned, everybody leaves the loop
   int hold;                  // the running task's results are on their way out: the producer starts no further stage (see produce_task)
 };
 struct Smem {

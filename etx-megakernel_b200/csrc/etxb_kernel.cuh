@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
   const Smem sm = smem_view();
   if (threadIdx.x == 0) {
     s_stop = 0;
-    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.cur = 0; s_vars.hold = 0;
+    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.cur = 0; s_vars.halt = 0; s_vars.hold = 0;
     s_deadline = globaltimer() + p.timeout_ns;
     for (int i = 0; i < ETXB_NSTAGE; ++i) { mbar_init(sm.full + i, 1); mbar_init(sm.empty + i, ETXB_EMPTY_COUNT); ((uint32_t*)(sm.empty + ETXB_NSTAGE))[i] = 0xffffffffu; }
     if constexpr (TC) {
@@ -414,6 +414,9 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
     if (tidx() == 0) {
       const int in_n = c->r.in_n;
       if (p.trace) p.trace[8 * (size_t)c->r.id] = globaltimer();
+      // Everybody must leave the loop at the same task, or a barrier waits for warps that have left.  s_stop may be set at any
+      // time (by the producer warp, by a warp whose wait in a body gives up), so only this thread looks at it, before the barrier.
+      const bool stopped = *(volatile int*)&s_stop != 0;
       bool ok = true;                                              // wait_event polls the abort word itself
       for (int i = 0; ok && i < in_n; ++i) {
         int word, cnt;
@@ -422,6 +425,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
         ok = wait_event(p, word, (int32_t)(p.epoch * (uint32_t)cnt), cur, s_deadline);
       }
       if (!ok) s_stop = 1;
+      s_vars.halt = stopped || !ok;
       s_vars.tr = p.trace ? p.trace + 8 * (size_t)c->r.id : nullptr;
       s_vars.cur = cur;
       if (p.trace) p.trace[8 * (size_t)c->r.id + 1] = globaltimer();
@@ -435,7 +439,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
       }
     }
     csync();
-    if (s_stop) break;
+    if (vars->halt) break;
     if (tidx() >= ETXB_CONSUMERS - 32) {                            // the last consumer warp keeps the contexts coming (asynchronously)
       const int q1 = vars->q1;
       fetch_ctx(p, ctx, vars->q0, cur + 2 < q1 ? cur + 2 : -1, cur + 1 < q1 ? cur + 1 : -1);
@@ -477,12 +481,22 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
     if (p.tc_on != 0u) {
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       csync();                                                     // nobody reads an accumulator any more
-      // an abandoned step may have loaded stages that no MMA took: wait (bounded) for those copies before the CTA's memory goes
-      if (tidx() == 32 && ld_relaxed(p.ctrl) != 0)
-        for (int i = 0; i < ETXB_TC_MAXSTAGE; ++i)
-          if (s_tc.lu[i] != s_tc.mu[i])
-            for (int spin = 0; spin < 2000000 && !mbar_try_wait(s_tc.full + i, (s_tc.lu[i] - 1) & 1); ++spin) {}
-      if (threadIdx.x < 32) tc_dealloc(s_tc.tmem);
+      if (threadIdx.x < 32) {
+        // an abandoned step may have loaded stages that no MMA took, and MMAs that nobody waited for may still be reading theirs
+        // and writing tensor memory: wait (bounded) for the copies, and for the commit behind each stage's last MMAs
+        if (__any_sync(0xffffffffu, ld_relaxed(p.ctrl) != 0)) {
+          for (int i = 0; i < ETXB_TC_MAXSTAGE; ++i) {
+            const uint32_t lu = s_tc.lu[i], mu = s_tc.mu[i];
+            if (lu != mu)
+              for (int spin = 0; spin < 2000000 && !mbar_try_wait(s_tc.full + i, (lu - 1) & 1); ++spin) {}
+            if (mu != 0)
+              for (int spin = 0; spin < 2000000 && !mbar_try_wait(s_tc.empty + i, (mu - 1) & 1); ++spin) {}
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          __syncwarp();
+        }
+        tc_dealloc(s_tc.tmem);
+      }
     }
   }
 }

@@ -21,7 +21,8 @@ def test_group_size_divides_the_heads_of_a_kv_head(G, NKV, maxlen):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("NH,NKV,qk_norm,seq,gq", [(12, 2, False, 1, 1), (12, 2, False, 127, 2), (12, 2, False, 128, 1), (12, 2, True, 129, 2),
-                                                   (12, 2, False, 1700, 2), (6, 2, True, 300, 1), (12, 1, False, 257, 4)])
+                                                   (12, 2, False, 1700, 2), (6, 2, True, 300, 1), (12, 1, False, 257, 4),
+                                                   (28, 4, False, 385, 1), (15, 1, True, 256, 1), (16, 1, False, 300, 8)])
 def test_grouped_phase_with_other_head_counts(NH, NKV, qk_norm, seq, gq):
     from tests.test_gpu_ops import test_attention_phase_fused as phase
     phase(NH, NKV, 128, qk_norm, seq, gq)

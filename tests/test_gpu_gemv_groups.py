@@ -1,11 +1,13 @@
 """The one-token GEMV at the edges of its rule for sharing a stage between the warps (rows at once, warps per stage): the
 widest row of each class, the next one, rows that fill a stage exactly or not, and several tasks behind each other on a
 worker so that a stage changes hands between groups."""
+import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
+from oracle import ref_decode as O  # noqa: E402
 from tests.test_gpu_ops import assert_bf16_close, gemv_case  # noqa: E402
 from tests.test_gpu_ops import test_moe_block_grouped_slots_and_summed_down as moe_block_grouped  # noqa: E402
 
@@ -18,6 +20,13 @@ def test_rows_per_warp_classes(K, N, tasks):
     # fp32 sums of K products in another order: a result may round to the neighbouring bf16 value when it lies within
     # the fp32 error of a rounding boundary, one in a few hundred
     assert_bf16_close(got, want, f"K={K} N={N} tasks={tasks}", min_exact=0.97 if N > 100 else 0.6)
+    if N == 3:
+        # too few for a share: each against its fp64 sum, half a bf16 ulp (2^-8 of the value at most) and the bound of a lane's
+        # chain of K / 32 fp32 steps with the butterfly behind it
+        rng = np.random.default_rng(K + N)
+        W, x = O.bfr(rng.standard_normal((N, K), dtype=np.float32) * np.float32(0.02)), O.bfr(rng.standard_normal((1, K), dtype=np.float32))
+        terms = W.astype(np.float64) * x.astype(np.float64)
+        assert np.all(np.abs(got[0] - terms.sum(1)) <= 2.0 ** -8 * np.abs(terms.sum(1)) + (K / 32 + 8) * 2.0 ** -24 * np.abs(terms).sum(1))
 
 
 # each slot with its own activation vector: 4 rows at once (short rows) and one (2048 and more), slots that straddle stages

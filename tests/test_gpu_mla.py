@@ -150,3 +150,22 @@ def test_blocks_outside_the_tile_are_refused():
     bad[60:64] = (2048).to_bytes(4, "little")                 # C beyond the tile's shared-memory layout, patched past the Python check
     with pytest.raises(EtxbError, match="mla_attn"):
         op_launch("mla_attn", bytes(bad), 2 * 5)
+
+
+def test_the_plan_gets_the_latent_attention_kernel_and_matches_the_full_one():
+    """The latent-attention plan runs on its lean kernel; the full kernel gives the same bits."""
+    d, layers, embed, final_norm, lm_head = small_model(2)
+    maxlen = 64
+    packed = {"embed": embed, "final_norm": final_norm, "lm_head": lm_head}
+    for L in range(d.L):
+        packed.update(M.pack_layer(d, L, layers[L]))
+    weights = M.to_device(d, packed, maxlen, DEV)
+    prompt = np.random.default_rng(6).integers(0, d.V, 7)
+    res = []
+    for full in (0, 1):
+        prog = M.MlaProgram(d, weights, device=0, maxlen=maxlen)
+        prog.session.set_option("full_kernel", full)
+        assert prog.session.status().kernel_variant == (0 if full else 10)
+        res.append((prog.generate(prompt, 6), *(prog.read(n) for n in ("logits", "ckv", "ti", "tw"))))
+        prog.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*res))

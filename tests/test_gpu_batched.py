@@ -208,3 +208,30 @@ def test_the_batched_plan_gets_its_own_kernel_and_matches_the_full_one(B, whole)
     mma = program(SMALL_MOE, O.SyntheticWeights(SMALL_MOE, seed=36, gamma="ones"), 2, 64, "mma")
     assert mma.session.status().kernel_variant == 0                                      # tiles the batched kernel does not hold
     mma.close()
+
+
+def test_a_batched_step_after_an_abandoned_one_is_correct():
+    """The host watchdog aborts a step of some milliseconds at once, in the middle of its tensor-core tiles (weight copies and
+    MMAs in flight, tensor memory held): the step reports it, the context stays usable, and the session then gives the tokens
+    of a fresh one."""
+    from etx_megakernel_b200.runtime.lib import EtxbError
+    d = Q.Dims(name="deep", H=1024, NH=16, NKV=4, HD=128, INTER=0, L=32, V=4096, qk_norm=True, moe=True, E=32, TOPK=8, MI=384, norm_topk=True)
+    w = D.random_packed_weights(d, 64, torch.device("cuda:0"), seed=4, gamma="ones")
+    prompts = np.random.default_rng(9).integers(0, d.V, (24, 4))
+    fresh = BT.BatchProgram(d, w, 24, device=0, maxlen=64)
+    want = fresh.generate(prompts, 5)
+    fresh.close()
+    prog = BT.BatchProgram(d, w, 24, device=0, maxlen=64)
+    aborted = 0
+    for _ in range(3):
+        prog.session.set_step(tok=0, pos=0, write_next=0)
+        prog.session.launch()
+        try:
+            prog.session.wait(1e-7)
+        except EtxbError as e:
+            assert e.status == "E_ABORTED"
+            aborted += 1
+        assert np.array_equal(prog.generate(prompts, 5), want)
+    prog.close()
+    if aborted == 0:
+        pytest.skip("every step finished before the host watchdog looked at it")

@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(ETXB_CONSUMERS, 1) etxb_attn_static_kernel(con
   Smem sm;
   sm.xs = (float*)st_smem;
   sm.scr = (float*)(st_smem + ETXB_GEN_BYTES);
-  sm.ring = nullptr; sm.full = nullptr; sm.empty = nullptr; sm.prod = nullptr; sm.deadline = nullptr; sm.stop = nullptr; sm.tc = nullptr; sm.geo = nullptr; sm.vars = nullptr;
+  sm.ring = nullptr; sm.full = nullptr; sm.empty = nullptr; sm.prod = nullptr; sm.deadline = nullptr; sm.stop = nullptr; sm.geo = nullptr; sm.vars = nullptr;
   tile_attn_fused((const unsigned char*)&d, (int)blockIdx.x, sm, S);
 }
 }  // namespace etxb

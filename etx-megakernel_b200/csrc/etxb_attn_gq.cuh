@@ -397,8 +397,8 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
 // ---------------------------------------------------------------------------------------------- a whole sequence per task
 // The same attention with one task per (sequence, group of GQ q heads): the task walks the context's partitions itself,
 // keeps every partition's partial output and statistics in shared memory and merges them at the end with the merge's
-// arithmetic (same partition boundaries, same order of sums: the results are those of the one-partition-per-task form bit
-// for bit).  This is the form of a batched step with enough sequences to fill the workers (sequences x kv heads x groups
+// arithmetic (same partition boundaries, same order of the partitions; inside a partition the products run on the tensor cores,
+// so the sums are in another order than in the one-partition-per-task form and most, not all, results have the same bits).  This is the form of a batched step with enough sequences to fill the workers (sequences x kv heads x groups
 // tasks): the q rows are prepared once per sequence instead of once per partition, the next partition's K (then V) is
 // copied asynchronously into shared memory while the current one is being worked on, so the cache latency hides behind
 // the softmax and the output sums, and nothing is published, polled or merged through global memory.

@@ -60,7 +60,6 @@ struct Smem {
   int32_t* prod;             // producer-warp scratch: 16 ids + 16 weights
   const unsigned long long* deadline;
   int* stop;                 // CTA-local: a wait inside a body gave up (the body's results are not to be announced)
-  struct TcShared* tc;       // state of the tensor-core tiles of a batched step (null where the kernel has none)
   const GemvGeom* geo;       // the running GEMV-family task's rows and how the warps share them
   CtaVars* vars;       // null outside the persistent kernel
   __device__ __forceinline__ int32_t* ctrl() const { return vars->ctrl; }
@@ -232,8 +231,8 @@ __device__ __forceinline__ int udiv_small(int a, int b) {
 }
 // Rows at once (R) and warps per stage (W): one row at a time is a chain of waits, shared-memory latencies and shuffles that
 // 4 warps per scheduler do not hide; several rows share the activation vector with its unpacking and are reduced together.
-// Rows of up to 1792 values (7 vectors per lane): 4 at once; of 2048 (6 rows per stage): 3; longer ones: a stage holds 3
-// rows or fewer, one warp each (so too where every range has its own activation vector and 3 rows share nothing).  Clocks
+// Rows of up to 1792 values (7 vectors per lane): 4 at once; of 2048 (6 rows per stage): 3; longer ones: a stage holds 5
+// rows or fewer (of 4096: 3), one warp each (so too where every range has its own activation vector and 3 rows share nothing).  Clocks
 // per task, weights already in the ring, against one row per warp and every warp on every stage:
 // 35 rows of 2048: 5816 -> 3786; 8 x 14 rows of 768: 8972 -> 6486; 48 of 1536: 6277 -> 3701; 18 of 4096: 5420 -> 5293.
 __device__ __forceinline__ void gemv_geom(int body, GemvGeom& g) {

@@ -193,7 +193,7 @@ __device__ __forceinline__ Smem smem_view() {
   sm.full = (uint64_t*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4);
   sm.empty = sm.full + ETXB_NSTAGE;
   sm.prod = (int32_t*)(sm.empty + ETXB_NSTAGE) + 8;                 // (behind the notes of the stages' uses)
-  sm.deadline = &s_deadline; sm.stop = &s_stop; sm.tc = &s_tc; sm.geo = &s_geo; sm.vars = &s_vars;
+  sm.deadline = &s_deadline; sm.stop = &s_stop; sm.geo = &s_geo; sm.vars = &s_vars;
   return sm;
 }
 // A tile of the full kernel or of the batched step.  These are calls: each tile gets the registers for itself (inlined side by
@@ -253,8 +253,9 @@ __device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, i
 // grouped attention tile with GQV q heads per task); ETXB_VARIANT_MLA = the lean kernel of a latent-attention model (the
 // same GEMV family with the latent-attention tile in place of the grouped one); ETXB_VARIANT_BATCH = the tiles of a batched step
 // on the tensor cores.  The host picks it from the plan (select_variant): the full
-// kernel is 550 KB of code, of which a decode step uses a fraction scattered through it, and the step runs about 10 %
-// faster from a 142 KB kernel (instruction fetch).
+// kernel is 1020 KB of code, of which a decode step uses a fraction scattered through it, and its tiles are calls.  From the
+// 142 KB kernel (same bits): 12 layers of a 128-expert model 794 -> 693 us, of a dense one 1393 -> 1253; 9 layers of a
+// latent-attention model 794 -> 689 from its 170 KB; the batched kernel (610 KB) gives 1 to 5 % (batched_plan).
 // XCH: the variants a sharded session launches -- the same bodies plus the exchange code (flagged-row folds of R = ranks
 // rows, row publishing after the body, the argmax exchange); compiled out of the others.
 #define ETXB_VARIANT_MLA 16

@@ -1,5 +1,5 @@
 // Batched decode on the Blackwell tensor cores: tcgen05.mma with the tokens as the M side (A operand, shared memory,
-// SWIZZLE_128B K-major), 128 or 256 weight rows as the N side (B operand, loaded by TMA tensor copies --
+// SWIZZLE_128B K-major), 64 .. 256 weight rows as the N side (B operand, loaded by TMA tensor copies --
 // cp.async.bulk.tensor.2d with SWIZZLE_128B, one tensor map per weight tensor, boxes of 64 k x 64 rows, up to four per
 // instruction) and fp32 accumulators in tensor memory, read back with tcgen05.ld for the epilogue.
 //
@@ -11,11 +11,11 @@
 // delivers (22.5), and all of a batch's tokens (up to 32 here) ride along for free -- mma.sync m16n8k16, the legacy
 // path, managed about a sixth of that with 8 tokens per pass.
 //
-// A task = a few tiles of up to 256 weight rows (two neighbouring blocks of 128 rows of a matrix, or an expert's 128 gate
-// rows and their 128 up rows) x all of K (or a K-slice) x up to 32 tokens.  Roles inside the CTA's consumer warps: every
-// thread stages the tokens' vectors into the swizzled layout, once per task; one thread issues the TMA loads of the
-// weight tiles, k-chunk by k-chunk, through a ring of 32 KB stages (as many as fit beside the tokens: 2 with 32 tokens
-// of 2048 columns, 5 with up to 8); one thread issues the MMAs (four k16 steps per 64-wide chunk) and commits each stage back to the loader; when the last
+// A task = a few tiles of 64 .. 256 weight rows (neighbouring rows of a matrix, or up to 128 of an expert's gate rows and
+// as many up rows) x all of K (or a K-slice) x up to 32 tokens.  Roles inside the CTA's consumer warps: one
+// warp issues the TMA loads of the weight tiles (a lane per box of 64 rows), k-chunk by k-chunk, through a ring of 32 KB stages
+// (as many as fit beside the tokens: 2 with 32 tokens of 2048 columns, 5 with up to 8), and starts before the tokens are there;
+// the other threads stage the tokens' vectors into the swizzled layout, once per task; one thread issues the MMAs (four k16 steps per 64-wide chunk) and commits each stage back to the loader; when the last
 // MMA of a tile has completed, four warps read its accumulators (one token per TMEM lane) and run the epilogue while
 // the next tile's MMAs fill the other accumulator buffer.  The weight ring of the one-token tiles is not in use during
 // a batched step (their producer warp has nothing to stream), so its shared memory and the general region form one

@@ -159,9 +159,13 @@ class MachineModel:
 
     def attention_groups(self, NH: int, NKV: int, HD: int, BS: int, maxlen: int) -> tuple:
         """(q heads per task, positions per task, partitions) of the grouped attention tile, or (0, 0, 0) when the
-        shape needs the general tile (12 q heads on 2 kv heads, 600 positions: 14.7 us per layer there, and the step on the
-        full kernel for its sake).  The fewest q heads per task that still gives every task its own SM: the merge
-        a group's last task runs reads gq * partitions partial rows, and the groups of a kv head share its K / V in L2."""
+        shape needs the general tile.  The fewest q heads per task that still gives every task its own SM: the merge
+        a group's last task runs reads gq * partitions partial rows, and the groups of a kv head share its K / V in L2.
+
+        Head counts that leave one q head per task (3, 5, 7 .. per kv head) read K and V once per q head and still gain
+        over the general tile, which also takes the step to the full kernel.  A layer of a small dense model at 600 / 2000 /
+        8000 positions, general -> grouped, us: 28 q heads on 4 kv heads 44 / 58 / 135 -> 32 / 48 / 103; 56 on 8
+        61 / 84 / 218 -> 42 / 69 / 181; 24 on 8 50 / 71 / 180 -> 32 / 43 / 98; 36 on 4 47 / 66 / 160 -> 37 / 48 / 125."""
         G = NH // NKV
         if HD != 128 or BS != 16:
             return (0, 0, 0)

@@ -12,6 +12,8 @@
 #include <chrono>
 #include <string>
 #include <thread>
+#include <array>
+#include <map>
 #include <vector>
 
 #include "../../include/etxb200.h"
@@ -118,7 +120,7 @@ static int32_t check_attnf_block(const etxb_attnf_args& a) {
     else if (a.gq * a.max_parts > 4096) why = "gq * max_parts <= 4096";
     else if ((a.part_len >> 24) & ~1) why = "part_len bits 25..31 are zero";
     else if ((a.part_len >> 24) && (a.nblocks > (uint32_t)(a.NH / a.gq) || 65536 + (size_t)a.max_parts * a.gq * 130 * 4 > ETXB_RING_BYTES))
-      why = "whole-sequence form: the grid is NH / gq tasks and 64 KB + max_parts * gq * 130 floats fit the idle weight ring";
+      why = "whole-sequence form: the grid is NH / gq tasks and 64 KB + max_parts * gq * 130 floats fit the weight ring (longer contexts: partitions)";
     else if (a.nblocks > (uint32_t)(a.max_parts * (a.NH / a.gq))) why = "the grid is at most max_parts * NH / gq tasks";
   } else {
     const int G = a.NH / a.NKV;
@@ -277,12 +279,12 @@ static int select_variant(const etxb_session* s, const std::vector<unsigned char
 // Entries 5..9: the same five with the exchange code of a sharded session compiled in (launch_kernel adds 5).
 // Entry 10: the lean decode kernel of a latent-attention model (no sharded form: such a session falls back to entry 5).
 // Entry 11: the kernel of a batched step on the tensor cores.
-static const void* const g_kernels[12] = {(const void*)etxb::etxb_megakernel<0>, (const void*)etxb::etxb_megakernel<1>, (const void*)etxb::etxb_megakernel<2>,
-                                          (const void*)etxb::etxb_megakernel<4>, (const void*)etxb::etxb_megakernel<8>,
-                                          (const void*)etxb::etxb_megakernel<0, true>, (const void*)etxb::etxb_megakernel<1, true>,
-                                          (const void*)etxb::etxb_megakernel<2, true>, (const void*)etxb::etxb_megakernel<4, true>,
-                                          (const void*)etxb::etxb_megakernel<8, true>, (const void*)etxb::etxb_megakernel<ETXB_VARIANT_MLA>,
-                                          (const void*)etxb::etxb_megakernel<ETXB_VARIANT_BATCH>};
+// (the group size of grouped attention is read from the argument block: entries 1..4, and 6..9, are one kernel)
+static const void* const g_lean = (const void*)etxb::etxb_megakernel<ETXB_VARIANT_LEAN>;
+static const void* const g_lean_x = (const void*)etxb::etxb_megakernel<ETXB_VARIANT_LEAN, true>;
+static const void* const g_kernels[12] = {(const void*)etxb::etxb_megakernel<0>, g_lean, g_lean, g_lean, g_lean,
+                                          (const void*)etxb::etxb_megakernel<0, true>, g_lean_x, g_lean_x, g_lean_x, g_lean_x,
+                                          (const void*)etxb::etxb_megakernel<ETXB_VARIANT_MLA>, (const void*)etxb::etxb_megakernel<ETXB_VARIANT_BATCH>};
 static int kernel_index(const etxb_session* s) {
   const int v = s->force_full ? 0 : s->variant;
   if (s->xbase == nullptr) return v;
@@ -631,6 +633,42 @@ static int32_t build_tensor_maps(etxb_session* s) {
   return ETXB_OK;
 }
 
+// Grouped attention over partitions: who merges a group's partials (attn_gq_tile).  Where every worker's queue holds the tasks of a grid
+// in ascending order, the workers' last tasks of that grid share the merge of each group between them; otherwise (and in single-tile
+// launches) the record says nothing and the task of the last partition does it.  Written into the record's `mirror` word, which
+// attention tasks have no other use for.
+static void share_merges(const etxb_session* s, std::vector<etxb_rec>& recs) {
+  std::vector<char> ascending(s->types.size(), 1);
+  std::vector<int> last(recs.size(), 0);
+  for (uint32_t w = 0; w < s->h.n_workers; ++w) {
+    std::vector<int> at(s->types.size(), -1);                      // the worker's latest task of each type
+    for (int32_t i = s->qbegin[w]; i < s->qbegin[w + 1]; ++i) {
+      const int ty = s->tasks[i].type;
+      if (s->types[ty].body != ETXB_BODY_ATTN_FUSED) continue;
+      if (at[ty] >= 0) { last[at[ty]] = 0; if (s->tasks[at[ty]].id > s->tasks[i].id) ascending[ty] = 0; }
+      at[ty] = i; last[i] = 1;
+    }
+  }
+  std::map<std::array<int, 3>, std::vector<int>> groups;           // (type, sequence, q group) -> its tasks
+  for (size_t i = 0; i < recs.size(); ++i) {
+    const etxb_task& t = s->tasks[i];
+    const etxb_type& ty = s->types[t.type];
+    if (ty.body != ETXB_BODY_ATTN_FUSED || !ascending[t.type] || ty.args[0] != 0 || ty.cst[0] < 0 || ty.cst[1] < 0) continue;
+    const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
+    etxb_attnf_args a;
+    if (off < 0 || (uint64_t)off + sizeof a > s->h_pool.size()) continue;
+    memcpy(&a, s->h_pool.data() + off, sizeof a);
+    if (a.gq <= 0 || a.gq > a.NH || (a.part_len & ETXB_GQ_WHOLE) || t.coord[0] < 0 || t.coord[0] >= (int)a.nblocks) continue;
+    groups[{t.type, t.coord[1], t.coord[0] % (a.NH / a.gq)}].push_back((int)i);
+  }
+  for (auto& g : groups) {
+    uint32_t count = 0, k = 0;
+    for (int i : g.second) count += last[i];
+    if (count == 0) continue;
+    for (int i : g.second) recs[i].mirror = last[i] ? (count << 16 | ++k) : 0xffffu;
+  }
+}
+
 static int32_t upload_type_args(etxb_session* s) {
   std::vector<void*> ta((size_t)s->h.n_types * ETXB_MAX_ARGS, nullptr);
   for (size_t t = 0; t < s->types.size(); ++t)
@@ -676,6 +714,7 @@ static int32_t upload_type_args(etxb_session* s) {
       if (rc) return rc;
     }
   }
+  share_merges(s, recs);
   if (!s->d_recs) CU(cudaMalloc((void**)&s->d_recs, recs.size() * sizeof(etxb_rec) + 96));
   CU(cudaMemcpy(s->d_recs, recs.data(), recs.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
   // the same records grouped by grid (type), worker by worker, for the one-launch-per-grid baseline

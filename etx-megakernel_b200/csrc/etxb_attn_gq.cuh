@@ -1,13 +1,19 @@
-// The attention phase of a decode step, the form tuned for head_dim 128 and 16-position cache blocks: one task per
-// (128-position partition, group of GQ q heads that share a kv head).  Same work as the general fused tile
-// (etxb_attn_fused.cuh: q/k RMSNorm + neox rotary, the new position's k / v rows into the paged cache, split-KV
-// attention, merge by the last task to finish) with two differences that shorten its critical path:
-//   * the partition's K and V go from the cache straight into registers (each thread keeps the 64 + 64 bytes it will
-//     multiply), no shared-memory staging;
-//   * a task covers few q heads and many positions, so the merge that the last task runs reads GQ * parts partial
-//     rows (2 * 9 at a 1K context) instead of G * parts of 32 positions (8 * 34): one round of loads.
-// The groups of one kv head read the same K / V (through L2); the first group of the kv head writes the cache slot.
-// The new position never comes from the cache: its k / v rows are taken from shared memory as one extra position.
+// The attention phase of a decode step, the form for head_dim 128 and 16-position cache blocks: one task per
+// (128-position partition, group of gq <= 8 q heads that share a kv head), or one per group that walks the whole context.  Same work
+// as the general fused tile (etxb_attn_fused.cuh: q/k RMSNorm + neox rotary, the new position's k / v rows into the paged cache,
+// split-KV attention, merge), built around what a decode step makes of it: a few microseconds of latency and a stream of K / V.
+//   * K and V come through the weight ring: a cache block of one kv head is 4 KB of K and 4 KB of V in one piece each (a UNIT
+//     of 16 positions), three units to a stage.  The producer warp copies them ahead of the task as it does weights -- the rows of earlier
+//     positions depend on nothing in this step -- so they lie in shared memory when the q rows arrive.
+//   * a warp takes a unit at a time and runs it alone: scores on the tensor cores (mma.sync, 16 positions x 8 heads, K rows by
+//     ldmatrix), its own running maximum and sum, the probabilities transposed by movmatrix into the second product's operand, 128
+//     output sums per head in its registers.  No barrier between units; the warps' results meet once, at the end.
+//   * the probabilities go into the product as a bf16 value plus the bf16 of what that rounding lost (2^-17 of the value).
+// Bound by the stream of K / V at long contexts, by the chain q rows -> norm -> scores -> publish -> merge at short ones.
+// A phase at 8150 positions (64 partitions, 256 tasks): 30 us -> 17; 8 sequences at 1033: 33 -> 22; 32 sequences, whole contexts of 1045:
+// 52 -> 21; one sequence at 1037: 8.3 -> 7.9.  The forms before multiplied out of registers on the fp32 pipes, or walked a context with
+// a barrier between any two of its steps.
+// The new position never comes from the cache: its k / v rows stand in for the stale slot of the staged unit.
 //
 // It stands where the reference runs dsl_attnprep (etx/ops/attnprep.py:86-211), vLLM's paged attention and its reduce
 // kernel (etx/importer/spec.py:243-244; grids examples/vllm_llm/model.py:78-84, 358-362); numerics follow
@@ -18,9 +24,12 @@
 namespace etxb {
 
 #define ETXB_GQ_PART 128   // positions per task
-#define ETXB_GQ_STAGE_BYTES 65536  // whole-sequence form: a partition's K and V pieces in shared memory (512 threads x 4 x 16 bytes each)
-#define ETXB_GQ_WHOLE (1 << 24)   // part_len bit: one task per (sequence, q group) walks all partitions (plans without streamed tiles)
+#define ETXB_GQ_WHOLE (1 << 24)   // part_len bit: one task per (sequence, q group) takes all partitions
 #define ETXB_GQ_PW 136     // 8-byte (value, flag) pairs a task publishes per q head and partition: 128 outputs, max, sum, padding
+#define ETXB_GQ_SHARE 64   // partials (gq x partitions) from which the merge is shared out.  Below: 144 tasks that all wait and poll made a phase of
+                           // 2 x 9 partials 9.5 us, one merging task per group 8.0.  Above: 8 x 64 partials are 512 KB for one merging task
+#define ETXB_GQ_UNIT 8192  // a unit in a ring stage: 16 positions' K (4 KB), then their V
+#define ETXB_GQ_UPS (ETXB_STAGE_BYTES / ETXB_GQ_UNIT)   // units per stage
 
 // Partial results travel as FLAGGED PAIRS: every fp32 value is stored together with a 32-bit flag derived from the step
 // (one aligned 8-byte store: value and flag become visible together), into `tmp_out` viewed as
@@ -60,16 +69,16 @@ __device__ __forceinline__ float poll_pair(const uint2* p, uint32_t fl, const Sm
   }
 }
 
-// Between two rounds of a poll of n pairs (from `p` on, a partition apart): false when the step is being abandoned (deadline or
+// Between two rounds of a poll of n pairs (from `p` on, `stride` pairs apart): false when the step is being abandoned (deadline or
 // abort, see poll_pair).  The flag that is missing is looked up again for the report, so that the poll need not keep it.
-__device__ __forceinline__ bool poll_again(uint32_t& spins, const uint2* p, int n, uint32_t fl, const Smem& sm) {
+__device__ __forceinline__ bool poll_again(uint32_t& spins, const uint2* p, int n, size_t stride, uint32_t fl, const Smem& sm) {
   if ((++spins & 15u) == 0) {
     if (ld_relaxed(sm.ctrl()) != 0) { *(volatile int*)sm.stop = 1; return false; }
     if ((spins & 255u) == 0 && globaltimer() > *sm.deadline) {
       if (atomicOr(sm.ctrl(), ETXB_CTRL_TIMEOUT) == 0) {
         uint32_t seen = fl;
 #pragma unroll 1
-        for (int u = 0; u < n && seen == fl; ++u) seen = ld_pair(p + (size_t)u * ETXB_GQ_PW).y;
+        for (int u = 0; u < n && seen == fl; ++u) seen = ld_pair(p + (size_t)u * stride).y;
         sm.ctrl()[1] = sm.cur(); sm.ctrl()[2] = -3; sm.ctrl()[3] = (int32_t)seen; sm.ctrl()[4] = (int32_t)fl;
       }
       *(volatile int*)sm.stop = 1;
@@ -80,600 +89,398 @@ __device__ __forceinline__ bool poll_again(uint32_t& spins, const uint2* p, int 
   return true;
 }
 
-template <int GQ>
-struct GqSmem {
-  static constexpr int HD = 128, PL = ETXB_GQ_PART;
-  float* raw;   // [GQ + 2][HD] raw q rows, new k row, new v row
-  float* cw;    // [3][HD] cos | sin row, q norm weight, k norm weight
-  float* qs;    // [GQ][HD] normed + roped q
-  float* knew;  // [HD] normed + roped new k (bf16 values)
-  float* vnew;  // [HD] new v (bf16 values)
-  float* ph;    // [4][GQ][PL] quarter dot products
-  float* sc;    // [GQ][PL] probabilities
-  float* st;    // [GQ] max, [GQ] sum, [GQ] probability of the new position
-  float* po;    // [4][GQ][HD] partial outputs
-  __device__ explicit GqSmem(float* b) {
-    raw = b; cw = raw + (GQ + 2) * HD; qs = cw + 3 * HD; knew = qs + GQ * HD; vnew = knew + HD;
-    ph = vnew + HD; sc = ph + 4 * GQ * PL; st = sc + GQ * PL; po = st + 32;
-  }
+// What a task covers: worked out alike by the consumer warps and by the producer warp.
+struct GqTask {
+  int part, hq0, h;          // partition (0 in the whole-context form), first q head of the group, its kv head
+  int t0, u0, nu;            // first position; first unit (cache block) and number of units
+  int seq;
+  long long pos;
+  bool whole, owner;         // owner: the task's positions hold the one being written
 };
-#ifndef ETXB_LAYOUT_EXPERIMENT
-static_assert(((8 + 2) + 3 + 8 + 2 + 32 + 8 + 32) * 128 * 4 + 128 <= ETXB_GEN_BYTES, "GQ = 8 layout fits the general region");
-#endif
-
-// out[hq][:] = bf16(sum_p w_p * tmp[p][:] / sum_p w_p * l_p), w_p = exp(m_p - max m), for q heads hq0 .. hq0 + GQ - 1.
-// Run by the task of the last partition; polls the flagged partials the other CTAs publish (L2).  GQ * np <= 4096.
-// The statistics AND the partial outputs are requested in one round (up to ETXB_GQ_NPR partitions out of registers), so the
-// tail of the attention phase is one L2 round trip after the slowest partition has published.
-template <int GQ>
-__device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Smem& sm, int hq0, int np, uint32_t fl) {
-#ifndef ETXB_GQ_NPR
-#define ETXB_GQ_NPR 12               // partitions merged out of registers in one round (a 1.5K context); measured against 16: 0.8 % faster
-#endif
-  constexpr int HD = 128, NPR = ETXB_GQ_NPR, NR = (GQ * HD + ETXB_CONSUMERS - 1) / ETXB_CONSUMERS;   // output values per thread
-  const int lane = tidx() & 31, warp = tidx() >> 5;
-  float* wl = sm.xs;                                              // [GQ][np] max logits, then weights
-  float* es = sm.xs + 4096;                                       // [GQ][np] exp sums
-  float* red = sm.scr + 200;                                      // [GQ] denominators
-  const uint2* pw = (const uint2*)d.tmp_out;
-  const int idx0 = tidx();                                        // this thread's output values (GQ * HD <= 1024: one or two)
-  float pv[NR][NPR];
-  const bool in_regs = np <= NPR;
-  if (in_regs) {
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const int idx = idx0 + r * ETXB_CONSUMERS;
-      if (idx < GQ * HD) {
-        const int g = idx >> 7, dd = idx & (HD - 1);
-        const uint2* tp = pw + (size_t)(hq0 + g) * d.max_parts * ETXB_GQ_PW + dd;
-        // all requests in flight at once, all again while one is missing (a poll per pair, inlined NPR times, is 20 KB of code
-        // that the instruction cache has to hold)
-        bool ok;
-        uint32_t spins = 0;
-        do {
-          ok = true;
-          uint2 first[NPR];
-#pragma unroll
-          for (int u = 0; u < NPR; ++u) first[u] = ld_pair(tp + (size_t)min(u, np - 1) * ETXB_GQ_PW);
-#pragma unroll
-          for (int u = 0; u < NPR; ++u) { pv[r][u] = __uint_as_float(first[u].x); ok = ok && first[u].y == fl; }
-        } while (!ok && poll_again(spins, tp, np, fl, sm));
-      }
-    }
-  }
-  for (int i = tidx(); i < GQ * np; i += ETXB_CONSUMERS) {
-    const int g = i / np, pp = i - g * np;
-    const uint2* st = pw + ((size_t)(hq0 + g) * d.max_parts + pp) * ETXB_GQ_PW + HD;
-    wl[i] = poll_pair(st, fl, sm);
-    es[i] = poll_pair(st + 1, fl, sm);
-  }
-  csync();
-  mark(sm, 0);
-  if (warp < GQ) {
-    const int g = warp;
-    float m = -INFINITY;
-    for (int pp = lane; pp < np; pp += 32) m = fmaxf(m, wl[g * np + pp]);
-    m = warp_max(m);
-    float L = 0.f;
-    for (int pp = lane; pp < np; pp += 32) {
-      const float w = expf(__fsub_rn(wl[g * np + pp], m));
-      wl[g * np + pp] = w;
-      L = __fmaf_rn(w, es[g * np + pp], L);
-    }
-    L = warp_sum(L);
-    if (lane == 0) red[g] = L;
-  }
-  csync();
-  mark(sm, 1);
-  if (in_regs) {
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const int idx = idx0 + r * ETXB_CONSUMERS;
-      if (idx < GQ * HD) {
-        const int g = idx >> 7;
-        const float* wg = wl + g * np;
-        float o = 0.f;
-#pragma unroll
-        for (int u = 0; u < NPR; ++u) o = __fmaf_rn(u < np ? wg[u] : 0.f, u < np ? pv[r][u] : 0.f, o);   // partitions in ascending order
-        ((__nv_bfloat16*)d.out)[(size_t)hq0 * HD + idx] = __float2bfloat16_rn(__fdiv_rn(o, red[g]));
-      }
-    }
-  } else {
-    // a long context: the partials in rounds of NPR requests per output value, partitions still in ascending order
-    for (int idx = tidx(); idx < GQ * HD; idx += ETXB_CONSUMERS) {
-      const int g = idx >> 7, dd = idx & (HD - 1);
-      const uint2* tp = pw + (size_t)(hq0 + g) * d.max_parts * ETXB_GQ_PW + dd;
-      const float* wg = wl + g * np;
-      float o = 0.f;
-      for (int p0 = 0; p0 < np; p0 += NPR) {
-        uint2 first[NPR];
-        bool ok;
-        uint32_t spins = 0;
-        do {
-          ok = true;
-#pragma unroll
-          for (int u = 0; u < NPR; ++u) first[u] = ld_pair(tp + (size_t)min(p0 + u, np - 1) * ETXB_GQ_PW);
-#pragma unroll
-          for (int u = 0; u < NPR; ++u) ok = ok && first[u].y == fl;
-        } while (!ok && poll_again(spins, tp + (size_t)p0 * ETXB_GQ_PW, min(NPR, np - p0), fl, sm));
-#pragma unroll
-        for (int u = 0; u < NPR; ++u)
-          if (p0 + u < np) o = __fmaf_rn(wg[p0 + u], __uint_as_float(first[u].x), o);
-      }
-      ((__nv_bfloat16*)d.out)[(size_t)(hq0 + g) * HD + dd] = __float2bfloat16_rn(__fdiv_rn(o, red[g]));
-    }
-  }
-  mark(sm, 2);
+__device__ __forceinline__ GqTask gq_task(const etxb_attnf_args& d, int blk, const etxb_stepv& S) {
+  GqTask t;
+  // the step's own buffers hold what the prologue wrote from the step parameters: take the values from there
+  t.pos = (const void*)d.positions == (const void*)S.positions ? (long long)S.pos : __ldcg((const long long*)d.positions);
+  t.seq = (const void*)d.seq_lens == (const void*)S.seq_lens ? S.pos + 1 : __ldcg(d.seq_lens);
+  t.whole = (d.part_len & ETXB_GQ_WHOLE) != 0;
+  const int lg = 31 - __clz(d.gq), NQG = d.NH >> lg;               // (gq: 1, 2, 4 or 8)
+  t.part = t.whole ? 0 : udiv_small(blk, NQG);
+  t.hq0 = (blk - t.part * NQG) << lg;
+  t.h = udiv_small(t.hq0 * d.NKV, d.NH);
+  t.t0 = t.part * ETXB_GQ_PART;
+  const int np = min((t.seq + ETXB_GQ_PART - 1) / ETXB_GQ_PART, d.max_parts);
+  const int tend = t.whole ? np * ETXB_GQ_PART : t.t0 + ETXB_GQ_PART;
+  t.owner = t.pos >= t.t0 && t.pos < tend;
+  const int lim = t.owner ? max(t.seq, (int)t.pos + 1) : t.seq;
+  t.u0 = t.t0 >> 4;
+  t.nu = t.t0 < t.seq && tend > t.t0 ? (min(tend, lim) - t.t0 + 15) >> 4 : 0;
+  return t;
 }
 
-// (inlined into the lean kernels, which hold one of it: a call takes the address of Smem, which then lives on the stack for
-// every tile of the kernel)
-template <int GQ>
-__device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S) {
-  constexpr int HD = 128, BS = 16, X = 8, PL = ETXB_GQ_PART, HV = HD / 8;
-  const int NKV = d.NKV, G = d.NH / NKV, NQG = d.NH / GQ;
-  const int part = blk / NQG, qg = blk - part * NQG;
-  const int hq0 = qg * GQ, h = hq0 / G;                           // first q head of the group, its kv head
-  const bool writer = hq0 - h * G == 0;                           // the kv head's first group stores the new k / v rows
-  // the step's own buffers hold what the prologue wrote from the step parameters: take the values from there
-  const long long pos = (const void*)d.positions == (const void*)S.positions ? (long long)S.pos : __ldcg((const long long*)d.positions);
-  const long long slot = (const void*)d.slot_mapping == (const void*)S.slot_mapping ? (long long)S.pos : __ldcg((const long long*)d.slot_mapping);
-  const int seq = (const void*)d.seq_lens == (const void*)S.seq_lens ? S.pos + 1 : __ldcg(d.seq_lens);
-  const int t0 = part * PL;
-  const int tid = tidx(), lane = tid & 31, warp = tid >> 5;
-  const uint32_t fl = pair_flag(sm.epoch(), d.part_len);
-  if (t0 < seq) {
-    const GqSmem<GQ> s(sm.xs);
-    const bool owner = pos >= t0 && pos < t0 + PL;                // this partition holds the position being written
-    const int tpos = owner ? (int)(pos - t0) : -1;
-    const int ntok = min(PL, seq - t0);
-    // positions taken from the cache: all of the partition's but the new one (its slot is stale until this step's write)
-    auto cached = [&](int tt) { return tt < ntok && tt != tpos; };
-    const int t = tid & (PL - 1), qr = tid >> 7;                  // K: position t, dims [32 qr, 32 qr + 32);  V: dim t, blocks 2 qr, 2 qr + 1
-    // ---- K and V of the partition: cache -> registers (nothing here depends on this step's q)
-    uint4 kreg[4], vreg[4];
-    {
-      const int lb = t0 / BS + (t >> 4);
-      const bool live = lb * BS < seq;
-      const long long pb = live ? __ldg(d.block_tables + lb) : 0;
-      const __nv_bfloat16* kp = (const __nv_bfloat16*)d.kc + ((((size_t)pb * NKV + h) * HV + qr * 4) * BS + (t & 15)) * X;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) kreg[j] = live ? ld_act16(kp + (size_t)j * BS * X) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int lv = t0 / BS + 2 * qr + u;
-        const bool lv_live = lv * BS < seq;
-        const long long pv = lv_live ? __ldg(d.block_tables + lv) : 0;
-        const __nv_bfloat16* vp = (const __nv_bfloat16*)d.vc + (((size_t)pv * NKV + h) * HD + t) * BS;
-        vreg[2 * u] = lv_live ? ld_act16(vp) : make_uint4(0u, 0u, 0u, 0u);
-        vreg[2 * u + 1] = lv_live ? ld_act16(vp + 8) : make_uint4(0u, 0u, 0u, 0u);
+// Producer warp: the task's units into the ring, three to a stage.  A unit past the context (possible only where positions and
+// seq_lens disagree) has no block: its place in the stage stays as it is.
+__device__ __forceinline__ bool produce_attn(const etxb_attnf_args& d, int blk, const etxb_stepv& S, uint32_t& n, const Smem& sm, int where) {
+  if (blk >= (int)d.nblocks) return true;
+  const GqTask t = gq_task(d, blk, S);
+  const int lane = tidx() & 31, ns = (t.nu + ETXB_GQ_UPS - 1) / ETXB_GQ_UPS;
+  const size_t piece = (size_t)128 * 16 * 2;                        // bytes of one kv head's K (or V) in a cache block
+  bool ok = true;
+  int tab = 0;
+  for (int s = 0; s < ns && ok; ++s) {
+    const uint32_t st = n % ETXB_NSTAGE, par = (n / ETXB_NSTAGE) & 1;
+    const int i0 = s * ETXB_GQ_UPS;
+    if (s % 10 == 0) {                                             // block-table entries of the next ten stages' units, one per lane
+      const int u = t.u0 + i0 + lane;
+      tab = i0 + lane < t.nu && (u << 4) < t.seq ? __ldg(d.block_tables + u) : 0;
+    }
+    const int i = i0 + (lane >> 1), u = t.u0 + i;
+    const bool live = lane < 2 * ETXB_GQ_UPS && i < t.nu && (u << 4) < t.seq;
+    const long long pb = __shfl_sync(0xffffffffu, tab, (i0 % (10 * ETXB_GQ_UPS) + (lane >> 1)) & 31);
+    const int pieces = __popc(__ballot_sync(0xffffffffu, live));
+    int good = 1;
+    if (lane == 0) {
+      good = mbar_wait(sm.empty + st, par ^ 1, sm, where) ? 1 : 0;
+      if (good) {
+        *((volatile uint32_t*)(sm.full + 2 * ETXB_NSTAGE) + st) = n;  // (see wait_use)
+        mbar_expect_tx(sm.full + st, (uint32_t)(pieces * piece));
       }
     }
-    // ---- this step's rows: raw q heads, (owner) new k and v rows; rotary row and norm weights
-    {
-      const __nv_bfloat16* qkv = (const __nv_bfloat16*)d.qkv;
-      const int nq = GQ * HV, nrow = nq + (owner ? 2 * HV : 0);
-      for (int i = tid; i < nrow + 3 * HV; i += ETXB_CONSUMERS) {
-        if (i < nrow) {
-          const __nv_bfloat16* src = i < nq ? qkv + (size_t)hq0 * HD + 8 * i
-                                            : (i < nq + HV ? qkv + (size_t)(d.NH + h) * HD + 8 * (i - nq)
-                                                           : qkv + (size_t)(d.NH + NKV + h) * HD + 8 * (i - nq - HV));
-          unpack8(ld_act16(src), s.raw + (i < nq ? 8 * i : GQ * HD + 8 * (i - nq)));
-        } else {
-          const int c = i - nrow, which = c / HV, v = c - which * HV;
-          const __nv_bfloat16* src = which == 0 ? (const __nv_bfloat16*)d.cos_sin + (size_t)pos * HD
-                                                : (const __nv_bfloat16*)(which == 1 ? d.qw : d.kw);
-          if (src != nullptr) unpack8(__ldg((const uint4*)src + v), s.cw + which * HD + 8 * v);
+    ok = __shfl_sync(0xffffffffu, good, 0) != 0;
+    if (ok && live)
+      bulk_g2s(sm.ring + (size_t)st * ETXB_STAGE_BYTES + (lane >> 1) * ETXB_GQ_UNIT + (lane & 1) * piece,
+               (const unsigned char*)((lane & 1) ? d.vc : d.kc) + ((size_t)pb * d.NKV + t.h) * piece, (uint32_t)piece, sm.full + st);
+    if (ok) ++n;
+  }
+  return ok;
+}
+
+// D += A (16 x 16, row-major) * B (16 x 8, column-major), bf16 operands, fp32 accumulators (the warp-level tensor-core form)
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&a)[4], uint32_t saddr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(saddr) : "memory");
+}
+__device__ __forceinline__ uint32_t movmatrix(uint32_t a) {        // transpose of an 8 x 8 matrix of 16-bit values spread over the warp
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
+
+// Shared memory of the tile in the general region: 47 KB.
+struct GqSmem {
+  float* raw;                // [10][128] raw rows: q heads, new k (each warp's own, for its norm)
+  uint32_t* qb;              // [8][68] words = [8 heads][136] bf16: q rows, normed and rotated (heads past gq: zero)
+  __nv_bfloat16* knew;       // [128] new k row
+  __nv_bfloat16* vnew;       // [128] new v row
+  float* st;                 // [8 slots][8 heads][2] running maximum, sum
+  float* po;                 // [8 slots][1152] a warp's output sums: as fragments (handed from warp w + 8 to w), then [head][132]
+  float* mg;                 // [16][32] partial sums of the merge
+  __device__ explicit GqSmem(float* b) {
+    raw = b; qb = (uint32_t*)(raw + 10 * 128); knew = (__nv_bfloat16*)(qb + 8 * 68); vnew = knew + 128;
+    st = (float*)(vnew + 128); po = st + 8 * 8 * 2; mg = po + 8 * 1152;
+  }
+};
+static_assert((10 * 128 + 8 * 68 + 128 + 128 + 8 * 1152 + 16 * 32) * 4 <= ETXB_GEN_BYTES, "the layout fits the general region");
+
+// One head row (lane holds elements 4 lane ..): optional RMSNorm with weight nw (mean in numpy's order), then neox rotary.  xh: 128
+// floats of the warp's own; o[j]: the bf16-rounded results.  Same arithmetic as head_norm_rope_s<128>, operands in registers.
+__device__ __forceinline__ void head_norm_rope_r(uint2 x, float* xh, bool norm, uint2 nw, uint2 cs, uint2 sn, float eps, float (&o)[4]) {
+  const int lane = tidx() & 31;
+  float v[4] = {bf_lo(x.x), bf_hi(x.x), bf_lo(x.y), bf_hi(x.y)};
+  if (norm) {
+    const float wf[4] = {bf_lo(nw.x), bf_hi(nw.x), bf_lo(nw.y), bf_hi(nw.y)};
+    *(float4*)(xh + 4 * lane) = make_float4(v[0], v[1], v[2], v[3]);
+    __syncwarp();
+    const float ss = sumsq128_numpy_order_warp(xh);
+    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.0f), eps)));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = bfr(__fmul_rn(wf[j], bfr(__fmul_rn(v[j], r))));
+  }
+  const float cf[4] = {bf_lo(cs.x), bf_hi(cs.x), bf_lo(cs.y), bf_hi(cs.y)}, sf[4] = {bf_lo(sn.x), bf_hi(sn.x), bf_lo(sn.y), bf_hi(sn.y)};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float other = __shfl_xor_sync(0xffffffffu, v[j], 16);    // element d +- 64 lives 16 lanes away
+    o[j] = bfr(__fadd_rn(bfr(__fmul_rn(v[j], cf[j])), bfr(__fmul_rn(lane < 16 ? -other : other, sf[j]))));
+  }
+}
+
+// out[h][:] = bf16(sum_p w_p * tmp[p][:] / sum_p w_p * l_p), w_p = exp(m_p - max m), for the 32-value slices mi, mi + mk, .. of the
+// group's gq * 128 output values.  Polls the flagged partials the other CTAs publish (L2).  A warp takes a slice and a share of the
+// partitions (its lane: one value); every warp works out its head's weights itself from the partitions' statistics.
+__device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Smem& sm, float* mg, int hq0, int np, uint32_t fl, int mi, int mk) {
+  constexpr int HD = 128, NF = 8;
+  const int lane = tidx() & 31, warp = tidx() >> 5;
+  const int nsl = (d.gq * 4 - mi + mk - 1) / mk;                   // slices of this task
+  const int wps = nsl > 8 ? 1 : nsl > 4 ? 2 : nsl > 2 ? 4 : nsl > 1 ? 8 : 16;   // warps per slice
+  const int per = 16 / wps, sub = warp / per;                      // slices per round; the warp's share of the partitions
+#pragma unroll 1
+  for (int s0 = 0; s0 < nsl; s0 += per) {
+    const int si = s0 + (warp & (per - 1));
+    const bool on = si < nsl;
+    const int sl = mi + min(si, nsl - 1) * mk, g = sl >> 2;
+    const uint2* tp = (const uint2*)d.tmp_out + (size_t)(hq0 + g) * d.max_parts * ETXB_GQ_PW;
+    const uint2* vp = tp + (sl & 3) * 32 + lane;
+    float o = 0.f, L = 0.f, M = -INFINITY;
+    if (on) {
+      // a round: up to 32 partitions' statistics (a lane each) and this warp's values of them, requested together -- the tail of the
+      // phase is one trip to L2 behind the slowest partition.  Between rounds the sums are rescaled to the larger maximum.
+      const int ch = min(32, NF * wps);
+#pragma unroll 1
+      for (int p0 = 0; p0 < np; p0 += ch) {
+        const int pe = min(np - p0, ch);
+        const uint2* sp = tp + (size_t)p0 * ETXB_GQ_PW + HD;
+        uint2 first[NF];
+        uint4 v;
+        uint32_t spins = 0;
+        for (;;) {
+          v = ld_volatile16(sp + (size_t)min(lane, pe - 1) * ETXB_GQ_PW);      // (maximum, flag, sum, flag)
+#pragma unroll
+          for (int u = 0; u < NF; ++u) first[u] = ld_pair(vp + (size_t)(p0 + min(sub + u * wps, pe - 1)) * ETXB_GQ_PW);
+          bool ok = v.y == fl && v.w == fl;
+#pragma unroll
+          for (int u = 0; u < NF; ++u) ok = ok && first[u].y == fl;
+          if (ok || !poll_again(spins, sp, pe, ETXB_GQ_PW, fl, sm)) break;
+        }
+        __syncwarp();
+        const float m = lane < pe ? __uint_as_float(v.x) : -INFINITY;
+        const float Mn = fmaxf(M, warp_max(m)), Mz = Mn == -INFINITY ? 0.f : Mn;
+        const float f = expf(__fsub_rn(M, Mz)), w = expf(__fsub_rn(m, Mz));    // (lanes past the round: 0)
+        M = Mn;
+        o = __fmul_rn(o, f);
+        L = __fmaf_rn(L, f, lane < pe ? __fmul_rn(w, __uint_as_float(v.z)) : 0.f);
+#pragma unroll
+        for (int u = 0; u < NF; ++u) {
+          const float wu = __shfl_sync(0xffffffffu, w, (sub + u * wps) & 31);
+          if (sub + u * wps < pe) o = __fmaf_rn(wu, __uint_as_float(first[u].x), o);
         }
       }
+      L = warp_sum(L);
     }
+    if (wps > 1) {
+      mg[warp * 32 + lane] = o;
+      csync();
+      if (sub == 0)
+        for (int q = 1; q < wps; ++q) o = __fadd_rn(o, mg[(warp + q * per) * 32 + lane]);
+    }
+    if (on && sub == 0) ((__nv_bfloat16*)d.out)[(size_t)hq0 * HD + sl * 32 + lane] = __float2bfloat16_rn(__fdiv_rn(o, L));
+    if (s0 + per < nsl && wps > 1) csync();
+  }
+}
+
+// One task.  n: the running stage count of the ring.  mg: how the merge of a context in partitions is shared out -- 0: the task of the
+// last partition merges the group (it comes last in the queues, and a task that waits only for tasks of lower index cannot be part of
+// a circle); else count << 16 | index + 1: the host has found that every worker's queue holds the grid in ascending order, so the
+// workers' LAST tasks of the grid may wait for all the others (whatever stands before them in a queue waits for nobody), and this is
+// one of `count` such tasks of the group, each of which merges a share; 0xffff: it is not one of them, others are.  Shared out from
+// gq * np = ETXB_GQ_SHARE on only: with few partials the last partition's task alone is as quick, and the other tasks are done.
+__device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S, uint32_t& n, uint32_t mg) {
+  constexpr int HD = 128, BS = 16;
+  const GqTask t = gq_task(d, blk, S);
+  const int NKV = d.NKV, gq = d.gq, tid = tidx(), lane = tid & 31, warp = tid >> 5;
+  const uint32_t fl = pair_flag(sm.epoch(), d.part_len);
+  const int np = min((t.seq + ETXB_GQ_PART - 1) / ETXB_GQ_PART, d.max_parts);
+  const GqSmem s(sm.xs);
+  const uint32_t n0 = n;
+  n += (uint32_t)((t.nu + ETXB_GQ_UPS - 1) / ETXB_GQ_UPS);
+  if (t.nu > 0) {
+    const bool newrow = t.owner || t.whole;
+    // ---- this step's rows, a warp each: q heads, the new k row, the new v row
+    if (warp < gq || (warp == gq && newrow)) {
+      const bool isq = warp < gq;
+      const void* nwp = isq ? d.qw : d.kw;
+      const uint2 x = __ldcg((const uint2*)((const __nv_bfloat16*)d.qkv + (size_t)(isq ? t.hq0 + warp : d.NH + t.h) * HD) + lane);
+      const uint2* cs = (const uint2*)((const __nv_bfloat16*)d.cos_sin + (size_t)t.pos * HD);
+      const uint2 nw = nwp ? __ldg((const uint2*)nwp + lane) : make_uint2(0u, 0u), c = __ldg(cs + (lane & 15)), sn = __ldg(cs + 16 + (lane & 15));
+      float o[4];
+      head_norm_rope_r(x, s.raw + warp * HD, nwp != nullptr, nw, c, sn, d.eps, o);
+      const uint2 r = make_uint2(pack_bf(o[0], o[1]), pack_bf(o[2], o[3]));
+      if (isq) *(uint2*)(s.qb + warp * 68 + 2 * lane) = r;
+      else {
+        *(uint2*)(s.knew + 4 * lane) = r;
+        if (t.hq0 * NKV == t.h * d.NH) {                          // the kv head's first group stores the new k / v rows
+          const long long slot = (const void*)d.slot_mapping == (const void*)S.slot_mapping ? (long long)S.pos : __ldcg((const long long*)d.slot_mapping);
+          *(uint2*)((__nv_bfloat16*)d.kc + ((((size_t)(slot / BS) * NKV + t.h) * (HD / 8) + (lane >> 1)) * BS + (int)(slot % BS)) * 8 + 4 * (lane & 1)) = r;
+        }
+      }
+    } else if (warp == gq + 1 && newrow) {
+      const uint2 x = __ldcg((const uint2*)((const __nv_bfloat16*)d.qkv + (size_t)(d.NH + NKV + t.h) * HD) + lane);
+      *(uint2*)(s.vnew + 4 * lane) = x;
+      if (t.hq0 * NKV == t.h * d.NH) {
+        const long long slot = (const void*)d.slot_mapping == (const void*)S.slot_mapping ? (long long)S.pos : __ldcg((const long long*)d.slot_mapping);
+        unsigned short* vc = (unsigned short*)d.vc + (((size_t)(slot / BS) * NKV + t.h) * HD + 4 * lane) * BS + (int)(slot % BS);
+        vc[0] = (unsigned short)x.x; vc[BS] = (unsigned short)(x.x >> 16); vc[2 * BS] = (unsigned short)x.y; vc[3 * BS] = (unsigned short)(x.y >> 16);
+      }
+    }
+    for (int i = gq * 68 + tid; i < 8 * 68; i += ETXB_CONSUMERS) s.qb[i] = 0u;
     csync();
     mark(sm, 0);
-    // ---- norm + rope of the q heads (warps 0..GQ-1), of the new k row (warp GQ); the new v row (warp GQ + 1)
-    if (warp < GQ || (warp == GQ && owner)) {                       // q heads, then the new k row: raw rows lie one behind the other
-      float o[8];
-      const bool isq = warp < GQ;
-      head_norm_rope_s<128>(s.raw + warp * HD, (isq ? d.qw : d.kw) ? s.cw + (isq ? HD : 2 * HD) : nullptr, s.cw, HD, d.eps, o);
-      const long long cb = slot / BS; const int off = (int)(slot % BS);
-      __nv_bfloat16* kc = (__nv_bfloat16*)d.kc;
-      float* dst = isq ? s.qs + warp * HD : s.knew;
+    // ---- the units, warp w: w, w + 16, ..
+    const int g8 = lane >> 2, t4 = lane & 3, nwarp = min(t.nu, ETXB_CONSUMER_WARPS), where = sm.cur();
+    float acc[8][4];                                               // [dims 16 i + g8, + 8][heads 2 t4, 2 t4 + 1]
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;      // of heads 2 t4, 2 t4 + 1 (l: this lane's positions)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int dd = lane * 4 + j;
-        dst[dd] = o[j];
-        if (!isq && writer) kc[((((size_t)cb * NKV + h) * HV + dd / X) * BS + off) * X + dd % X] = __float2bfloat16_rn(o[j]);
+    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    if (warp < nwarp) {
+      const uint32_t* qw = s.qb + g8 * 68 + t4;                     // (read again for every unit: 16 registers fewer)
+#pragma unroll 1
+      for (int i = warp; i < t.nu; i += ETXB_CONSUMER_WARPS) {
+        const int si = i / ETXB_GQ_UPS, ui = i - si * ETXB_GQ_UPS, p0 = (t.u0 + i) << 4;
+        const uint32_t k = n0 + (uint32_t)si, st = k % ETXB_NSTAGE;
+        // (the parity of a stage tells use k from use k - 1 only, and the use before this one may be another warp's: see wait_use)
+        bool ok = wait_use((volatile const uint32_t*)(sm.full + 2 * ETXB_NSTAGE) + st, k, sm, where) && mbar_wait(sm.full + st, (k / ETXB_NSTAGE) & 1, sm, where);
+        if (!__all_sync(0xffffffffu, ok)) break;                   // step abandoned: touch nothing
+        unsigned char* unit = sm.ring + (size_t)st * ETXB_STAGE_BYTES + ui * ETXB_GQ_UNIT;
+        // the unit at the end of the context: the new position's rows over its stale slot; a slot beyond the context may hold anything:
+        // it is never multiplied (V: zero, K: the score below)
+        const bool ragged = p0 + 16 > t.seq || (t.pos >= p0 && t.pos < p0 + 16);
+        if (ragged) {
+          const int rn = t.owner && t.pos >= p0 && t.pos < p0 + 16 ? (int)t.pos - p0 : -1;
+          if (rn >= 0) *(uint2*)(unit + ((lane >> 1) * 16 + rn) * 16 + 8 * (lane & 1)) = *(const uint2*)(s.knew + 4 * lane);
+          const int nv = max(0, min(16, t.seq - p0));              // cached positions
+#pragma unroll 1
+          for (int j = lane; j < 128 * 8; j += 32) {               // pairs of positions: dim j / 8, positions 2 (j % 8) ..
+            const int pa = 2 * (j & 7);
+            uint32_t* w = (uint32_t*)(unit + 4096) + j;
+            const uint32_t vn = ((const unsigned short*)s.vnew)[j >> 3];
+            uint32_t v = *w;
+            if (pa >= nv) v &= 0xffff0000u;
+            if (pa + 1 >= nv) v &= 0xffffu;
+            if (pa == rn) v = (v & 0xffff0000u) | vn;
+            if (pa + 1 == rn) v = (v & 0xffffu) | vn << 16;
+            *w = v;
+          }
+          __syncwarp();
+        }
+        const uint32_t ks = smem_u32(unit) + lane * 16, vs = smem_u32(unit) + 4096 + ((lane >> 4) << 4) + ((lane & 15) << 5);
+        // (four fragments at a time, then their products: a load in front of every product is a chain of their latencies)
+        float c[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+        for (int q = 0; q < 8; q += 4) {
+          uint32_t a[4][4], b[4][2];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            ldmatrix_x4(a[u], ks + (q + u) * 512);                 // 16 positions x 16 dims
+            b[u][0] = qw[8 * (q + u)]; b[u][1] = qw[8 * (q + u) + 4];
+          }
+#pragma unroll
+          for (int u = 0; u < 4; u += 2) { mma16816(c, a[u], b[u][0], b[u][1]); mma16816(e, a[u + 1], b[u + 1][0], b[u + 1][1]); }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = __fadd_rn(c[j], e[j]);
+        // softmax of the unit: positions g8 (c[0], c[1]) and g8 + 8 (c[2], c[3]), heads 2 t4 and 2 t4 + 1
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = __fmul_rn(c[j], d.scale);
+        if (ragged) {
+          const int pa = p0 + g8, pb = pa + 8;
+          if (pa >= t.seq && !(t.owner && pa == (int)t.pos)) c[0] = c[1] = -INFINITY;
+          if (pb >= t.seq && !(t.owner && pb == (int)t.pos)) c[2] = c[3] = -INFINITY;
+        }
+        float n0m = fmaxf(c[0], c[2]), n1m = fmaxf(c[1], c[3]);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) { n0m = fmaxf(n0m, __shfl_xor_sync(0xffffffffu, n0m, o)); n1m = fmaxf(n1m, __shfl_xor_sync(0xffffffffu, n1m, o)); }
+        n0m = fmaxf(m0, n0m); n1m = fmaxf(m1, n1m);
+        const float b0 = n0m == -INFINITY ? 0.f : n0m, b1 = n1m == -INFINITY ? 0.f : n1m;   // (nothing valid yet: every probability is 0)
+        if (i != warp) {
+          const float f0 = expf(__fsub_rn(m0, b0)), f1 = expf(__fsub_rn(m1, b1));
+          l0 = __fmul_rn(l0, f0); l1 = __fmul_rn(l1, f1);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { acc[j][0] *= f0; acc[j][1] *= f1; acc[j][2] *= f0; acc[j][3] *= f1; }
+        }
+        m0 = n0m; m1 = n1m;
+        c[0] = expf(__fsub_rn(c[0], b0)); c[1] = expf(__fsub_rn(c[1], b1)); c[2] = expf(__fsub_rn(c[2], b0)); c[3] = expf(__fsub_rn(c[3], b1));
+        l0 = __fadd_rn(l0, __fadd_rn(c[0], c[2])); l1 = __fadd_rn(l1, __fadd_rn(c[1], c[3]));
+        float r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = __fsub_rn(c[j], bfr(c[j]));
+        const uint32_t h0 = movmatrix(pack_bf(c[0], c[1])), h1 = movmatrix(pack_bf(c[2], c[3]));
+        const uint32_t w0 = movmatrix(pack_bf(r[0], r[1])), w1 = movmatrix(pack_bf(r[2], r[3]));
+#pragma unroll
+        for (int j = 0; j < 8; j += 4) {
+          uint32_t a[4][4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) ldmatrix_x4(a[u], vs + (j + u) * 512);   // 16 dims x 16 positions (matrices: dims 0-7, 8-15 of positions 0-7, then of 8-15)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mma16816(acc[j + u], a[u], h0, h1);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mma16816(acc[j + u], a[u], w0, w1);
+        }
+        if (ragged) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // (this warp's writes, before the next copy into the place)
+        __syncwarp();
+        const int in_stage = min(t.nu - si * ETXB_GQ_UPS, ETXB_GQ_UPS), share = ETXB_EMPTY_COUNT / ETXB_GQ_UPS;
+        if (lane == 0) mbar_arrive_n(sm.empty + st, ui == in_stage - 1 ? ETXB_EMPTY_COUNT - ui * share : share);
       }
-    } else if (warp == GQ + 1 && owner) {
-      const long long cb = slot / BS; const int off = (int)(slot % BS);
-      __nv_bfloat16* vc = (__nv_bfloat16*)d.vc;
-      for (int dd = lane; dd < HD; dd += 32) {
-        const float v = s.raw[(GQ + 1) * HD + dd];
-        s.vnew[dd] = v;
-        if (writer) vc[(((size_t)cb * NKV + h) * HD + dd) * BS + off] = __float2bfloat16_rn(v);
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) { l0 += __shfl_xor_sync(0xffffffffu, l0, o); l1 += __shfl_xor_sync(0xffffffffu, l1, o); }
+    }
+    // ---- the warps' results: warp w + 8 hands its fragments to warp w, then the eight meet in shared memory
+    if (nwarp > 8) {
+      float4* box = (float4*)(s.po + (warp & 7) * 1152);
+      if (warp >= 8 && warp < nwarp) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) box[j * 32 + lane] = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+        box[256 + lane] = make_float4(m0, m1, l0, l1);
       }
+      csync();
+      if (warp + 8 < nwarp) {
+        const float4 o = box[256 + lane];
+        const float a0 = fmaxf(m0, o.x), a1 = fmaxf(m1, o.y), z0 = a0 == -INFINITY ? 0.f : a0, z1 = a1 == -INFINITY ? 0.f : a1;
+        const float f0 = expf(__fsub_rn(m0, z0)), f1 = expf(__fsub_rn(m1, z1)), e0 = expf(__fsub_rn(o.x, z0)), e1 = expf(__fsub_rn(o.y, z1));
+        m0 = a0; m1 = a1;
+        l0 = __fmaf_rn(l0, f0, __fmul_rn(o.z, e0)); l1 = __fmaf_rn(l1, f1, __fmul_rn(o.w, e1));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 v = box[j * 32 + lane];
+          acc[j][0] = __fmaf_rn(acc[j][0], f0, __fmul_rn(v.x, e0)); acc[j][1] = __fmaf_rn(acc[j][1], f1, __fmul_rn(v.y, e1));
+          acc[j][2] = __fmaf_rn(acc[j][2], f0, __fmul_rn(v.z, e0)); acc[j][3] = __fmaf_rn(acc[j][3], f1, __fmul_rn(v.w, e1));
+        }
+        __syncwarp();
+      }
+    }
+    const int nslot = min(nwarp, 8);
+    if (warp < nslot) {
+      float* po = s.po + warp * 1152 + (2 * t4) * 132 + g8;
+      const bool hA = 2 * t4 < gq, hB = 2 * t4 + 1 < gq;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (hA) { po[16 * j] = acc[j][0]; po[16 * j + 8] = acc[j][2]; }
+        if (hB) { po[132 + 16 * j] = acc[j][1]; po[132 + 16 * j + 8] = acc[j][3]; }
+      }
+      if (g8 == 0) *(float4*)(s.st + (warp * 8 + 2 * t4) * 2) = make_float4(m0, l0, m1, l1);
     }
     csync();
     mark(sm, 1);
-    // ---- scores: thread (qr, t) holds 32 dims of position t; quarter sums to shared memory
-    {
-      float acc[GQ];
-#pragma unroll
-      for (int g = 0; g < GQ; ++g) acc[g] = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float kf[8];
-        unpack8(kreg[j], kf);
-#pragma unroll
-        for (int g = 0; g < GQ; ++g) {
-          const float4 qa = *(const float4*)(s.qs + g * HD + (qr * 4 + j) * 8), qb = *(const float4*)(s.qs + g * HD + (qr * 4 + j) * 8 + 4);
-          acc[g] = __fmaf_rn(kf[0], qa.x, acc[g]); acc[g] = __fmaf_rn(kf[1], qa.y, acc[g]);
-          acc[g] = __fmaf_rn(kf[2], qa.z, acc[g]); acc[g] = __fmaf_rn(kf[3], qa.w, acc[g]);
-          acc[g] = __fmaf_rn(kf[4], qb.x, acc[g]); acc[g] = __fmaf_rn(kf[5], qb.y, acc[g]);
-          acc[g] = __fmaf_rn(kf[6], qb.z, acc[g]); acc[g] = __fmaf_rn(kf[7], qb.w, acc[g]);
-        }
-      }
-#pragma unroll
-      for (int g = 0; g < GQ; ++g) s.ph[(qr * GQ + g) * PL + t] = acc[g];
-    }
-    csync();
-    // ---- softmax statistics: one warp per q head, lane holds positions lane + 32 k
-    if (warp < GQ) {
-      const int g = warp;
-      float sv[4], m = -INFINITY;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int tt = lane + 32 * k;
-        const float dot = __fadd_rn(__fadd_rn(__fadd_rn(s.ph[g * PL + tt], s.ph[(GQ + g) * PL + tt]), s.ph[(2 * GQ + g) * PL + tt]), s.ph[(3 * GQ + g) * PL + tt]);
-        sv[k] = cached(tt) ? __fmul_rn(dot, d.scale) : -INFINITY;
-        m = fmaxf(m, sv[k]);
-      }
-      float snew = -INFINITY;
-      if (owner) {                                                 // the new position: q . k_new from shared memory
-        float a = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) a = __fmaf_rn(s.qs[g * HD + lane * 4 + j], s.knew[lane * 4 + j], a);
-        snew = __fmul_rn(warp_sum(a), d.scale);
-      }
-      m = fmaxf(warp_max(m), snew);
-      float l = 0.f;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float pr = cached(lane + 32 * k) ? expf(__fsub_rn(sv[k], m)) : 0.f;
-        s.sc[g * PL + lane + 32 * k] = pr;
-        l = __fadd_rn(l, pr);
-      }
-      l = warp_sum(l);
-      const float pn = owner ? expf(__fsub_rn(snew, m)) : 0.f;
-      if (lane == 0) { s.st[g] = m; s.st[GQ + g] = __fadd_rn(l, pn); s.st[2 * GQ + g] = pn; }
-    }
-    csync();
-    mark(sm, 2);
-    // ---- output: thread (qr, dd = t) multiplies its two blocks of 16 positions; quarter sums to shared memory
-    {
-      float acc[GQ];
-#pragma unroll
-      for (int g = 0; g < GQ; ++g) acc[g] = 0.f;
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int tb = (2 * qr + u) * BS;
-        if (tb < ntok) {
-          float f[16];
-          unpack8(vreg[2 * u], f); unpack8(vreg[2 * u + 1], f + 8);
-#pragma unroll
-          for (int o = 0; o < 16; ++o) f[o] = cached(tb + o) ? f[o] : 0.f;   // stale slots may hold anything: never multiply them
-#pragma unroll
-          for (int g = 0; g < GQ; ++g) {
-#pragma unroll
-            for (int o4 = 0; o4 < 4; ++o4) {
-              const float4 pr = *(const float4*)(s.sc + g * PL + tb + 4 * o4);
-              acc[g] = __fmaf_rn(pr.x, f[4 * o4], acc[g]); acc[g] = __fmaf_rn(pr.y, f[4 * o4 + 1], acc[g]);
-              acc[g] = __fmaf_rn(pr.z, f[4 * o4 + 2], acc[g]); acc[g] = __fmaf_rn(pr.w, f[4 * o4 + 3], acc[g]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int g = 0; g < GQ; ++g) s.po[(qr * GQ + g) * HD + t] = acc[g];
-    }
-    csync();
-    for (int idx = tid; idx < GQ * HD; idx += ETXB_CONSUMERS) {
+    for (int idx = tid; idx < gq * HD; idx += ETXB_CONSUMERS) {
       const int g = idx >> 7, dd = idx & (HD - 1);
-      float o = __fadd_rn(__fadd_rn(__fadd_rn(s.po[g * HD + dd], s.po[(GQ + g) * HD + dd]), s.po[(2 * GQ + g) * HD + dd]), s.po[(3 * GQ + g) * HD + dd]);
-      if (owner) o = __fmaf_rn(s.st[2 * GQ + g], s.vnew[dd], o);
-      uint2* pw = (uint2*)d.tmp_out + ((size_t)(hq0 + g) * d.max_parts + part) * ETXB_GQ_PW;
-      st_pair(pw + dd, o, fl);
-      if (dd == 0) { st_pair(pw + HD, s.st[g], fl); st_pair(pw + HD + 1, s.st[GQ + g], fl); }
-    }
-  }
-  mark(sm, 3);
-  // the context's last partition merges (never past the partitions the grid computed, whatever seq_lens says)
-  const int np = min((seq + PL - 1) / PL, d.max_parts);
-  if (part == np - 1) {
-    csync();                                                       // every thread is done with the tile's shared memory
-    attn_gq_merge<GQ>(d, sm, hq0, np, fl);
-  }
-}
-
-// ---------------------------------------------------------------------------------------------- a whole sequence per task
-// The same attention with one task per (sequence, group of GQ q heads): the task walks the context's partitions itself,
-// keeps every partition's partial output and statistics in shared memory and merges them at the end with the merge's
-// arithmetic (same partition boundaries, same order of the partitions; inside a partition the products run on the tensor cores,
-// so the sums are in another order than in the one-partition-per-task form and most, not all, results have the same bits).  This is the form of a batched step with enough sequences to fill the workers (sequences x kv heads x groups
-// tasks): the q rows are prepared once per sequence instead of once per partition, the next partition's K (then V) is
-// copied asynchronously into shared memory while the current one is being worked on, so the cache latency hides behind
-// the softmax and the output sums, and nothing is published, polled or merged through global memory.
-// The partials live in the weight ring, which is idle in a batched plan (no streamed tiles): part_len bit 24 selects
-// this form, and only builders of plans without streamed tiles may set it.  (64 KB of K / V pieces + np * GQ * 130 floats <= the ring.)
-// D += A (16 x 16, row-major) * B (16 x 8, column-major), bf16 operands, fp32 accumulators (the warp-level tensor-core form)
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-template <int GQ>
-__device__ __forceinline__ void attn_gq_seq(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S) {
-  constexpr int HD = 128, BS = 16, X = 8, PL = ETXB_GQ_PART, HV = HD / 8;
-  const int NKV = d.NKV, G = d.NH / NKV;
-  const int hq0 = blk * GQ, h = hq0 / G;
-  const bool writer = hq0 - h * G == 0;
-  const long long pos = (const void*)d.positions == (const void*)S.positions ? (long long)S.pos : __ldcg((const long long*)d.positions);
-  const long long slot = (const void*)d.slot_mapping == (const void*)S.slot_mapping ? (long long)S.pos : __ldcg((const long long*)d.slot_mapping);
-  const int seq = (const void*)d.seq_lens == (const void*)S.seq_lens ? S.pos + 1 : __ldcg(d.seq_lens);
-  const int np = min(min((seq + PL - 1) / PL, d.max_parts), (ETXB_RING_BYTES - ETXB_GQ_STAGE_BYTES) / (GQ * (HD + 2) * 4));
-  if (np < 1) return;
-  const int tid = tidx(), lane = tid & 31, warp = tid >> 5;
-  const GqSmem<GQ> s(sm.xs);
-  // the weight ring: [4][512] 16-byte K pieces, [4][512] V pieces (piece j of thread tid at [j][tid]: every thread copies
-  // and reads only its own), then the partitions' partial outputs and statistics
-  uint4* KB = (uint4*)sm.ring;
-  uint4* VB = KB + 4 * ETXB_CONSUMERS;
-  // bf16 operands of the tensor-core products, rows padded to 68 words (bank-conflict-free fragment loads): the q heads,
-  // and a partition's probabilities split into a bf16 value and the bf16 of what that rounding lost
-  uint32_t* QB = (uint32_t*)(s.po + 4 * GQ * HD);                  // [8][68] words = [8 heads][136] bf16 (heads >= GQ: zero)
-  uint32_t* PH = QB + 8 * 68;                                      // [8][68] high parts of the probabilities
-  uint32_t* PLo = PH + 8 * 68;                                     // [8][68] low parts
-  for (int i = tid; i < 3 * 8 * 68; i += ETXB_CONSUMERS) QB[i] = 0u;
-  float* PO = (float*)(sm.ring + ETXB_GQ_STAGE_BYTES);            // [np][GQ][HD] partial outputs
-  float* PS = PO + (size_t)np * GQ * HD;                           // [np][GQ][2] max logit, exp sum
-  const int t = tid & (PL - 1), qr = tid >> 7;                     // K: position t, dims [32 qr, 32 qr + 32);  V: dim t, blocks 2 qr, 2 qr + 1
-  // Asynchronous copies (cp.async, 16 bytes each, zero-filled where the context ends) bring a partition's K and V pieces
-  // from the cache to shared memory while the previous partition is being worked on: K of the next partition as soon as
-  // the scores have consumed this one's, V of the next as soon as the output sums have.  One commit group per request, in
-  // that order, so "all but the latest group" is always the piece about to be read.  Nothing waits in registers: a
-  // 17-warp CTA has 96 of them per thread, and a partition of K and V ahead would take 32.
-  // (the block-table entries a request needs are fetched a phase earlier: tab[0] the block of the thread's K position,
-  // tab[1], tab[2] the blocks of its V positions, of the partition that is requested next)
-  int tab[3];
-  auto fetch_tab = [&](int part) {
-    const int lb = part * (PL / BS) + (t >> 4), lv = part * (PL / BS) + 2 * qr;
-    tab[0] = part < np && lb * BS < seq ? __ldg(d.block_tables + lb) : 0;
-    tab[1] = part < np && lv * BS < seq ? __ldg(d.block_tables + lv) : 0;
-    tab[2] = part < np && (lv + 1) * BS < seq ? __ldg(d.block_tables + lv + 1) : 0;
-  };
-  auto request_k = [&](int part) {
-    if (part < np) {
-      const int lb = part * (PL / BS) + (t >> 4);
-      const bool live = lb * BS < seq;
-      const long long pb = tab[0];
-      const __nv_bfloat16* kp = (const __nv_bfloat16*)d.kc + ((((size_t)pb * NKV + h) * HV + qr * 4) * BS + (t & 15)) * X;
+      float M = -INFINITY;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) cp_async16(KB + j * ETXB_CONSUMERS + tid, kp + (size_t)j * BS * X, live);
-    }
-    cp_async_commit();
-  };
-  auto request_v = [&](int part) {
-    if (part < np) {
+      for (int w = 0; w < 8; ++w) M = fmaxf(M, w < nslot ? s.st[(w * 8 + g) * 2] : -INFINITY);
+      const float Mz = M == -INFINITY ? 0.f : M;
+      float o = 0.f, L = 0.f;
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int lv = part * (PL / BS) + 2 * qr + u;
-        const bool live = lv * BS < seq;
-        const long long pv = tab[1 + u];
-        const __nv_bfloat16* vp = (const __nv_bfloat16*)d.vc + (((size_t)pv * NKV + h) * HD + t) * BS;
-        cp_async16(VB + (2 * u) * ETXB_CONSUMERS + tid, vp, live);
-        cp_async16(VB + (2 * u + 1) * ETXB_CONSUMERS + tid, vp + 8, live);
-      }
-    }
-    cp_async_commit();
-  };
-  fetch_tab(0);
-  request_k(0);
-  request_v(0);
-  // ---- this step's rows: raw q heads, new k and v rows; rotary row and norm weights
-  {
-    const __nv_bfloat16* qkv = (const __nv_bfloat16*)d.qkv;
-    const int nq = GQ * HV, nrow = nq + 2 * HV;
-    for (int i = tid; i < nrow + 3 * HV; i += ETXB_CONSUMERS) {
-      if (i < nrow) {
-        const __nv_bfloat16* src = i < nq ? qkv + (size_t)hq0 * HD + 8 * i
-                                          : (i < nq + HV ? qkv + (size_t)(d.NH + h) * HD + 8 * (i - nq)
-                                                         : qkv + (size_t)(d.NH + NKV + h) * HD + 8 * (i - nq - HV));
-        unpack8(ld_act16(src), s.raw + (i < nq ? 8 * i : GQ * HD + 8 * (i - nq)));
+      for (int w = 0; w < 8; ++w)
+        if (w < nslot) {
+          const float f = expf(__fsub_rn(s.st[(w * 8 + g) * 2], Mz));
+          L = __fmaf_rn(f, s.st[(w * 8 + g) * 2 + 1], L);
+          o = __fmaf_rn(f, s.po[w * 1152 + g * 132 + dd], o);
+        }
+      if (t.whole || np == 1) {
+        ((__nv_bfloat16*)d.out)[(size_t)t.hq0 * HD + idx] = __float2bfloat16_rn(__fdiv_rn(o, L));
       } else {
-        const int c = i - nrow, which = c / HV, v = c - which * HV;
-        const __nv_bfloat16* src = which == 0 ? (const __nv_bfloat16*)d.cos_sin + (size_t)pos * HD
-                                              : (const __nv_bfloat16*)(which == 1 ? d.qw : d.kw);
-        if (src != nullptr) unpack8(__ldg((const uint4*)src + v), s.cw + which * HD + 8 * v);
+        uint2* pw = (uint2*)d.tmp_out + ((size_t)(t.hq0 + g) * d.max_parts + t.part) * ETXB_GQ_PW;
+        st_pair(pw + dd, o, fl);
+        if (dd == 0) { st_pair(pw + HD, M, fl); st_pair(pw + HD + 1, L, fl); }
       }
     }
   }
-  csync();
-  mark(sm, 0);
-  if (warp < GQ) {
-    float o[8];
-    head_norm_rope_s<128>(s.raw + warp * HD, d.qw ? s.cw + HD : nullptr, s.cw, HD, d.eps, o);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) s.qs[warp * HD + lane * 4 + j] = o[j];
-    QB[warp * 68 + 2 * lane] = pack_bf(o[0], o[1]);                // (the rotated q values are bf16 values already)
-    QB[warp * 68 + 2 * lane + 1] = pack_bf(o[2], o[3]);
-  } else if (warp == GQ) {
-    float o[8];
-    head_norm_rope_s<128>(s.raw + GQ * HD, d.kw ? s.cw + 2 * HD : nullptr, s.cw, HD, d.eps, o);
-    const long long cb = slot / BS; const int off = (int)(slot % BS);
-    __nv_bfloat16* kc = (__nv_bfloat16*)d.kc;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int dd = lane * 4 + j;
-      s.knew[dd] = o[j];
-      if (writer) kc[((((size_t)cb * NKV + h) * HV + dd / X) * BS + off) * X + dd % X] = __float2bfloat16_rn(o[j]);
-    }
-  } else if (warp == GQ + 1) {
-    const long long cb = slot / BS; const int off = (int)(slot % BS);
-    __nv_bfloat16* vc = (__nv_bfloat16*)d.vc;
-    for (int dd = lane; dd < HD; dd += 32) {
-      const float v = s.raw[(GQ + 1) * HD + dd];
-      s.vnew[dd] = v;
-      if (writer) vc[(((size_t)cb * NKV + h) * HD + dd) * BS + off] = __float2bfloat16_rn(v);
-    }
-  }
-  csync();
-  mark(sm, 1);
-  for (int part = 0; part < np; ++part) {
-    const int t0 = part * PL;
-    const bool owner = pos >= t0 && pos < t0 + PL;
-    const int tpos = owner ? (int)(pos - t0) : -1;
-    const int ntok = min(PL, seq - t0);
-    auto cached = [&](int tt) { return tt < ntok && tt != tpos; };
-    fetch_tab(part + 1);
-    // ---- scores on the tensor cores: S[position][head] = K[position][:] . q[head][:].  Warp = (16 positions, half of the
-    //      128 dims): four m16n8k16 steps; A fragments straight from the staged K pieces (piece of dims chunk c and
-    //      position p sits at [c & 3][c >> 2][p]), B fragments from the bf16 q rows.  The two halves go to s.ph.
-    cp_async_wait1();                                              // this thread's K pieces have landed (its V may still travel)
-    csync();                                                       // .. and everybody else's: the fragments cross threads
-    {
-      const int mt = warp & 7, kh = warp >> 3, g8 = lane >> 2, t4 = lane & 3;
-      const uint32_t* KW = (const uint32_t*)KB;
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-      const int p0 = 16 * mt + g8;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int ks = 4 * kh + q, c0 = 2 * ks, c1 = 2 * ks + 1;
-        const uint32_t a0 = KW[(((c0 & 3) * ETXB_CONSUMERS + (c0 >> 2) * PL + p0) << 2) + t4];
-        const uint32_t a1 = KW[(((c0 & 3) * ETXB_CONSUMERS + (c0 >> 2) * PL + p0 + 8) << 2) + t4];
-        const uint32_t a2 = KW[(((c1 & 3) * ETXB_CONSUMERS + (c1 >> 2) * PL + p0) << 2) + t4];
-        const uint32_t a3 = KW[(((c1 & 3) * ETXB_CONSUMERS + (c1 >> 2) * PL + p0 + 8) << 2) + t4];
-        mma16816(c, a0, a1, a2, a3, QB[g8 * 68 + 8 * ks + t4], QB[g8 * 68 + 8 * ks + 4 + t4]);
-      }
-      const int h0 = 2 * t4;
-      if (h0 < GQ) { s.ph[(kh * GQ + h0) * PL + p0] = c[0]; s.ph[(kh * GQ + h0) * PL + p0 + 8] = c[2]; }
-      if (h0 + 1 < GQ) { s.ph[(kh * GQ + h0 + 1) * PL + p0] = c[1]; s.ph[(kh * GQ + h0 + 1) * PL + p0 + 8] = c[3]; }
-    }
-    csync();
-    request_k(part + 1);                                           // every warp is done with the K pieces: the next partition's may land
-    // ---- softmax statistics: one warp per q head, lane holds positions lane + 32 k
-    if (warp < GQ) {
-      const int g = warp;
-      float sv[4], m = -INFINITY;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int tt = lane + 32 * k;
-        const float dot = __fadd_rn(s.ph[g * PL + tt], s.ph[(GQ + g) * PL + tt]);
-        sv[k] = cached(tt) ? __fmul_rn(dot, d.scale) : -INFINITY;
-        m = fmaxf(m, sv[k]);
-      }
-      float snew = -INFINITY;
-      if (owner) {
-        float a = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) a = __fmaf_rn(s.qs[g * HD + lane * 4 + j], s.knew[lane * 4 + j], a);
-        snew = __fmul_rn(warp_sum(a), d.scale);
-      }
-      m = fmaxf(warp_max(m), snew);
-      float l = 0.f;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float pr = cached(lane + 32 * k) ? expf(__fsub_rn(sv[k], m)) : 0.f;
-        const __nv_bfloat16 hi = __float2bfloat16_rn(pr), lo = __float2bfloat16_rn(__fsub_rn(pr, __bfloat162float(hi)));
-        ((__nv_bfloat16*)PH)[g * 136 + lane + 32 * k] = hi;
-        ((__nv_bfloat16*)PLo)[g * 136 + lane + 32 * k] = lo;
-        l = __fadd_rn(l, pr);
-      }
-      l = warp_sum(l);
-      const float pn = owner ? expf(__fsub_rn(snew, m)) : 0.f;
-      if (lane == 0) { s.st[g] = m; s.st[GQ + g] = __fadd_rn(l, pn); s.st[2 * GQ + g] = pn; }
-    }
-    // ---- output on the tensor cores: O[dim][head] = sum_pos V[dim][pos] P[head][pos].  Warp = (16 dims, half of the
-    //      partition's eight cache blocks): per block one m16n8k16 step for the high and one for the low part of the
-    //      probabilities; A fragments straight from the staged V pieces (block b, positions 8 v .. of dim d at
-    //      [2 (b & 1) + v][b >> 1][d]).  Slots that are not cached yet (last partition only) are zeroed first: a
-    //      probability of 0 does not neutralise whatever bits a stale slot holds.
-    cp_async_wait1();                                              // this thread's V pieces have landed (the next K may still travel)
-    if (part == np - 1) {
-      __nv_bfloat16* vb = (__nv_bfloat16*)VB;
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int v = 0; v < 2; ++v) {
-          const int base = (2 * qr + u) * BS + 8 * v;
-          if (base + 8 > ntok || (tpos >= base && tpos < base + 8))
-#pragma unroll
-            for (int o = 0; o < 8; ++o)
-              if (!cached(base + o)) vb[(((2 * u + v) * ETXB_CONSUMERS + tid) << 3) + o] = __float2bfloat16_rn(0.f);
-        }
-    }
-    csync();                                                       // the probabilities and everybody's V pieces are in place
-    {
-      const int mt = warp & 7, kh = warp >> 3, g8 = lane >> 2, t4 = lane & 3;
-      const uint32_t* VW = (const uint32_t*)VB;
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-      const int d0 = 16 * mt + g8;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int b = 4 * kh + q;
-        if (b * BS < ntok) {
-          const int pu = 2 * (b & 1), pq = (b >> 1) * PL;
-          const uint32_t a0 = VW[((pu * ETXB_CONSUMERS + pq + d0) << 2) + t4];
-          const uint32_t a1 = VW[((pu * ETXB_CONSUMERS + pq + d0 + 8) << 2) + t4];
-          const uint32_t a2 = VW[(((pu + 1) * ETXB_CONSUMERS + pq + d0) << 2) + t4];
-          const uint32_t a3 = VW[(((pu + 1) * ETXB_CONSUMERS + pq + d0 + 8) << 2) + t4];
-          mma16816(c, a0, a1, a2, a3, PH[g8 * 68 + 8 * b + t4], PH[g8 * 68 + 8 * b + 4 + t4]);
-          mma16816(c, a0, a1, a2, a3, PLo[g8 * 68 + 8 * b + t4], PLo[g8 * 68 + 8 * b + 4 + t4]);
-        }
-      }
-      const int h0 = 2 * t4;
-      if (h0 < GQ) { s.po[(kh * GQ + h0) * HD + d0] = c[0]; s.po[(kh * GQ + h0) * HD + d0 + 8] = c[2]; }
-      if (h0 + 1 < GQ) { s.po[(kh * GQ + h0 + 1) * HD + d0] = c[1]; s.po[(kh * GQ + h0 + 1) * HD + d0 + 8] = c[3]; }
-    }
-    csync();
-    request_v(part + 1);                                           // every warp is done with the V pieces
-    for (int idx = tid; idx < GQ * HD; idx += ETXB_CONSUMERS) {
-      const int g = idx >> 7, dd = idx & (HD - 1);
-      float o = __fadd_rn(s.po[g * HD + dd], s.po[(GQ + g) * HD + dd]);
-      if (owner) o = __fmaf_rn(s.st[2 * GQ + g], s.vnew[dd], o);
-      PO[((size_t)part * GQ + g) * HD + dd] = o;
-      if (dd == 0) { PS[(part * GQ + g) * 2] = s.st[g]; PS[(part * GQ + g) * 2 + 1] = s.st[GQ + g]; }
-    }
-    // (the next partition's score sums go to s.ph, its statistics to s.sc / s.st only after the barrier that follows them:
-    // nothing this loop still reads is overwritten early)
-  }
-  csync();
   mark(sm, 2);
-  // ---- merge, with the arithmetic of attn_gq_merge: weights exp(m_p - max m), sums in ascending partition order
-  float* wl = s.ph;                                                // [GQ][np]
-  float* red = s.st + 24;                                          // [GQ]
-  if (warp < GQ) {
-    const int g = warp;
-    float m = -INFINITY;
-    for (int pp = lane; pp < np; pp += 32) m = fmaxf(m, PS[(pp * GQ + g) * 2]);
-    m = warp_max(m);
-    float L = 0.f;
-    for (int pp = lane; pp < np; pp += 32) {
-      const float w = expf(__fsub_rn(PS[(pp * GQ + g) * 2], m));
-      wl[g * np + pp] = w;
-      L = __fmaf_rn(w, PS[(pp * GQ + g) * 2 + 1], L);
-    }
-    L = warp_sum(L);
-    if (lane == 0) red[g] = L;
-  }
-  csync();
-  for (int idx = tid; idx < GQ * HD; idx += ETXB_CONSUMERS) {
-    const int g = idx >> 7, dd = idx & (HD - 1);
-    float o = 0.f;
-    for (int pp = 0; pp < np; ++pp) o = __fmaf_rn(wl[g * np + pp], PO[((size_t)pp * GQ + g) * HD + dd], o);
-    ((__nv_bfloat16*)d.out)[(size_t)(hq0 + g) * HD + dd] = __float2bfloat16_rn(__fdiv_rn(o, red[g]));
+  // (a merge never looks past the partitions the grid computed, whatever seq_lens says)
+  if (gq * np < ETXB_GQ_SHARE) mg = 0u;
+  if (!t.whole && np > 1) {
+    if (mg == 0u ? t.part == np - 1 : mg != 0xffffu) attn_gq_merge(d, sm, s.mg, t.hq0, np, fl, mg == 0u ? 0 : (int)(mg & 0xffffu) - 1, mg == 0u ? 1 : (int)(mg >> 16));
   }
   mark(sm, 3);
-  cp_async_wait0();
-  csync();                                                         // the next task may overwrite the partials
 }
 
 }  // namespace etxb

@@ -48,6 +48,7 @@ struct CtaVars {
   uint32_t epoch;            // the step (sharded sessions: the flag of this step's exchanged words derives from it)
   int cur;                   // the running task's index in the queue order (reported when a wait gives up)
   int q0, q1;                // the CTA's queue
+  int done;                  // tasks of the queue before this one are over (kernels whose other tiles use the ring's memory too)
   int halt;                  // thread 0's word before a task: the step is being abandoned, everybody leaves the loop
   int hold;                  // the running task's results are on their way out: the producer starts no further stage (see produce_task)
 };
@@ -97,6 +98,23 @@ __device__ __forceinline__ bool wait_use(volatile const uint32_t* use, uint32_t 
       if (ld_relaxed(sm.ctrl()) != 0) { *(volatile int*)sm.stop = 1; return false; }
       if ((n & 4095u) == 0 && globaltimer() > *sm.deadline) {
         if (atomicOr(sm.ctrl(), ETXB_CTRL_TIMEOUT) == 0) { sm.ctrl()[1] = where; sm.ctrl()[2] = -1; sm.ctrl()[3] = (int32_t)*use; sm.ctrl()[4] = (int32_t)k; }
+        *(volatile int*)sm.stop = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
+// Bounded wait until the tasks of the queue before `cur` are over; gives up like mbar_wait.
+__device__ __forceinline__ bool wait_done(const Smem& sm, int cur) {
+  volatile const int* done = &sm.vars->done;
+  uint32_t n = 0;
+  while (*done < cur) {
+    __nanosleep(20);
+    if ((++n & 255u) == 0) {
+      if (ld_relaxed(sm.ctrl()) != 0) return false;
+      if ((n & 1023u) == 0 && globaltimer() > *sm.deadline) {
+        if (atomicOr(sm.ctrl(), ETXB_CTRL_TIMEOUT) == 0) { sm.ctrl()[1] = cur; sm.ctrl()[2] = -1; sm.ctrl()[3] = *done; sm.ctrl()[4] = cur; }
         *(volatile int*)sm.stop = 1;
         return false;
       }

@@ -207,7 +207,6 @@ __device__ __noinline__ void batch_call(const unsigned char* args, int c0, int c
   else if constexpr (B == 20) tile_gemv_tc(args, c0, sm, s_tc, cur);
   else if constexpr (B == 21) tile_moe_up_tc(args, c0, sm, s_tc, cur);
   else if constexpr (B == 22) tile_moe_down_tc(args, c0, sm, s_tc, cur);
-  else if constexpr (B == 23) tile_mla_attn(args, c0, sm, S);
   else if constexpr (B == 7) tile_attnprep(args, c0, sm, S);
   else if constexpr (B == 8) tile_attn(args, c0, sm, S);
   else if constexpr (B == 9) tile_attn_reduce(args, c0, sm, S);
@@ -218,39 +217,31 @@ __device__ __noinline__ void argmax_col_call(const etxb_params& p, const unsigne
   const int nb = ((const etxb_batch_args*)args)->nb;
   if (c0 < nb) tile_argmax<false>(p, smem_view(), c0, nb);
 }
-// Attention out of a kernel that holds all its forms, a call each: the grouped forms (gq > 0 in the argument block; head_dim
-// 128, cache blocks of 16, partitions of 128), one task per partition or (part_len bit 24) one per sequence and q group ..
-template <int GQ, bool WHOLE>
-__device__ __noinline__ void attn_call(const etxb_attnf_args& d, int blk, const etxb_stepv& S) {
-  if constexpr (WHOLE) attn_gq_seq<GQ>(d, blk, smem_view(), S);
-  else attn_gq_tile<GQ>(d, blk, smem_view(), S);
+// Attention out of a kernel that holds all its forms, a call each: the grouped form (gq > 0 in the argument block; head_dim 128,
+// cache blocks of 16) and, in the full kernel, the general tile and latent attention.  They return the running stage count of the ring.
+__device__ __noinline__ uint32_t attn_call(const etxb_attnf_args& d, int blk, const etxb_stepv& S, uint32_t n, uint32_t mg) {
+  attn_gq_tile(d, blk, smem_view(), S, n, mg);
+  return n;
 }
-// .. and, in the full kernel, the general tile.
+__device__ __noinline__ uint32_t mla_call(const unsigned char* args, int blk, const etxb_stepv& S, uint32_t n) {
+  tile_mla_attn(args, blk, smem_view(), S, n);
+  return n;
+}
 template <bool GENERAL>
-__device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, int cur, const etxb_stepv& S) {
+__device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, int cur, const etxb_stepv& S, uint32_t& n, uint32_t mg) {
   const etxb_attnf_args& d = *(const etxb_attnf_args*)a;
   if (blk >= (int)d.nblocks || d.gq < 0) return;
   if (d.gq == 0) {
     if constexpr (GENERAL) { if (attn_fused_128(d)) batch_call<12 + 128>(a, blk, cur, S); else batch_call<12>(a, blk, cur, S); }
     return;
   }
-  const int form = (d.gq == 1 ? 0 : d.gq == 2 ? 1 : d.gq == 4 ? 2 : 3) + ((d.part_len & ETXB_GQ_WHOLE) ? 4 : 0);
-  switch (form) {
-    case 0: attn_call<1, false>(d, blk, S); break;
-    case 1: attn_call<2, false>(d, blk, S); break;
-    case 2: attn_call<4, false>(d, blk, S); break;
-    case 3: attn_call<8, false>(d, blk, S); break;
-    case 4: attn_call<1, true>(d, blk, S); break;
-    case 5: attn_call<2, true>(d, blk, S); break;
-    case 6: attn_call<4, true>(d, blk, S); break;
-    default: attn_call<8, true>(d, blk, S); break;
-  }
+  n = attn_call(d, blk, S, n, mg);
 }
 
 // Run the body of the task whose context is `c` on the consumer warps.
-// GQV: the kernel variant.  0 = every tile.  1, 2, 4, 8 = the lean decode kernel: only the tiles of a fused decode step
+// KV: the kernel variant.  0 = every tile.  ETXB_VARIANT_LEAN = the lean decode kernel: only the tiles of a fused decode step
 // (prologue, argmax, the GEMV family with norm folds of at most one row and top-k folds over at most 128 experts, the
-// grouped attention tile with GQV q heads per task); ETXB_VARIANT_MLA = the lean kernel of a latent-attention model (the
+// grouped attention tile); ETXB_VARIANT_MLA = the lean kernel of a latent-attention model (the
 // same GEMV family with the latent-attention tile in place of the grouped one); ETXB_VARIANT_BATCH = the tiles of a batched step
 // on the tensor cores.  The host picks it from the plan (select_variant): the full
 // kernel is 1020 KB of code, of which a decode step uses a fraction scattered through it, and its tiles are calls.  From the
@@ -258,15 +249,16 @@ __device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, i
 // latent-attention model 794 -> 689 from its 170 KB; the batched kernel (610 KB) gives 1 to 5 % (batched_plan).
 // XCH: the variants a sharded session launches -- the same bodies plus the exchange code (flagged-row folds of R = ranks
 // rows, row publishing after the body, the argmax exchange); compiled out of the others.
+#define ETXB_VARIANT_LEAN 1
 #define ETXB_VARIANT_MLA 16
 #define ETXB_VARIANT_BATCH 32         // the batched step on the tensor cores: its tiles and the attention tiles, nothing else
-template <int GQV, bool XCH>
+template <int KV, bool XCH>
 __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c, int cur, const Smem& sm, uint32_t& n) {
   const unsigned char* args = c->args;
   const int c0 = c->r.c0, c1 = c->r.c1;
-  constexpr bool LEAN = GQV != 0;
-  constexpr bool SH = GQV == 0 || GQV == ETXB_VARIANT_MLA;         // always-on (shared) experts: the full kernel and the latent-attention variant
-  constexpr bool FULL = GQV == 0, BATCHED = GQV == ETXB_VARIANT_BATCH;
+  constexpr bool LEAN = KV != 0;
+  constexpr bool SH = KV == 0 || KV == ETXB_VARIANT_MLA;         // always-on (shared) experts: the full kernel and the latent-attention variant
+  constexpr bool FULL = KV == 0, BATCHED = KV == ETXB_VARIANT_BATCH;
   // (a body this variant does not hold: the host picks the variant from the plan's bodies, so this is a corrupted record)
 #define ETXB_TILE(cond, call) if constexpr (cond) { call; } else { if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK); } break
   switch (c->r.body) {
@@ -275,10 +267,11 @@ __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c,
     case 2: ETXB_TILE(!BATCHED, tile_argmax<XCH>(p, sm));
     case 3: case 4: case 5: ETXB_TILE(!BATCHED, (tile_gemv_family<LEAN, XCH, SH>(c->r.body, args, c0, sm, n, cur)));
     case 12:
-      if constexpr (GQV == ETXB_VARIANT_MLA) { if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK); }      // (the latent-attention variant has no GQA tile)
-      else if constexpr (BATCHED) tile_attn_any<false>(args, c0, cur, p.step);
-      else if constexpr (LEAN) { if (c0 < (int)((const etxb_attnf_args*)args)->nblocks) attn_gq_tile<GQV ? GQV : 1>(*(const etxb_attnf_args*)args, c0, sm, p.step); }
-      else tile_attn_any<true>(args, c0, cur, p.step);
+      if constexpr (KV == ETXB_VARIANT_MLA) { if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK); }      // (the latent-attention variant has no GQA tile)
+      else if constexpr (KV == ETXB_VARIANT_LEAN) {
+        const etxb_attnf_args& d = *(const etxb_attnf_args*)args;
+        if (c0 < (int)d.nblocks && d.gq > 0) attn_gq_tile(d, c0, sm, p.step, n, c->r.mirror);
+      } else tile_attn_any<FULL>(args, c0, cur, p.step, n, c->r.mirror);
       break;
     case 6: ETXB_TILE(!LEAN, tile_topk(args, c0, sm));
     case 7: ETXB_TILE(!LEAN, batch_call<7>(args, c0, cur, p.step));
@@ -300,8 +293,8 @@ __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c,
     case 21: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<21>(args, c0, cur, p.step));
     case 22: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<22>(args, c0, cur, p.step));
     case 23:
-      if constexpr (GQV == ETXB_VARIANT_MLA) tile_mla_attn(args, c0, sm, p.step);
-      else { ETXB_TILE(FULL, batch_call<23>(args, c0, cur, p.step)); }
+      if constexpr (KV == ETXB_VARIANT_MLA) tile_mla_attn(args, c0, sm, p.step, n);
+      else { ETXB_TILE(FULL, n = mla_call(args, c0, p.step, n)); }
       break;
     default:
       if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK);
@@ -310,10 +303,29 @@ __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c,
 #undef ETXB_TILE
 }
 
+// Producer warp: waits for what the addresses of a task's stream depend on; false when the step is being abandoned.
+__device__ __forceinline__ bool producer_wait(const etxb_params& p, const Smem& sm, const etxb_rec* t, int cur) {
+  const int sw = t->stream_word;
+  if (sw == -1) return ld_relaxed(p.ctrl) == 0;
+  int good = 1;
+  if ((tidx() & 31) == 0) {
+    if (sw >= 0) good = wait_event(p, sw, (int32_t)(p.epoch * (uint32_t)p.evcount[sw]), cur, *sm.deadline) ? 1 : 0;
+    else
+      for (int i = 0; good && i < t->in_n; ++i) {
+        const int word = i < 4 ? t->in_word[i] : p.inwords[t->in_off + i];
+        good = wait_event(p, word, (int32_t)(p.epoch * (uint32_t)p.evcount[word]), cur, *sm.deadline) ? 1 : 0;
+      }
+  }
+  return __shfl_sync(0xffffffffu, good, 0) != 0;
+}
+
 // The producer warp: walks the same queue ahead of the consumers and streams the weight rows of every GEMV-family
 // task into the ring.  It waits only for what the weight ADDRESSES depend on (nothing for static weights, the router's
 // event for expert weights), never for the task's activations.
-template <bool LEAN, bool SH = !LEAN>
+// Attention tasks: the K / V units of their positions (GQ: grouped), W_UK and the cached rows (MLA: latent attention).  In a kernel whose
+// other tiles use the ring's memory as their own (TC: the tensor-core tiles) the copies wait until every task before this one is over;
+// they still run ahead of the task's events.
+template <bool LEAN, bool SH, bool GEMV, bool GQ, bool MLA, bool TC>
 __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& sm, int q0, int q1) {
   uint32_t n = 0;
   const int lane = tidx() & 31;
@@ -321,7 +333,26 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
   for (int cur = q0; cur < q1 && ok; ++cur) {
     const etxb_rec* t = p.recs + cur;
     const int body = t->body;
-    if (body < 3 || body > 5) continue;
+    if constexpr (GQ || MLA) {
+      if ((GQ && body == 12) || (MLA && body == 23)) {
+        etxb_attnf_args* aa = (etxb_attnf_args*)(sm.prod + 32);
+        __syncwarp();
+        if (lane < (int)(sizeof(etxb_attnf_args) / 8)) ((uint64_t*)aa)[lane] = __ldg((const uint64_t*)t->args + lane);   // (at least as long as the other block)
+        __syncwarp();
+        if (body == 12 && aa->gq <= 0) continue;
+        if constexpr (TC) {
+          int good = 1;
+          if (lane == 0) good = wait_done(sm, cur) ? 1 : 0;
+          if (__shfl_sync(0xffffffffu, good, 0) == 0) break;
+        }
+        if (!producer_wait(p, sm, t, cur)) break;
+        if constexpr (GQ && MLA) ok = body == 12 ? produce_attn(*aa, t->c0, p.step, n, sm, cur) : produce_mla(*(const etxb_mla_args*)aa, t->c0, p.step, n, sm, cur);
+        else if constexpr (GQ) ok = produce_attn(*aa, t->c0, p.step, n, sm, cur);
+        else ok = produce_mla(*(const etxb_mla_args*)aa, t->c0, p.step, n, sm, cur);
+        continue;
+      }
+    }
+    if (!GEMV || body < 3 || body > 5) continue;
     // the argument block through shared memory, fetched BEFORE the wait below (it depends on no event)
     etxb_gemv_args* pa = (etxb_gemv_args*)(sm.prod + 32);
     if (lane < 20) ((uint64_t*)pa)[lane] = __ldg((const uint64_t*)t->args + lane);
@@ -330,22 +361,7 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
     gg.t = gemv_task(body, *pa, t->c0);
     gemv_geom(body, gg);
     const GemvTask gt = gg.t;
-    const int sw = t->stream_word;
-    if (sw != -1) {
-      int good = 1;
-      if (lane == 0) {
-        if (sw >= 0) good = wait_event(p, sw, (int32_t)(p.epoch * (uint32_t)p.evcount[sw]), cur, *sm.deadline) ? 1 : 0;
-        else
-          for (int i = 0; good && i < t->in_n; ++i) {
-            const int word = i < 4 ? t->in_word[i] : p.inwords[t->in_off + i];
-            good = wait_event(p, word, (int32_t)(p.epoch * (uint32_t)p.evcount[word]), cur, *sm.deadline) ? 1 : 0;
-          }
-      }
-      good = __shfl_sync(0xffffffffu, good, 0);
-      if (!good) break;
-    } else if (ld_relaxed(p.ctrl) != 0) {
-      break;
-    }
+    if (!producer_wait(p, sm, t, cur)) break;
     if (gt.n > 0 && body != 3) gemv_routing<LEAN, SH>(*pa, sm.prod, (float*)(sm.prod + 16));
     ok = produce_task<SH>(body, *pa, gt, gg.rps, sm.prod, n, sm, cur, p.trace ? p.trace + 8 * (size_t)t->id : nullptr);
   }
@@ -360,14 +376,14 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
   }
 }
 
-template <int GQV, bool XCH = false>
+template <int KV, bool XCH = false>
 __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_constant__ etxb_params p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  constexpr bool TC = (GQV == 0 || GQV == ETXB_VARIANT_BATCH) && !XCH;
+  constexpr bool TC = (KV == 0 || KV == ETXB_VARIANT_BATCH) && !XCH;
   const Smem sm = smem_view();
   if (threadIdx.x == 0) {
     s_stop = 0;
-    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.cur = 0; s_vars.halt = 0; s_vars.hold = 0;
+    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.cur = 0; s_vars.halt = 0; s_vars.hold = 0; s_vars.done = -1;
     s_deadline = globaltimer() + p.timeout_ns;
     for (int i = 0; i < ETXB_NSTAGE; ++i) { mbar_init(sm.full + i, 1); mbar_init(sm.empty + i, ETXB_EMPTY_COUNT); ((uint32_t*)(sm.empty + ETXB_NSTAGE))[i] = 0xffffffffu; }
     if constexpr (TC) {
@@ -382,8 +398,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
   {
   const int q0 = p.qbegin[blockIdx.x], q1 = p.qbegin[blockIdx.x + 1];
   if (threadIdx.x >= ETXB_CONSUMERS) {
-    if constexpr (GQV != ETXB_VARIANT_BATCH)                        // (nothing is streamed through the ring in a batched plan)
-      producer_loop<GQV != 0, GQV == 0 || GQV == ETXB_VARIANT_MLA>(p, sm, q0, q1);
+    producer_loop<KV != 0, KV == 0 || KV == ETXB_VARIANT_MLA, KV != ETXB_VARIANT_BATCH, KV != ETXB_VARIANT_MLA, KV == 0 || KV == ETXB_VARIANT_MLA, TC>(p, sm, q0, q1);
     return;
   }
   TaskCtx* const ctx = (TaskCtx*)(smem_raw + ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4 + 512);
@@ -393,7 +408,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
     if (p.tc_on != 0u && threadIdx.x < 32) tc_alloc(&s_tc.tmem);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
-  if (threadIdx.x == 0) { s_vars.q0 = q0; s_vars.q1 = q1; s_vars.cur = q0; }
+  if (threadIdx.x == 0) { s_vars.q0 = q0; s_vars.q1 = q1; s_vars.cur = q0; *(volatile int*)&s_vars.done = q0; }
   if (threadIdx.x >= ETXB_CONSUMERS - 32 && q0 < q1) {
     fetch_ctx(p, ctx, q0, q0, -1);
     fetch_ctx(p, ctx, q0, q0 + 1 < q1 ? q0 + 1 : -1, -1);
@@ -430,7 +445,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
       s_vars.tr = p.trace ? p.trace + 8 * (size_t)c->r.id : nullptr;
       s_vars.cur = cur;
       if (p.trace) p.trace[8 * (size_t)c->r.id + 1] = globaltimer();
-    } else if (GQV != ETXB_VARIANT_BATCH && tidx() == 32) {   // meanwhile: what the task multiplies and how the warps share it
+    } else if (KV != ETXB_VARIANT_BATCH && tidx() == 32) {   // meanwhile: what the task multiplies and how the warps share it
       const int body = c->r.body;
       if (body >= 3 && body <= 5) {
         GemvGeom g;
@@ -445,7 +460,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
       const int q1 = vars->q1;
       fetch_ctx(p, ctx, vars->q0, cur + 2 < q1 ? cur + 2 : -1, cur + 1 < q1 ? cur + 1 : -1);
     }
-    run_body<GQV, XCH>(p, c, cur, smem_view(), n);
+    run_body<KV, XCH>(p, c, cur, smem_view(), n);
     cur = vars->cur;                                               // (before the barrier: thread 0 moves it on behind it)
     c = ctx + ((cur - vars->q0) & (ETXB_CTX_SLOTS - 1));
     if (tidx() >= ETXB_CONSUMERS - 32) cp_async_wait_all();
@@ -454,7 +469,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
     // grid's block of every rank's exchange region, its own included -- plain 4-byte stores, over NVLink for the peers.
     // Value and flag travel in one word, so nothing has to be ordered: no fence, no barrier, no remote counter; the
     // arrival below only tells this rank's consumers that the local phase is over, the folds then poll the flags.
-    const uint32_t mirror = XCH ? c->r.mirror : 0u;                  // 0 unless the grid is exchanged
+    const uint32_t mirror = XCH && c->r.body != 12 ? c->r.mirror : 0u;   // 0 unless the grid is exchanged
     if (XCH && mirror != 0u && s_stop == 0 && (threadIdx.x >> 5) == 1) {   // (an abandoned body publishes nothing)
       const etxb_gemv_args& d = *(const etxb_gemv_args*)c->args;
       const int r0 = (c->r.body == 3 ? c->r.c0 : c->r.c0 % d.tpe) * d.rpt;
@@ -474,6 +489,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
           red_release_add(p.events + (size_t)word * ETXB_EV_STRIDE, 1);
         }
       vars->hold = 0;
+      if constexpr (TC) vars->done = cur + 1;
       if (p.trace) { p.trace[8 * (size_t)id + 2] = globaltimer(); p.trace[8 * (size_t)id + 3] = blockIdx.x; }
       if (p.exec_count) atomicAdd(p.exec_count + id, 1);
     }

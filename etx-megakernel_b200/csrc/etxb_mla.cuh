@@ -16,8 +16,12 @@
 // memory -- the task (head 0, last partition) also stores it into the cache --, folds W_UK into its head's query, and
 // produces its partition's softmax statistics and weighted latent.  The partials travel as flagged (value, step) pairs
 // like those of the grouped GQA tile (etxb_attn_gq.cuh); four finishing tasks per head, placed after the partition tasks
-// in the grid, poll them, merge them in ascending partition order and apply a quarter of W_UV's rows each.  The cached
-// rows come from L2 (all heads read the same rows).
+// in the grid, poll them, merge them in ascending partition order and apply a quarter of W_UV's rows each.
+//
+// W_UK's rows and the cached rows come through the weight ring (the producer warp copies them ahead of the task, as it does
+// weights; all heads read the same cached rows, from L2): a partition task is 128 KB of W_UK and 147 KB of cache, and with loads
+// into registers, eight in flight per thread, it spent its time waiting for them.
+// A phase of 16 heads at 1043 positions: 19.5 us -> 16.5.  (Two positions at a time per warp: 72 bytes of spills, 18.)
 #pragma once
 #include "etxb_attn_gq.cuh"
 
@@ -133,23 +137,67 @@ __device__ __forceinline__ void mla_finish(const etxb_mla_args& d, const Smem& s
   csync();
 }
 
-__device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, const Smem& sm, const etxb_stepv& S) {
+// What a partition task covers and streams, worked out alike by the consumer warps and by the producer warp: first the head's W_UK
+// (DN rows of C), then the partition's cached rows (C + DR each), as many whole rows to a ring stage as fit.
+struct MlaTask {
+  int part, h, np;           // np: partitions of the context;  part >= max_parts: a finishing task
+  int tbase, ncached;        // first position; rows that come from the cache (the new one, last of its partition, does not)
+  bool owner, work;          // owner: the new position falls into the partition
+  int ra, rb, na, nb;        // rows per stage and stages, of W_UK and of the cache
+  long long pos;
+};
+__device__ __forceinline__ MlaTask mla_task(const etxb_mla_args& d, int blk, const etxb_stepv& S) {
+  MlaTask t;
+  t.part = udiv_small(blk, d.NH); t.h = blk - t.part * d.NH;
+  t.pos = (const void*)d.positions == (const void*)S.positions ? (long long)S.pos : __ldcg((const long long*)d.positions);
+  t.work = t.pos >= 0 && t.pos < d.maxlen && t.pos < ETXB_MLA_MAXCTX;
+  const int seq = t.work ? (int)t.pos + 1 : 0;
+  t.np = min((seq + ETXB_MLA_PART - 1) / ETXB_MLA_PART, d.max_parts);
+  t.tbase = t.part * ETXB_MLA_PART;
+  t.owner = t.work && (int)t.pos >= t.tbase && (int)t.pos < t.tbase + ETXB_MLA_PART;
+  t.ncached = t.owner ? (int)t.pos - t.tbase : min(seq - t.tbase, ETXB_MLA_PART);
+  t.ra = udiv_small(ETXB_STAGE_BYTES, d.C * 2); t.rb = udiv_small(ETXB_STAGE_BYTES, (d.C + d.DR) * 2);
+  const bool streams = t.work && t.part < d.max_parts && t.part < t.np;
+  t.na = streams ? udiv_small(d.DN + t.ra - 1, t.ra) : 0; t.nb = streams ? udiv_small(t.ncached + t.rb - 1, t.rb) : 0;
+  return t;
+}
+__device__ __forceinline__ bool produce_mla(const etxb_mla_args& d, int blk, const etxb_stepv& S, uint32_t& n, const Smem& sm, int where) {
+  if (blk >= (int)d.nblocks) return true;
+  const MlaTask t = mla_task(d, blk, S);
+  bool ok = true;
+  if ((tidx() & 31) == 0) {
+    const unsigned char* wa = (const unsigned char*)d.wkvb + (size_t)t.h * (d.DN + d.DV) * d.C * 2;
+    const unsigned char* wb = (const unsigned char*)d.cache + (size_t)t.tbase * (d.C + d.DR) * 2;
+    for (int s = 0; s < t.na + t.nb && ok; ++s) {
+      const uint32_t st = n % ETXB_NSTAGE, par = (n / ETXB_NSTAGE) & 1;
+      ok = mbar_wait(sm.empty + st, par ^ 1, sm, where);
+      if (!ok) break;
+      const bool A = s < t.na;
+      const int r0 = A ? s * t.ra : (s - t.na) * t.rb, nr = A ? min(t.ra, d.DN - r0) : min(t.rb, t.ncached - r0), rbytes = A ? d.C * 2 : (d.C + d.DR) * 2;
+      *((volatile uint32_t*)(sm.full + 2 * ETXB_NSTAGE) + st) = n;
+      mbar_expect_tx(sm.full + st, (uint32_t)(nr * rbytes));
+      bulk_g2s(sm.ring + (size_t)st * ETXB_STAGE_BYTES, (A ? wa : wb) + (size_t)r0 * rbytes, (uint32_t)(nr * rbytes), sm.full + st);
+      ++n;
+    }
+  }
+  ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+  n = __shfl_sync(0xffffffffu, n, 0);
+  return ok;
+}
+
+__device__ __forceinline__ void unpack16(const uint4 a, const uint4 b, float (&f)[16]) { unpack8(a, f); unpack8(b, f + 8); }
+
+__device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, const Smem& sm, const etxb_stepv& S, uint32_t& n) {
   const etxb_mla_args& d = *(const etxb_mla_args*)a;
   if (blk >= (int)d.nblocks || blk >= d.NH * (d.max_parts + ETXB_MLA_FIN)) return;
-  const int part_i = blk / d.NH, h = blk - part_i * d.NH;            // part_i >= max_parts: finishing task part_i - max_parts of the head
-  const int C = d.C, DN = d.DN, DR = d.DR, DV = d.DV, QH = DN + DR, ROW = C + DR, PW = C + 8;
-  const long long pos = (const void*)d.positions == (const void*)S.positions ? (long long)S.pos : __ldcg((const long long*)d.positions);
-  if (pos < 0 || pos >= d.maxlen || pos >= ETXB_MLA_MAXCTX) return;
-  const int seq_all = (int)pos + 1;
-  const int np = min((seq_all + ETXB_MLA_PART - 1) / ETXB_MLA_PART, d.max_parts);
-  if (part_i >= d.max_parts) { mla_finish(d, sm, h, part_i - d.max_parts, np); return; }
-  if (part_i >= np) return;
-  const int tbase = part_i * ETXB_MLA_PART;                        // first position of this task
-  const int seq = min(seq_all - tbase, ETXB_MLA_PART);               // its positions: tbase .. tbase + seq - 1
-  const bool owner = pos >= tbase && pos < tbase + ETXB_MLA_PART;    // the new position falls into this partition
-  const int lpos = owner ? (int)pos - tbase : -1;
+  const MlaTask tk = mla_task(d, blk, S);
+  if (!tk.work) return;
+  if (tk.part >= d.max_parts) { mla_finish(d, sm, tk.h, tk.part - d.max_parts, tk.np); return; }
+  if (tk.part >= tk.np) return;
+  const int h = tk.h, C = d.C, DN = d.DN, DR = d.DR, QH = DN + DR, ROW = C + DR, PW = C + 8;
+  const bool owner = tk.owner;
   const uint32_t fl = pair_flag(sm.epoch(), d.tag << 16);
-  const int tid = tidx(), lane = tid & 31, warp = tid >> 5;
+  const int tid = tidx(), lane = tid & 31, warp = tid >> 5, where = sm.cur();
   float* qf = sm.xs;            // [QH <= 256] this head's q row
   float* kvf = qf + 256;        // [ROW <= 640] the raw kv_a row
   float* cn = kvf + 640;        // [C <= 512] the new position's latent (bf16 values)
@@ -157,22 +205,51 @@ __device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, c
   float* qpe = kpn + 64;        // [DR] this head's rotated q_pe (bf16 values)
   float* cs = qpe + 64;         // [2 DR] cos | sin of the position
   float* qc = cs + 128;         // [C] q_nope W_UK
-  float* part = qc + 512;       // [8][C] partial sums of the eight thread groups (q_c, then o_c)
-  float* red = part + 4096;     // [64]
-  float* sc = red + 64;         // [128] the partition's scores, then exp(s - m); the merge keeps its weights and sums here
+  float* part = qc + 512;       // [16][512] the warps' partial sums (q_c, then o_c)
+  float* red = part + 16 * 512; // [64]
+  float* st = red + 64;         // [16][2] the warps' maximum and sum
   const __nv_bfloat16* qkv = (const __nv_bfloat16*)d.qkv;
-  for (int i = tid; i < QH + ROW + 2 * DR; i += ETXB_CONSUMERS) {
+  for (int i = tid; i < QH + 2 * DR + (owner ? ROW : 0); i += ETXB_CONSUMERS) {
     if (i < QH) qf[i] = ld_bf(qkv, (size_t)h * QH + i);
-    else if (i < QH + ROW) kvf[i - QH] = ld_bf(qkv, (size_t)d.NH * QH + (i - QH));
-    else cs[i - QH - ROW] = __ldg((const float*)d.cos_sin + (size_t)pos * 2 * DR + (i - QH - ROW));
+    else if (i < QH + 2 * DR) cs[i - QH] = __ldg((const float*)d.cos_sin + (size_t)tk.pos * 2 * DR + (i - QH));
+    else kvf[i - QH - 2 * DR] = ld_bf(qkv, (size_t)d.NH * QH + (i - QH - 2 * DR));
   }
   csync();
-  // ---- the new position's cache row: latent = rmsnorm(kv_a[:C]) (rounded twice), k_pe = rope(kv_a[C:]); this head's q_pe
-  const float ss = sumsq_numpy_order(kvf, C, red);
-  const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)C), d.eps)));
-  for (int i = tid; i < C; i += ETXB_CONSUMERS)
-    cn[i] = bfr(__fmul_rn(bfr(__fmul_rn(kvf[i], r)), __bfloat162float(__ldg((const __nv_bfloat16*)d.kvln + i))));
-  if (tid < 2 * DR) {
+  mark(sm, 0);
+  // ---- q_c[j] = sum_i q_nope[i] W_UK[h][i][j]: a warp takes rows w, w + 16, .. (they lie in the ring), its lanes the columns
+  //      8 lane .. and 256 + 8 lane ..; the warps' sums are added in warp order
+  const bool c0 = 8 * lane < C, c1 = 256 + 8 * lane < C;
+  const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
+  float acc[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) acc[u] = 0.f;
+  // (every warp walks every stage and gives back its sixteenth, so a stage's parity says which use it is)
+  uint32_t k = n;
+  n += (uint32_t)(tk.na + tk.nb);
+  bool ok = true;
+  int i0 = 0;
+#pragma unroll 1
+  for (int s = 0; s < tk.na && ok; ++s, i0 += tk.ra, ++k) {
+    const uint32_t sx = k % ETXB_NSTAGE;
+    ok = mbar_wait(sm.full + sx, (k / ETXB_NSTAGE) & 1, sm, where);
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) break;
+    const int ie = min(DN, i0 + tk.ra);
+    for (int i = i0 + ((warp - i0) & 15); i < ie; i += 16) {
+      const uint4* row = (const uint4*)(sm.ring + (size_t)sx * ETXB_STAGE_BYTES + (size_t)(i - i0) * C * 2);
+      float f[16];
+      unpack16(c0 ? row[lane] : z4, c1 ? row[32 + lane] : z4, f);
+      const float q = qf[i];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) acc[u] = __fmaf_rn(q, f[u], acc[u]);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive_n(sm.empty + sx, ETXB_EMPTY_COUNT / ETXB_CONSUMER_WARPS);
+  }
+#pragma unroll
+  for (int u = 0; u < 16; u += 4) *(float4*)(part + warp * 512 + (u >> 3) * 256 + 8 * lane + (u & 7)) = make_float4(acc[u], acc[u + 1], acc[u + 2], acc[u + 3]);
+  // ---- meanwhile: the rotated q_pe, and, for the new position, its cache row: latent = rmsnorm(kv_a[:C]) (rounded twice), k_pe = rope(kv_a[C:])
+  if (tid < 2 * DR && (owner || tid >= DR)) {
     // de-interleave (even elements first, then odd), then the half rotation: y cos + rot(y) sin
     const int i = tid < DR ? tid : tid - DR, half = DR >> 1;
     const float* x = tid < DR ? kvf + C : qf + DN;
@@ -181,138 +258,100 @@ __device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, c
     const float v = bfr(__fadd_rn(__fmul_rn(y, cs[i]), __fmul_rn(rot, cs[DR + i])));
     (tid < DR ? kpn : qpe)[i] = v;
   }
+  if (owner) {
+    const float ss = sumsq_numpy_order(kvf, C, red);               // (with barriers; owner is the same for all threads)
+    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)C), d.eps)));
+    for (int i = tid; i < C; i += ETXB_CONSUMERS)
+      cn[i] = bfr(__fmul_rn(bfr(__fmul_rn(kvf[i], r)), __bfloat162float(__ldg((const __nv_bfloat16*)d.kvln + i))));
+  }
   csync();
+  if (tid < C) {
+    float v = part[tid];
+#pragma unroll
+    for (int w = 1; w < 16; ++w) v = __fadd_rn(v, part[w * 512 + tid]);
+    qc[tid] = v;
+  }
   if (h == 0 && owner) {
-    __nv_bfloat16* row = (__nv_bfloat16*)d.cache + (size_t)pos * ROW;
+    __nv_bfloat16* row = (__nv_bfloat16*)d.cache + (size_t)tk.pos * ROW;
     for (int i = tid; i < ROW; i += ETXB_CONSUMERS) row[i] = __float2bfloat16_rn(i < C ? cn[i] : kpn[i - C]);
   }
-  // Every loop below keeps eight 16-byte loads per thread in flight before it uses the first: the rows come from L2 (a
-  // microsecond away) and a thread that consumed each load before issuing the next spent the phase waiting.
-  // ---- q_c[j] = sum_i q_nope[i] W_UK[h][i][j]: thread = (group of DN / 8 rows, 8 columns); groups added in ascending order
-  const __nv_bfloat16* wuk = (const __nv_bfloat16*)d.wkvb + (size_t)h * (DN + DV) * C;
-  const int nocts = C >> 3, grp = tid >> 6, oct = tid & 63;
-  {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const int per = (DN + 7) >> 3, i0 = grp * per, i1 = min(DN, i0 + per);
-    if (oct < nocts) {
-      for (int ib = i0; ib < i1; ib += 8) {
-        uint4 w[8];
+  csync();
+  mark(sm, 1);
+  // ---- the positions, one at a time per warp (rows w, w + 16, ..; the new one after them): score, running maximum and sum, and the
+  //      weighted latent in the lanes' registers -- a row is read once
+  float q[16], qp[2];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) w[u] = ib + u < i1 ? __ldg((const uint4*)(wuk + (size_t)(ib + u) * C) + oct) : make_uint4(0u, 0u, 0u, 0u);
+  for (int u = 0; u < 8; ++u) { q[u] = c0 ? qc[8 * lane + u] : 0.f; q[8 + u] = c1 ? qc[256 + 8 * lane + u] : 0.f; }
+  qp[0] = 2 * lane < DR ? qpe[2 * lane] : 0.f; qp[1] = 2 * lane < DR ? qpe[2 * lane + 1] : 0.f;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float q = ib + u < i1 ? qf[ib + u] : 0.f;
-          acc[0] = __fmaf_rn(q, bf_lo(w[u].x), acc[0]); acc[1] = __fmaf_rn(q, bf_hi(w[u].x), acc[1]);
-          acc[2] = __fmaf_rn(q, bf_lo(w[u].y), acc[2]); acc[3] = __fmaf_rn(q, bf_hi(w[u].y), acc[3]);
-          acc[4] = __fmaf_rn(q, bf_lo(w[u].z), acc[4]); acc[5] = __fmaf_rn(q, bf_hi(w[u].z), acc[5]);
-          acc[6] = __fmaf_rn(q, bf_lo(w[u].w), acc[6]); acc[7] = __fmaf_rn(q, bf_hi(w[u].w), acc[7]);
-        }
-      }
+  for (int u = 0; u < 16; ++u) acc[u] = 0.f;
+  float m = -INFINITY, l = 0.f;
+  auto take = [&](const float (&f)[16], float p0, float p1) {
+    float sa = 0.f, sb = 0.f;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) part[grp * 512 + 8 * oct + u] = acc[u];
+    for (int u = 0; u < 8; ++u) { sa = __fmaf_rn(f[u], q[u], sa); sb = __fmaf_rn(f[8 + u], q[8 + u], sb); }
+    sa = __fmaf_rn(p0, qp[0], sa); sb = __fmaf_rn(p1, qp[1], sb);
+    const float sc = __fmul_rn(warp_sum(__fadd_rn(sa, sb)), d.scale);
+    if (sc > m) {                                                  // (the same in every lane)
+      const float g = expf(__fsub_rn(m, sc));
+      m = sc; l = __fmul_rn(l, g);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) acc[u] = __fmul_rn(acc[u], g);
     }
-  }
-  csync();
-  for (int j = tid; j < C; j += ETXB_CONSUMERS) {
-    float v = part[j];
+    const float e = expf(__fsub_rn(sc, m));
+    l = __fadd_rn(l, e);
 #pragma unroll
-    for (int g = 1; g < 8; ++g) v = __fadd_rn(v, part[g * 512 + j]);
-    qc[j] = v;
-  }
-  csync();
-  // ---- scores: four lanes per position (lane q of the four takes the 16-byte pieces q, q + 4, ..), eight positions per
-  //      warp and round; the new position's row comes from shared memory
-  const __nv_bfloat16* cache = (const __nv_bfloat16*)d.cache + (size_t)tbase * ROW;    // (positions below are relative to the partition)
-  const int npiece = ROW >> 3, quad = lane >> 2, ql = lane & 3;
-  for (int t0 = warp * 8; t0 < seq; t0 += ETXB_CONSUMER_WARPS * 8) {
-    const int t = t0 + quad;
-    float acc = 0.f;
-    if (t < seq) {
-      const uint4* row = (const uint4*)(cache + (size_t)t * ROW);
-      for (int p0 = ql; p0 < npiece; p0 += 32) {
-        uint4 w[8];
-        if (t == lpos) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int e = 8 * (p0 + 4 * u);
-            if (e < ROW) {
-              const float* src = e < C ? cn + e : kpn + (e - C);
-              w[u] = make_uint4(pack_bf(src[0], src[1]), pack_bf(src[2], src[3]), pack_bf(src[4], src[5]), pack_bf(src[6], src[7]));
-            } else w[u] = make_uint4(0u, 0u, 0u, 0u);
-          }
-        } else {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) w[u] = p0 + 4 * u < npiece ? __ldcg(row + p0 + 4 * u) : make_uint4(0u, 0u, 0u, 0u);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int e = 8 * (p0 + 4 * u);
-          if (e < ROW) {
-            const float* qv = e < C ? qc + e : qpe + (e - C);
-            acc = __fmaf_rn(bf_lo(w[u].x), qv[0], acc); acc = __fmaf_rn(bf_hi(w[u].x), qv[1], acc);
-            acc = __fmaf_rn(bf_lo(w[u].y), qv[2], acc); acc = __fmaf_rn(bf_hi(w[u].y), qv[3], acc);
-            acc = __fmaf_rn(bf_lo(w[u].z), qv[4], acc); acc = __fmaf_rn(bf_hi(w[u].z), qv[5], acc);
-            acc = __fmaf_rn(bf_lo(w[u].w), qv[6], acc); acc = __fmaf_rn(bf_hi(w[u].w), qv[7], acc);
-          }
-        }
-      }
+    for (int u = 0; u < 16; ++u) acc[u] = __fmaf_rn(e, f[u], acc[u]);
+  };
+  i0 = 0;
+#pragma unroll 1
+  for (int s = 0; s < tk.nb && ok; ++s, i0 += tk.rb, ++k) {
+    const uint32_t sx = k % ETXB_NSTAGE;
+    ok = mbar_wait(sm.full + sx, (k / ETXB_NSTAGE) & 1, sm, where);
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) break;
+    const int ie = min(tk.ncached, i0 + tk.rb);
+#pragma unroll 1
+    for (int i = i0 + ((warp - i0) & 15); i < ie; i += 16) {
+      const unsigned char* base = sm.ring + (size_t)sx * ETXB_STAGE_BYTES + (size_t)(i - i0) * ROW * 2;
+      const uint4* row = (const uint4*)base;
+      float f[16];
+      unpack16(c0 ? row[lane] : z4, c1 ? row[32 + lane] : z4, f);
+      const uint32_t pe = 2 * lane < DR ? *(const uint32_t*)(base + 2 * C + 4 * lane) : 0u;
+      take(f, bf_lo(pe), bf_hi(pe));
     }
-    acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 1));
-    acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 2));
-    if (ql == 0 && t < seq) sc[t] = __fmul_rn(acc, d.scale);
+    __syncwarp();
+    if (lane == 0) mbar_arrive_n(sm.empty + sx, ETXB_EMPTY_COUNT / ETXB_CONSUMER_WARPS);
   }
-  csync();
-  // ---- softmax statistics of the partition: m = max score, e_t = exp(s_t - m) (kept unnormalised), l = sum e_t
-  float m = -INFINITY;
-  for (int t = tid; t < seq; t += ETXB_CONSUMERS) m = fmaxf(m, sc[t]);
-  m = warp_max(m);
-  if (lane == 0) red[warp] = m;
-  csync();
-  m = red[0];
-  for (int w = 1; w < ETXB_CONSUMER_WARPS; ++w) m = fmaxf(m, red[w]);
-  csync();
-  float l = 0.f;
-  for (int t = tid; t < seq; t += ETXB_CONSUMERS) { const float e = expf(__fsub_rn(sc[t], m)); sc[t] = e; l = __fadd_rn(l, e); }
-  l = block_sum(l, red);
-  csync();
-  // ---- o_c[j] = sum_t e_t c[t][j]: thread = (group g of eight: cached positions g, g + 8, .., 8 columns); the new
-  //      position's term is added by group 0 from shared memory; groups added in ascending order
-  {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (oct < nocts) {
-      const int ncached = owner ? lpos : seq;                      // the partition's rows that come from the cache (the new one is its last)
-      for (int tb = grp; tb < ncached; tb += 64) {
-        uint4 w[8];
+  if (owner && warp == (tk.ncached & 15)) {
+    float f[16];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) w[u] = tb + 8 * u < ncached ? __ldcg((const uint4*)(cache + (size_t)(tb + 8 * u) * ROW) + oct) : make_uint4(0u, 0u, 0u, 0u);
+    for (int u = 0; u < 8; ++u) { f[u] = c0 ? cn[8 * lane + u] : 0.f; f[8 + u] = c1 ? cn[256 + 8 * lane + u] : 0.f; }
+    take(f, 2 * lane < DR ? kpn[2 * lane] : 0.f, 2 * lane < DR ? kpn[2 * lane + 1] : 0.f);
+  }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float pr = tb + 8 * u < ncached ? sc[tb + 8 * u] : 0.f;
-          acc[0] = __fmaf_rn(pr, bf_lo(w[u].x), acc[0]); acc[1] = __fmaf_rn(pr, bf_hi(w[u].x), acc[1]);
-          acc[2] = __fmaf_rn(pr, bf_lo(w[u].y), acc[2]); acc[3] = __fmaf_rn(pr, bf_hi(w[u].y), acc[3]);
-          acc[4] = __fmaf_rn(pr, bf_lo(w[u].z), acc[4]); acc[5] = __fmaf_rn(pr, bf_hi(w[u].z), acc[5]);
-          acc[6] = __fmaf_rn(pr, bf_lo(w[u].w), acc[6]); acc[7] = __fmaf_rn(pr, bf_hi(w[u].w), acc[7]);
-        }
-      }
-      if (grp == 0 && owner) {
-        const float pr = sc[lpos];
+  for (int u = 0; u < 16; u += 4) *(float4*)(part + warp * 512 + (u >> 3) * 256 + 8 * lane + (u & 7)) = make_float4(acc[u], acc[u + 1], acc[u + 2], acc[u + 3]);
+  if (lane == 0) { st[2 * warp] = m; st[2 * warp + 1] = l; }
+  csync();
+  mark(sm, 2);
+  // ---- publish the partition's partial as flagged pairs: weighted latent [C], then max and sum (the warps' in warp order)
+  uint2* pw = (uint2*)d.tmp + ((size_t)h * d.max_parts + tk.part) * PW;
+  if (tid < C) {
+    float M = st[0];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc[u] = __fmaf_rn(pr, cn[8 * oct + u], acc[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) part[grp * 512 + 8 * oct + u] = acc[u];
+    for (int w = 1; w < 16; ++w) M = fmaxf(M, st[2 * w]);
+    const float Mz = M == -INFINITY ? 0.f : M;                     // (a warp without a position: maximum -inf, weight 0)
+    float L = 0.f, v = 0.f;
+#pragma unroll 4
+    for (int w = 0; w < 16; ++w) {
+      const float g = expf(__fsub_rn(st[2 * w], Mz));
+      L = __fmaf_rn(g, st[2 * w + 1], L);
+      v = __fmaf_rn(g, part[w * 512 + tid], v);
     }
+    st_pair(pw + tid, v, fl);
+    if (tid == 0) { st_pair(pw + C, M, fl); st_pair(pw + C + 1, L, fl); }
   }
-  csync();
-  // ---- publish the partition's partial as flagged pairs: weighted latent [C], then max and sum
-  uint2* pw = (uint2*)d.tmp + ((size_t)h * d.max_parts + part_i) * PW;
-  for (int j = tid; j < C; j += ETXB_CONSUMERS) {
-    float v = part[j];
-#pragma unroll
-    for (int g = 1; g < 8; ++g) v = __fadd_rn(v, part[g * 512 + j]);
-    st_pair(pw + j, v, fl);
-  }
-  if (tid == 0) { st_pair(pw + C, m, fl); st_pair(pw + C + 1, l, fl); }
+  mark(sm, 3);
 }
 
 }  // namespace etxb

@@ -375,6 +375,7 @@ __device__ __forceinline__ void tile_gemv_tc(const unsigned char* a, int blk, co
     const float v = tile[rl * ld + tok];
     out[(size_t)tok * d.sout + r] = __float2bfloat16_rn(bias ? __fadd_rn(v, __bfloat162float(bias[r])) : v);
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // (the producer warp may copy into this memory as soon as the task is over)
   csync();
 }
 

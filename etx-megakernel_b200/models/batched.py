@@ -89,13 +89,13 @@ def build_graph(d: Q.Dims, ptr, B: int, maxlen: int = 1072, machine: MachineMode
     scale = float(np.float32(1.0 / np.sqrt(d.HD)))
     state = {"prev": None}
 
-    def add(name, symbol, blob, grid, n_out, two_d=False, stride=0):
+    def add(name, symbol, blob, grid, n_out, two_d=False, stride=0, after=None):
         off = pool.add(blob)
         pool.rows.append((name, symbol, "", 0, off, n_out, 0, 0))
         ev = "E_" + name
         g.etensor(ev, (1,), wait_count=n_out)
         imap = "ij->(0)" if two_d else "i->(0)"
-        g.call_device(name, grid, cuda_link(SRC, symbol), resource=res, args=["impargs"], consts=(off, stride),
+        g.call_device(name, grid, cuda_link(SRC, symbol, stream_after=after), resource=res, args=["impargs"], consts=(off, stride),
                       in_edges={state["prev"]: imap} if state["prev"] else {}, out_edges={ev: imap})
         state["prev"] = ev
 
@@ -147,7 +147,8 @@ def build_graph(d: Q.Dims, ptr, B: int, maxlen: int = 1072, machine: MachineMode
                 tmp_out=ptr("tmp_out") + b * d.NH * gparts * op_attn.GQ_PARTIAL_FLOATS * 4, out=ptr("attn_out") + b * d.NH * d.HD * 2,
                 counters=ptr("attn_counters") + 4 * (L * B + b) * d.NH, scale=scale, eps=d.eps, NH=d.NH, NKV=d.NKV, HD=d.HD, BS=BS, X=X,
                 max_parts=gparts, gq=gq, part_len=op_attn.tagged_part_len(L, whole))
-        add(f"attn_{L}", "etx_tile_attn_fused", blobs, (ntask, B), ntask * B, two_d=True, stride=op_attn.F_ARG_BYTES)
+        add(f"attn_{L}", "etx_tile_attn_fused", blobs, (ntask, B), ntask * B, two_d=True, stride=op_attn.F_ARG_BYTES,
+            after="E_prologue")                                        # (the cached rows a task reads depend on its sequence's position alone)
         dense(f"o_proj_{L}", Wl("wo"), "attn_out", "o", d.H, d.NH * d.HD)
         norm(f"norm2_{L}", "o", 1, None, d.H, "resid", "resid2", "o_norm", Wl("ln2"))
         dense(f"router_{L}", Wl("wr"), "o_norm", "rlog", d.E, d.H)

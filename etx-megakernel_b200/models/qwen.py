@@ -460,7 +460,7 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
                                        counters=ptr("attn_counters") + 4 * L * d.NH, scale=scale, eps=d.eps, NH=d.NH, NKV=d.NKV, HD=d.HD,
                                        BS=BS, X=X, max_parts=nparts, gq=gq, part_len=op_attn.tagged_part_len(L) if gq else plen)
             prev = add(f"attn_{L}", "attn_fused", "attn_fused", L, blob, ntask, (ntask,), prev, "i->(0)",
-                       f"E_red_{L}", "i->(0)", (1,), ntask)
+                       f"E_red_{L}", "i->(0)", (1,), ntask, after="E_pro")    # (cached rows depend on the step's position alone)
         else:
             # ---- attention prep per kv head
             blob = argblock.pack_named(ent["dsl_attnprep"], (d.NKV, 1, 1), qkv=ptr("qkv"), qw=W("qn") if d.qk_norm else 0,

@@ -35,19 +35,20 @@ F_PARAMS = [("qkv", "ptr addrspace(1)", 0, 8), ("qw", "ptr addrspace(1)", 8, 8),
             ("gq", "i32", 152, 4), ("part_len", "i32", 156, 4)]
 GQ_PART = 128
 GQ_WHOLE = 1 << 24
-RING_BYTES = 6 * 24576     # shared memory of the weight ring, where the whole-sequence form keeps its partials
+RING_BYTES = 6 * 24576     # shared memory of the weight ring
 
 
 def tagged_part_len(tag: int, whole: bool = False) -> int:
     """part_len word of a grouped attention block: 128 positions per task, and in bits 16..23 a tag that differs between the
     grids of a step that share the partial buffers (the layer index): a merger only accepts partials carrying its own.
-    whole: bit 24, the form with one task per (sequence, q group) that walks all partitions itself -- for plans without
-    streamed tiles (the batched step), whose idle weight ring holds the partials."""
+    whole: bit 24, the form with one task per (sequence, q group) that takes all partitions itself (the batched step)."""
     return GQ_PART | ((tag & 0xff) << 16) | (GQ_WHOLE if whole else 0)
 
 
 def whole_sequence_fits(gq: int, max_parts: int) -> bool:
-    return 65536 + max_parts * gq * 130 * 4 <= RING_BYTES      # a partition of K / V pieces + the partials
+    """The longest context of the whole-sequence form, 2432 positions at 8 q heads per task: a longer one is cut into partitions, so that
+    a step is not as long as its longest sequence's one task."""
+    return 65536 + max_parts * gq * 130 * 4 <= RING_BYTES
 
 
 GQ_PARTIAL_FLOATS = 272   # grouped form: floats of `tmp_out` per (q head, partition) -- 136 (value, flag) pairs: 128 outputs, max, sum, padding

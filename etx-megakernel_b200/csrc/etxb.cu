@@ -617,6 +617,7 @@ static int32_t build_tensor_maps(etxb_session* s) {
     cuuint64_t gdim[2] = {(cuuint64_t)a.K, rows};
     cuuint64_t gstr[1] = {(cuuint64_t)a.K * 2};
     cuuint32_t box[2] = {64, ETXB_TC_BOXROWS};
+    if (ty.body == ETXB_BODY_GEMV_TC && a.tpe > 1) box[1] = (cuuint32_t)etxb::narrow_box(a.rpt, a.tpe);
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)a.W, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

@@ -253,9 +253,8 @@ __device__ __forceinline__ void tile_moe_down_g(const unsigned char* a, int blk,
 // ---------------------------------------------------------------------------------------------- per-column prologue
 // Columns of a batched step: token_in / token_out are [step][nb]; every column is at the step's position; column b owns
 // the cache slots [b * slot_span, (b + 1) * slot_span) of the shared block pool.
-// `zero`: optional, ETXB_SPLITK_COUNTERS int32 counters that column 0's prologue task clears (the arrival counters of the
-// split-K dense grids: they return to a multiple of the split in every completed step, and an abandoned step must not
-// leave them off one).
+// `zero`: optional, ETXB_SPLITK_COUNTERS int32 counters that column 0's prologue task clears (arrival counters of dense
+// grids whose tasks meet in partial sums; none of the present tiles do).
 #define ETXB_SPLITK_COUNTERS 768
 struct etxb_batch_args { int32_t nb, slot_span; int32_t* zero; uint32_t grid[3], nblocks; };
 __device__ __forceinline__ void tile_prologue_nb(const unsigned char* a, int b, const etxb_stepv& S) {

@@ -223,6 +223,10 @@ __device__ __noinline__ uint32_t attn_call(const etxb_attnf_args& d, int blk, co
   attn_gq_tile(d, blk, smem_view(), S, n, mg);
   return n;
 }
+__device__ __noinline__ uint32_t narrow_call(const unsigned char* args, int blk, uint32_t n) {
+  tile_gemv_narrow(args, blk, smem_view(), n);
+  return n;
+}
 __device__ __noinline__ uint32_t mla_call(const unsigned char* args, int blk, const etxb_stepv& S, uint32_t n) {
   tile_mla_attn(args, blk, smem_view(), S, n);
   return n;
@@ -289,7 +293,12 @@ __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c,
     case 17: ETXB_TILE(!LEAN, tile_moe_down_g(args, c0, sm));
     case 18: ETXB_TILE(FULL || BATCHED, batch_call<18>(args, c0, cur, p.step));
     case 19: ETXB_TILE(FULL || BATCHED, argmax_col_call(p, args, c0));
-    case 20: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<20>(args, c0, cur, p.step));
+    case 20:
+      if constexpr ((FULL || BATCHED) && !XCH) {
+        if (((const etxb_gemv_args*)args)->tpe > 1) n = narrow_call(args, c0, n);
+        else batch_call<20>(args, c0, cur, p.step);
+      } else if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK);
+      break;
     case 21: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<21>(args, c0, cur, p.step));
     case 22: ETXB_TILE((FULL || BATCHED) && !XCH, batch_call<22>(args, c0, cur, p.step));
     case 23:
@@ -334,16 +343,24 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
     const etxb_rec* t = p.recs + cur;
     const int body = t->body;
     if constexpr (GQ || MLA) {
-      if ((GQ && body == 12) || (MLA && body == 23)) {
+      if ((GQ && body == 12) || (MLA && body == 23) || (TC && body == 20)) {
         etxb_attnf_args* aa = (etxb_attnf_args*)(sm.prod + 32);
         __syncwarp();
         if (lane < (int)(sizeof(etxb_attnf_args) / 8)) ((uint64_t*)aa)[lane] = __ldg((const uint64_t*)t->args + lane);   // (at least as long as the other block)
         __syncwarp();
         if (body == 12 && aa->gq <= 0) continue;
+        if (TC && body == 20 && ((const etxb_gemv_args*)aa)->tpe <= 1) continue;
         if constexpr (TC) {
           int good = 1;
           if (lane == 0) good = wait_done(sm, cur) ? 1 : 0;
           if (__shfl_sync(0xffffffffu, good, 0) == 0) break;
+        }
+        if constexpr (TC) {
+          if (body == 20) {                                        // (static weights)
+            if (ld_relaxed(p.ctrl) != 0) break;
+            ok = produce_narrow(*(const etxb_gemv_args*)aa, t->c0, n, sm, cur);
+            continue;
+          }
         }
         if (!producer_wait(p, sm, t, cur)) break;
         if constexpr (GQ && MLA) ok = body == 12 ? produce_attn(*aa, t->c0, p.step, n, sm, cur) : produce_mla(*(const etxb_mla_args*)aa, t->c0, p.step, n, sm, cur);

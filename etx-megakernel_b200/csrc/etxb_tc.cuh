@@ -275,108 +275,187 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
 // out[b * sout + r] = bf16(W[r,:] . x[b] (+ bias[r])) for the nb columns b.  The GEMV block of gemv_nb; `ln` = the tensor
 // map of W (rows M, box 64 x 64), put there by the host library when the plan is bound.
 //
-// tpe = the K-split S of the grid (1: none).  Task blk covers rows [(blk / S) * rpt, ...) and the K-slice blk % S.  A
-// matrix of a few thousand rows has too few 128-row tiles for 148 workers (qkv: 40, o_proj: 16, router: 1) and an
-// instruction cannot take fewer rows without paying the same time, so the narrow matrices are cut along K instead: every
-// slice task stores its fp32 partial sums to `rows` ([S][M][nb] floats) and counts itself in `resid_in` (one int32 per row
-// block); the S-th arrival adds the partials in slice order, adds the bias and writes the bf16 result -- the same sum
-// whoever comes last.
+// tpe = 1: task blk covers rows [blk * rpt, ...) through the tcgen05 engine above.
 __device__ __forceinline__ void tile_gemv_tc(const unsigned char* a, int blk, const Smem& sm, TcShared& tc, int where) {
   const etxb_gemv_args& d = *(const etxb_gemv_args*)a;
   if (blk >= (int)d.nblocks) return;
-  const int S = max(1, d.tpe), rb = blk / S, ksl = blk - rb * S, Ks = d.K / S;
-  const int r0 = rb * d.rpt, r1 = min(d.M, r0 + d.rpt);
+  const int r0 = blk * d.rpt, r1 = min(d.M, r0 + d.rpt);
   if (r0 >= r1) return;
   const __nv_bfloat16* bias = (d.mode & ETXB_MODE_BIAS) ? (const __nv_bfloat16*)d.wts : nullptr;
   __nv_bfloat16* out = (__nv_bfloat16*)d.out;
-  float* part = S > 1 ? (float*)d.rows + (size_t)ksl * d.nb * d.M : nullptr;   // this slice's [M][nb] partial sums
   const TcSeg seg = {r0, 0, (r1 - r0 + ETXB_TC_BOXROWS - 1) & -ETXB_TC_BOXROWS, 2 * ETXB_TC_ROWS};
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // what other tiles left in this memory: ordered before the copies
   csync();
   for (int b0 = 0; b0 < d.nb; b0 += ETXB_TC_MAXTOK) {
     const int nt = min(ETXB_TC_MAXTOK, d.nb - b0);
     int pre = 0;
-    tc_task<false>(sm, tc, d.ln, seg, seg, 0, pre, ksl * Ks, Ks, nt, where,
+    tc_task<false>(sm, tc, d.ln, seg, seg, 0, pre, 0, d.K, nt, where,
             [&](int n) { return (const __nv_bfloat16*)d.x + (size_t)(b0 + n) * d.sx; },
             [&](int i, int tok, int j, const float (&v)[8], const float (&)[8]) {
               const int rr = r0 + 2 * i * ETXB_TC_ROWS + j;
-              if (part != nullptr) {                              // [slice][row][column]: the 32 lanes of a store are 32 consecutive floats
+              float y[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) if (rr + u < r1) __stcg(part + (size_t)(rr + u) * d.nb + b0 + tok, v[u]);
-              } else {
-                float y[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) y[u] = (bias && rr + u < r1) ? __fadd_rn(v[u], __bfloat162float(bias[rr + u])) : v[u];
-                tc_store8(out + (size_t)(b0 + tok) * d.sout, rr, r1, y);
-              }
+              for (int u = 0; u < 8; ++u) y[u] = (bias && rr + u < r1) ? __fadd_rn(v[u], __bfloat162float(bias[rr + u])) : v[u];
+              tc_store8(out + (size_t)(b0 + tok) * d.sout, rr, r1, y);
             });
   }
-  if (S == 1) return;
-  // (tc_task ended with a barrier: every partial of this task is stored)
-  int* last = (int*)(sm.scr + 90);
-  if (tidx() == 0) {
-    int old;                                                       // release: the CTA's partials (seen through the barrier); acquire: the other slices'
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"((int*)d.resid_in + rb) : "memory");
-    *last = ((old + 1) % S) == 0;
-  }
-  csync();
-  if (*last == 0) return;
-  const float* p0 = (const float*)d.rows;
-  const size_t sstride = (size_t)d.nb * d.M;
-  // Sums with the column index fastest (the partials are [row][column]: coalesced reads), eight loads of four columns in
-  // flight per thread (the partials come from L2, a microsecond away); every output is the sum of its slices in slice order.
-  // The sums go through shared memory ([row][nb + 1] floats in the area the tile's tokens and stages have left) so that
-  // the bf16 results leave with the row index fastest: rows of `out` are contiguous, columns are sout apart.
-  const int nr = r1 - r0, nout = d.nb * nr, ld = d.nb + 1;
-  float* tile = (float*)(((uintptr_t)sm.ring + 1023) & ~(uintptr_t)1023);
-  if ((d.nb & 3) == 0 && (((uintptr_t)p0) & 15) == 0) {
-    // four columns per 16-byte load; two such groups x four slices in flight per thread and round
-    const int gpr = d.nb >> 2, ngrp = nr * gpr;
-    for (int g0 = tidx(); g0 < ngrp; g0 += 2 * ETXB_CONSUMERS) {
-      float4 acc[2];
-      acc[0] = acc[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int q0 = 0; q0 < S; q0 += 4) {
-        float4 t[2][4];
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
-          const int gi = min(g0 + w * ETXB_CONSUMERS, ngrp - 1);
-          const float4* src = (const float4*)(p0 + (size_t)(r0 + gi / gpr) * d.nb) + (gi - (gi / gpr) * gpr);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) t[w][u] = q0 + u < S ? __ldcg((const float4*)((const float*)src + (size_t)(q0 + u) * sstride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// ---------------------------------------------------------------------------------------------- narrow dense GEMV
+// The same grid with tpe = S > 1: a matrix of a few thousand rows (qkv, o_proj, the router), S tasks per block of rpt rows.  Task blk
+// takes the rows [(blk / S) * rpt + (blk % S) * R, + R), R = rpt / S rounded up to 16, over ALL of K: no partial sums leave the SM.
+// With so few rows a tcgen05.mma (the same time for 16 rows as for 256) would take K / 16 times its 156 clocks, so these tiles run on
+// mma.sync: sub-blocks of up to 128 rows as m16 tiles, the tokens as n8 tiles, K shared out between the warps.
+//   weights  boxes of (rows of a sub-block) x 64 k through the ring, issued by the producer warp as soon as the task before is over
+//            (they depend on no event): up to 144 KB lie in shared memory when the activations arrive
+//   tokens   staged by all threads in rows of 64 k (pieces XOR-ed with the row, as the boxes: no bank conflicts for ldmatrix), all of K
+//            at once where it fits 64 KB, else in two alternating windows of 32 KB with asynchronous copies
+//   warps    16 = (16-row tiles of a sub-block) x (K groups): chunk c of 64 k belongs to K group c % KG; the groups' sums meet in
+//            shared memory and are added in group order
+// Against cutting K between the tasks (fp32 partial sums through L2, the last task to arrive adds them), us: qkv (5120 x 2048) 18.5 -> 12.5
+// with 8 tokens and 23 -> 16.5 with 32, o_proj (2048 x 4096) 15 -> 9 and 20 -> 15, the router (128 x 2048) 9.5 -> 5 and 11 -> 8.5.  What is
+// left is the staging of the tokens (2 .. 4) behind the event and the release.
+struct NarrowGeo {
+  int r0, r1, R, nsub;       // rows [r0, r1) of the task; rows of a sub-block (16, 32, 64, 128); sub-blocks
+  int nmt, KG, cps, cnt;     // m16 tiles of a sub-block, K groups, 64-k chunks per ring stage, arrivals per warp and chunk
+  int nchunk, ns;            // chunks of K; stages of one sub-block and pass
+};
+// rows of a task, a multiple of 16, and of its sub-blocks (the box of the grid's tensor map)
+__host__ __device__ __forceinline__ int narrow_rows(int rpt, int S) { return ((rpt + S - 1) / S + 15) & -16; }
+__host__ __device__ __forceinline__ int narrow_box(int rpt, int S) {
+  const int per = narrow_rows(rpt, S);
+  return per <= 16 ? 16 : per <= 32 ? 32 : per <= 64 ? 64 : 128;
+}
+__device__ __forceinline__ NarrowGeo narrow_geo(const etxb_gemv_args& d, int blk) {
+  NarrowGeo g;
+  const int S = d.tpe, rb = udiv_small(blk, S), ksl = blk - rb * S, per = narrow_rows(d.rpt, S);
+  const int e = min(d.M, rb * d.rpt + d.rpt);
+  g.r0 = min(e, rb * d.rpt + ksl * per); g.r1 = blk < (int)d.nblocks ? min(e, g.r0 + per) : g.r0;
+  g.R = narrow_box(d.rpt, S);
+  g.nmt = g.R >> 4; g.KG = ETXB_CONSUMER_WARPS / g.nmt;
+  g.nsub = (g.r1 - g.r0 + g.R - 1) / g.R;
+  g.cps = ETXB_STAGE_BYTES / (g.R * 128);                          // 12, 6, 3, 1
+  g.cnt = ETXB_EMPTY_COUNT / (g.cps * g.nmt);                      // 4, 4, 4, 6
+  g.nchunk = d.K >> 6;
+  g.ns = udiv_small(g.nchunk + g.cps - 1, g.cps);
+  return g;
+}
+__device__ __forceinline__ bool produce_narrow(const etxb_gemv_args& d, int blk, uint32_t& n, const Smem& sm, int where) {
+  const NarrowGeo g = narrow_geo(d, blk);
+  const int lane = tidx() & 31, npass = (d.nb + ETXB_TC_MAXTOK - 1) / ETXB_TC_MAXTOK;
+  bool ok = true;
+  for (int p = 0; p < npass && ok; ++p)
+    for (int b = 0; b < g.nsub && ok; ++b)
+      for (int s = 0; s < g.ns && ok; ++s) {
+        const uint32_t st = n % ETXB_NSTAGE, par = (n / ETXB_NSTAGE) & 1;
+        const int c0 = s * g.cps, nc = min(g.cps, g.nchunk - c0);
+        int good = 1;
+        if (lane == 0) {
+          good = mbar_wait(sm.empty + st, par ^ 1, sm, where) ? 1 : 0;
+          if (good) {
+            *((volatile uint32_t*)(sm.full + 2 * ETXB_NSTAGE) + st) = n;  // (see wait_use)
+            mbar_expect_tx(sm.full + st, (uint32_t)(nc * g.R * 128));
+          }
         }
-#pragma unroll
-        for (int w = 0; w < 2; ++w)
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (q0 + u < S) {
-              acc[w].x = __fadd_rn(acc[w].x, t[w][u].x); acc[w].y = __fadd_rn(acc[w].y, t[w][u].y);
-              acc[w].z = __fadd_rn(acc[w].z, t[w][u].z); acc[w].w = __fadd_rn(acc[w].w, t[w][u].w);
-            }
+        ok = __shfl_sync(0xffffffffu, good, 0) != 0;
+        if (ok && lane < nc)
+          tma_load_2d(sm.ring + (size_t)st * ETXB_STAGE_BYTES + lane * g.R * 128, d.ln, (c0 + lane) * 64, g.r0 + b * g.R, sm.full + st);
+        if (ok) ++n;
       }
-#pragma unroll
-      for (int w = 0; w < 2; ++w) {
-        const int gi = g0 + w * ETXB_CONSUMERS;
-        if (gi >= ngrp) break;
-        float* dst = tile + (gi / gpr) * ld + 4 * (gi - (gi / gpr) * gpr);
-        dst[0] = acc[w].x; dst[1] = acc[w].y; dst[2] = acc[w].z; dst[3] = acc[w].w;
+  return ok;
+}
+__device__ __forceinline__ void tile_gemv_narrow(const unsigned char* a, int blk, const Smem& sm, uint32_t& n) {
+  const etxb_gemv_args& d = *(const etxb_gemv_args*)a;
+  const NarrowGeo g = narrow_geo(d, blk);
+  if (g.nsub <= 0) return;
+  const int tid = tidx(), warp = tid >> 5, lane = tid & 31, where = sm.cur();
+  const int mt = warp & (g.nmt - 1), kg = warp / g.nmt, g8 = lane >> 2, t4 = lane & 3;
+  const __nv_bfloat16* bias = (d.mode & ETXB_MODE_BIAS) ? (const __nv_bfloat16*)d.wts : nullptr;
+  __nv_bfloat16* out = (__nv_bfloat16*)d.out;
+  unsigned char* xs = (unsigned char*)sm.xs;                       // tokens; then the K groups' sums
+  volatile const uint32_t* use = (volatile const uint32_t*)(sm.full + 2 * ETXB_NSTAGE);
+  for (int b0 = 0; b0 < d.nb; b0 += ETXB_TC_MAXTOK) {
+    const int nt = min(ETXB_TC_MAXTOK, d.nb - b0);
+    const int n8 = nt <= 8 ? 1 : nt <= 16 ? 2 : 4, tp = 8 * n8;    // n8 tiles the products take; token rows in a chunk
+    const int lw = n8 == 1 ? 5 : n8 == 2 ? 4 : 3;                  // log2 of the chunks of a 32 KB window
+    const bool whole = g.nchunk <= 2 << lw;                        // all of K fits both windows
+    const int nwin = whole ? 1 : (g.nchunk + (1 << lw) - 1) >> lw, wlen = whole ? g.nchunk : 1 << lw;
+    auto stage = [&](int w) {                                      // window w of the tokens -> its buffer, asynchronously (tokens past nt: zero)
+      const int c0 = w * wlen, nc = min(wlen, g.nchunk - c0);
+      unsigned char* dst = xs + (whole ? 0 : (w & 1) * 32768);
+      for (int i = tid; i < nc * 8 * tp; i += ETXB_CONSUMERS) {
+        const int j = i & 7, q = i >> 3, c = n8 == 1 ? q >> 3 : n8 == 2 ? q >> 4 : q >> 5, r = q & (tp - 1);   // piece, then token, then chunk
+        const bool live = r < nt;
+        cp_async16(dst + (size_t)(c * tp + r) * 128 + ((j ^ (r & 7)) << 4),
+                   (const __nv_bfloat16*)d.x + (size_t)(b0 + (live ? r : 0)) * d.sx + (c0 + c) * 64 + 8 * j, live);
       }
-    }
-  } else {
-    for (int i = tidx(); i < nout; i += ETXB_CONSUMERS) {
-      const int rl = i / d.nb, tok = i - rl * d.nb;
-      float v = 0.f;
-      for (int q = 0; q < S; ++q) v = __fadd_rn(v, __ldcg(p0 + (size_t)q * sstride + (size_t)(r0 + rl) * d.nb + tok));
-      tile[rl * ld + tok] = v;
+      cp_async_commit();
+    };
+    for (int b = 0; b < g.nsub; ++b) {
+      const uint32_t n0 = n;
+      n += (uint32_t)g.ns;
+      float acc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+      stage(0);
+      bool ok = true;
+      for (int w = 0; w < nwin; ++w) {
+        cp_async_wait0();
+        csync();                                                   // everybody's copies of window w; everybody is done with window w - 1
+        if (w + 1 < nwin) stage(w + 1);
+        if (w == 0 && b == 0 && b0 == 0) mark(sm, 0);
+        const int c0 = w * wlen, ce = min(g.nchunk, c0 + wlen);
+        const uint32_t xw = smem_u32(xs + (whole ? 0 : (w & 1) * 32768));
+        for (int c = c0 + ((kg - c0) & (g.KG - 1)); c < ce && ok; c += g.KG) {
+          const int s = g.cps == 1 ? c : udiv_small(c, g.cps), ci = c - s * g.cps;
+          const uint32_t k = n0 + (uint32_t)s, st = k % ETXB_NSTAGE;
+          ok = wait_use(use + st, k, sm, where) && mbar_wait(sm.full + st, (k / ETXB_NSTAGE) & 1, sm, where);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          const int br = lane & 7;
+          const uint32_t aw = smem_u32(sm.ring) + st * ETXB_STAGE_BYTES + ci * g.R * 128 + (16 * mt + (lane & 15)) * 128;
+          const uint32_t bw = xw + ((c - c0) * tp + br) * 128, ap = (aw >> 7) & 7;   // (the copies' swizzle goes by the address)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {                            // 32 k: two k16 steps
+            uint32_t a0[4], a1[4], x[4][4];                        // (all fragments, then their products: the loads' latencies overlap)
+            ldmatrix_x4(a0, aw + (((4 * h + (lane >> 4)) ^ ap) << 4));
+            ldmatrix_x4(a1, aw + (((4 * h + 2 + (lane >> 4)) ^ ap) << 4));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) if (i < n8) ldmatrix_x4(x[i], bw + i * 1024 + (((4 * h + (lane >> 3)) ^ br) << 4));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) if (i < n8) mma16816(acc[i], a0, x[i][0], x[i][1]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) if (i < n8) mma16816(acc[i], a1, x[i][2], x[i][3]);
+          }
+          __syncwarp();
+          // (the last chunk of a stage that is not full gives back the missing ones' arrivals too)
+          const int in_stage = min(g.cps, g.nchunk - s * g.cps);
+          if (lane == 0) mbar_arrive_n(sm.empty + st, (uint32_t)(g.cnt * (ci == in_stage - 1 ? g.cps - ci : 1)));
+        }
+      }
+      csync();                                                     // (the sums lie where the tokens were)
+      if (b == 0 && b0 == 0) mark(sm, 1);
+      // the K groups' sums: [group][token][R + 4] floats
+      float* red = (float*)xs;
+      const int ld = g.R + 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < n8) {
+          float* q = red + (size_t)(kg * tp + 8 * i + 2 * t4) * ld + 16 * mt + g8;
+          q[0] = acc[i][0]; q[ld] = acc[i][1]; q[8] = acc[i][2]; q[ld + 8] = acc[i][3];
+        }
+      csync();
+      const int rows = min(g.R, g.r1 - g.r0 - b * g.R);
+      for (int i = tid; i < nt * g.R; i += ETXB_CONSUMERS) {
+        const int tok = i >> (31 - __clz(g.R)), r = i & (g.R - 1), row = g.r0 + b * g.R + r;
+        float v = red[tok * ld + r];
+        for (int q = 1; q < g.KG; ++q) v = __fadd_rn(v, red[(size_t)(q * tp + tok) * ld + r]);
+        if (r < rows) out[(size_t)(b0 + tok) * d.sout + row] = __float2bfloat16_rn(bias ? __fadd_rn(v, __bfloat162float(bias[row])) : v);
+      }
+      if (b + 1 < g.nsub || b0 + ETXB_TC_MAXTOK < d.nb) csync();   // the tokens of the next sub-block or pass may come
     }
   }
-  csync();
-  for (int i = tidx(); i < nout; i += ETXB_CONSUMERS) {
-    const int tok = i / nr, rl = i - tok * nr, r = r0 + rl;
-    const float v = tile[rl * ld + tok];
-    out[(size_t)tok * d.sout + r] = __float2bfloat16_rn(bias ? __fadd_rn(v, __bfloat162float(bias[r])) : v);
-  }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // (the producer warp may copy into this memory as soon as the task is over)
-  csync();
+  mark(sm, 2);
 }
 
 // ---------------------------------------------------------------------------------------------- expert-grouped gate+up / down

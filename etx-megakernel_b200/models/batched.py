@@ -112,7 +112,7 @@ def build_graph(d: Q.Dims, ptr, B: int, maxlen: int = 1072, machine: MachineMode
     def dense(name, Wp, x, out, M, K, bias=0):
         mode = op_gemv.MODE_BIAS if bias else 0
         if engine == "tc":
-            # row blocks of 256 (one instruction's worth); narrow matrices are also cut along K to fill the workers
+            # row blocks of 256 (one instruction's worth); those of narrow matrices are shared by several tasks
             t, rpt, S = op_batch.split_k(M, K, W)
             blocks = t // S
             if S > 1 and ((M, K, S) not in skc and skc["n"] + blocks > op_batch.SPLITK_COUNTERS or S * B * M > SKP_FLOATS):

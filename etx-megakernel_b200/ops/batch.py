@@ -14,8 +14,9 @@ prologue / argmax have small blocks of their own.
   moe_up_g      task (expert e, row chunk): act[b][slot][r] for every (b, slot) of e's list
   moe_down_g    task (expert e, row chunk): y[b][slot][r] = bf16(bf16(W2_e[r,:] . act[b][slot]) * wts[b][slot])
   gemv_tc       the dense grid on tcgen05.mma (K % 64 == 0); `ln` is filled by the library with the address of the grid's TMA
-                tensor map.  tpe = S > 1 splits K: task blk = (row block blk // S, K-slice blk % S), fp32 partials in `rows`
-                ([S][M][nb]), arrival counters in `resid_in`; the S-th arrival of a row block sums the slices in order
+                tensor map.  tpe = S > 1: S tasks per block of rpt rows, task blk takes rows
+                (blk % S) * ceil16(rpt / S) .. of block blk // S over all of K (mma.sync; `rows` and `resid_in` have to be
+                set and are not read: a block of the plans that cut K between the tasks stays a valid one)
   moe_up_tc, moe_down_tc   the expert grids on tcgen05.mma, scheduled by share: nblocks = workers, task blk takes an equal
                 share of (active experts x row tiles); ids = the step's routing ids [nb][R] (the tiles build the
                 per-expert lists themselves), E set; moe_up_tc's resid_out = optional counter += active experts
@@ -60,9 +61,9 @@ def check_batch(nb: int, K: int) -> None:
 
 
 def split_k(M: int, K: int, workers: int) -> tuple:
-    """(tasks, rows per task, K-split) of a dense tcgen05 grid: row blocks of TC_ROWS (128 for a matrix of at most 128 rows),
-    and the largest power-of-two split of K up to 8 (slices of at least 256 columns: the task that arrives last adds
-    the slices' partial sums, which it reads from L2) that keeps the grid within one wave of the workers.  A matrix with a wave of row blocks of its own is not split."""
+    """(tasks, rows per block, split) of a dense batched grid: row blocks of TC_ROWS (128 for a matrix of at most 128 rows), each
+    shared by the largest power of two of tasks up to 8 (K of at least 256 columns for each) that keeps the grid within one wave of the
+    workers.  A matrix with a wave of row blocks of its own is not split."""
     rpt = TC_ROWS if M > 128 else 128
     blocks = -(-M // rpt)
     if blocks >= workers:

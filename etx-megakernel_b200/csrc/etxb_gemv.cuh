@@ -146,7 +146,7 @@ __device__ __forceinline__ void warp_topk_n(const void* logits, int E, int K, bo
   // Selection keys: a probability is a non-negative float, so its bit pattern orders like the value; + 1 keeps a valid
   // zero probability above "no candidate" (0).  A candidate is the 64-bit pair (key, ~expert): the larger pair is the
   // larger probability or, on a tie, the lower expert.  Each lane sorts its NK candidates once (descending), so a
-  // round only looks at the lane's head: two warp reductions (redux.sync) find the winner, whose lane pops its head.
+  // round only looks at the lanes' heads: a warp reduction (redux.sync) finds the winner, whose lane pops its head.
   // A NaN anywhere in the row makes the sum, and so every probability, NaN: no candidate is valid then and every round
   // writes id 0x7fffffff with weight -1 (the behaviour the reference's model pins for its wave path,
   // etx/ops/topk_key32.py:122-147; the expert tiles map such an id to expert 0 before they form an address).
@@ -170,7 +170,10 @@ __device__ __forceinline__ void warp_topk_n(const void* logits, int E, int K, bo
   for (int t = 0; t < K; ++t) {
     const uint32_t hk = (uint32_t)(c[0] >> 32), hi_ = (uint32_t)c[0];
     const uint32_t top = __reduce_max_sync(0xffffffffu, hk);
-    const uint32_t wl = __reduce_max_sync(0xffffffffu, hk == top ? hi_ : 0u);
+    const uint32_t who = __ballot_sync(0xffffffffu, hk == top);
+    uint32_t wl;
+    if (who & (who - 1u)) wl = __reduce_max_sync(0xffffffffu, hk == top ? hi_ : 0u);    // (several lanes' heads are as probable)
+    else wl = __shfl_sync(0xffffffffu, hi_, __ffs(who) - 1);
     const bool any = top != 0u;
     if (any && hk == top && hi_ == wl) {                            // the winner's lane pops its head
 #pragma unroll
@@ -179,7 +182,7 @@ __device__ __forceinline__ void warp_topk_n(const void* logits, int E, int K, bo
     }
     if (lane == t) { myw = any ? __uint_as_float(top - 1u) : -1.f; myid = any ? (int)(0xffffffffu - wl) : 0x7fffffff; }
   }
-  if (renorm) {
+  if (wts != nullptr && renorm) {
     // numpy's order for the sum of the K selected weights: K < 8 left to right, else 8 accumulators + tree + tail
     float tot;
     if (K < 8) {
@@ -199,7 +202,7 @@ __device__ __forceinline__ void warp_topk_n(const void* logits, int E, int K, bo
     myw = __fdiv_rn(myw, tot);
   }
   if (bf16w) myw = bfr(myw);
-  if (lane < K) { ids[lane] = myid; wts[lane] = myw; if (tei) tei[lane] = lane; }
+  if (lane < K) { ids[lane] = myid; if (wts != nullptr) wts[lane] = myw; if (tei) tei[lane] = lane; }
   __syncwarp();
 }
 
@@ -269,7 +272,7 @@ __device__ __forceinline__ void gemv_geom(int body, GemvGeom& g) {
   g.wmul = udiv_small(255 + g.W, g.W);                              // ceil(256 / W): exact for 16 warps and for ETXB_EMPTY_COUNT / W
 }
 
-// Expert ids (and routing weights) of the task's slots into `lids` / `lwts` (indexed by global slot).  One warp, all
+// Expert ids (and routing weights, unless lwts is null) of the task's slots into `lids` / `lwts` (indexed by global slot).  One warp, all
 // lanes call.  Top-k fold: recomputed from the logits; else read from the ids / wts buffers; no ids: expert 0.
 // SH: the kernel variant supports always-on (shared) experts -- mode bits 24..27: ns experts that every token uses, stored
 // after the E routed ones; they take the last ns slots with weight 1, the top-k picks the others.  (A template parameter
@@ -282,7 +285,7 @@ __device__ __forceinline__ void gemv_routing(const etxb_gemv_args& d, int32_t* l
       const int ns = (d.mode >> 24) & 0xf;
       warp_topk<LEAN>(d.logits, d.E, d.R - ns, fold == 3, (d.mode & ETXB_MODE_BF16_WTS) != 0, lids, lwts, nullptr);
       if (ns > 0) {
-        if (lane < ns) { lids[d.R - ns + lane] = d.E + lane; lwts[d.R - ns + lane] = 1.f; }
+        if (lane < ns) { lids[d.R - ns + lane] = d.E + lane; if (lwts != nullptr) lwts[d.R - ns + lane] = 1.f; }
         __syncwarp();
       }
     } else {
@@ -291,7 +294,7 @@ __device__ __forceinline__ void gemv_routing(const etxb_gemv_args& d, int32_t* l
   } else {
     if (lane < 16) {
       lids[lane] = (d.ids && lane < d.R) ? __ldcg(d.ids + lane) : 0;
-      lwts[lane] = (d.wts && lane < d.R) ? __ldcg(d.wts + lane) : 1.f;
+      if (lwts != nullptr) lwts[lane] = (d.wts && lane < d.R) ? __ldcg(d.wts + lane) : 1.f;
     }
     __syncwarp();
   }
@@ -549,7 +552,7 @@ __device__ __forceinline__ void stage_norm_col(const void* rows, const void* rin
     }
     csync();
   }
-  const int nv = K >> 3;
+  const int nv = K >> 3, pad = K <= 4096 ? 8 : 0;                  // (blocks of 128 values apart: see sumsq_numpy_order)
   uint4 lw0 = make_uint4(0, 0, 0, 0), lw1 = lw0;                   // norm weights of this thread's (at most two) vectors, fetched with the rows
 #pragma unroll 1
   for (int i = tidx(), it = 0; i < nv; i += ETXB_CONSUMERS, ++it) {
@@ -619,13 +622,14 @@ __device__ __forceinline__ void stage_norm_col(const void* rows, const void* rin
 #pragma unroll
       for (int j = 0; j < 8; ++j) z[j] = bfr(__fadd_rn(rf[j], acc[j]));
     }
-    *(float4*)(xf + 8 * i) = make_float4(z[0], z[1], z[2], z[3]);
-    *(float4*)(xf + 8 * i + 4) = make_float4(z[4], z[5], z[6], z[7]);
+    float* zx = xf + 8 * i + (i >> 4) * pad;
+    *(float4*)zx = make_float4(z[0], z[1], z[2], z[3]);
+    *(float4*)(zx + 4) = make_float4(z[4], z[5], z[6], z[7]);
     if (store && rout != nullptr)
       *(uint4*)((__nv_bfloat16*)rout + 8 * i) = make_uint4(pack_bf(z[0], z[1]), pack_bf(z[2], z[3]), pack_bf(z[4], z[5]), pack_bf(z[6], z[7]));
   }
   csync();
-  const float ss = sumsq_numpy_order(xf, K, scr);
+  const float ss = sumsq_numpy_order<true>(xf, K, scr, pad);
   const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
 #pragma unroll 1
   for (int i = tidx(), it = 0; i < nv; i += ETXB_CONSUMERS, ++it) {
@@ -633,7 +637,7 @@ __device__ __forceinline__ void stage_norm_col(const void* rows, const void* rin
     const float wf[8] = {bf_lo(w.x), bf_hi(w.x), bf_lo(w.y), bf_hi(w.y), bf_lo(w.z), bf_hi(w.z), bf_lo(w.w), bf_hi(w.w)};
     float v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = bfr(__fmul_rn(wf[j], bfr(__fmul_rn(xf[8 * i + j], r))));
+    for (int j = 0; j < 8; ++j) v[j] = bfr(__fmul_rn(wf[j], bfr(__fmul_rn(xf[8 * i + (i >> 4) * pad + j], r))));
     const uint4 o = make_uint4(pack_bf(v[0], v[1]), pack_bf(v[2], v[3]), pack_bf(v[4], v[5]), pack_bf(v[6], v[7]));
     ((uint4*)xb)[i] = o;
     if (store && xout != nullptr) *(uint4*)((__nv_bfloat16*)xout + 8 * i) = o;
@@ -670,7 +674,7 @@ __device__ __forceinline__ void tile_gemv_family(int body, const unsigned char* 
         lwts[tidx()] = tidx() < d.R ? __ldcg(d.wts + tidx()) : 1.f;
       }
       __syncwarp();
-    } else if (body == 5 || fold >= 2) {
+    } else if (body == 5 || (fold >= 2 && blk - t.group * d.tpe == 0)) {    // (gate+up needs the routing only to publish it)
       gemv_routing<LEAN, SH>(d, lids, lwts);
     }
     if (body == 4 && fold >= 2 && blk - t.group * d.tpe == 0 && tidx() < spt) {   // the group's first chunk publishes its slots' routing

@@ -379,7 +379,7 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
     gemv_geom(body, gg);
     const GemvTask gt = gg.t;
     if (!producer_wait(p, sm, t, cur)) break;
-    if (gt.n > 0 && body != 3) gemv_routing<LEAN, SH>(*pa, sm.prod, (float*)(sm.prod + 16));
+    if (gt.n > 0 && body != 3) gemv_routing<LEAN, SH>(*pa, sm.prod, nullptr);    // (the ids alone: the stream waits for them)
     ok = produce_task<SH>(body, *pa, gt, gg.rps, sm.prod, n, sm, cur, p.trace ? p.trace + 8 * (size_t)t->id : nullptr);
   }
   // Nothing is left in flight on a normal exit (the consumers waited for every stage).  When the step was abandoned,

@@ -190,25 +190,28 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // ref_numpy.py:71-73): blocks of 128 with 8 strided accumulators each, combined ((r0+r1)+(r2+r3))+((r4+r5)+(r6+r7)),
 // blocks combined by a balanced binary tree.  Exact for n = 128 * 2^j, 128 <= n <= 16 * blockDim; other n fall back
 // to block_sum (same value up to fp32 rounding).  x in shared memory; red >= 32 floats; all threads call.
-__device__ __forceinline__ float sumsq_numpy_order(const float* x, int n, float* red) {
+// pad: floats between two blocks of 128 (8: the eight accumulators of four blocks lie in 32 different banks).  FRESH: the caller
+// has just passed a barrier, nobody reads `red` any more.
+template <bool FRESH = false>
+__device__ __forceinline__ float sumsq_numpy_order(const float* x, int n, float* red, int pad = 0) {
   const bool pow2 = n >= 128 && (n & (n - 1)) == 0 && n <= 16 * ETXB_CONSUMERS;
   if (!pow2) {
     float s = 0.f;
-    for (int i = tidx(); i < n; i += ETXB_CONSUMERS) s = __fmaf_rn(x[i], x[i], s);
+    for (int i = tidx(); i < n; i += ETXB_CONSUMERS) { const float v = x[i + (i >> 7) * pad]; s = __fmaf_rn(v, v, s); }
     return block_sum(s, red);
   }
   const int nacc = n >> 4;                                         // 8 accumulators per 128-element block
   const int t = tidx();
   float r = 0.f;
   if (t < nacc) {
-    const float* b = x + (t >> 3) * 128 + (t & 7);
+    const float* b = x + (t >> 3) * (128 + pad) + (t & 7);
     r = __fmul_rn(b[0], b[0]);
 #pragma unroll
     for (int i = 1; i < 16; ++i) r = __fadd_rn(r, __fmul_rn(b[8 * i], b[8 * i]));
   }
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, o));   // accumulators, then 4 blocks
-  csync();
+  if (!FRESH) csync();
   if ((t & 31) == 0) red[t >> 5] = r;
   csync();
   const int nw = (nacc + 31) >> 5;                                 // power of two (or 1)

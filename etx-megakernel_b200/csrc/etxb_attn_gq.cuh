@@ -8,7 +8,8 @@
 //   * a warp takes a unit at a time and runs it alone: scores on the tensor cores (mma.sync, 16 positions x 8 heads, K rows by
 //     ldmatrix), its own running maximum and sum, the probabilities transposed by movmatrix into the second product's operand, 128
 //     output sums per head in its registers.  No barrier between units; the warps' results meet once, at the end.
-//   * the probabilities go into the product as a bf16 value plus the bf16 of what that rounding lost (2^-17 of the value).
+//   * the probabilities go into the product as a bf16 value, the bf16 of what that rounding lost and that of what the second one lost: the
+//     24 bits of their fp32 value, as they were multiplied before.  Whole contexts: the first two (2^-17 of the value), as before too.
 // Bound by the stream of K / V at long contexts, by the chain q rows -> norm -> scores -> publish -> merge at short ones.
 // A phase at 8150 positions (64 partitions, 256 tasks): 30 us -> 17; 8 sequences at 1033: 33 -> 22; 32 sequences, whole contexts of 1045:
 // 52 -> 21; one sequence at 1037: 8.3 -> 7.9.  The forms before multiplied out of registers on the fp32 pipes, or walked a context with
@@ -354,21 +355,24 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
           __syncwarp();
         }
         const uint32_t ks = smem_u32(unit) + lane * 16, vs = smem_u32(unit) + 4096 + ((lane >> 4) << 4) + ((lane & 15) << 5);
-        // (four fragments at a time, then their products: a load in front of every product is a chain of their latencies)
-        float c[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-        for (int q = 0; q < 8; q += 4) {
+        // Four fragments at a time, then their products (a load in front of every product is a chain of their latencies); sums over a
+        // quarter of the dims each, added pairwise: chains of two products instead of eight.
+        float c[4], qs[4][4];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) qs[j >> 2][j & 3] = 0.f;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
           uint32_t a[4][4], b[4][2];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            ldmatrix_x4(a[u], ks + (q + u) * 512);                 // 16 positions x 16 dims
-            b[u][0] = qw[8 * (q + u)]; b[u][1] = qw[8 * (q + u) + 4];
+            ldmatrix_x4(a[u], ks + (4 * h + u) * 512);             // 16 positions x 16 dims
+            b[u][0] = qw[8 * (4 * h + u)]; b[u][1] = qw[8 * (4 * h + u) + 4];
           }
 #pragma unroll
-          for (int u = 0; u < 4; u += 2) { mma16816(c, a[u], b[u][0], b[u][1]); mma16816(e, a[u + 1], b[u + 1][0], b[u + 1][1]); }
+          for (int u = 0; u < 4; u += 2) { mma16816(qs[2 * h], a[u >> 1], b[u >> 1][0], b[u >> 1][1]); mma16816(qs[2 * h + 1], a[2 + (u >> 1)], b[2 + (u >> 1)][0], b[2 + (u >> 1)][1]); }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = __fadd_rn(c[j], e[j]);
+        for (int j = 0; j < 4; ++j) c[j] = __fadd_rn(__fadd_rn(qs[0][j], qs[1][j]), __fadd_rn(qs[2][j], qs[3][j]));
         // softmax of the unit: positions g8 (c[0], c[1]) and g8 + 8 (c[2], c[3]), heads 2 t4 and 2 t4 + 1
 #pragma unroll
         for (int j = 0; j < 4; ++j) c[j] = __fmul_rn(c[j], d.scale);
@@ -396,6 +400,12 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
         for (int j = 0; j < 4; ++j) r[j] = __fsub_rn(c[j], bfr(c[j]));
         const uint32_t h0 = movmatrix(pack_bf(c[0], c[1])), h1 = movmatrix(pack_bf(c[2], c[3]));
         const uint32_t w0 = movmatrix(pack_bf(r[0], r[1])), w1 = movmatrix(pack_bf(r[2], r[3]));
+        uint32_t x0 = 0u, x1 = 0u;
+        if (!t.whole) {                                            // what the second rounding lost
+#pragma unroll
+          for (int j = 0; j < 4; ++j) r[j] = __fsub_rn(r[j], bfr(r[j]));
+          x0 = movmatrix(pack_bf(r[0], r[1])); x1 = movmatrix(pack_bf(r[2], r[3]));
+        }
 #pragma unroll
         for (int j = 0; j < 8; j += 4) {
           uint32_t a[4][4];
@@ -405,6 +415,9 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
           for (int u = 0; u < 4; ++u) mma16816(acc[j + u], a[u], h0, h1);
 #pragma unroll
           for (int u = 0; u < 4; ++u) mma16816(acc[j + u], a[u], w0, w1);
+          if (!t.whole)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) mma16816(acc[j + u], a[u], x0, x1);
         }
         if (ragged) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // (this warp's writes, before the next copy into the place)
         __syncwarp();

@@ -210,11 +210,15 @@ __device__ __forceinline__ void head_norm_rope_r(uint2 x, float* xh, bool norm, 
 // out[h][:] = bf16(sum_p w_p * tmp[p][:] / sum_p w_p * l_p), w_p = exp(m_p - max m), for the 32-value slices mi, mi + mk, .. of the
 // group's gq * 128 output values.  Polls the flagged partials the other CTAs publish (L2).  A warp takes a slice and a share of the
 // partitions (its lane: one value); every warp works out its head's weights itself from the partitions' statistics.
+// The order of the sums is a matter of gq and np alone (warps per slice, partitions per round): how many tasks share the merge (mk) differs between
+// the sequences of a batch and between plans, and equal columns get equal bits.  Past 16 partitions shared merges fetch 32 at a time, four
+// warps a slice; below, a warp a slice (all 16 slices of a round at once): against two warps, a phase of 8 sequences at 1033 positions 21.4 us /
+// 22.3, of 16 at 1400 48.9 / 50.7, of 3 at 1400 13.3 / 13.4.  (As many warps as the slices of a task left free, 1 to 16: 22.4, 49.2 and 14.1.)
 __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Smem& sm, float* mg, int hq0, int np, uint32_t fl, int mi, int mk) {
   constexpr int HD = 128, NF = 8;
   const int lane = tidx() & 31, warp = tidx() >> 5;
   const int nsl = (d.gq * 4 - mi + mk - 1) / mk;                   // slices of this task
-  const int wps = nsl > 8 ? 1 : nsl > 4 ? 2 : nsl > 2 ? 4 : nsl > 1 ? 8 : 16;   // warps per slice
+  const int wps = np > 16 && d.gq * np >= ETXB_GQ_SHARE ? 4 : d.gq > 2 ? 1 : d.gq == 2 ? 2 : 4;   // warps per slice
   const int per = 16 / wps, sub = warp / per;                      // slices per round; the warp's share of the partitions
 #pragma unroll 1
   for (int s0 = 0; s0 < nsl; s0 += per) {

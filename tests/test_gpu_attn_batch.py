@@ -1,0 +1,82 @@
+"""The grouped attention tile in plans of several sequences (one argument block each) and of long contexts: what a column gets may not depend
+on its place in the batch, on the other columns or on how large the cache is."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import etx_megakernel_b200  # noqa: E402,F401
+from etx_megakernel_b200 import ops  # noqa: E402
+from etx_megakernel_b200.frontends import cuda_link  # noqa: E402
+from etx_megakernel_b200.importer import argblock  # noqa: E402
+from etx_megakernel_b200.ir import Graph  # noqa: E402
+from etx_megakernel_b200.models import qwen as Q  # noqa: E402
+from etx_megakernel_b200.passes import compile_graph  # noqa: E402
+from etx_megakernel_b200.runtime import Session  # noqa: E402
+from oracle import ref_decode as O  # noqa: E402
+from tests.test_gpu_ops import dev_bf16, host  # noqa: E402
+
+DEV, HD, SCALE = "cuda:0", 128, float(np.float32(1.0 / np.sqrt(128)))
+
+
+def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True):
+    """One attention grid over B sequences.  K, V: per sequence [seq][NKV][HD], the last position being the new one (its cache row holds NaN and comes from qkv
+    [B][NH + 2 NKV][HD] instead).  Returns (out [B][NH][HD] bf16 values, the cached k rows at the new positions [B][NKV][HD])."""
+    B, nblk, parts = len(K), maxlen // 16, -(-maxlen // 128)
+    pools = []
+    for b in range(B):
+        pad = np.full((maxlen - len(K[b]) + 1, NKV, HD), np.nan, np.float32)
+        pools.append(O.paged_from_contig(np.concatenate([K[b][:-1], pad]), np.concatenate([V[b][:-1], pad]), nblk))
+    table = np.random.default_rng(1).permutation(B * nblk).astype(np.int32)                # any block order
+    inv = np.argsort(table)
+    kc, vc = (dev_bf16(np.concatenate([p[i] for p in pools])[inv]) for i in (0, 1))
+    seq = np.array([len(k) for k in K])
+    tab = Q.rope_table(1e6, HD, maxlen).view(np.int16)
+    if not rotary:
+        tab = np.concatenate([O.f32_to_bf16_bits(np.ones((maxlen, HD // 2), np.float32)).view(np.int16), np.zeros((maxlen, HD // 2), np.int16)], 1)
+    t = {"qkv": dev_bf16(qkv), "cos_sin": torch.from_numpy(tab).to(DEV).view(torch.bfloat16), "kc": kc, "vc": vc,
+         "block_tables": torch.from_numpy(table).to(DEV), "seq_lens": torch.from_numpy(seq.astype(np.int32)).to(DEV),
+         "positions": torch.from_numpy(seq - 1).to(DEV), "tmp_out": torch.zeros((B, NH, parts, ops.attn.GQ_PARTIAL_FLOATS), dtype=torch.float32, device=DEV),
+         "slot_mapping": torch.from_numpy(np.array([int(table[b * nblk + (s - 1) // 16]) * 16 + (s - 1) % 16 for b, s in enumerate(seq)], np.int64)).to(DEV),
+         "out": torch.zeros((B, NH, HD), dtype=torch.bfloat16, device=DEV)}
+    step = {"qkv": (NH + 2 * NKV) * HD * 2, "block_tables": nblk * 4, "seq_lens": 4, "positions": 8, "slot_mapping": 8,
+            "tmp_out": NH * parts * ops.attn.GQ_PARTIAL_FLOATS * 4, "out": NH * HD * 2}
+    ntask = NH // gq * (1 if whole else parts)
+    blobs = b"".join(argblock.pack_named(ops.all_entries()["attn_fused"], (ntask, 1, 1), **{n: x.data_ptr() + b * step.get(n, 0) for n, x in t.items()}, scale=scale,
+                                         eps=1e-6, NH=NH, NKV=NKV, HD=HD, BS=16, X=8, max_parts=parts, gq=gq, part_len=ops.attn.tagged_part_len(3, whole)) for b in range(B))
+    g = Graph("attn")
+    g.tensor("impargs", (len(blobs),), role="weight", bytes_per_elem=1)
+    g.etensor("E_done", (1,), wait_count=ntask * B)
+    g.call_device("attn", (ntask, B), cuda_link("", "etx_tile_attn_fused"), args=["impargs"], consts=(0, ops.attn.F_ARG_BYTES), out_edges={"E_done": "ij->(0)"})
+    s = Session(compile_graph(g, "b200", {}), {}, blobs, 0)
+    outs = []
+    for _ in range(2):
+        t["out"].zero_()
+        s.run(10.0)
+        outs.append(host(t["out"]).copy())
+    s.close()
+    assert np.array_equal(outs[0], outs[1], equal_nan=True)
+    slot = host(t["slot_mapping"])
+    return outs[0], np.stack([host(kc)[s // 16, :, :, s % 16].reshape(NKV, HD) for s in slot])
+
+
+@pytest.mark.parametrize("seq,gq", [(1030, 8), (1030, 2), (900, 8), (4200, 8)])
+def test_equal_columns_get_equal_bits_wherever_they_stand(seq, gq):
+    """Ten equal sequences, 9 partitions: the numbers of tasks that share a group's merge differ between the columns; one sequence, and one in a larger
+    cache: other numbers again.  V alternates by partition, so that the sum over the partitions is small beside its terms and
+    another order of them would show."""
+    NH, NKV, G = 32, 4, 8
+    rng = np.random.default_rng(seq)
+    V = O.bfr(rng.standard_normal((seq, NKV, HD), dtype=np.float32) + np.where(np.arange(seq) // 128 % 2, -900.0, 900.0).astype(np.float32)[:, None, None])
+    K = O.bfr(rng.standard_normal((seq, NKV, HD), dtype=np.float32) * np.float32(0.3))
+    qkv = O.bfr(rng.standard_normal((NH + 2 * NKV, HD), dtype=np.float32))
+    maxlen = -(-seq // 128) * 128
+    one, _ = run(NH, NKV, [K], [V], qkv[None], maxlen, gq)
+    ten, _ = run(NH, NKV, [K] * 10, [V] * 10, np.stack([qkv] * 10), maxlen, gq)
+    large, _ = run(NH, NKV, [K] * 3, [V] * 3, np.stack([qkv] * 3), maxlen + 640, gq)
+    assert np.isfinite(one).all() and np.abs(one).max() < 900
+    for b in range(10):
+        assert np.array_equal(ten[b], one[0]), f"column {b}: {np.mean(ten[b] != one[0]):.4f} of the values differ"
+    for b in range(3):
+        assert np.array_equal(large[b], one[0]), f"larger cache, column {b}: {np.mean(large[b] != one[0]):.4f} of the values differ"

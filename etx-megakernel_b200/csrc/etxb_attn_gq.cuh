@@ -10,6 +10,8 @@
 //     output sums per head in its registers.  No barrier between units; the warps' results meet once, at the end.
 //   * the probabilities go into the product as a bf16 value, the bf16 of what that rounding lost and that of what the second one lost: the
 //     24 bits of their fp32 value, as they were multiplied before.  Whole contexts: the first two (2^-17 of the value), as before too.
+//     Sums meet in fp32, so that the partials are no further from 64-bit ones than plain fp32 chains of 32 terms leave them: 1.3e-7 at 1038
+//     and 8151 positions against 1.6e-7 (summed up inside the products 1.8e-7).
 // Bound by the stream of K / V at long contexts, by the chain q rows -> norm -> scores -> publish -> merge at short ones.
 // A phase at 8150 positions (64 partitions, 256 tasks): 30 us -> 17; 8 sequences at 1033: 33 -> 22; 32 sequences, whole contexts of 1045:
 // 52 -> 21; one sequence at 1037: 8.3 -> 7.9.  The forms before multiplied out of registers on the fp32 pipes, or walked a context with
@@ -359,24 +361,28 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
           __syncwarp();
         }
         const uint32_t ks = smem_u32(unit) + lane * 16, vs = smem_u32(unit) + 4096 + ((lane >> 4) << 4) + ((lane & 15) << 5);
-        // Four fragments at a time, then their products (a load in front of every product is a chain of their latencies); sums over a
-        // quarter of the dims each, added pairwise: chains of two products instead of eight.
-        float c[4], qs[4][4];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) qs[j >> 2][j & 3] = 0.f;
+        // Four fragments at a time, then their products (a load in front of every product is a chain of their latencies).  A tensor-core sum is
+        // cut off, not rounded, where it leaves the 24 bits: every product begins at zero and the eight are added pairwise in fp32.
+        float c[4];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t a[4][4], b[4][2];
+          float qs[4][4];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) qs[j >> 2][j & 3] = 0.f;
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             ldmatrix_x4(a[u], ks + (4 * h + u) * 512);             // 16 positions x 16 dims
             b[u][0] = qw[8 * (4 * h + u)]; b[u][1] = qw[8 * (4 * h + u) + 4];
           }
 #pragma unroll
-          for (int u = 0; u < 4; u += 2) { mma16816(qs[2 * h], a[u >> 1], b[u >> 1][0], b[u >> 1][1]); mma16816(qs[2 * h + 1], a[2 + (u >> 1)], b[2 + (u >> 1)][0], b[2 + (u >> 1)][1]); }
-        }
+          for (int u = 0; u < 4; ++u) mma16816(qs[u], a[u], b[u][0], b[u][1]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = __fadd_rn(__fadd_rn(qs[0][j], qs[1][j]), __fadd_rn(qs[2][j], qs[3][j]));
+          for (int j = 0; j < 4; ++j) {
+            const float v = __fadd_rn(__fadd_rn(qs[0][j], qs[1][j]), __fadd_rn(qs[2][j], qs[3][j]));
+            c[j] = h == 0 ? v : __fadd_rn(c[j], v);
+          }
+        }
         // softmax of the unit: positions g8 (c[0], c[1]) and g8 + 8 (c[2], c[3]), heads 2 t4 and 2 t4 + 1
 #pragma unroll
         for (int j = 0; j < 4; ++j) c[j] = __fmul_rn(c[j], d.scale);
@@ -410,18 +416,28 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
           for (int j = 0; j < 4; ++j) r[j] = __fsub_rn(r[j], bfr(r[j]));
           x0 = movmatrix(pack_bf(r[0], r[1])); x1 = movmatrix(pack_bf(r[2], r[3]));
         }
+        // (two fragments at a time, four spill; the small parts first, and their sum rounded into the large one's: see the scores)
 #pragma unroll
-        for (int j = 0; j < 8; j += 4) {
-          uint32_t a[4][4];
+        for (int j = 0; j < 8; j += 2) {
+          uint32_t a[2][4];
+          float lo[2][4], hi[2][4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) ldmatrix_x4(a[u], vs + (j + u) * 512);   // 16 dims x 16 positions (matrices: dims 0-7, 8-15 of positions 0-7, then of 8-15)
+          for (int u = 0; u < 2; ++u) {
+            ldmatrix_x4(a[u], vs + (j + u) * 512);                 // 16 dims x 16 positions (matrices: dims 0-7, 8-15 of positions 0-7, then of 8-15)
 #pragma unroll
-          for (int u = 0; u < 4; ++u) mma16816(acc[j + u], a[u], h0, h1);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) mma16816(acc[j + u], a[u], w0, w1);
+            for (int e = 0; e < 4; ++e) lo[u][e] = hi[u][e] = 0.f;
+          }
           if (!t.whole)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) mma16816(acc[j + u], a[u], x0, x1);
+            for (int u = 0; u < 2; ++u) mma16816(lo[u], a[u], x0, x1);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) mma16816(lo[u], a[u], w0, w1);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) mma16816(hi[u], a[u], h0, h1);
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[j + u][e] = __fadd_rn(acc[j + u][e], __fadd_rn(hi[u][e], lo[u][e]));
         }
         if (ragged) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // (this warp's writes, before the next copy into the place)
         __syncwarp();

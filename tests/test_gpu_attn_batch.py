@@ -22,7 +22,8 @@ DEV, HD, SCALE = "cuda:0", 128, float(np.float32(1.0 / np.sqrt(128)))
 
 def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True):
     """One attention grid over B sequences.  K, V: per sequence [seq][NKV][HD], the last position being the new one (its cache row holds NaN and comes from qkv
-    [B][NH + 2 NKV][HD] instead).  Returns (out [B][NH][HD] bf16 values, the cached k rows at the new positions [B][NKV][HD])."""
+    [B][NH + 2 NKV][HD] instead).  Returns (out [B][NH][HD] bf16 values, the cached k rows at the new positions [B][NKV][HD], the partials
+    [B][NH][partitions][128 sums, maximum, sum of the probabilities])."""
     B, nblk, parts = len(K), maxlen // 16, -(-maxlen // 128)
     pools = []
     for b in range(B):
@@ -58,7 +59,8 @@ def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True):
     s.close()
     assert np.array_equal(outs[0], outs[1], equal_nan=True)
     slot = host(t["slot_mapping"])
-    return outs[0], np.stack([host(kc)[s // 16, :, :, s % 16].reshape(NKV, HD) for s in slot])
+    tmp = host(t["tmp_out"]).reshape(B, NH, parts, ops.attn.GQ_PARTIAL_FLOATS // 2, 2)[..., :HD + 2, 0]
+    return outs[0], np.stack([host(kc)[s // 16, :, :, s % 16].reshape(NKV, HD) for s in slot]), tmp
 
 
 @pytest.mark.parametrize("seq,gq", [(1030, 8), (1030, 2), (900, 8), (4200, 8)])
@@ -72,11 +74,56 @@ def test_equal_columns_get_equal_bits_wherever_they_stand(seq, gq):
     K = O.bfr(rng.standard_normal((seq, NKV, HD), dtype=np.float32) * np.float32(0.3))
     qkv = O.bfr(rng.standard_normal((NH + 2 * NKV, HD), dtype=np.float32))
     maxlen = -(-seq // 128) * 128
-    one, _ = run(NH, NKV, [K], [V], qkv[None], maxlen, gq)
-    ten, _ = run(NH, NKV, [K] * 10, [V] * 10, np.stack([qkv] * 10), maxlen, gq)
-    large, _ = run(NH, NKV, [K] * 3, [V] * 3, np.stack([qkv] * 3), maxlen + 640, gq)
+    one, _, _ = run(NH, NKV, [K], [V], qkv[None], maxlen, gq)
+    ten, _, _ = run(NH, NKV, [K] * 10, [V] * 10, np.stack([qkv] * 10), maxlen, gq)
+    large, _, _ = run(NH, NKV, [K] * 3, [V] * 3, np.stack([qkv] * 3), maxlen + 640, gq)
     assert np.isfinite(one).all() and np.abs(one).max() < 900
     for b in range(10):
         assert np.array_equal(ten[b], one[0]), f"column {b}: {np.mean(ten[b] != one[0]):.4f} of the values differ"
     for b in range(3):
         assert np.array_equal(large[b], one[0]), f"larger cache, column {b}: {np.mean(large[b] != one[0]):.4f} of the values differ"
+
+
+def chains(terms, n=32):
+    """Sum over the last axis in fp32: chains of n terms (each step rounded once), their results added one by one."""
+    out = None
+    for c in range(0, terms.shape[-1], n):
+        acc = np.zeros(terms.shape[:-1], np.float32)
+        for i in range(c, min(c + n, terms.shape[-1])):
+            acc = (acc.astype(np.float64) + terms[..., i]).astype(np.float32)
+        out = acc if out is None else (out + acc).astype(np.float32)
+    return out
+
+
+@pytest.mark.parametrize("seq,NH,NKV,gq", [(1030, 8, 1, 8), (334, 12, 2, 1), (2100, 8, 2, 4)])
+def test_partials_are_as_exact_as_fp32_chains(seq, NH, NKV, gq):
+    """What the tasks publish, put together in 64 bits, against attention in 64 bits: no further off than fp32 arithmetic in chains of 32 terms (scores over 32
+    dims, outputs over 32 positions), which is what the products ran in before they went to the tensor cores.  The rounding of the result to
+    bf16 hides all of it, so the partials are looked at."""
+    G, got, plain = NH // NKV, [], []
+    for seed in range(3):
+        rng = np.random.default_rng(100 * seed + seq)
+        K, V, qkv = (O.bfr(rng.standard_normal(s, dtype=np.float32)) for s in ((seq, NKV, HD), (seq, NKV, HD), (NH + 2 * NKV, HD)))
+        cos, sin = O.rope_tables(1e6, HD, seq)
+        q = np.stack([O.apply_rope(h, cos[-1], sin[-1]) for h in qkv[:NH]])
+        _, _, tmp = run(NH, NKV, [K], [V], qkv[None], -(-seq // 128) * 128, gq)
+        K[-1], V[-1] = np.stack([O.apply_rope(h, cos[-1], sin[-1]) for h in qkv[NH:NH + NKV]]), qkv[NH + NKV:]
+        for h in range(NH):
+            k, v = K[:, h // G].astype(np.float64), V[:, h // G].astype(np.float64)
+            s = k @ q[h].astype(np.float64) * SCALE
+            p = np.exp(s - s.max())
+            want = p @ v / p.sum()
+            pr = tmp[0, h].astype(np.float64)
+            w = np.exp(pr[:, HD] - pr[:, HD].max())
+            got.append((w @ pr[:, :HD] / (w @ pr[:, HD + 1]) - want) / np.linalg.norm(want))
+            sf = chains(k * q[h].astype(np.float64)) * np.float32(SCALE)
+            o, l, m = [], [], []
+            for a in range(0, seq, 128):
+                sp = sf[a:a + 128]
+                pf = np.exp(sp - sp.max()).astype(np.float32)
+                o.append(chains((pf[:, None].astype(np.float64) * v[a:a + 128]).T)); l.append(pf.astype(np.float64).sum()); m.append(sp.max())
+            w = np.exp(np.float64(m) - np.max(m))
+            plain.append((w @ np.float64(o) / (w @ l) - want) / np.linalg.norm(want))
+    got, plain = np.sqrt(np.mean(np.square(got)) * HD), np.sqrt(np.mean(np.square(plain)) * HD)
+    print(f"{seq} positions, gq {gq}: {got:.3e}, fp32 chains {plain:.3e}")
+    assert got <= plain

@@ -9,7 +9,8 @@
 //     ldmatrix), its own running maximum and sum, the probabilities transposed by movmatrix into the second product's operand, 128
 //     output sums per head in its registers.  No barrier between units; the warps' results meet once, at the end.
 //   * the probabilities go into the product as a bf16 value, the bf16 of what that rounding lost and that of what the second one lost: the
-//     24 bits of their fp32 value, as they were multiplied before.  Whole contexts: the first two (2^-17 of the value), as before too.
+//     24 bits of their fp32 value, as they were multiplied before.  Whole contexts: the first two (2^-17 of the value), as before too, but
+//     all three for the unit of the new position, whose probability was multiplied in fp32.
 //     Sums meet in fp32, so that the partials are no further from 64-bit ones than plain fp32 chains of 32 terms leave them: 1.3e-7 at 1038
 //     and 8151 positions against 1.6e-7 (summed up inside the products 1.8e-7).
 // Bound by the stream of K / V at long contexts, by the chain q rows -> norm -> scores -> publish -> merge at short ones.
@@ -411,7 +412,8 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
         const uint32_t h0 = movmatrix(pack_bf(c[0], c[1])), h1 = movmatrix(pack_bf(c[2], c[3]));
         const uint32_t w0 = movmatrix(pack_bf(r[0], r[1])), w1 = movmatrix(pack_bf(r[2], r[3]));
         uint32_t x0 = 0u, x1 = 0u;
-        if (!t.whole) {                                            // what the second rounding lost
+        const bool third = !t.whole || ragged;
+        if (third) {                                               // what the second rounding lost
 #pragma unroll
           for (int j = 0; j < 4; ++j) r[j] = __fsub_rn(r[j], bfr(r[j]));
           x0 = movmatrix(pack_bf(r[0], r[1])); x1 = movmatrix(pack_bf(r[2], r[3]));
@@ -427,7 +429,7 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
 #pragma unroll
             for (int e = 0; e < 4; ++e) lo[u][e] = hi[u][e] = 0.f;
           }
-          if (!t.whole)
+          if (third)
 #pragma unroll
             for (int u = 0; u < 2; ++u) mma16816(lo[u], a[u], x0, x1);
 #pragma unroll

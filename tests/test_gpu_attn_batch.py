@@ -127,3 +127,26 @@ def test_partials_are_as_exact_as_fp32_chains(seq, NH, NKV, gq):
     got, plain = np.sqrt(np.mean(np.square(got)) * HD), np.sqrt(np.mean(np.square(plain)) * HD)
     print(f"{seq} positions, gq {gq}: {got:.3e}, fp32 chains {plain:.3e}")
     assert got <= plain
+
+
+@pytest.mark.parametrize("whole", [True, False])
+def test_the_new_position_keeps_all_bits_of_its_probability(whole):
+    """Two cached positions of probability 1 take away the first two bf16 parts of the new position's, so what is left of the sum is its third part (2^-18
+    of it and less): 0 if that part were not multiplied.  A difference of two units in the last place of exp() is 2^-5 of what is left."""
+    NH, gq = 8, 8
+    d = np.arange(1, 4096, dtype=np.float32) / np.float32(1024)                          # bf16-exact differences of the scores, the third parts largest
+    d = d[O.bfr(d) == d]
+    p = np.exp(-d.astype(np.float64)).astype(np.float32)
+    first = O.bfr(p)
+    second = O.bfr(p - first)
+    third = p - first - second
+    best = np.argsort(-np.abs(third) / p)[:NH]
+    d, first, second, third, p = (x[best].astype(np.float64) for x in (d, first, second, third, p))
+    assert np.all(np.abs(third) / p > 2.0 ** -19)
+    K, V, qkv = np.zeros((3, 1, HD), np.float32), np.zeros((3, 1, HD), np.float32), np.zeros((NH + 2, HD), np.float32)
+    K[:2, 0, 0], qkv[:NH, 0] = 1.0, d                                                    # score of a cached position: d of the head, of the new one: 0
+    V[0, 0, :NH], V[1, 0, :NH], qkv[NH + 1, :NH] = -first, -second, 1.0
+    out, _, _ = run(NH, 1, [K], [V], qkv[None], 128, gq, whole=whole, scale=1.0, rotary=False)
+    want = third / (2.0 + p)
+    got = out[0, np.arange(NH), np.arange(NH)]
+    assert np.all(np.abs(got - want) <= 2.0 ** -4 * np.abs(want)), (got, want)

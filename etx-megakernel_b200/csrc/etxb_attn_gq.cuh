@@ -439,7 +439,11 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
 #pragma unroll
           for (int u = 0; u < 2; ++u)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[j + u][e] = __fadd_rn(acc[j + u][e], __fadd_rn(hi[u][e], lo[u][e]));
+            for (int e = 0; e < 4; ++e) {
+              // (an infinite V: its product with a small part is NaN where the part is 0 or has another sign than the probability)
+              const float v = fabsf(hi[u][e]) < INFINITY ? __fadd_rn(hi[u][e], lo[u][e]) : hi[u][e];
+              acc[j + u][e] = __fadd_rn(acc[j + u][e], v);
+            }
         }
         if (ragged) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // (this warp's writes, before the next copy into the place)
         __syncwarp();

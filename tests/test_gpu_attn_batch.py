@@ -150,3 +150,28 @@ def test_the_new_position_keeps_all_bits_of_its_probability(whole):
     want = third / (2.0 + p)
     got = out[0, np.arange(NH), np.arange(NH)]
     assert np.all(np.abs(got - want) <= 2.0 ** -4 * np.abs(want)), (got, want)
+
+
+@pytest.mark.parametrize("seq,NH,NKV,gq,whole", [(300, 8, 2, 4, False), (40, 8, 1, 8, False), (300, 8, 2, 4, True)])
+def test_infinite_values_in_the_cache_stay_infinite(seq, NH, NKV, gq, whole):
+    """V rows that overflowed bf16: the sum of an infinite value and finite ones is that value, in its dim alone; values of both signs give NaN.  A key row of
+    minus infinity (against positive q values) takes its position out."""
+    rng = np.random.default_rng(seq)
+    K, V, qkv = (O.bfr(rng.standard_normal(s, dtype=np.float32)) for s in ((seq, NKV, HD), (seq, NKV, HD), (NH + 2 * NKV, HD)))
+    qkv = np.abs(qkv)
+    K[5, :, 7] = -np.inf
+    V[5], V[3, :, 10], V[seq // 2, :, 11] = 3.0, np.inf, -np.inf
+    V[2, :, 12], V[9, :, 12] = np.inf, -np.inf
+    qkv[NH + NKV:, 13] = np.inf                                                           # the new position's own row
+    out, _, _ = run(NH, NKV, [K], [V], qkv[None], -(-seq // 128) * 128, gq, whole=whole, rotary=False)
+    K[-1], V[-1] = qkv[NH:NH + NKV], qkv[NH + NKV:]
+    for h in range(NH):
+        k, v = K[:, h * NKV // NH].astype(np.float64), V[:, h * NKV // NH].astype(np.float64)
+        s = k @ qkv[h].astype(np.float64) * SCALE
+        assert s[5] == -np.inf
+        p = np.exp(s - s.max())
+        want = np.where(p[:, None] > 0, p[:, None] * v, 0.0).sum(0) / p.sum()
+        fin = np.isfinite(want)
+        assert np.array_equal(np.flatnonzero(~fin), [10, 11, 12, 13])
+        assert np.array_equal(out[0, h, ~fin], want[~fin].astype(np.float32), equal_nan=True), out[0, h, ~fin]
+        assert np.all(np.abs(out[0, h, fin] - want[fin]) <= 2.0 ** -8 * np.abs(want[fin]) + np.abs(want[fin]).max() * 2.0 ** -13)

@@ -346,18 +346,29 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
         if (ragged) {
           const int rn = t.owner && t.pos >= p0 && t.pos < p0 + 16 ? (int)t.pos - p0 : -1;
           if (rn >= 0) *(uint2*)(unit + ((lane >> 1) * 16 + rn) * 16 + 8 * (lane & 1)) = *(const uint2*)(s.knew + 4 * lane);
-          const int nv = max(0, min(16, t.seq - p0));              // cached positions
-#pragma unroll 1
-          for (int j = lane; j < 128 * 8; j += 32) {               // pairs of positions: dim j / 8, positions 2 (j % 8) ..
-            const int pa = 2 * (j & 7);
-            uint32_t* w = (uint32_t*)(unit + 4096) + j;
-            const uint32_t vn = ((const unsigned short*)s.vnew)[j >> 3];
-            uint32_t v = *w;
-            if (pa >= nv) v &= 0xffff0000u;
-            if (pa + 1 >= nv) v &= 0xffffu;
-            if (pa == rn) v = (v & 0xffff0000u) | vn;
-            if (pa + 1 == rn) v = (v & 0xffffu) | vn << 16;
-            *w = v;
+          const int nv = max(0, min(16, t.seq - p0));              // positions of the context
+          // Every 32nd piece of 16 bytes is the lane's: eight positions of one dim, the same eight for all its pieces.  (As 32 words a lane, one read,
+          // change and write behind the other, the new position's task came 1.1 us after all others: a phase of a small dense model at
+          // 200 positions, one q head a task, 8.0 us -> 7.4.)
+          uint32_t keep[4], put[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int p = 8 * (lane & 1) + 2 * q;
+            put[q] = (p == rn ? 0xffffu : 0u) | (p + 1 == rn ? 0xffff0000u : 0u);
+            keep[q] = ((p < nv ? 0xffffu : 0u) | (p + 1 < nv ? 0xffff0000u : 0u)) & ~put[q];
+          }
+          uint4* vp = (uint4*)(unit + 4096) + lane;
+          const unsigned short* vn = (const unsigned short*)s.vnew + (lane >> 1);
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            uint4 v[2];
+            uint32_t x[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) { v[u] = vp[32 * (j + u)]; x[u] = vn[16 * (j + u)]; x[u] |= x[u] << 16; }
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+              vp[32 * (j + u)] = make_uint4((v[u].x & keep[0]) | (x[u] & put[0]), (v[u].y & keep[1]) | (x[u] & put[1]),
+                                            (v[u].z & keep[2]) | (x[u] & put[2]), (v[u].w & keep[3]) | (x[u] & put[3]));
           }
           __syncwarp();
         }

@@ -298,7 +298,7 @@ __device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, c
 #pragma unroll
       for (int u = 0; u < 16; ++u) acc[u] = __fmul_rn(acc[u], g);
     }
-    const float e = expf(__fsub_rn(sc, m));
+    const float e = expf(__fsub_rn(sc, m == -INFINITY ? 0.f : m)); // (a first row of score -inf: probability 0)
     l = __fadd_rn(l, e);
 #pragma unroll
     for (int u = 0; u < 16; ++u) acc[u] = __fmaf_rn(e, f[u], acc[u]);

@@ -328,12 +328,19 @@ __device__ __forceinline__ bool producer_wait(const etxb_params& p, const Smem& 
   return __shfl_sync(0xffffffffu, good, 0) != 0;
 }
 
+// .. until every task of the queue before `cur` is over; false when the step is being abandoned.
+__device__ __forceinline__ bool queue_done(const Smem& sm, int cur) {
+  int good = 1;
+  if ((tidx() & 31) == 0) good = wait_done(sm, cur) ? 1 : 0;
+  return __shfl_sync(0xffffffffu, good, 0) != 0;
+}
+
 // The producer warp: walks the same queue ahead of the consumers and streams the weight rows of every GEMV-family
 // task into the ring.  It waits only for what the weight ADDRESSES depend on (nothing for static weights, the router's
 // event for expert weights), never for the task's activations.
 // Attention tasks: the K / V units of their positions (GQ: grouped), W_UK and the cached rows (MLA: latent attention).  In a kernel whose
 // other tiles use the ring's memory as their own (TC: the tensor-core tiles) the copies wait until every task before this one is over;
-// they still run ahead of the task's events.
+// they still run ahead of the task's events.  The same for weights in a plan that has such tiles (none of the bundled ones mixes them).
 template <bool LEAN, bool SH, bool GEMV, bool GQ, bool MLA, bool TC>
 __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& sm, int q0, int q1) {
   uint32_t n = 0;
@@ -350,11 +357,7 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
         __syncwarp();
         if (body == 12 && aa->gq <= 0) continue;
         if (TC && body == 20 && ((const etxb_gemv_args*)aa)->tpe <= 1) continue;
-        if constexpr (TC) {
-          int good = 1;
-          if (lane == 0) good = wait_done(sm, cur) ? 1 : 0;
-          if (__shfl_sync(0xffffffffu, good, 0) == 0) break;
-        }
+        if constexpr (TC) { if (!queue_done(sm, cur)) break; }
         if constexpr (TC) {
           if (body == 20) {                                        // (static weights)
             if (ld_relaxed(p.ctrl) != 0) break;
@@ -378,6 +381,7 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
     gg.t = gemv_task(body, *pa, t->c0);
     gemv_geom(body, gg);
     const GemvTask gt = gg.t;
+    if constexpr (TC) { if (p.tc_on != 0u && !queue_done(sm, cur)) break; }
     if (!producer_wait(p, sm, t, cur)) break;
     if (gt.n > 0 && body != 3) gemv_routing<LEAN, SH>(*pa, sm.prod, nullptr);    // (the ids alone: the stream waits for them)
     ok = produce_task<SH>(body, *pa, gt, gg.rps, sm.prod, n, sm, cur, p.trace ? p.trace + 8 * (size_t)t->id : nullptr);

@@ -634,19 +634,43 @@ static int32_t build_tensor_maps(etxb_session* s) {
   return ETXB_OK;
 }
 
-// Grouped attention over partitions: who merges a group's partials (attn_gq_tile).  Where every worker's queue holds the tasks of a grid
-// in ascending order, the workers' last tasks of that grid share the merge of each group between them; otherwise (and in single-tile
-// launches) the record says nothing and the task of the last partition does it.  Written into the record's `mirror` word, which
-// attention tasks have no other use for.
+// Grids whose last tasks on each worker may wait for all other tasks of the grid (a merge shared between them): 1 per such type.  The wait is none
+// of the plan's events, so it must not close a circle with them.  It cannot where every queue is in ascending task order and no task waits for
+// an event that a later one arrives on -- all that a task waits for has a lower number then -- and the grid's tasks are consecutive numbers
+// that wait for none of the grid: before the first of them nothing waits for the grid, and what the others still need is done without it.
+static std::vector<char> waiting_grids(const etxb_session* s) {
+  const size_t N = s->tasks.size(), T = s->types.size();
+  std::vector<char> ok(T, 0);
+  for (uint32_t w = 0; w < s->h.n_workers; ++w)
+    for (int32_t i = s->qbegin[w] + 1; i < s->qbegin[w + 1]; ++i)
+      if (s->tasks[i].id < s->tasks[i - 1].id) return ok;
+  std::vector<int> arrives(s->h.n_events, -1), lo(T, (int)N), hi(T, -1), count(T, 0);   // latest task that arrives on an event; the grids' numbers
+  for (const etxb_task& t : s->tasks) {
+    for (int k = 0; k < t.out_n; ++k) arrives[s->outwords[t.out_off + k]] = std::max(arrives[s->outwords[t.out_off + k]], t.id);
+    lo[t.type] = std::min(lo[t.type], t.id); hi[t.type] = std::max(hi[t.type], t.id); ++count[t.type];
+  }
+  for (size_t y = 0; y < T; ++y) ok[y] = s->types[y].body == ETXB_BODY_ATTN_FUSED && hi[y] - lo[y] + 1 == count[y];
+  for (const etxb_task& t : s->tasks)
+    for (int k = 0; k < t.in_n; ++k) {
+      const int a = arrives[s->inwords[t.in_off + k]];
+      if (a >= t.id) return std::vector<char>(T, 0);
+      if (a >= lo[t.type]) ok[t.type] = 0;
+    }
+  return ok;
+}
+
+// Grouped attention over partitions: who merges a group's partials (attn_gq_tile).  Where they may wait (above), the workers' last tasks of a grid
+// share the merge of each group between them; otherwise (and in single-tile launches) the record says nothing and the task of the last
+// partition does it.  Written into the record's `mirror` word, which attention tasks have no other use for.
 static void share_merges(const etxb_session* s, std::vector<etxb_rec>& recs) {
-  std::vector<char> ascending(s->types.size(), 1);
+  const std::vector<char> waits = waiting_grids(s);
   std::vector<int> last(recs.size(), 0);
   for (uint32_t w = 0; w < s->h.n_workers; ++w) {
     std::vector<int> at(s->types.size(), -1);                      // the worker's latest task of each type
     for (int32_t i = s->qbegin[w]; i < s->qbegin[w + 1]; ++i) {
       const int ty = s->tasks[i].type;
-      if (s->types[ty].body != ETXB_BODY_ATTN_FUSED) continue;
-      if (at[ty] >= 0) { last[at[ty]] = 0; if (s->tasks[at[ty]].id > s->tasks[i].id) ascending[ty] = 0; }
+      if (!waits[ty]) continue;
+      if (at[ty] >= 0) last[at[ty]] = 0;
       at[ty] = i; last[i] = 1;
     }
   }
@@ -654,7 +678,7 @@ static void share_merges(const etxb_session* s, std::vector<etxb_rec>& recs) {
   for (size_t i = 0; i < recs.size(); ++i) {
     const etxb_task& t = s->tasks[i];
     const etxb_type& ty = s->types[t.type];
-    if (ty.body != ETXB_BODY_ATTN_FUSED || !ascending[t.type] || ty.args[0] != 0 || ty.cst[0] < 0 || ty.cst[1] < 0) continue;
+    if (!waits[t.type] || ty.args[0] != 0 || ty.cst[0] < 0 || ty.cst[1] < 0) continue;
     const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
     etxb_attnf_args a;
     if (off < 0 || (uint64_t)off + sizeof a > s->h_pool.size()) continue;

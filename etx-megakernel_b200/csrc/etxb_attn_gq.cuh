@@ -279,9 +279,8 @@ __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Sm
 
 // One task.  n: the running stage count of the ring.  mg: how the merge of a context in partitions is shared out -- 0: the task of the
 // last partition merges the group (it comes last in the queues, and a task that waits only for tasks of lower index cannot be part of
-// a circle); else count << 16 | index + 1: the host has found that every worker's queue holds the grid in ascending order, so the
-// workers' LAST tasks of the grid may wait for all the others (whatever stands before them in a queue waits for nobody), and this is
-// one of `count` such tasks of the group, each of which merges a share; 0xffff: it is not one of them, others are.  Shared out from
+// a circle); else count << 16 | index + 1: the host has found that the workers' LAST tasks of the grid may wait for all the others (the order of the
+// queues and the events leave no circle: waiting_grids), and this is one of `count` such tasks of the group, each of which merges a share; 0xffff: it is not one of them, others are.  Shared out from
 // gq * np = ETXB_GQ_SHARE on only: with few partials the last partition's task alone is as quick, and the other tasks are done.
 __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S, uint32_t& n, uint32_t mg) {
   constexpr int HD = 128, BS = 16;

@@ -20,10 +20,11 @@ from tests.test_gpu_ops import dev_bf16, host  # noqa: E402
 DEV, HD, SCALE = "cuda:0", 128, float(np.float32(1.0 / np.sqrt(128)))
 
 
-def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True):
+def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True, behind=None):
     """One attention grid over B sequences.  K, V: per sequence [seq][NKV][HD], the last position being the new one (its cache row holds NaN and comes from qkv
     [B][NH + 2 NKV][HD] instead).  Returns (out [B][NH][HD] bf16 values, the cached k rows at the new positions [B][NKV][HD], the partials
-    [B][NH][partitions][128 sums, maximum, sum of the probabilities])."""
+    [B][NH][partitions][128 sums, maximum, sum of the probabilities]).  behind: a second grid of one empty task that waits for the first attention task
+    alone, and the queues of the plan as a function of the attention tasks' and its number."""
     B, nblk, parts = len(K), maxlen // 16, -(-maxlen // 128)
     pools = []
     for b in range(B):
@@ -48,9 +49,19 @@ def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True):
                                          eps=1e-6, NH=NH, NKV=NKV, HD=HD, BS=16, X=8, max_parts=parts, gq=gq, part_len=ops.attn.tagged_part_len(3, whole)) for b in range(B))
     g = Graph("attn")
     g.tensor("impargs", (len(blobs),), role="weight", bytes_per_elem=1)
-    g.etensor("E_done", (1,), wait_count=ntask * B)
-    g.call_device("attn", (ntask, B), cuda_link("", "etx_tile_attn_fused"), args=["impargs"], consts=(0, ops.attn.F_ARG_BYTES), out_edges={"E_done": "ij->(0)"})
-    s = Session(compile_graph(g, "b200", {}), {}, blobs, 0)
+    if behind is None:
+        g.etensor("E_done", (1,), wait_count=ntask * B)
+        g.call_device("attn", (ntask, B), cuda_link("", "etx_tile_attn_fused"), args=["impargs"], consts=(0, ops.attn.F_ARG_BYTES), out_edges={"E_done": "ij->(0)"})
+    else:
+        g.etensor("E_done", (ntask, B), wait_count=1)
+        g.etensor("E_empty", (1,), wait_count=1)
+        g.call_device("attn", (ntask, B), cuda_link("", "etx_tile_attn_fused"), args=["impargs"], consts=(0, ops.attn.F_ARG_BYTES), out_edges={"E_done": "ij->ij"})
+        g.call_device("empty", (1,), cuda_link("", "nop"), args=["impargs"], consts=(0, 0), in_edges={"E_done": "i->(0)(0)"}, out_edges={"E_empty": "i->(0)"})
+    plan = compile_graph(g, "b200", {})
+    if behind is not None:
+        queues = behind([i for i, t in enumerate(plan.tasks) if t.grid == "attn"], [i for i, t in enumerate(plan.tasks) if t.grid == "empty"][0])
+        plan.static_queues = {(0, w): queues[w] if w < len(queues) else [] for w in range(plan.workers_per_device())}
+    s = Session(plan, {}, blobs, 0)
     outs = []
     for _ in range(2):
         t["out"].zero_()
@@ -82,6 +93,16 @@ def test_equal_columns_get_equal_bits_wherever_they_stand(seq, gq):
         assert np.array_equal(ten[b], one[0]), f"column {b}: {np.mean(ten[b] != one[0]):.4f} of the values differ"
     for b in range(3):
         assert np.array_equal(large[b], one[0]), f"larger cache, column {b}: {np.mean(large[b] != one[0]):.4f} of the values differ"
+
+
+def test_a_merge_waits_for_nothing_that_waits_for_its_task():
+    """Eight partitions of one group, 64 partials.  The first worker has the first attention task alone; the second one an empty task that waits for it, then the other
+    attention tasks.  If the first task, the last of its worker, waited for the others' partials, they would wait for it too."""
+    rng = np.random.default_rng(3)
+    K, V, qkv = (O.bfr(rng.standard_normal(s, dtype=np.float32)) for s in ((1000, 1, HD), (1000, 1, HD), (10, HD)))
+    want, _, _ = run(8, 1, [K], [V], qkv[None], 1024, 8)
+    got, _, _ = run(8, 1, [K], [V], qkv[None], 1024, 8, behind=lambda attn, empty: [attn[:1], [empty] + attn[1:]])
+    assert np.array_equal(got, want)
 
 
 def chains(terms, n=32):

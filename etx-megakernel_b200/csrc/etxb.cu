@@ -9,11 +9,10 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <chrono>
 #include <string>
 #include <thread>
-#include <array>
-#include <map>
 #include <vector>
 
 #include "../../include/etxb200.h"
@@ -73,6 +72,7 @@ struct etxb_session {
   unsigned char* xbase = nullptr; size_t xbytes = 0;
   unsigned char* xpeer[ETXB_MAX_PEERS] = {};
   uint32_t xargmax = 0;                // byte offset of the sharded argmax block in a region (0: the lm_head is whole on every rank)
+  std::vector<uint32_t> merge;         // per task: its share in the merge of a group's partials (share_merges)
   bool has_exchange = false;           // the plan is one rank's step of a sharded model (some grid is marked exchanged)
   bool tc_on = false;                  // the plan has tensor-core tiles (tcgen05): the kernel allocates tensor memory
   void* d_maps = nullptr;              // their TMA tensor maps, one per grid (128 bytes each)
@@ -324,6 +324,78 @@ extern "C" int32_t etxb_device_info(int device, etxb_device_info_t* out) {
   return ETXB_OK;
 }
 
+// Grids whose last tasks on each worker may wait for all other tasks of the grid (a merge shared between them): 1 per such type.  The wait is none
+// of the plan's events, so it must not close a circle with them.  It cannot where every queue is in ascending task order and no task waits for
+// an event that a later one arrives on -- all that a task waits for has a lower number then -- and the grid's tasks are consecutive numbers
+// that wait for none of the grid: before the first of them nothing waits for the grid, and what the others still need is done without it.
+static std::vector<char> waiting_grids(const etxb_session* s) {
+  const size_t N = s->tasks.size(), T = s->types.size();
+  std::vector<char> ok(T, 0);
+  for (uint32_t w = 0; w < s->h.n_workers; ++w)
+    for (int32_t i = s->qbegin[w] + 1; i < s->qbegin[w + 1]; ++i)
+      if (s->tasks[i].id < s->tasks[i - 1].id) return ok;
+  std::vector<int> arrives(s->h.n_events, -1), lo(T, (int)N), hi(T, -1), count(T, 0);   // latest task that arrives on an event; the grids' numbers
+  for (const etxb_task& t : s->tasks) {
+    for (int k = 0; k < t.out_n; ++k) arrives[s->outwords[t.out_off + k]] = std::max(arrives[s->outwords[t.out_off + k]], t.id);
+    lo[t.type] = std::min(lo[t.type], t.id); hi[t.type] = std::max(hi[t.type], t.id); ++count[t.type];
+  }
+  for (size_t y = 0; y < T; ++y) ok[y] = s->types[y].body == ETXB_BODY_ATTN_FUSED && hi[y] - lo[y] + 1 == count[y];
+  for (const etxb_task& t : s->tasks)
+    for (int k = 0; k < t.in_n; ++k) {
+      const int a = arrives[s->inwords[t.in_off + k]];
+      if (a >= t.id) return std::vector<char>(T, 0);
+      if (a >= lo[t.type]) ok[t.type] = 0;
+    }
+  return ok;
+}
+
+// Grouped attention over partitions: who merges a group's partials (attn_gq_tile).  Where they may wait (above), the workers' last tasks of a grid
+// share the merge of each group between them; otherwise (and in single-tile launches) the record says nothing and the task of the last
+// partition does it.  Goes into the record's `mirror` word, which attention tasks have no other use for.  Worked out once, when the session is
+// created: it depends on the queues and the argument pool alone.
+static void share_merges(etxb_session* s) {
+  const size_t N = s->tasks.size(), T = s->types.size();
+  s->merge.assign(N, 0u);
+  const std::vector<char> waits = waiting_grids(s);
+  if (std::find(waits.begin(), waits.end(), 1) == waits.end()) return;
+  // groups in a row: per type its sequences (second coordinates), per sequence its NH / gq groups
+  struct Seq { int first, groups, tasks; };
+  std::vector<std::vector<Seq>> seqs(T);
+  int n = 0;
+  for (const etxb_task& t : s->tasks) {
+    const etxb_type& ty = s->types[t.type];
+    if (!waits[t.type] || ty.args[0] != 0 || ty.cst[0] < 0 || ty.cst[1] < 0 || t.coord[1] < 0 || (size_t)t.coord[1] >= N) continue;
+    std::vector<Seq>& q = seqs[t.type];
+    if ((size_t)t.coord[1] < q.size() && q[t.coord[1]].first >= 0) continue;
+    if (q.size() <= (size_t)t.coord[1]) q.resize((size_t)t.coord[1] + 1, Seq{-1, 0, 0});
+    Seq& k = q[t.coord[1]];
+    k.first = n;
+    const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
+    etxb_attnf_args a;
+    if (off < 0 || (uint64_t)off + sizeof a > s->h_pool.size()) continue;
+    memcpy(&a, s->h_pool.data() + off, sizeof a);
+    if (a.gq <= 0 || a.gq > a.NH || a.NH > (1 << 16) || (a.part_len & ETXB_GQ_WHOLE)) continue;
+    k.groups = a.NH / a.gq; k.tasks = (int)std::min<uint32_t>(a.nblocks, 1u << 30);
+    n += k.groups;
+  }
+  std::vector<int> group(N, -1), at(T, -1);
+  std::vector<char> last(N, 0);
+  std::vector<uint32_t> count((size_t)n, 0u), next((size_t)n, 0u);
+  for (uint32_t w = 0; w < s->h.n_workers; ++w)
+    for (int32_t i = s->qbegin[w + 1] - 1; i >= s->qbegin[w]; --i) {   // (from the queue's end: the first of a type is its last)
+      const etxb_task& t = s->tasks[i];
+      if (!waits[t.type]) continue;
+      last[i] = at[t.type] != (int)w; at[t.type] = (int)w;
+      if (t.coord[1] < 0 || (size_t)t.coord[1] >= seqs[t.type].size()) continue;
+      const Seq& k = seqs[t.type][t.coord[1]];
+      if (k.groups == 0 || t.coord[0] < 0 || t.coord[0] >= k.tasks) continue;
+      group[i] = k.first + t.coord[0] % k.groups;
+      count[group[i]] += (uint32_t)last[i];
+    }
+  for (size_t i = 0; i < N; ++i)
+    if (group[i] >= 0 && count[group[i]] > 0) s->merge[i] = last[i] ? (count[group[i]] << 16 | ++next[group[i]]) : 0xffffu;
+}
+
 // ---- plan blob ------------------------------------------------------------------------------------------------
 static size_t al8(size_t x) { return (x + 7) & ~size_t(7); }
 
@@ -401,6 +473,7 @@ static int32_t parse_plan(etxb_session* s, const unsigned char* b, size_t n) {
   CU(up((void**)&s->d_outwords, s->outwords.data(), h.n_out * 4));
   s->variant = select_variant(s, pool);
   s->h_pool = pool;
+  share_merges(s);
   for (const etxb_type& ty : s->types) s->has_exchange = s->has_exchange || ty.exchange != 0;
   pool.resize(pool.size() + 256, 0);                               // the context prefetch reads 192 bytes from a block start
   CU(up((void**)&s->d_pool, pool.data(), pool.size()));
@@ -634,66 +707,6 @@ static int32_t build_tensor_maps(etxb_session* s) {
   return ETXB_OK;
 }
 
-// Grids whose last tasks on each worker may wait for all other tasks of the grid (a merge shared between them): 1 per such type.  The wait is none
-// of the plan's events, so it must not close a circle with them.  It cannot where every queue is in ascending task order and no task waits for
-// an event that a later one arrives on -- all that a task waits for has a lower number then -- and the grid's tasks are consecutive numbers
-// that wait for none of the grid: before the first of them nothing waits for the grid, and what the others still need is done without it.
-static std::vector<char> waiting_grids(const etxb_session* s) {
-  const size_t N = s->tasks.size(), T = s->types.size();
-  std::vector<char> ok(T, 0);
-  for (uint32_t w = 0; w < s->h.n_workers; ++w)
-    for (int32_t i = s->qbegin[w] + 1; i < s->qbegin[w + 1]; ++i)
-      if (s->tasks[i].id < s->tasks[i - 1].id) return ok;
-  std::vector<int> arrives(s->h.n_events, -1), lo(T, (int)N), hi(T, -1), count(T, 0);   // latest task that arrives on an event; the grids' numbers
-  for (const etxb_task& t : s->tasks) {
-    for (int k = 0; k < t.out_n; ++k) arrives[s->outwords[t.out_off + k]] = std::max(arrives[s->outwords[t.out_off + k]], t.id);
-    lo[t.type] = std::min(lo[t.type], t.id); hi[t.type] = std::max(hi[t.type], t.id); ++count[t.type];
-  }
-  for (size_t y = 0; y < T; ++y) ok[y] = s->types[y].body == ETXB_BODY_ATTN_FUSED && hi[y] - lo[y] + 1 == count[y];
-  for (const etxb_task& t : s->tasks)
-    for (int k = 0; k < t.in_n; ++k) {
-      const int a = arrives[s->inwords[t.in_off + k]];
-      if (a >= t.id) return std::vector<char>(T, 0);
-      if (a >= lo[t.type]) ok[t.type] = 0;
-    }
-  return ok;
-}
-
-// Grouped attention over partitions: who merges a group's partials (attn_gq_tile).  Where they may wait (above), the workers' last tasks of a grid
-// share the merge of each group between them; otherwise (and in single-tile launches) the record says nothing and the task of the last
-// partition does it.  Written into the record's `mirror` word, which attention tasks have no other use for.
-static void share_merges(const etxb_session* s, std::vector<etxb_rec>& recs) {
-  const std::vector<char> waits = waiting_grids(s);
-  std::vector<int> last(recs.size(), 0);
-  for (uint32_t w = 0; w < s->h.n_workers; ++w) {
-    std::vector<int> at(s->types.size(), -1);                      // the worker's latest task of each type
-    for (int32_t i = s->qbegin[w]; i < s->qbegin[w + 1]; ++i) {
-      const int ty = s->tasks[i].type;
-      if (!waits[ty]) continue;
-      if (at[ty] >= 0) last[at[ty]] = 0;
-      at[ty] = i; last[i] = 1;
-    }
-  }
-  std::map<std::array<int, 3>, std::vector<int>> groups;           // (type, sequence, q group) -> its tasks
-  for (size_t i = 0; i < recs.size(); ++i) {
-    const etxb_task& t = s->tasks[i];
-    const etxb_type& ty = s->types[t.type];
-    if (!waits[t.type] || ty.args[0] != 0 || ty.cst[0] < 0 || ty.cst[1] < 0) continue;
-    const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
-    etxb_attnf_args a;
-    if (off < 0 || (uint64_t)off + sizeof a > s->h_pool.size()) continue;
-    memcpy(&a, s->h_pool.data() + off, sizeof a);
-    if (a.gq <= 0 || a.gq > a.NH || (a.part_len & ETXB_GQ_WHOLE) || t.coord[0] < 0 || t.coord[0] >= (int)a.nblocks) continue;
-    groups[{t.type, t.coord[1], t.coord[0] % (a.NH / a.gq)}].push_back((int)i);
-  }
-  for (auto& g : groups) {
-    uint32_t count = 0, k = 0;
-    for (int i : g.second) count += last[i];
-    if (count == 0) continue;
-    for (int i : g.second) recs[i].mirror = last[i] ? (count << 16 | ++k) : 0xffffu;
-  }
-}
-
 static int32_t upload_type_args(etxb_session* s) {
   std::vector<void*> ta((size_t)s->h.n_types * ETXB_MAX_ARGS, nullptr);
   for (size_t t = 0; t < s->types.size(); ++t)
@@ -734,12 +747,12 @@ static int32_t upload_type_args(etxb_session* s) {
     r.args = has_block ? (uint64_t)(uintptr_t)ta[(size_t)t.type * ETXB_MAX_ARGS] + (uint64_t)ty.cst[0] + (uint64_t)t.coord[1] * (uint64_t)ty.cst[1]
                        : (uint64_t)(uintptr_t)s->d_pool;
     r.stream_word = ty.stream_word;
+    r.mirror = s->merge[i];
     if (s->xbase != nullptr && ty.exchange) {
       int32_t rc = exchange_rows(s, ty, t, &r.mirror);
       if (rc) return rc;
     }
   }
-  share_merges(s, recs);
   if (!s->d_recs) CU(cudaMalloc((void**)&s->d_recs, recs.size() * sizeof(etxb_rec) + 96));
   CU(cudaMemcpy(s->d_recs, recs.data(), recs.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
   // the same records grouped by grid (type), worker by worker, for the one-launch-per-grid baseline

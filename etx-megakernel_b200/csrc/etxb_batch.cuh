@@ -253,9 +253,7 @@ __device__ __forceinline__ void tile_moe_down_g(const unsigned char* a, int blk,
 // ---------------------------------------------------------------------------------------------- per-column prologue
 // Columns of a batched step: token_in / token_out are [step][nb]; every column is at the step's position; column b owns
 // the cache slots [b * slot_span, (b + 1) * slot_span) of the shared block pool.
-// `zero`: optional, ETXB_SPLITK_COUNTERS int32 counters that column 0's prologue task clears (arrival counters of dense
-// grids whose tasks meet in partial sums; none of the present tiles do).
-#define ETXB_SPLITK_COUNTERS 768
+// `zero`: not read (it named counters that the first column's task cleared; no tile counts arrivals any more).
 struct etxb_batch_args { int32_t nb, slot_span; int32_t* zero; uint32_t grid[3], nblocks; };
 __device__ __forceinline__ void tile_prologue_nb(const unsigned char* a, int b, const etxb_stepv& S) {
   const etxb_batch_args& d = *(const etxb_batch_args*)a;
@@ -265,8 +263,6 @@ __device__ __forceinline__ void tile_prologue_nb(const unsigned char* a, int b, 
     if (S.token_time && b == 0) S.token_time[2 * t] = globaltimer();
     S.positions[b] = S.pos; S.seq_lens[b] = S.pos + 1; S.slot_mapping[b] = (long long)b * d.slot_span + S.pos;
   }
-  if (b == 0 && d.zero != nullptr)
-    for (int i = tidx(); i < ETXB_SPLITK_COUNTERS; i += ETXB_CONSUMERS) d.zero[i] = 0;
   const int id = __ldcg(S.token_in + (size_t)t * d.nb + b);
   const uint4* src = (const uint4*)((const __nv_bfloat16*)S.embed + (size_t)id * S.H);
   uint4* dst = (uint4*)((__nv_bfloat16*)S.resid + (size_t)b * S.H);

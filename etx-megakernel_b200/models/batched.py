@@ -34,7 +34,6 @@ from .qwen import BS, SRC, X, ArgPool
 
 _DT = {"bf16": torch.bfloat16, "f32": torch.float32, "i32": torch.int32, "i64": torch.int64}
 UP_ROWS, DOWN_ROWS = 256, 512      # mma.sync engine: rows of one expert a gate+up / down task covers (blocks of 128 inside the tile)
-SKP_FLOATS = 4 << 20               # fp32 partial sums of a split-K dense grid ([split][rows][B])
 
 
 def buffer_shapes(d: Q.Dims, B: int, maxlen: int, steps: int, parts: int) -> dict:
@@ -50,7 +49,7 @@ def buffer_shapes(d: Q.Dims, B: int, maxlen: int, steps: int, parts: int) -> dic
             "kc": ((d.L, B * nblk, d.NKV, d.HD // X, BS, X), "bf16"), "vc": ((d.L, B * nblk, d.NKV, d.HD, BS), "bf16"),
             "attn_counters": ((d.L, B, d.NH), "i32"), "rlog": ((B, d.E), "bf16"), "tw": ((B, d.TOPK), "f32"), "ti": ((B, d.TOPK), "i32"),
             "mc2": ((B, d.TOPK, d.MI), "bf16"), "mc3": ((B, d.TOPK, d.H), "bf16"), "ecount": ((d.E,), "i32"), "elist": ((d.E, B), "i32"), "active": ((d.L,), "i32"),
-            "skp": ((SKP_FLOATS,), "f32"), "skc": ((op_batch.SPLITK_COUNTERS,), "i32")}
+            "skp": ((32,), "f32"), "skc": ((32,), "i32")}                       # named by the blocks of shared row blocks, not read (ops/batch.py)
 
 
 def build_graph(d: Q.Dims, ptr, B: int, maxlen: int = 1072, machine: MachineModel | str = "b200", engine: str = "tc"):
@@ -107,28 +106,25 @@ def build_graph(d: Q.Dims, ptr, B: int, maxlen: int = 1072, machine: MachineMode
                                           ln=ln, ids=ptr(ids) if ids else 0, R=R, K=d.H, M=d.H, rpt=1, tpe=1, eps=d.eps, nb=B, sx=d.H, srows=srows,
                                           srin=d.H, srout=d.H), (B,), B)
 
-    skc = {"n": 0}                                                     # arrival counters handed out so far; grids of one shape share theirs
+    skc = {"n": 0}                                                     # a word per shared row block (a block that is not set is refused); one shape, one range
 
     def dense(name, Wp, x, out, M, K, bias=0):
         mode = op_gemv.MODE_BIAS if bias else 0
         if engine == "tc":
             # row blocks of 256 (one instruction's worth); those of narrow matrices are shared by several tasks
             t, rpt, S = op_batch.split_k(M, K, W)
-            blocks = t // S
-            if S > 1 and ((M, K, S) not in skc and skc["n"] + blocks > op_batch.SPLITK_COUNTERS or S * B * M > SKP_FLOATS):
-                t, rpt, S = blocks, rpt, 1
             extra = {}
             if S > 1:
                 if (M, K, S) not in skc:
                     skc[(M, K, S)] = skc["n"]
-                    skc["n"] += blocks
+                    skc["n"] += t // S
                 extra = dict(rows=ptr("skp"), resid_in=ptr("skc") + 4 * skc[(M, K, S)])
             add(name, "etx_tile_gemv_tc", gb("gemv_tc", t, W=Wp, x=ptr(x), out=ptr(out), M=M, K=K, rpt=rpt, tpe=S, nb=B, sx=K, sout=M, wts=bias, mode=mode, **extra), (t,), t)
             return
         t, rpt = m.gemv_tasks(M)
         add(name, "etx_tile_gemv_nb", gb("gemv_nb", t, W=Wp, x=ptr(x), out=ptr(out), M=M, K=K, rpt=rpt, tpe=1, nb=B, sx=K, sout=M, wts=bias, mode=mode), (t,), t)
 
-    cols = argblock.pack_named(ent["cols"], (B, 1, 1), nb=B, slot_span=nblk * BS, zero=ptr("skc"))
+    cols = argblock.pack_named(ent["cols"], (B, 1, 1), nb=B, slot_span=nblk * BS)
     add("prologue", "vl_prologue_nb", cols, (B,), B)
     for L in range(d.L):
         Wl = lambda n, L=L: ptr(f"{L}.{n}")                                  # noqa: E731

@@ -20,7 +20,7 @@ prologue / argmax have small blocks of their own.
   moe_up_tc, moe_down_tc   the expert grids on tcgen05.mma, scheduled by share: nblocks = workers, task blk takes an equal
                 share of (active experts x row tiles); ids = the step's routing ids [nb][R] (the tiles build the
                 per-expert lists themselves), E set; moe_up_tc's resid_out = optional counter += active experts
-  prologue_nb   task b: residual <- embedding row of column b's token, positions / slot of column b
+  prologue_nb   task b: residual <- embedding row of column b's token, positions / slot of column b (`zero`: not read)
   argmax_nb     task b: greedy token of column b
 """
 from __future__ import annotations
@@ -35,7 +35,6 @@ ROUTE_PARAMS = [("logits", "ptr addrspace(1)", 0, 8), ("wts", "ptr addrspace(1)"
                 ("E", "i32", 48, 4), ("K", "i32", 52, 4), ("mode", "i32", 56, 4), ("nb", "i32", 60, 4), ("cap", "i32", 64, 4)]
 COLS_BYTES, COLS_GRID = 32, 16
 COLS_PARAMS = [("nb", "i32", 0, 4), ("slot_span", "i32", 4, 4), ("zero", "ptr addrspace(1)", 8, 8)]
-SPLITK_COUNTERS = 768       # int32 arrival counters `zero` names (cleared by column 0's prologue task every step)
 TC_ROWS = 256               # weight rows one tcgen05 instruction takes (four TMA boxes of 64)
 XBYTES = 40960              # shared memory for the token vectors of a pass: min(8, XBYTES // (2 K + 64)) columns per pass
 GROUP_ROWS = 128            # weight rows a block of the tensor-core loop covers

@@ -51,10 +51,9 @@ def run(shapes=SHAPES, iters: int = 12, device: int = 0, peak_gbs: float | None 
         if tc:
             from . import batch as _batch
             tasks, rpt, S = _batch.split_k(N, K, m.workers())
-            part = torch.zeros((S * N * M,), dtype=torch.float32, device=dev)
-            count = torch.zeros((tasks // S,), dtype=torch.int32, device=dev)
+            word = torch.zeros((32,), dtype=torch.float32, device=dev)          # (set in the blocks of shared row blocks, not read)
             blob = argblock.pack_named(ent["gemv_tc"], (tasks, 1, 1), W=W.data_ptr(), x=x.data_ptr(), out=out.data_ptr(), M=N, K=K, rpt=rpt, tpe=S, nb=M,
-                                       sx=K, sout=N, rows=part.data_ptr() if S > 1 else 0, resid_in=count.data_ptr() if S > 1 else 0)
+                                       sx=K, sout=N, rows=word.data_ptr() if S > 1 else 0, resid_in=word.data_ptr() if S > 1 else 0)
             g = Graph(f"gemv_tc_{M}x{K}x{N}")
             g.tensor("impargs", (len(blob),), role="weight", bytes_per_elem=1)
             g.etensor("E_done", (1,), wait_count=tasks)

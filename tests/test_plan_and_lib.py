@@ -178,3 +178,13 @@ def test_batched_graph_phases_and_argument_blocks():
         assert struct.unpack_from("<4I", blk, 160) == (info["attn_tasks"], 1, 1, info["attn_tasks"])
     with pytest.raises(ValueError, match="MoE"):
         BT.build_graph(Q.load_dims("qwen3-8b", layers=1), _fake_ptr, 4, 1072)
+
+
+def test_batched_buffers_hold_what_the_tiles_read():
+    """No tile sums partials of a dense grid through memory: beside caches, attention partials and logits a batch of 8 needs under a megabyte."""
+    import math
+    from etx_megakernel_b200.models import batched as BT
+    d = Q.load_dims("qwen3-30b-a3b", layers=2)
+    size = {"bf16": 2, "f32": 4, "i32": 4, "i64": 8}
+    shapes = BT.buffer_shapes(d, 8, 1072, 8, 9)
+    assert sum(math.prod(shape) * size[dt] for n, (shape, dt) in shapes.items() if n not in ("kc", "vc", "tmp_out", "logits")) < 1 << 20

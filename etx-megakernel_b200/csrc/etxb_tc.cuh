@@ -12,14 +12,14 @@
 // path, managed about a sixth of that with 8 tokens per pass.
 //
 // A task = a few tiles of 64 .. 256 weight rows (neighbouring rows of a matrix, or up to 128 of an expert's gate rows and
-// as many up rows) x all of K (or a K-slice) x up to 32 tokens.  Roles inside the CTA's consumer warps: one
+// as many up rows) x all of K x up to 32 tokens.  Roles inside the CTA's consumer warps: one
 // warp issues the TMA loads of the weight tiles (a lane per box of 64 rows), k-chunk by k-chunk, through a ring of 32 KB stages
 // (as many as fit beside the tokens: 2 with 32 tokens of 2048 columns, 5 with up to 8), and starts before the tokens are there;
 // the other threads stage the tokens' vectors into the swizzled layout, once per task; one thread issues the MMAs (four k16 steps per 64-wide chunk) and commits each stage back to the loader; when the last
 // MMA of a tile has completed, four warps read its accumulators (one token per TMEM lane) and run the epilogue while
-// the next tile's MMAs fill the other accumulator buffer.  The weight ring of the one-token tiles is not in use during
-// a batched step (their producer warp has nothing to stream), so its shared memory and the general region form one
-// area for tokens and stages here.  Every wait is bounded by the step's deadline; tensor memory is allocated once per
+// the next tile's MMAs fill the other accumulator buffer.  The weight ring's memory and the general region form one area for
+// tokens and stages here: the producer warp copies into the ring (units of attention, rows of the narrow tiles, streamed
+// weights) only when every task before the one it copies for is over.  Every wait is bounded by the step's deadline; tensor memory is allocated once per
 // launch by the kernel and freed on every exit path.
 #pragma once
 #include <cuda.h>
@@ -34,7 +34,7 @@ namespace etxb {
 #define ETXB_TC_STAGE (4 * ETXB_TC_BOX)   // one k-chunk of a tile: up to 256 rows
 #define ETXB_TC_MAXSTAGE 6
 #define ETXB_TC_TAIL 8192              // end of the area: the routing tables of the expert tiles
-#define ETXB_TC_AREA (ETXB_RING_BYTES + ETXB_GEN_BYTES - 1024 - ETXB_TC_TAIL)   // the idle weight ring and the general region, 1024-byte aligned inside
+#define ETXB_TC_AREA (ETXB_RING_BYTES + ETXB_GEN_BYTES - 1024 - ETXB_TC_TAIL)   // the weight ring and the general region, 1024-byte aligned inside
 #define ETXB_TC_XBYTES 131072          // at most this much of it holds tokens (32 tokens x 2048 columns); the rest are weight stages
 #define ETXB_TC_MAXTOK 32              // tokens per job (M = 64 up to 8 tokens, 128 above)
 #define ETXB_TC_COLS 512               // tensor-memory columns the kernel allocates: two accumulator buffers of 256
@@ -112,10 +112,9 @@ __device__ __forceinline__ int tc_stages(int K, int ntok) {
 
 // One task: for every tile i of the segment, h = height(i) rows, D_i[tok][j] = sum_k x_tok[k] * W[y0 + i tmax + j][k] for j < h, then
 // epi(i, tok, j, v0, v1) for every tok < ntok and j = 0, 8, .. h - 8 with v0[u] = D_i[tok][j + u]; TWO: v1[u] = the same of the second run
-// (one instruction multiplies both, N = 2 h).  The sum runs over the K columns from
-// `kofs` on (a K-slice of the matrix: both multiples of 64).  xsrc(n): the bf16 row of token n (column 0);
+// (one instruction multiplies both, N = 2 h).  K: a multiple of 64.  xsrc(n): the bf16 row of token n;
 // map: the tensor map of the weight tensor (rows x all columns, box 64 x 64).  All consumer threads call; ends with a barrier.
-// nx, nx_tok: the segment that the same caller runs next with the same map, kofs and K, and its tokens (0: none).
+// nx, nx_tok: the segment that the same caller runs next with the same map and K, and its tokens (0: none).
 // pre: in, how many stages an earlier call has already filled for this segment; out, for the next one.
 //
 // The tokens are staged ONCE per task (the tiles of a task share them) whenever all of K fits the token area; the tiles
@@ -127,7 +126,7 @@ __device__ __forceinline__ int tc_stages(int K, int ntok) {
 // place whatever the number of tokens): the step from one expert to the next, which a third of the workers take, does not
 // drain the stream.
 template <bool TWO, typename XSrc, typename Epi>
-__device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void* map, const TcSeg seg, const TcSeg nx, int nx_tok, int& pre, int kofs, int K, int ntok,
+__device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void* map, const TcSeg seg, const TcSeg nx, int nx_tok, int& pre, int K, int ntok,
                                         int where, XSrc xsrc, Epi epi) {
   const int tid = tidx(), warp = tid >> 5, lane = tid & 31;
   unsigned char* area = (unsigned char*)(((uintptr_t)sm.ring + 1023) & ~(uintptr_t)1023);
@@ -158,7 +157,7 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
       __syncwarp();
       if (lane < nb) {
         const bool second = TWO && lane >= per;
-        tma_load_2d(ws - (size_t)st * ETXB_TC_STAGE + lane * ETXB_TC_BOX, map, kofs + (w0 + c) * 64,
+        tma_load_2d(ws - (size_t)st * ETXB_TC_STAGE + lane * ETXB_TC_BOX, map, (w0 + c) * 64,
                     (second ? g.y1 - per * ETXB_TC_BOXROWS : g.y0) + i * g.tmax + lane * ETXB_TC_BOXROWS, tc.full + st);
       }
       return true;
@@ -183,7 +182,7 @@ __device__ __forceinline__ void tc_task(const Smem& sm, TcShared& tc, const void
     const int first = warp == 0 ? lane : tid - 32, step = alive0 ? ETXB_CONSUMERS - 32 : ETXB_CONSUMERS;   // (an abandoned step: whatever)
     for (int i = first; i < ntok * nc * 8; i += step) {
       const int n = i / (nc * 8), v = i - n * (nc * 8), c = v >> 3, j = v & 7, r = n & 7;
-      const uint4 val = ld_act16((const __nv_bfloat16*)xsrc(n) + (size_t)(kofs + w0 * 64 + v * 8));
+      const uint4 val = ld_act16((const __nv_bfloat16*)xsrc(n) + (size_t)(w0 * 64 + v * 8));
       *(uint4*)(area + (size_t)(c * groups + (n >> 3)) * 1024 + r * 128 + ((j ^ r) << 4)) = val;
     }
     }
@@ -289,7 +288,7 @@ __device__ __forceinline__ void tile_gemv_tc(const unsigned char* a, int blk, co
   for (int b0 = 0; b0 < d.nb; b0 += ETXB_TC_MAXTOK) {
     const int nt = min(ETXB_TC_MAXTOK, d.nb - b0);
     int pre = 0;
-    tc_task<false>(sm, tc, d.ln, seg, seg, 0, pre, 0, d.K, nt, where,
+    tc_task<false>(sm, tc, d.ln, seg, seg, 0, pre, d.K, nt, where,
             [&](int n) { return (const __nv_bfloat16*)d.x + (size_t)(b0 + n) * d.sx; },
             [&](int i, int tok, int j, const float (&v)[8], const float (&)[8]) {
               const int rr = r0 + 2 * i * ETXB_TC_ROWS + j;
@@ -566,7 +565,7 @@ __device__ __forceinline__ void tile_moe_tc(const unsigned char* a, int blk, con
       const int nt = min(ETXB_TC_MAXTOK, cnt - p0), nxt = p0 + nt < cnt ? 0 : ntn;
       const int32_t* ent = rt.ent + p0;
       if constexpr (UP) {
-        tc_task<true>(sm, tc, d.ln, seg, nseg, nxt, pre, 0, d.K, nt, where,
+        tc_task<true>(sm, tc, d.ln, seg, nseg, nxt, pre, d.K, nt, where,
                 [&](int n) { return (const __nv_bfloat16*)d.x + (size_t)(ent[n] >> 8) * d.sx; },
                 [&](int i, int tok, int j, const float (&g)[8], const float (&up)[8]) {
                   const int r = r0 + i * TMAX + j, en = ent[tok];
@@ -577,7 +576,7 @@ __device__ __forceinline__ void tile_moe_tc(const unsigned char* a, int blk, con
                 });
       } else {
         const float* wt = rt.wt + p0;
-        tc_task<false>(sm, tc, d.ln, seg, nseg, nxt, pre, 0, d.K, nt, where,
+        tc_task<false>(sm, tc, d.ln, seg, nseg, nxt, pre, d.K, nt, where,
                 [&](int n) { return (const __nv_bfloat16*)d.x + ((size_t)(ent[n] >> 8) * d.R + (ent[n] & 0xff)) * d.K; },
                 [&](int i, int tok, int j, const float (&v)[8], const float (&)[8]) {
                   const int r = r0 + i * TMAX + j, en = ent[tok];

@@ -20,28 +20,34 @@ from tests.test_gpu_ops import dev_bf16, host  # noqa: E402
 DEV, HD, SCALE = "cuda:0", 128, float(np.float32(1.0 / np.sqrt(128)))
 
 
-def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True, behind=None):
+def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True, behind=None, norm=None, seqs=None, pos=None):
     """One attention grid over B sequences.  K, V: per sequence [seq][NKV][HD], the last position being the new one (its cache row holds NaN and comes from qkv
     [B][NH + 2 NKV][HD] instead).  Returns (out [B][NH][HD] bf16 values, the cached k rows at the new positions [B][NKV][HD], the partials
     [B][NH][partitions][128 sums, maximum, sum of the probabilities]).  behind: a second grid of one empty task that waits for the first attention task
-    alone, and the queues of the plan as a function of the attention tasks' and its number."""
+    alone, and the queues of the plan as a function of the attention tasks' and its number.  norm: weights of the q and k norms.  seqs, pos: sequence
+    lengths and new positions where the new one is not the last (its cache row and all rows behind the length hold NaN)."""
     B, nblk, parts = len(K), maxlen // 16, -(-maxlen // 128)
+    seq = np.array(seqs if seqs is not None else [len(k) for k in K])
+    pos = np.array(pos) if pos is not None else seq - 1
     pools = []
     for b in range(B):
-        pad = np.full((maxlen - len(K[b]) + 1, NKV, HD), np.nan, np.float32)
-        pools.append(O.paged_from_contig(np.concatenate([K[b][:-1], pad]), np.concatenate([V[b][:-1], pad]), nblk))
+        kv = np.full((2, maxlen, NKV, HD), np.nan, np.float32)
+        kv[0, :seq[b]], kv[1, :seq[b]] = K[b][:seq[b]], V[b][:seq[b]]
+        kv[:, pos[b]] = np.nan
+        pools.append(O.paged_from_contig(kv[0], kv[1], nblk))
     table = np.random.default_rng(1).permutation(B * nblk).astype(np.int32)                # any block order
     inv = np.argsort(table)
     kc, vc = (dev_bf16(np.concatenate([p[i] for p in pools])[inv]) for i in (0, 1))
-    seq = np.array([len(k) for k in K])
     tab = Q.rope_table(1e6, HD, maxlen).view(np.int16)
     if not rotary:
         tab = np.concatenate([O.f32_to_bf16_bits(np.ones((maxlen, HD // 2), np.float32)).view(np.int16), np.zeros((maxlen, HD // 2), np.int16)], 1)
     t = {"qkv": dev_bf16(qkv), "cos_sin": torch.from_numpy(tab).to(DEV).view(torch.bfloat16), "kc": kc, "vc": vc,
          "block_tables": torch.from_numpy(table).to(DEV), "seq_lens": torch.from_numpy(seq.astype(np.int32)).to(DEV),
-         "positions": torch.from_numpy(seq - 1).to(DEV), "tmp_out": torch.zeros((B, NH, parts, ops.attn.GQ_PARTIAL_FLOATS), dtype=torch.float32, device=DEV),
-         "slot_mapping": torch.from_numpy(np.array([int(table[b * nblk + (s - 1) // 16]) * 16 + (s - 1) % 16 for b, s in enumerate(seq)], np.int64)).to(DEV),
+         "positions": torch.from_numpy(pos.astype(np.int64)).to(DEV), "tmp_out": torch.zeros((B, NH, parts, ops.attn.GQ_PARTIAL_FLOATS), dtype=torch.float32, device=DEV),
+         "slot_mapping": torch.from_numpy(np.array([int(table[b * nblk + p // 16]) * 16 + p % 16 for b, p in enumerate(pos)], np.int64)).to(DEV),
          "out": torch.zeros((B, NH, HD), dtype=torch.bfloat16, device=DEV)}
+    if norm is not None:
+        t["qw"], t["kw"] = (dev_bf16(w) for w in norm)
     step = {"qkv": (NH + 2 * NKV) * HD * 2, "block_tables": nblk * 4, "seq_lens": 4, "positions": 8, "slot_mapping": 8,
             "tmp_out": NH * parts * ops.attn.GQ_PARTIAL_FLOATS * 4, "out": NH * HD * 2}
     ntask = NH // gq * (1 if whole else parts)
@@ -196,3 +202,44 @@ def test_infinite_values_in_the_cache_stay_infinite(seq, NH, NKV, gq, whole):
         assert np.array_equal(np.flatnonzero(~fin), [10, 11, 12, 13])
         assert np.array_equal(out[0, h, ~fin], want[~fin].astype(np.float32), equal_nan=True), out[0, h, ~fin]
         assert np.all(np.abs(out[0, h, fin] - want[fin]) <= 2.0 ** -8 * np.abs(want[fin]) + np.abs(want[fin]).max() * 2.0 ** -13)
+
+
+@pytest.mark.parametrize("norm", [True, False])
+@pytest.mark.parametrize("whole", [False, True])
+def test_sequences_of_different_lengths_in_a_large_cache(norm, whole):
+    """One plan over sequences of 1 to 1000 positions (1 to 8 partitions of 8 q heads: both sides of the number of partials from which the merge is shared) in a cache of
+    1280, most of whose tasks have nothing to do; with and without the q / k norms; positions that are not the last of their sequence -- inside it, where the
+    cached row is replaced, behind it in its last block, and in a block behind that."""
+    NH, NKV, gq, maxlen = 16, 2, 8, 1280
+    seqs, pos = (1, 16, 129, 700, 1000, 890, 333, 97, 100, 100), (0, 15, 128, 699, 999, 889, 200, 0, 105, 125)
+    rng = np.random.default_rng(7)
+    nw, kw = (O.bfr(1 + 0.1 * rng.standard_normal(HD, dtype=np.float32)) for _ in range(2))
+    K, V = ([O.bfr(rng.standard_normal((max(s, p + 1), NKV, HD), dtype=np.float32)) for s, p in zip(seqs, pos)] for _ in range(2))
+    qkv = O.bfr(rng.standard_normal((len(seqs), NH + 2 * NKV, HD), dtype=np.float32))
+    out, rows, _ = run(NH, NKV, K, V, qkv, maxlen, gq, whole=whole, norm=(nw, kw) if norm else None, seqs=seqs, pos=pos)
+    cos, sin = O.rope_tables(1e6, HD, maxlen)
+    for b, (s, p) in enumerate(zip(seqs, pos)):
+        x = qkv[b]
+        q, k = (np.stack([O.rmsnorm(h, w, 1e-6) for h in y]) if norm else y for y, w in ((x[:NH], nw), (x[NH:NH + NKV], kw)))
+        q, k = (np.stack([O.apply_rope(h, cos[p], sin[p]) for h in y]) for y in (q, k))
+        assert np.array_equal(rows[b], k), f"column {b}: the cached k row"
+        used = sorted(set(range(s)) | {p})
+        for h in range(NH):
+            kk, vv = K[b][:, h * NKV // NH].astype(np.float64), V[b][:, h * NKV // NH].astype(np.float64)
+            kk[p], vv[p] = k[h * NKV // NH], x[NH + NKV + h * NKV // NH]
+            sc = kk[used] @ q[h].astype(np.float64) * SCALE
+            w = np.exp(sc - sc.max())
+            want = w @ vv[used] / w.sum()
+            # the bf16 rounding of the result (2^-9 of it), and fp32 sums with probabilities exact to 2^-17
+            assert np.all(np.abs(out[b, h] - want) <= 2.0 ** -8 * np.abs(want) + np.abs(want).max() * 2.0 ** -13), (b, h)
+
+
+def test_shared_and_single_merges_give_the_same_bits():
+    """64 partials of a group, merged by eight tasks, by the last ones of two workers, and by the last partition's task alone (a queue that is not in ascending order)."""
+    rng = np.random.default_rng(11)
+    V = O.bfr(rng.standard_normal((1000, 1, HD), dtype=np.float32) + np.where(np.arange(1000) // 128 % 2, -900.0, 900.0).astype(np.float32)[:, None, None])
+    K, qkv = (O.bfr(rng.standard_normal(s, dtype=np.float32) * np.float32(0.3)) for s in ((1000, 1, HD), (10, HD)))
+    eight, _, _ = run(8, 1, [K], [V], qkv[None], 1024, 8)
+    two, _, _ = run(8, 1, [K], [V], qkv[None], 1024, 8, behind=lambda attn, empty: [attn[4:], attn[:4] + [empty]])
+    alone, _, _ = run(8, 1, [K], [V], qkv[None], 1024, 8, behind=lambda attn, empty: [attn[4:], attn[3::-1] + [empty]])
+    assert np.array_equal(two, eight) and np.array_equal(alone, eight)

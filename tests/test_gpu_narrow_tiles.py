@@ -26,3 +26,18 @@ def test_rows_shared_between_tasks(M, K, rpt, S, nb):
     want = O.bfr((x.astype(np.float64) @ W.astype(np.float64).T + bias).astype(np.float32))
     assert_bf16_close(host(out)[:nb], want, f"M={M} K={K} nb={nb}", min_exact=0.97)
     assert not host(out)[nb:].any() and not word.any()        # nothing behind the last column, no partial sums
+
+
+@pytest.mark.parametrize("nb", [5, 33])
+def test_token_and_result_rows_further_apart_than_their_length(nb):
+    M, K, rpt, S, sx, sout = 300, 512, 256, 4, 520, 311
+    rng = np.random.default_rng(nb)
+    W, x = O.bfr(rng.standard_normal((M, K), dtype=np.float32) * np.float32(0.02)), np.full((nb, sx), np.nan, np.float32)
+    x[:, :K] = O.bfr(rng.standard_normal((nb, K), dtype=np.float32))
+    Wd, xd, out = dev_bf16(W), dev_bf16(x), torch.full((nb, sout), 7.0, dtype=torch.bfloat16, device=DEV)
+    word = torch.zeros(64, dtype=torch.float32, device=DEV)
+    run_grid("gemv_tc", -(-M // rpt) * S, W=Wd.data_ptr(), x=xd.data_ptr(), out=out.data_ptr(), M=M, K=K, rpt=rpt, tpe=S, nb=nb, sx=sx, sout=sout,
+             rows=word.data_ptr(), resid_in=word.data_ptr())
+    want = O.bfr((x[:, :K].astype(np.float64) @ W.astype(np.float64).T).astype(np.float32))
+    assert_bf16_close(host(out)[:, :M], want, f"nb={nb}", min_exact=0.97)
+    assert (host(out)[:, M:] == 7.0).all()                    # nothing between the columns' rows

@@ -119,8 +119,8 @@ static int32_t check_attnf_block(const etxb_attnf_args& a) {
     else if (a.HD != 128 || a.BS != 16 || (a.part_len & 0xffff) != 128) why = "the grouped form is head_dim 128, cache blocks of 16, partitions of 128";
     else if (a.gq * a.max_parts > 4096) why = "gq * max_parts <= 4096";
     else if ((a.part_len >> 24) & ~1) why = "part_len bits 25..31 are zero";
-    else if ((a.part_len >> 24) && (a.nblocks > (uint32_t)(a.NH / a.gq) || 65536 + (size_t)a.max_parts * a.gq * 130 * 4 > ETXB_RING_BYTES))
-      why = "whole-sequence form: the grid is NH / gq tasks and 64 KB + max_parts * gq * 130 floats fit the weight ring (longer contexts: partitions)";
+    else if ((a.part_len >> 24) && (a.nblocks > (uint32_t)(a.NH / a.gq) || a.max_parts * a.gq > ETXB_GQ_WHOLE_MAX))
+      why = "whole-sequence form: the grid is NH / gq tasks and max_parts * gq <= 157 (longer contexts: partitions)";
     else if (a.nblocks > (uint32_t)(a.max_parts * (a.NH / a.gq))) why = "the grid is at most max_parts * NH / gq tasks";
   } else {
     const int G = a.NH / a.NKV;
@@ -168,7 +168,7 @@ static int32_t check_batch_block(int body, const unsigned char* blk, size_t byte
   else if ((body == ETXB_BODY_MOE_UP_TC || body == ETXB_BODY_MOE_DOWN_TC) && (a.R < 1 || a.R > 16 || a.nb * a.R > 1024 || !a.ids || a.E > 256))
     why = "share-scheduled expert tile: 1 <= R <= 16, nb * R <= 1024, E <= 256, the step's routing ids set";
   else if (body >= ETXB_BODY_GEMV_TC && (a.K % 64 || ((uintptr_t)a.W & 15))) why = "tensor-core tile: K % 64 == 0 and W 16-byte aligned (TMA tensor copies of 64-wide chunks)";
-  else if (body == ETXB_BODY_GEMV_TC && a.tpe > 1 && (a.K % (64 * a.tpe) || !a.rows || !a.resid_in)) why = "split-K dense tile: K a multiple of 64 x the split, partial sums (rows) and arrival counters (resid_in) set";
+  else if (body == ETXB_BODY_GEMV_TC && a.tpe > 1 && (a.K % (64 * a.tpe) || !a.rows || !a.resid_in)) why = "row blocks shared by several tasks: K a multiple of 64 x their number, rows and resid_in set";
   else if ((body == ETXB_BODY_MOE_UP_TC || body == ETXB_BODY_MOE_DOWN_TC) && (a.E < 1 || a.estride <= 0 || a.estride % a.K)) why = "tensor-core expert tile: E >= 1 and estride a multiple of K (the experts form one [E * rows][K] matrix)";
   if (!why) return ETXB_OK;
   snprintf(m, sizeof m, "batched block (body %d, M=%d, K=%d, rpt=%d, tpe=%d, R=%d, nb=%d) outside the tile: %s", body, a.M, a.K, a.rpt, a.tpe, a.R, a.nb, why);
@@ -241,7 +241,8 @@ static bool batched_plan(const etxb_session* s, const std::vector<unsigned char>
 // Which kernel can run this plan?  The lean decode kernels hold only the tiles of a fused decode step; a plan qualifies
 // when every grid is one of those tiles with its argument block in the pool (one block per grid) and the blocks stay
 // inside what the lean forms cover: norm folds of at most one row (or the flagged rows of a sharded model), top-k folds over at most 128 experts, grouped
-// attention (head_dim 128, cache blocks of 16, partitions of 128) with the same group size everywhere.
+// attention (head_dim 128, cache blocks of 16, partitions of 128) with the same group size everywhere: the variant's number names it in
+// the session's status, although one lean kernel serves all sizes; a plan of several runs on the full kernel, as it always has.
 static int select_variant(const etxb_session* s, const std::vector<unsigned char>& pool) {
   if (batched_plan(s, pool)) return 11;
   int gq = 0;
@@ -274,8 +275,8 @@ static int select_variant(const etxb_session* s, const std::vector<unsigned char
   return gq == 1 ? 1 : gq == 2 ? 2 : gq == 4 ? 3 : 4;
 }
 
-// The kernel variants: index 0 = the full kernel, 1..4 = the lean decode kernels for grouped attention with 1, 2, 4, 8
-// q heads per task (etxb_kernel.cuh, run_body).
+// The kernel variants: index 0 = the full kernel, 1..4 = the lean decode kernel, by the 1, 2, 4 or 8 q heads that a grouped attention task of the
+// plan has (etxb_kernel.cuh, run_body).
 // Entries 5..9: the same five with the exchange code of a sharded session compiled in (launch_kernel adds 5).
 // Entry 10: the lean decode kernel of a latent-attention model (no sharded form: such a session falls back to entry 5).
 // Entry 11: the kernel of a batched step on the tensor cores.

@@ -14,9 +14,10 @@
 //     Sums meet in fp32, so that the partials are no further from 64-bit ones than plain fp32 chains of 32 terms leave them: 1.3e-7 at 1038
 //     and 8151 positions against 1.6e-7 (summed up inside the products 1.8e-7).
 // Bound by the stream of K / V at long contexts, by the chain q rows -> norm -> scores -> publish -> merge at short ones.
-// A phase at 8150 positions (64 partitions, 256 tasks): 30 us -> 17; 8 sequences at 1033: 33 -> 22; 32 sequences, whole contexts of 1045:
-// 52 -> 21; one sequence at 1037: 8.3 -> 7.9.  The forms before multiplied out of registers on the fp32 pipes, or walked a context with
-// a barrier between any two of its steps.
+// From the last q row to the last output: one sequence at 8150 positions (64 partitions, 256 tasks) 28.1 us -> 16.5, at 1037 9.3 -> 7.8, a
+// small dense model at 601 (one q head a task) 8.4 -> 7.6; 8 sequences at 1033 33.4 -> 22.9, 13 at 333 31.5 -> 24.0; 32 sequences, whole
+// contexts of 1045: 53.5 -> 25.0.  The forms before multiplied out of registers on the fp32 pipes, or walked a context with a barrier between
+// any two of its steps.
 // The new position never comes from the cache: its k / v rows stand in for the stale slot of the staged unit.
 //
 // It stands where the reference runs dsl_attnprep (etx/ops/attnprep.py:86-211), vLLM's paged attention and its reduce
@@ -29,9 +30,11 @@ namespace etxb {
 
 #define ETXB_GQ_PART 128   // positions per task
 #define ETXB_GQ_WHOLE (1 << 24)   // part_len bit: one task per (sequence, q group) takes all partitions
+#define ETXB_GQ_WHOLE_MAX 157     // .. of partitions x q heads at most (the builder's rule: ops/attn.py)
 #define ETXB_GQ_PW 136     // 8-byte (value, flag) pairs a task publishes per q head and partition: 128 outputs, max, sum, padding
-#define ETXB_GQ_SHARE 64   // partials (gq x partitions) from which the merge is shared out.  Below: 144 tasks that all wait and poll made a phase of
-                           // 2 x 9 partials 9.5 us, one merging task per group 8.0.  Above: 8 x 64 partials are 512 KB for one merging task
+#define ETXB_GQ_SHARE 64   // partials (gq x partitions) from which the merge is shared out.  Shared / by one task, us of a phase: 72 partials (8 sequences)
+                           // 22.3 / 23.9, 88 (3 sequences) 13.3 / 15.9; 8 x 64 partials are 512 KB for one task.  Few partials: 144 tasks that all wait and poll
+                           // made a phase of 2 x 9 partials 9.5, one merging task per group 8.0.  (Between them sharing gains too: 5 x 8 partials 23.6 / 24.5.)
 #define ETXB_GQ_UNIT 8192  // a unit in a ring stage: 16 positions' K (4 KB), then their V
 #define ETXB_GQ_UPS (ETXB_STAGE_BYTES / ETXB_GQ_UNIT)   // units per stage
 

@@ -58,7 +58,7 @@ struct Smem {
   unsigned char* ring;       // ETXB_NSTAGE stages
   uint64_t* full;            // [ETXB_NSTAGE] stage filled (transaction bytes landed)
   uint64_t* empty;           // [ETXB_NSTAGE] stage drained by the warps it belongs to; behind it [8] uint32: the use the producer fills it for
-  int32_t* prod;             // producer-warp scratch: 16 ids + 16 weights
+  int32_t* prod;             // producer-warp scratch: 16 expert ids; from word 32 on the argument block of the task it copies for
   const unsigned long long* deadline;
   int* stop;                 // CTA-local: a wait inside a body gave up (the body's results are not to be announced)
   const GemvGeom* geo;       // the running GEMV-family task's rows and how the warps share them

@@ -250,7 +250,8 @@ __device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, i
 // on the tensor cores.  The host picks it from the plan (select_variant): the full
 // kernel is 1020 KB of code, of which a decode step uses a fraction scattered through it, and its tiles are calls.  From the
 // 142 KB kernel (same bits): 12 layers of a 128-expert model 794 -> 693 us, of a dense one 1393 -> 1253; 9 layers of a
-// latent-attention model 794 -> 689 from its 170 KB; the batched kernel (610 KB) gives 1 to 5 % (batched_plan).
+// latent-attention model 794 -> 689 from its 170 KB; the batched kernel (610 KB) gives 1 to 5 % (batched_plan).  (Sizes as measured
+// then; since the attention tile is one for all group sizes 721, 150, 160 and 315 KB.)
 // XCH: the variants a sharded session launches -- the same bodies plus the exchange code (flagged-row folds of R = ranks
 // rows, row publishing after the body, the argmax exchange); compiled out of the others.
 #define ETXB_VARIANT_LEAN 1

@@ -164,8 +164,9 @@ class MachineModel:
 
         Head counts that leave one q head per task (3, 5, 7 .. per kv head) read K and V once per q head and still gain
         over the general tile, which also takes the step to the full kernel.  A layer of a small dense model at 600 / 2000 /
-        8000 positions, general -> grouped, us: 28 q heads on 4 kv heads 44 / 58 / 135 -> 32 / 48 / 103; 56 on 8
-        61 / 84 / 218 -> 42 / 69 / 181; 24 on 8 50 / 71 / 180 -> 32 / 43 / 98; 36 on 4 47 / 66 / 160 -> 37 / 48 / 125."""
+        8000 positions, general -> grouped, us: 28 q heads on 4 kv heads 52 / 63 / 121 -> 43 / 58 / 105; 56 on 8
+        68 / 86 / 190 -> 56 / 83 / 177; 24 on 8 58 / 73 / 159 -> 44 / 54 / 100; 36 on 4 55 / 68 / 137 -> 49 / 60 / 128.  (The rule itself, fewest
+        heads, is from a tile whose time grew with them; on the tensor cores it does not up to 8, and larger groups were not measured again.)"""
         G = NH // NKV
         if HD != 128 or BS != 16:
             return (0, 0, 0)

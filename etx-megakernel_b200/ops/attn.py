@@ -35,7 +35,7 @@ F_PARAMS = [("qkv", "ptr addrspace(1)", 0, 8), ("qw", "ptr addrspace(1)", 8, 8),
             ("gq", "i32", 152, 4), ("part_len", "i32", 156, 4)]
 GQ_PART = 128
 GQ_WHOLE = 1 << 24
-RING_BYTES = 6 * 24576     # shared memory of the weight ring
+GQ_WHOLE_MAX = 157         # partitions x q heads per task that a whole-sequence task takes
 
 
 def tagged_part_len(tag: int, whole: bool = False) -> int:
@@ -46,9 +46,10 @@ def tagged_part_len(tag: int, whole: bool = False) -> int:
 
 
 def whole_sequence_fits(gq: int, max_parts: int) -> bool:
-    """The longest context of the whole-sequence form, 2432 positions at 8 q heads per task: a longer one is cut into partitions, so that
-    a step is not as long as its longest sequence's one task."""
-    return 65536 + max_parts * gq * 130 * 4 <= RING_BYTES
+    """Whether the whole-sequence form takes a context: up to 2432 positions at 8 q heads per task.  The number is what the partials of an earlier
+    tile left of the ring's memory; the present one keeps none there, and at 2380 positions it is still far quicker than partitions are (3 layers
+    of a 128-expert model, us: 20 sequences 984 / 1205, 32 sequences 1071 / 1490, 48 sequences 1414 / 1985), so the line could lie higher."""
+    return max_parts * gq <= GQ_WHOLE_MAX
 
 
 GQ_PARTIAL_FLOATS = 272   # grouped form: floats of `tmp_out` per (q head, partition) -- 136 (value, flag) pairs: 128 outputs, max, sum, padding

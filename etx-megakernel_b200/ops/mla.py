@@ -9,8 +9,8 @@ It stands where the reference's DeepSeek-V2-Lite graph runs q_absorb, the chunke
   wkvb      bf16 [NH * (DN + DV)][C]         kv_b_proj: per head DN rows of W_UK, then DV rows of W_UV
   cache     bf16 [maxlen][C + DR]            the layer's latent cache (row `pos` is written by head 0's task)
   positions int64 [1],  out bf16 [NH * DV]
-  tmp       (value, flag) pairs [NH][max_parts][C + 8] (8 bytes each): the partitions' partial results; the task of the
-            four finishing tasks per head merge them and apply a quarter of W_UV each.  max_parts * 128 >= maxlen; grid =
+  tmp       (value, flag) pairs [NH][max_parts][C + 8] (8 bytes each): the partitions' partial results; the four
+            finishing tasks per head merge them and apply a quarter of W_UV each.  max_parts * 128 >= maxlen; grid =
             (max_parts + 4) * NH tasks (task = partition * NH + head, then the finishing tasks); tag = a number that differs between the grids sharing tmp (the layer)
 """
 from __future__ import annotations
@@ -29,7 +29,7 @@ PARAMS = [("qkv", "ptr addrspace(1)", 0, 8), ("kvln", "ptr addrspace(1)", 8, 8),
 
 
 def import_entries(threads: int = 544) -> dict:
-    return {"mla_attn": entry("mla_attn", "mla_attn", PARAMS, ARG_BYTES, GRID_OFF, threads, "absorbed multi-head latent attention, one (head, 128 positions) per task, merged by the last partition's task")}
+    return {"mla_attn": entry("mla_attn", "mla_attn", PARAMS, ARG_BYTES, GRID_OFF, threads, "absorbed multi-head latent attention, one (head, 128 positions) per task, merged by four finishing tasks per head")}
 
 
 def partitions(maxlen: int) -> int:

@@ -94,9 +94,8 @@ def test_columns_do_not_depend_on_their_neighbours():
 def test_whole_sequence_attention_agrees_with_the_partitioned_form():
     """20 sequences of a 150-token prompt (two partitions of 128 positions) through ONE layer, so that nothing but the
     attention phase separates the two forms: at B = 20 the attention grid has one task per (sequence, kv head) that
-    walks the partitions itself with its products on the tensor cores (bf16 q / K / V, the probabilities as a bf16 value
-    plus the bf16 of its rounding error, fp32 accumulation); at B = 10 it has one task per partition on the fp32 pipes
-    and a merge through flagged partials.  Same partition boundaries and merge order, sums in another order: the KV
+    takes the whole context (the probabilities of cached positions as a bf16 value plus the bf16 of its rounding error);
+    at B = 10 it has one task per partition (a third bf16 part) and a merge through flagged partials.  Sums in another order: the KV
     caches are bit-identical, the attention output agrees within 2 bf16 ulps per element with >= 90 % of the elements
     identical.  (Through several MoE layers a one-ulp difference can flip a near-tie routing decision, which is why the
     multi-layer comparisons are made against the oracle with its tie rule, not between the two forms.)"""

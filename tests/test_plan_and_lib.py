@@ -140,7 +140,7 @@ def test_weight_pack_round_trip():
 def test_batched_graph_phases_and_argument_blocks():
     """The batched step (several sequences per launch): phase order, one argument block per sequence for the attention grid
     (addressed by the grid's second coordinate), a valid plan; tensor-core engine: one routing task per column, expert grids
-    of one share per worker, narrow dense grids cut along K; mma.sync engine: one routing task, E x chunks expert tasks."""
+    of one share per worker, row blocks of narrow dense grids shared by several tasks; mma.sync engine: one routing task, E x chunks expert tasks."""
     from etx_megakernel_b200.models import batched as BT
     from etx_megakernel_b200.ops import attn as op_attn
     from etx_megakernel_b200.sim.protocol import simulate
@@ -159,8 +159,8 @@ def test_batched_graph_phases_and_argument_blocks():
     rows = {r[0]: r for r in pool.rows}
     pb = pool.bytes()
     q0, q1, o0 = (pb[rows[n][4]: rows[n][4] + 160] for n in ("qkv_0", "qkv_1", "o_proj_0"))
-    assert struct.unpack_from("<2i", q0, 56) == (256, 4) and struct.unpack_from("<2i", o0, 56) == (256, 8)          # rows per task, K-split
-    assert struct.unpack_from("<Q", q0, 72)[0] == struct.unpack_from("<Q", q1, 72)[0] == _fake_ptr("skc")            # layers share a shape's counters
+    assert struct.unpack_from("<2i", q0, 56) == (256, 4) and struct.unpack_from("<2i", o0, 56) == (256, 8)          # rows per block, tasks that share it
+    assert struct.unpack_from("<Q", q0, 72)[0] == struct.unpack_from("<Q", q1, 72)[0] == _fake_ptr("skc")            # layers share a shape's words
     assert struct.unpack_from("<Q", o0, 72)[0] == _fake_ptr("skc") + 4 * 20 and struct.unpack_from("<Q", o0, 64)[0] == _fake_ptr("skp")
     g3, pool3, info3 = BT.build_graph(d, _fake_ptr, 32, 1072)              # enough sequences: one attention task per (sequence, kv head)
     shape3 = compile_graph(g3, "b200", {"POOL": len(pool3.bytes())}).inst.grid_shapes

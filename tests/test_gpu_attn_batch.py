@@ -80,10 +80,10 @@ def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True, b
     return outs[0], np.stack([host(kc)[s // 16, :, :, s % 16].reshape(NKV, HD) for s in slot]), tmp
 
 
-@pytest.mark.parametrize("seq,gq", [(1030, 8), (1030, 2), (900, 8), (4200, 8)])
-def test_equal_columns_get_equal_bits_wherever_they_stand(seq, gq):
-    """Ten equal sequences, 9 partitions: the numbers of tasks that share a group's merge differ between the columns; one sequence, and one in a larger
-    cache: other numbers again.  V alternates by partition, so that the sum over the partitions is small beside its terms and
+@pytest.mark.parametrize("seq,gq,B", [(1030, 8, 10), (1030, 2, 10), (900, 8, 10), (4200, 8, 10), (1000, 8, 40)])
+def test_equal_columns_get_equal_bits_wherever_they_stand(seq, gq, B):
+    """Ten equal sequences, 9 partitions: the numbers of tasks that share a group's merge differ between the columns; 40 sequences: more groups than workers,
+    some with no worker's last task among theirs; one sequence, and three in a larger cache: other numbers again.  V alternates by partition, so that the sum over the partitions is small beside its terms and
     another order of them would show."""
     NH, NKV, G = 32, 4, 8
     rng = np.random.default_rng(seq)
@@ -92,11 +92,11 @@ def test_equal_columns_get_equal_bits_wherever_they_stand(seq, gq):
     qkv = O.bfr(rng.standard_normal((NH + 2 * NKV, HD), dtype=np.float32))
     maxlen = -(-seq // 128) * 128
     one, _, _ = run(NH, NKV, [K], [V], qkv[None], maxlen, gq)
-    ten, _, _ = run(NH, NKV, [K] * 10, [V] * 10, np.stack([qkv] * 10), maxlen, gq)
+    many, _, _ = run(NH, NKV, [K] * B, [V] * B, np.stack([qkv] * B), maxlen, gq)
     large, _, _ = run(NH, NKV, [K] * 3, [V] * 3, np.stack([qkv] * 3), maxlen + 640, gq)
     assert np.isfinite(one).all() and np.abs(one).max() < 900
-    for b in range(10):
-        assert np.array_equal(ten[b], one[0]), f"column {b}: {np.mean(ten[b] != one[0]):.4f} of the values differ"
+    for b in range(B):
+        assert np.array_equal(many[b], one[0]), f"column {b}: {np.mean(many[b] != one[0]):.4f} of the values differ"
     for b in range(3):
         assert np.array_equal(large[b], one[0]), f"larger cache, column {b}: {np.mean(large[b] != one[0]):.4f} of the values differ"
 

@@ -102,8 +102,8 @@ def test_latent_attention_block_layout_and_checks():
 
 
 def test_split_k_keeps_one_wave_and_whole_slices():
-    """The K-split of the dense tensor-core grids: tasks stay within one wave of the workers, slices are multiples of 64
-    columns and at least 256 wide, a matrix with a wave of row blocks of its own is not split."""
+    """How many tasks share a row block of the dense batched grids: tasks stay within one wave of the workers, K is a multiple of 64 x their
+    number and at least 256 for each, the blocks of a matrix with a wave of its own are not shared."""
     from etx_megakernel_b200.ops import batch as op_batch
     for M, K in ((5120, 2048), (2048, 4096), (128, 2048), (151936, 2048), (3648, 2048), (64, 2048), (2048, 1408), (102400, 2048)):
         tasks, rpt, S = op_batch.split_k(M, K, 148)

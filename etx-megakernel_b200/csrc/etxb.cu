@@ -10,6 +10,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <string>
 #include <thread>
@@ -60,6 +61,7 @@ struct etxb_session {
   int32_t* h_tok = nullptr;            // pinned staging of the host decode loop
   bool args_dirty = true, trace = false, launched = false;
   uint32_t epoch = 0;
+  uint32_t salt = 0;                   // added to the epoch in the flags of words: sessions that share buffers do not take each other's
   unsigned long long timeout_ns = 2000000000ull;
   etxb_stepv step{};
   cudaStream_t stream = nullptr, own_stream = nullptr;
@@ -109,6 +111,28 @@ static int32_t check_gemv_block(int body, const etxb_gemv_args& a) {
   snprintf(m, sizeof m, "GEMV-family block (body %d, M=%d, K=%d, rpt=%d, tpe=%d, R=%d, E=%d, mode=0x%x) outside the tile: %s", body, a.M, a.K, a.rpt, a.tpe, a.R, a.E, a.mode, why);
   return fail(ETXB_E_UNSUPPORTED, m);
 }
+// The words a block of the GEMV family reads and writes (behind the block: `bytes` readable from its beginning).
+static int32_t check_gemv_words(int body, const etxb_gemv_args& a, const unsigned char* blk, size_t bytes) {
+  if (!(a.mode & (ETXB_MODE_WORDS_IN | ETXB_MODE_WORDS_OUT))) return ETXB_OK;
+  if (bytes < sizeof a + sizeof(etxb_gemv_words)) return fail(ETXB_E_ARG, "hand-off as words: the argument block is 192 bytes");
+  etxb_gemv_words w;
+  memcpy(&w, blk + sizeof a, sizeof w);
+  auto off = [](const void* p, uintptr_t n) { return ((uintptr_t)p & (n - 1)) != 0; };
+  const bool in = (a.mode & ETXB_MODE_WORDS_IN) != 0, norm = (a.mode & 0xff) == ETXB_MODE_NORM, topk = (a.mode & 0xff) >= 2;
+  const char* why = nullptr;
+  if ((a.mode & ETXB_MODE_FLAGGED) || a.nb > 1) why = "one token, not a sharded grid";
+  else if ((a.mode & ETXB_MODE_WORDS_OUT) && a.rpt > ETXB_XF_FLOATS) why = "at most 8192 rows per task";
+  else if (norm && (a.R > 1 || !a.resid_in || !a.ln || off(a.ln, 8) || off(a.resid_in, 8) || off(a.rows, 8) || off(a.resid_out, 8) || off(a.x, 8))) why = "a norm fold adds at most one row, vectors 8-byte aligned";
+  else if (norm && in && (!a.rows || off(a.rows, 16) || off(a.resid_in, 16))) why = "rows and resid_in name words, 16-byte aligned";
+  else if (!norm && in && (!a.x || off(a.x, 16))) why = "x names words, 16-byte aligned";
+  else if (topk && in && off(a.logits, 4)) why = "logits name words";
+  else if (in && topk && body == ETXB_BODY_MOE_DOWN && (a.mode & ETXB_MODE_ROUTE_READY) && (!w.route || off(w.route, 8))) why = "the routing as words, 8-byte aligned";
+  else if ((a.mode & ETXB_MODE_WORDS_OUT) && ((!w.out && !w.z && !w.x) || off(w.out, 4) || off(w.z, 16) || off(w.x, 16) || off(w.route, 8))) why = "words of the results; z and x 16-byte, routing 8-byte aligned";
+  if (!why) return ETXB_OK;
+  char m[256];
+  snprintf(m, sizeof m, "GEMV-family block (body %d, M=%d, K=%d, mode=0x%x) outside the hand-off as words: %s", body, a.M, a.K, a.mode, why);
+  return fail(ETXB_E_UNSUPPORTED, m);
+}
 static int32_t check_attnf_block(const etxb_attnf_args& a) {
   const char* why = nullptr;
   if (a.NKV < 1 || a.NH < a.NKV || a.NH % a.NKV) why = "NH must be a positive multiple of NKV";
@@ -118,8 +142,10 @@ static int32_t check_attnf_block(const etxb_attnf_args& a) {
     if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8) || G % a.gq) why = "gq is 1, 2, 4 or 8 and divides NH / NKV";
     else if (a.HD != 128 || a.BS != 16 || (a.part_len & 0xffff) != 128) why = "the grouped form is head_dim 128, cache blocks of 16, partitions of 128";
     else if (a.gq * a.max_parts > 4096) why = "gq * max_parts <= 4096";
-    else if ((a.part_len >> 24) & ~1) why = "part_len bits 25..31 are zero";
-    else if ((a.part_len >> 24) && (a.nblocks > (uint32_t)(a.NH / a.gq) || a.max_parts * a.gq > ETXB_GQ_WHOLE_MAX))
+    else if (a.part_len < 0 || ((a.part_len & ETXB_GQ_WHOLE) && (a.part_len >> ETXB_GQ_LIM_SHIFT))) why = "part_len bit 31 is zero, bits 26..30 with partitions only";
+    else if ((a.part_len & ETXB_GQ_WORDS) && ((a.part_len & ETXB_GQ_WHOLE) || !a.exp_sums || ((uintptr_t)a.exp_sums & 3) || ((uintptr_t)a.qkv & 15)))
+      why = "hand-off as words: partitions, qkv 16-byte aligned, exp_sums names the words of the outputs";
+    else if ((a.part_len & ETXB_GQ_WHOLE) && (a.nblocks > (uint32_t)(a.NH / a.gq) || a.max_parts * a.gq > ETXB_GQ_WHOLE_MAX))
       why = "whole-sequence form: the grid is NH / gq tasks and max_parts * gq <= 157 (longer contexts: partitions)";
     else if (a.nblocks > (uint32_t)(a.max_parts * (a.NH / a.gq))) why = "the grid is at most max_parts * NH / gq tasks";
   } else {
@@ -200,7 +226,8 @@ static int32_t check_block(int body, const unsigned char* blk, size_t bytes) {
     if (bytes < sizeof(etxb_gemv_args)) return fail(ETXB_E_ARG, "GEMV-family tile: the argument block is 160 bytes");
     etxb_gemv_args a;
     memcpy(&a, blk, sizeof a);
-    return check_gemv_block(body, a);
+    const int32_t rc = check_gemv_block(body, a);
+    return rc ? rc : check_gemv_words(body, a, blk, bytes);
   }
   if (body == ETXB_BODY_ATTN_FUSED) {
     if (bytes < sizeof(etxb_attnf_args)) return fail(ETXB_E_ARG, "attn_fused tile: the argument block is 176 bytes");
@@ -233,7 +260,7 @@ static bool batched_plan(const etxb_session* s, const std::vector<unsigned char>
     etxb_attnf_args a;
     if (off < 0 || (uint64_t)off + sizeof a > pool.size()) return false;
     memcpy(&a, pool.data() + off, sizeof a);
-    if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8)) return false;
+    if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8) || (a.part_len & ETXB_GQ_WORDS)) return false;
   }
   return true;
 }
@@ -258,7 +285,7 @@ static int select_variant(const etxb_session* s, const std::vector<unsigned char
       if (off + sizeof(etxb_attnf_args) > pool.size()) return 0;
       etxb_attnf_args a;
       memcpy(&a, pool.data() + off, sizeof a);
-      if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8) || a.HD != 128 || a.BS != 16 || (a.part_len & 0xffff) != 128 || (a.part_len >> 24)) return 0;
+      if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8) || a.HD != 128 || a.BS != 16 || (a.part_len & 0xffff) != 128 || (a.part_len & ETXB_GQ_WHOLE)) return 0;
       if (any_attn && a.gq != gq) return 0;
       gq = a.gq; any_attn = true;
     } else {
@@ -398,6 +425,38 @@ static void share_merges(etxb_session* s) {
 }
 
 // ---- plan blob ------------------------------------------------------------------------------------------------
+// Tasks whose producer need not find the expert ids again: the streaming task before in the same queue has a top-k fold over the same logits with
+// the same parameters, and waited for the event that this one waits for before it reads them (whoever rewrites the logits in between
+// would have to know that this task is done).
+static void share_routing(const etxb_session* s, std::vector<etxb_rec>& recs) {
+  auto block = [&](int32_t i, etxb_gemv_args& a) {
+    const etxb_task& t = s->tasks[i];
+    const etxb_type& ty = s->types[t.type];
+    const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
+    if (ty.args[0] != 0 || off < 0 || (uint64_t)off + sizeof a > s->h_pool.size()) return false;
+    memcpy(&a, s->h_pool.data() + off, sizeof a);
+    const int j = t.coord[0];
+    return (a.mode & 0xff) >= 2 && a.tpe > 0 && a.rpt > 0 && j >= 0 && j < (int)a.nblocks && (long long)(j % a.tpe) * a.rpt < a.M;   // (a task with rows: its producer looks)
+  };
+  for (uint32_t w = 0; w < s->h.n_workers; ++w) {
+    int32_t prev = -1;                                             // the streaming task before
+    for (int32_t i = s->qbegin[w]; i < s->qbegin[w + 1]; ++i) {
+      const int body = s->types[s->tasks[i].type].body;
+      if (body < ETXB_BODY_GEMV || body > ETXB_BODY_MOE_DOWN) continue;
+      etxb_gemv_args a, b;
+      if (body != ETXB_BODY_GEMV && prev >= 0 && s->types[s->tasks[prev].type].body != ETXB_BODY_GEMV && block(prev, b) && block(i, a)) {
+        const uint32_t same = 0x0f0000ffu | ETXB_MODE_WORDS_IN;    // fold, always-on experts, where the logits come from
+        const int32_t ev = s->types[s->tasks[i].type].stream_word, pev = s->types[s->tasks[prev].type].stream_word;
+        bool waited = pev == ev;
+        if (pev == -2)
+          for (int k = 0; k < s->tasks[prev].in_n; ++k) waited = waited || s->inwords[s->tasks[prev].in_off + k] == ev;
+        if (ev >= 0 && waited && a.logits == b.logits && a.E == b.E && a.R == b.R && ((a.mode ^ b.mode) & same) == 0 && recs[i].in_n < ETXB_IN_ROUTED) recs[i].in_n |= ETXB_IN_ROUTED;
+      }
+      prev = i;
+    }
+  }
+}
+
 static size_t al8(size_t x) { return (x + 7) & ~size_t(7); }
 
 static int32_t parse_plan(etxb_session* s, const unsigned char* b, size_t n) {
@@ -496,6 +555,8 @@ extern "C" int32_t etxb_create(const void* plan_blob, size_t bytes, int device, 
   *out = nullptr;
   etxb_session* s = new etxb_session();
   s->device = device;
+  static std::atomic<uint32_t> sessions{0};
+  s->salt = sessions.fetch_add(1u) * 2749u;
   int32_t rc = prepare_kernel(device, &s->workers);
   if (rc == ETXB_OK) rc = parse_plan(s, (const unsigned char*)plan_blob, bytes);
   if (rc == ETXB_OK && (int)s->h.n_workers > s->workers) rc = fail(ETXB_E_RESIDENCY, "plan wants more workers than the device has SMs");
@@ -747,6 +808,24 @@ static int32_t upload_type_args(etxb_session* s) {
     const bool has_block = ty.body >= ETXB_BODY_GEMV && ty.args[0] >= 0;
     r.args = has_block ? (uint64_t)(uintptr_t)ta[(size_t)t.type * ETXB_MAX_ARGS] + (uint64_t)ty.cst[0] + (uint64_t)t.coord[1] * (uint64_t)ty.cst[1]
                        : (uint64_t)(uintptr_t)s->d_pool;
+    // a grid whose readers look at words announces itself without waiting for its stores
+    const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
+    bool words = false;
+    if (ty.args[0] == 0 && off >= 0 && (ty.body == ETXB_BODY_GEMV || ty.body == ETXB_BODY_MOE_UP || ty.body == ETXB_BODY_MOE_DOWN) && (uint64_t)off + sizeof(etxb_gemv_args) <= s->h_pool.size()) {
+      etxb_gemv_args a;
+      memcpy(&a, s->h_pool.data() + off, sizeof a);
+      etxb_gemv_words w;
+      if ((a.mode & ETXB_MODE_WORDS_OUT) && (uint64_t)off + sizeof a + sizeof w <= s->h_pool.size()) {
+        memcpy(&w, s->h_pool.data() + off + sizeof a, sizeof w);
+        words = w.out != nullptr;                                  // (null: its readers take the bf16 vector)
+      }
+    } else if (ty.args[0] == 0 && off >= 0 && ty.body == ETXB_BODY_ATTN_FUSED && (uint64_t)off + sizeof(etxb_attnf_args) <= s->h_pool.size()) {
+      etxb_attnf_args a;
+      memcpy(&a, s->h_pool.data() + off, sizeof a);
+      words = a.gq > 0 && (a.part_len & ETXB_GQ_WORDS) != 0;
+    }
+    if (words && s->xbase != nullptr) return fail(ETXB_E_UNSUPPORTED, "a sharded session hands rows over as flagged words of its exchange region only");
+    if (words && t.out_n < ETXB_OUT_RELAXED) r.out_n |= ETXB_OUT_RELAXED;
     r.stream_word = ty.stream_word;
     r.mirror = s->merge[i];
     if (s->xbase != nullptr && ty.exchange) {
@@ -754,9 +833,11 @@ static int32_t upload_type_args(etxb_session* s) {
       if (rc) return rc;
     }
   }
+  std::vector<etxb_rec> routed = recs;
+  share_routing(s, routed);
   if (!s->d_recs) CU(cudaMalloc((void**)&s->d_recs, recs.size() * sizeof(etxb_rec) + 96));
-  CU(cudaMemcpy(s->d_recs, recs.data(), recs.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
-  // the same records grouped by grid (type), worker by worker, for the one-launch-per-grid baseline
+  CU(cudaMemcpy(s->d_recs, routed.data(), routed.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
+  // the same records (every launch finds its own expert ids) grouped by grid (type), worker by worker, for the one-launch-per-grid baseline
   const uint32_t W = s->h.n_workers, NT = s->h.n_types;
   std::vector<etxb_rec> ug; ug.reserve(recs.size());
   std::vector<int32_t> uq((size_t)NT * (W + 1), 0);
@@ -788,7 +869,7 @@ static void fill_params(etxb_session* s, etxb_params& p) {
   p.events = s->d_events; p.evcount = s->d_evcount; p.inwords = s->d_inwords; p.outwords = s->d_outwords;
   p.ctrl = s->d_ctrl; p.trace = s->trace ? s->d_trace : nullptr; p.exec_count = s->trace ? s->d_exec : nullptr;
   p.step_dev = nullptr; p.timeout_ns = s->timeout_ns; p.epoch = s->epoch; p.n_workers = (int32_t)s->h.n_workers;
-  p.step = s->step;
+  p.step = s->step; p.salt = s->salt;
   p.n_peers = s->n_ranks - 1; p.rank = s->rank; p.xargmax = s->xargmax; p.tc_on = s->tc_on ? 1u : 0u; p.xbase = s->xbase;
   for (int q = 0; q < ETXB_MAX_PEERS; ++q) p.xpeer[q] = s->xpeer[q];
 }
@@ -993,6 +1074,10 @@ extern "C" int32_t etxb_op_launch(int device, int32_t body, const void* argblock
   if (!(body == ETXB_BODY_GEMV && bytes >= sizeof(etxb_gemv_args) && ((const etxb_gemv_args*)argblock)->nb > 1)) {
     rc = check_block(body, (const unsigned char*)argblock, bytes);      // (the column-batched kernel checks its own limits below)
     if (rc) return rc;
+    bool words = false;
+    if (body == ETXB_BODY_GEMV || body == ETXB_BODY_MOE_UP || body == ETXB_BODY_MOE_DOWN) words = (((const etxb_gemv_args*)argblock)->mode & (ETXB_MODE_WORDS_IN | ETXB_MODE_WORDS_OUT)) != 0;
+    else if (body == ETXB_BODY_ATTN_FUSED) words = ((const etxb_attnf_args*)argblock)->gq > 0 && (((const etxb_attnf_args*)argblock)->part_len & ETXB_GQ_WORDS) != 0;
+    if (words) return fail(ETXB_E_UNSUPPORTED, "hand-off as words: the flags are a session's step, a single tile has none");
   }
   cudaStream_t st = (cudaStream_t)cuda_stream;
   if (body == ETXB_BODY_GEMV && bytes >= sizeof(etxb_gemv_args) && ((const etxb_gemv_args*)argblock)->nb > 1) {

@@ -46,6 +46,8 @@
 #define ETXB_CTX_BYTES 288           // one prefetched task context: 96-byte record + 192 bytes of argument block
 #define ETXB_CTX_SLOTS 4
 #define ETXB_SMEM_BYTES (ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4 + 512 + ETXB_CTX_SLOTS * ETXB_CTX_BYTES)
+#define ETXB_OUT_RELAXED 0x10000     // etxb_rec.out_n: the arrivals need not wait for the task's stores (its readers look at words)
+#define ETXB_IN_ROUTED 0x10000        // etxb_rec.in_n: the streaming task before this one in the queue waited for the same event and found the same expert ids
 #define ETXB_ATTN_PART 32            // KV positions per attention task
 #define ETXB_MAX_PEERS 7           // ranks of a sharded model besides this one
 #define ETXB_MAX_NB 8                // activation columns of the stand-alone batched GEMV kernel
@@ -132,6 +134,7 @@ struct etxb_params {
                                                    // argmax (lm_head split by vocabulary); 0 = every rank holds all logits
   unsigned char* xbase;
   unsigned char* xpeer[ETXB_MAX_PEERS];
+  uint32_t salt, pad;                              // added to the epoch in the flags of words on this GPU: sessions that share buffers differ
 };
 
 // ctrl[0] bits
@@ -165,9 +168,22 @@ struct etxb_gemv_args {
 #define ETXB_MODE_ROUTE_READY 0x800   // MoE down with the top-k fold: the gate/up tiles it waits for have published the routing in
                                       // ids / wts, so the consumer warps read it there (one load) instead of redoing the top-k;
                                       // the producer warp, which runs ahead of the gate/up phase, still derives it from the logits
+// Hand-off as words (one GPU, one token; excludes ETXB_MODE_FLAGGED).  A value travels as a 4-byte word, bf16 in the low half and a flag of the
+// step in the high half: the words say themselves whether they have arrived, so the grid that writes them announces itself without
+// waiting for its stores (a relaxed arrival), and the grid that reads them looks at the flags.  The block is followed by an
+// etxb_gemv_words.
+#define ETXB_MODE_WORDS_IN 0x2000     // x (plain, gate+up, down), rows and resid_in (norm fold), logits (top-k fold) name words; down: routing from words, too
+#define ETXB_MODE_WORDS_OUT 0x4000    // results (and z, x of a norm fold, routing of a gate+up grid) are also written as words
 // bits 16..23 of mode: expert slots per task of the MoE forms (0 = 1)
 // bits 24..27 of mode (top-k fold): ns always-on experts stored after the E routed ones (DeepSeek's shared experts as
 // experts E .. E + ns - 1): the fold picks R - ns experts from the logits and gives the last ns slots weight 1
+
+// Behind the block of a grid with a words mode bit (bytes 160..191).  A word is written once per step: every grid has words of its own.
+struct etxb_gemv_words {
+  uint32_t* out;             // results: [M] (gate+up: [slots][M])
+  uint32_t* z; uint32_t* x;  // norm fold: [K] sum, [K] normed vector; null: nobody reads it
+  uint32_t* route;           // gate+up writes, down reads: 16 expert ids, then 16 (weight, flag) pairs
+};
 
 // top-k: the reference's 64-byte block (etx/ops/topk.py:16-23), grid words at 48.
 struct etxb_topk_args {
@@ -205,6 +221,8 @@ struct etxb_attnf_args {
   int32_t gq, part_len;   // 152..159: gq > 0 selects the grouped form (gq q heads x 128 positions per task, task = part * (NH / gq) + group);
                           // part_len: bits 0..15 = 128, bits 16..23 = a tag that tells the grids sharing the partial buffers apart (the layer),
                           // bit 24 = whole-sequence form: task = q group, takes every partition (the batched step)
+                          // bits 26..30: contexts of up to so many partitions are taken whole, by the tasks of the first partition
+                          // bit 25 = hand-off as words (partitions): qkv names words, the outputs are also written as words at exp_sums
   uint32_t grid[3], nblocks;                                                                                    // 160..175
 };
 

@@ -30,6 +30,8 @@ namespace etxb {
 
 #define ETXB_GQ_PART 128   // positions per task
 #define ETXB_GQ_WHOLE (1 << 24)   // part_len bit: one task per (sequence, q group) takes all partitions
+#define ETXB_GQ_WORDS (1 << 25)   // part_len bit: qkv names words, the outputs are also written as words (at exp_sums)
+#define ETXB_GQ_LIM_SHIFT 26      // part_len bits 26..31: contexts of up to so many partitions are taken whole, by the tasks of the first one
 #define ETXB_GQ_WHOLE_MAX 157     // .. of partitions x q heads at most (the builder's rule: ops/attn.py)
 #define ETXB_GQ_PW 136     // 8-byte (value, flag) pairs a task publishes per q head and partition: 128 outputs, max, sum, padding
 #define ETXB_GQ_SHARE 64   // partials (gq x partitions) from which the merge is shared out.  Shared / by one task, us of a phase: 72 partials (8 sequences)
@@ -102,25 +104,26 @@ struct GqTask {
   int t0, u0, nu;            // first position; first unit (cache block) and number of units
   int seq;
   long long pos;
-  bool whole, owner;         // owner: the task's positions hold the one being written
+  bool whole, owner;         // whole: one task per group takes all of the context; owner: the task's positions hold the one being written
 };
 __device__ __forceinline__ GqTask gq_task(const etxb_attnf_args& d, int blk, const etxb_stepv& S) {
   GqTask t;
   // the step's own buffers hold what the prologue wrote from the step parameters: take the values from there
   t.pos = (const void*)d.positions == (const void*)S.positions ? (long long)S.pos : __ldcg((const long long*)d.positions);
   t.seq = (const void*)d.seq_lens == (const void*)S.seq_lens ? S.pos + 1 : __ldcg(d.seq_lens);
-  t.whole = (d.part_len & ETXB_GQ_WHOLE) != 0;
+  const bool form = (d.part_len & ETXB_GQ_WHOLE) != 0;
   const int lg = 31 - __clz(d.gq), NQG = d.NH >> lg;               // (gq: 1, 2, 4 or 8)
-  t.part = t.whole ? 0 : udiv_small(blk, NQG);
+  t.part = form ? 0 : udiv_small(blk, NQG);
   t.hq0 = (blk - t.part * NQG) << lg;
   t.h = udiv_small(t.hq0 * d.NKV, d.NH);
   t.t0 = t.part * ETXB_GQ_PART;
   const int np = min((t.seq + ETXB_GQ_PART - 1) / ETXB_GQ_PART, d.max_parts);
-  const int tend = t.whole ? np * ETXB_GQ_PART : t.t0 + ETXB_GQ_PART;
-  t.owner = t.pos >= t.t0 && t.pos < tend;
+  t.whole = form || np <= (int)((uint32_t)d.part_len >> ETXB_GQ_LIM_SHIFT);    // (the tasks of the other partitions have nothing to do then)
+  const int tend = t.whole && t.part == 0 ? np * ETXB_GQ_PART : t.t0 + ETXB_GQ_PART;
+  t.owner = t.pos >= t.t0 && t.pos < tend && !(t.whole && t.part > 0);
   const int lim = t.owner ? max(t.seq, (int)t.pos + 1) : t.seq;
   t.u0 = t.t0 >> 4;
-  t.nu = t.t0 < t.seq && tend > t.t0 ? (min(tend, lim) - t.t0 + 15) >> 4 : 0;
+  t.nu = t.t0 < t.seq && tend > t.t0 && !(t.whole && t.part > 0) ? (min(tend, lim) - t.t0 + 15) >> 4 : 0;
   return t;
 }
 
@@ -201,7 +204,7 @@ __device__ __forceinline__ void head_norm_rope_r(uint2 x, float* xh, bool norm, 
     *(float4*)(xh + 4 * lane) = make_float4(v[0], v[1], v[2], v[3]);
     __syncwarp();
     const float ss = sumsq128_numpy_order_warp(xh);
-    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, 128.0f), eps)));
+    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(ss, 0.0078125f), eps)));
 #pragma unroll
     for (int j = 0; j < 4; ++j) v[j] = bfr(__fmul_rn(wf[j], bfr(__fmul_rn(v[j], r))));
   }
@@ -213,6 +216,19 @@ __device__ __forceinline__ void head_norm_rope_r(uint2 x, float* xh, bool norm, 
   }
 }
 
+template <bool WD>
+__device__ __forceinline__ void gq_out(const etxb_attnf_args& d, const Smem& sm, int i, float v) {
+  if (WD && (d.part_len & ETXB_GQ_WORDS)) st_word((uint32_t*)d.exp_sums + i, bf_bits(v) | s_vars.flag);
+  ((__nv_bfloat16*)d.out)[i] = __float2bfloat16_rn(v);
+}
+// one row of 128 values of this step's qkv, four per lane
+template <bool WD>
+__device__ __forceinline__ uint2 gq_row(const etxb_attnf_args& d, const Smem& sm, int row) {
+  const int lane = tidx() & 31;
+  if (WD && (d.part_len & ETXB_GQ_WORDS)) return words_pack(poll_words4((const uint32_t*)d.qkv + row * 128 + 4 * lane, s_vars.flag));
+  return __ldcg((const uint2*)((const __nv_bfloat16*)d.qkv + (size_t)row * 128) + lane);
+}
+
 // out[h][:] = bf16(sum_p w_p * tmp[p][:] / sum_p w_p * l_p), w_p = exp(m_p - max m), for the 32-value slices mi, mi + mk, .. of the
 // group's gq * 128 output values.  Polls the flagged partials the other CTAs publish (L2).  A warp takes a slice and a share of the
 // partitions (its lane: one value); every warp works out its head's weights itself from the partitions' statistics.
@@ -220,6 +236,7 @@ __device__ __forceinline__ void head_norm_rope_r(uint2 x, float* xh, bool norm, 
 // the sequences of a batch and between plans, and equal columns get equal bits.  Past 16 partitions shared merges fetch 32 at a time, four
 // warps a slice; below, a warp a slice (all 16 slices of a round at once): against two warps, a phase of 8 sequences at 1033 positions 21.4 us /
 // 22.3, of 16 at 1400 48.9 / 50.7, of 3 at 1400 13.3 / 13.4.  (As many warps as the slices of a task left free, 1 to 16: 22.4, 49.2 and 14.1.)
+template <bool WD>
 __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Smem& sm, float* mg, int hq0, int np, uint32_t fl, int mi, int mk) {
   constexpr int HD = 128, NF = 8;
   const int lane = tidx() & 31, warp = tidx() >> 5;
@@ -275,7 +292,7 @@ __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Sm
       if (sub == 0)
         for (int q = 1; q < wps; ++q) o = __fadd_rn(o, mg[(warp + q * per) * 32 + lane]);
     }
-    if (on && sub == 0) ((__nv_bfloat16*)d.out)[(size_t)hq0 * HD + sl * 32 + lane] = __float2bfloat16_rn(__fdiv_rn(o, L));
+    if (on && sub == 0) gq_out<WD>(d, sm, hq0 * HD + sl * 32 + lane, __fdiv_rn(o, L));
     if (s0 + per < nsl && wps > 1) csync();
   }
 }
@@ -285,6 +302,8 @@ __device__ __forceinline__ void attn_gq_merge(const etxb_attnf_args& d, const Sm
 // a circle); else count << 16 | index + 1: the host has found that the workers' LAST tasks of the grid may wait for all the others (the order of the
 // queues and the events leave no circle: waiting_grids), and this is one of `count` such tasks of the group, each of which merges a share; 0xffff: it is not one of them, others are.  Shared out from
 // gq * np = ETXB_GQ_SHARE on only: with few partials the last partition's task alone is as quick, and the other tasks are done.
+// WD: the kernel's plans may hand the rows over as words.
+template <bool WD>
 __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, const Smem& sm, const etxb_stepv& S, uint32_t& n, uint32_t mg) {
   constexpr int HD = 128, BS = 16;
   const GqTask t = gq_task(d, blk, S);
@@ -300,7 +319,7 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
     if (warp < gq || (warp == gq && newrow)) {
       const bool isq = warp < gq;
       const void* nwp = isq ? d.qw : d.kw;
-      const uint2 x = __ldcg((const uint2*)((const __nv_bfloat16*)d.qkv + (size_t)(isq ? t.hq0 + warp : d.NH + t.h) * HD) + lane);
+      const uint2 x = gq_row<WD>(d, sm, isq ? t.hq0 + warp : d.NH + t.h);
       const uint2* cs = (const uint2*)((const __nv_bfloat16*)d.cos_sin + (size_t)t.pos * HD);
       const uint2 nw = nwp ? __ldg((const uint2*)nwp + lane) : make_uint2(0u, 0u), c = __ldg(cs + (lane & 15)), sn = __ldg(cs + 16 + (lane & 15));
       float o[4];
@@ -315,7 +334,7 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
         }
       }
     } else if (warp == gq + 1 && newrow) {
-      const uint2 x = __ldcg((const uint2*)((const __nv_bfloat16*)d.qkv + (size_t)(d.NH + NKV + t.h) * HD) + lane);
+      const uint2 x = gq_row<WD>(d, sm, d.NH + NKV + t.h);
       *(uint2*)(s.vnew + 4 * lane) = x;
       if (t.hq0 * NKV == t.h * d.NH) {
         const long long slot = (const void*)d.slot_mapping == (const void*)S.slot_mapping ? (long long)S.pos : __ldcg((const long long*)d.slot_mapping);
@@ -425,7 +444,7 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
         const uint32_t h0 = movmatrix(pack_bf(c[0], c[1])), h1 = movmatrix(pack_bf(c[2], c[3]));
         const uint32_t w0 = movmatrix(pack_bf(r[0], r[1])), w1 = movmatrix(pack_bf(r[2], r[3]));
         uint32_t x0 = 0u, x1 = 0u;
-        const bool third = !t.whole || ragged;
+        const bool third = !(d.part_len & ETXB_GQ_WHOLE) || ragged;
         if (third) {                                               // what the second rounding lost
 #pragma unroll
           for (int j = 0; j < 4; ++j) r[j] = __fsub_rn(r[j], bfr(r[j]));
@@ -504,21 +523,24 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
     csync();
     mark(sm, 1);
     for (int idx = tid; idx < gq * HD; idx += ETXB_CONSUMERS) {
-      const int g = idx >> 7, dd = idx & (HD - 1);
-      float M = -INFINITY;
+      // a warp's 32 outputs are one head's: lane w works out slot w's factor (one exponential instead of eight), the sums take them by shuffle.
+      // (Every thread for itself: 1900 clocks of the phase with one q head to 1100 outputs.)
+      const int g = idx >> 7, dd = idx & (HD - 1), w0 = lane & 7;
+      const float2 ml = w0 < nslot ? *(const float2*)(s.st + (w0 * 8 + g) * 2) : make_float2(-INFINITY, 0.f);
+      float M = ml.x;
 #pragma unroll
-      for (int w = 0; w < 8; ++w) M = fmaxf(M, w < nslot ? s.st[(w * 8 + g) * 2] : -INFINITY);
-      const float Mz = M == -INFINITY ? 0.f : M;
-      float o = 0.f, L = 0.f;
+      for (int o = 1; o < 8; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+      const float f = expf(__fsub_rn(ml.x, M == -INFINITY ? 0.f : M));
+      float o = 0.f, L = __fmul_rn(f, ml.y);
 #pragma unroll
-      for (int w = 0; w < 8; ++w)
-        if (w < nslot) {
-          const float f = expf(__fsub_rn(s.st[(w * 8 + g) * 2], Mz));
-          L = __fmaf_rn(f, s.st[(w * 8 + g) * 2 + 1], L);
-          o = __fmaf_rn(f, s.po[w * 1152 + g * 132 + dd], o);
-        }
+      for (int x = 1; x < 8; x <<= 1) L = __fadd_rn(L, __shfl_xor_sync(0xffffffffu, L, x));
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        const float fw = __shfl_sync(0xffffffffu, f, w);
+        if (w < nslot) o = __fmaf_rn(fw, s.po[w * 1152 + g * 132 + dd], o);
+      }
       if (t.whole || np == 1) {
-        ((__nv_bfloat16*)d.out)[(size_t)t.hq0 * HD + idx] = __float2bfloat16_rn(__fdiv_rn(o, L));
+        gq_out<WD>(d, sm, t.hq0 * HD + idx, __fdiv_rn(o, L));
       } else {
         uint2* pw = (uint2*)d.tmp_out + ((size_t)(t.hq0 + g) * d.max_parts + t.part) * ETXB_GQ_PW;
         st_pair(pw + dd, o, fl);
@@ -530,7 +552,7 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
   // (a merge never looks past the partitions the grid computed, whatever seq_lens says)
   if (gq * np < ETXB_GQ_SHARE) mg = 0u;
   if (!t.whole && np > 1) {
-    if (mg == 0u ? t.part == np - 1 : mg != 0xffffu) attn_gq_merge(d, sm, s.mg, t.hq0, np, fl, mg == 0u ? 0 : (int)(mg & 0xffffu) - 1, mg == 0u ? 1 : (int)(mg >> 16));
+    if (mg == 0u ? t.part == np - 1 : mg != 0xffffu) attn_gq_merge<WD>(d, sm, s.mg, t.hq0, np, fl, mg == 0u ? 0 : (int)(mg & 0xffffu) - 1, mg == 0u ? 1 : (int)(mg >> 16));
   }
   mark(sm, 3);
 }

@@ -33,12 +33,19 @@ struct GemvTask {
 };
 // How the consumer warps share a task's stages.  Worked out by one warp while the task's event is being waited for (the
 // few integer divisions in it take longer than a short task's multiplications) and read by all through shared memory.
-//   rps    rows per stage,  ns  stages of the task
+//   rps    rows per stage (at most),  ns  stages of the task,  spr  stages per range where no stage crosses a range's end, else 0
 //   W      warps per stage (a divisor of ETXB_EMPTY_COUNT),  NG <= min(16 / W, ETXB_NSTAGE) groups: group g takes stages g, g + NG, ..
-//   R      rows a warp multiplies at once: rows wi, wi + W, .. of the stage
-struct GemvGeom {
+//   S      warps that share a row: warp h of them multiplies the vectors h * 32 + lane, (h + S) * 32 + lane, ..
+//   R      rows a warp multiplies at once: rows wi / S, wi / S + rw, .. of the stage, rw = W / S
+struct __align__(16) GemvGeom {
   GemvTask t;
-  int rps, ns, W, NG, R, wmul;                                     // wmul: warp w belongs to group (w * wmul) >> 8
+  int rps, ns, W, NG, R, S, rw, spr;
+  int wmul;                                                        // warp w belongs to group (w * wmul) >> 8
+  int cnt, shared;                                                 // arrivals of a warp per stage; a stage's uses may belong to different groups (see consume_task)
+  int few;                                                         // at most 16 rows, of at most 2048 values
+  int direct;                                                      // results go straight to memory: a plain task whose vector nobody takes as words
+  int one;                                                         // rows longer than 2048 values that go one at a time
+  float rspr;                                                      // 1 / spr (0: no ranges): stage s belongs to range (s + 0.5) * rspr
 };
 
 // What the tiles read of the running launch and task now and then: kept in shared memory, where it costs no registers.
@@ -46,6 +53,7 @@ struct CtaVars {
   int32_t* ctrl;
   uint64_t* tr;              // 8 stamps of the running task when tracing, else null (slots 4..7 are in-body marks)
   uint32_t epoch;            // the step (sharded sessions: the flag of this step's exchanged words derives from it)
+  uint32_t flag;             // flag of this step's words on this GPU (of the step and the session)
   int cur;                   // the running task's index in the queue order (reported when a wait gives up)
   int q0, q1;                // the CTA's queue
   int done;                  // tasks of the queue before this one are over (kernels whose other tiles use the ring's memory too)
@@ -68,8 +76,14 @@ struct Smem {
   __device__ __forceinline__ uint32_t epoch() const { return vars ? vars->epoch : 0u; }
   __device__ __forceinline__ int cur() const { return vars->cur; }
 };
+// The persistent kernel's shared memory beside the dynamic part.  At namespace scope so that the tiles that are calls find
+// it at known addresses too: passed by reference, Smem would live on the stack; passed by value, in registers.
+__shared__ int s_stop;
+__shared__ unsigned long long s_deadline;
+__shared__ GemvGeom s_geo;
+__shared__ CtaVars s_vars;
 // in-body time stamp k (0..3) of the running task; thread 0 only, no-op unless tracing
-__device__ __forceinline__ void mark(const Smem& sm, int k) { if (sm.tr() != nullptr && tidx() == 0) sm.tr()[4 + k] = globaltimer(); }
+__device__ __forceinline__ void mark(const Smem& sm, int k) { if (tidx() == 0 && sm.tr() != nullptr) sm.tr()[4 + k] = globaltimer(); }
 __device__ __forceinline__ __nv_bfloat16* smem_xb(const Smem& sm) { return (__nv_bfloat16*)((unsigned char*)sm.xs + ETXB_XB_OFF); }
 __device__ __forceinline__ float* smem_g(const Smem& sm) { return (float*)((unsigned char*)sm.xs + ETXB_G_OFF); }
 
@@ -122,20 +136,59 @@ __device__ __forceinline__ bool wait_done(const Smem& sm, int cur) {
   }
   return true;
 }
+// Between two looks at words that are not there yet: false when the step is being abandoned (see mbar_wait).
+__device__ __noinline__ bool words_again(uint32_t& spins, uint32_t fl) {
+  if ((++spins & 63u) == 0) {
+    int32_t* ctrl = s_vars.ctrl;
+    if (ld_relaxed(ctrl) != 0) { *(volatile int*)&s_stop = 1; return false; }
+    if ((spins & 1023u) == 0 && globaltimer() > s_deadline) {
+      if (atomicOr(ctrl, ETXB_CTRL_TIMEOUT) == 0) { ctrl[1] = s_vars.cur; ctrl[2] = -4; ctrl[3] = 0; ctrl[4] = (int32_t)(fl >> 16); }
+      *(volatile int*)&s_stop = 1;
+      return false;
+    }
+    __nanosleep(32);
+  }
+  return true;
+}
+__device__ __forceinline__ uint32_t poll_word(const uint32_t* p, uint32_t fl) {
+  uint32_t v, spins = 0;
+  do v = ld_word(p); while (((v ^ fl) >> 16) != 0u && words_again(spins, fl));
+  return v;
+}
+__device__ __forceinline__ uint4 poll_words4(const uint32_t* p, uint32_t fl) {
+  uint4 v;
+  uint32_t spins = 0;
+  do v = ld_words4(p); while (words_miss(v, fl) != 0u && words_again(spins, fl));
+  return v;
+}
 // ---------------------------------------------------------------------------------------------- top-k
 // softmax over E bf16 logits (fp32), K rounds of argmax with the lower index winning ties, optional renormalisation
 // over the selected weights (numpy's summation order for <= 16 values), optional bf16 rounding of the weights.
-// One warp (all 32 lanes call); E <= 256, K <= 16.  ids / wts / tei may point to shared or global memory.
+// One warp (all 32 lanes call); E <= 256, K <= 16.  fl: 0, or the flag of the words that `logits` names.  ids / wts / tei may point to shared or global memory.
 template <int NK>
-__device__ __forceinline__ void warp_topk_n(const void* logits, int E, int K, bool renorm, bool bf16w,
+__device__ __forceinline__ void warp_topk_n(const void* logits, uint32_t fl, int E, int K, bool renorm, bool bf16w,
                                             int32_t* ids, float* wts, int32_t* tei) {
   const int lane = tidx() & 31;
   float p[NK];
   float m = -INFINITY;
+  if (fl != 0u) {                                                  // (all loads, then a look at their flags)
+    uint32_t u[NK], spins = 0, miss;
+    do {
+      miss = 0u;
+#pragma unroll
+      for (int k = 0; k < NK; ++k) u[k] = ld_word((const uint32_t*)logits + min(lane + 32 * k, E - 1));
+#pragma unroll
+      for (int k = 0; k < NK; ++k) miss |= (u[k] ^ fl) >> 16;
+    } while (miss != 0u && words_again(spins, fl));
+#pragma unroll
+    for (int k = 0; k < NK; ++k) p[k] = bf_lo(u[k]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < NK; ++k) p[k] = ld_bf(logits, min(lane + 32 * k, E - 1));
+  }
 #pragma unroll
   for (int k = 0; k < NK; ++k) {
-    const int e = lane + 32 * k;
-    p[k] = e < E ? ld_bf(logits, e) : -INFINITY;
+    if (lane + 32 * k >= E) p[k] = -INFINITY;
     m = fmaxf(m, p[k]);
   }
   m = warp_max(m);
@@ -208,10 +261,10 @@ __device__ __forceinline__ void warp_topk_n(const void* logits, int E, int K, bo
 
 // LEAN: the form the host picks when every top-k of the plan has E <= 128 (no code for more experts in that kernel).
 template <bool LEAN>
-__device__ __noinline__ void warp_topk(const void* logits, int E, int K, bool renorm, bool bf16w,
+__device__ __noinline__ void warp_topk(const void* logits, uint32_t fl, int E, int K, bool renorm, bool bf16w,
                                        int32_t* ids, float* wts, int32_t* tei) {
-  if (LEAN || E <= 128) warp_topk_n<4>(logits, E, K, renorm, bf16w, ids, wts, tei);
-  else warp_topk_n<8>(logits, E, K, renorm, bf16w, ids, wts, tei);
+  if (LEAN || E <= 128) warp_topk_n<4>(logits, fl, E, K, renorm, bf16w, ids, wts, tei);
+  else warp_topk_n<8>(logits, fl, E, K, renorm, bf16w, ids, wts, tei);
 }
 
 __device__ __forceinline__ void tile_topk(const unsigned char* a, int blk, const Smem& sm) {
@@ -220,7 +273,7 @@ __device__ __forceinline__ void tile_topk(const unsigned char* a, int blk, const
   const int nb = (d.nbsv & 0xff) ? (d.nbsv & 0xff) : 1, sv = d.nbsv >> 8;
   const int w = tidx() >> 5;
   if (w >= nb) return;
-  warp_topk<false>((const __nv_bfloat16*)d.logits + (size_t)w * d.E, d.E, d.K, (d.mode & 0xff) == 1, (d.mode & ETXB_MODE_BF16_WTS) != 0,
+  warp_topk<false>((const __nv_bfloat16*)d.logits + (size_t)w * d.E, 0u, d.E, d.K, (d.mode & 0xff) == 1, (d.mode & ETXB_MODE_BF16_WTS) != 0,
             d.ids + (size_t)w * sv, d.wts + (size_t)w * sv, d.tei ? d.tei + (size_t)w * sv : nullptr);
 }
 
@@ -250,26 +303,62 @@ __device__ __forceinline__ int udiv_small(int a, int b) {
   if (r < 0) --q; else if (r >= b) ++q;
   return q;
 }
-// Rows at once (R) and warps per stage (W): one row at a time is a chain of waits, shared-memory latencies and shuffles that
-// 4 warps per scheduler do not hide; several rows share the activation vector with its unpacking and are reduced together.
-// Rows of up to 1792 values (7 vectors per lane): 4 at once; of 2048 (6 rows per stage): 3; longer ones: a stage holds 5
-// rows or fewer (of 4096: 3), one warp each (so too where every range has its own activation vector and 3 rows share nothing).  Clocks
-// per task, weights already in the ring, against one row per warp and every warp on every stage:
-// 35 rows of 2048: 5816 -> 3786; 8 x 14 rows of 768: 8972 -> 6486; 48 of 1536: 6277 -> 3701; 18 of 4096: 5420 -> 5293.
-__device__ __forceinline__ void gemv_geom(int body, GemvGeom& g) {
+// Rows at once (R), rows per stage and warps per stage (W).  The products are bound by the unpacking of bf16 on the integer pipe and by their
+// latencies: several rows at once share the activation vector with its unpacking and are reduced together, and 12 to 16 warps have to be at it.
+//   up to 16 rows of up to 2048 values: a warp each (or several, S), in stages that all have a group at once
+//   longer tasks, rows of up to 1792 values (7 vectors per lane): 4 at once; of 2048 (6 rows per stage): 3
+//   longer rows (5 to 1 per stage): 3 or 4 at once (of 2 or 1 per stage one) by two warps, a half of the row each; by four where the task is a stream of
+//   more stages than the ring has: a stage is given back sooner, and the last one is multiplied in a quarter of the time (a stand-alone 4096 -> 12288 GEMV
+//   ends 14.5 us after its start, 15.3 with a row per warp; 12 dense layers 1142 us with two warps everywhere, 1126 now)
+//   down grids of several slots: every slot has its own activations, so a stage holds rows of one slot
+// Clocks per task, weights already in the ring, before / now: 14 rows of 4096 (a row per warp before) 2650 / 2100; 8 x 14 rows of 768 (16-row stages
+// across the slots, activations unpacked per row) 6000 / 3700; 1 row of 2048 (three times by one warp) 1800 / 500; 11 of 1536 (by four warps) 1700 / 700.
+// 35 of 2048: 2400, 60 bytes per clock; the same loop without its loads 2800 (with indexing), without its products 2000.
+__device__ __forceinline__ int gemv_groups(int W) { return W <= 2 ? ETXB_NSTAGE : W == 3 ? 5 : W == 4 ? 4 : W <= 8 ? 2 : 1; }
+// rows per stage (0: a row longer than a stage) and stages per range: what the producer has to know
+__device__ __forceinline__ void gemv_stages(int body, int mode, GemvGeom& g) {
   const int total = g.t.nranges * g.t.n;
-  const int nvl = ((g.t.row_bytes >> 4) + 31) >> 5;
   g.rps = g.t.row_bytes > 0 && g.t.row_bytes <= ETXB_STAGE_BYTES ? udiv_small(ETXB_STAGE_BYTES, g.t.row_bytes) : 0;
-  g.ns = 0; g.W = 1; g.NG = ETXB_NSTAGE; g.R = 1;
-  if (total > 0 && g.rps > 0) {
-    g.ns = total < (1 << 21) ? udiv_small(total + g.rps - 1, g.rps) : (total + g.rps - 1) / g.rps;
-    g.R = nvl <= 7 ? 4 : (nvl <= 8 && !(body == 5 && g.t.nranges > 1) ? 3 : 1);
-    const int m = min(g.rps, total);
-    const int w = g.R == 4 ? (m + 3) >> 2 : (g.R == 3 ? udiv_small(m + 2, 3) : m);
-    g.W = w <= 4 ? w : w <= 6 ? 6 : w <= 8 ? 8 : w <= 12 ? 12 : 16;
-    g.NG = g.W <= 2 ? ETXB_NSTAGE : g.W == 3 ? 5 : g.W == 4 ? 4 : g.W <= 8 ? 2 : 1;
+  g.spr = 0;
+  // (a row's sums are the same whichever way the results go: S does not depend on it)
+  g.direct = body == 3 && total > ETXB_XF_FLOATS / 4 && !(mode & ETXB_MODE_WORDS_OUT);
+  g.few = total <= ETXB_CONSUMER_WARPS && g.t.row_bytes <= 4096;
+  if (total <= 0 || g.rps <= 0) return;
+  if (g.few) {
+    int r = min(g.rps, total);
+    r = r >= 16 ? 16 : r >= 12 ? 12 : r >= 8 ? 8 : r >= 6 ? 6 : r >= 4 ? 4 : r;
+#pragma unroll 1
+    while (r > 1 && r * gemv_groups(r) < total) r = r > 12 ? 12 : r > 8 ? 8 : r > 6 ? 6 : r > 4 ? 4 : r - 1;
+    g.rps = r;
   }
-  g.wmul = udiv_small(255 + g.W, g.W);                              // ceil(256 / W): exact for 16 warps and for ETXB_EMPTY_COUNT / W
+  if (body == 5 && g.t.nranges > 1) {
+    g.spr = udiv_small(g.t.n + g.rps - 1, g.rps);
+    g.rps = udiv_small(g.t.n + g.spr - 1, g.spr);
+  }
+}
+__device__ __forceinline__ void gemv_geom(int body, int mode, GemvGeom& g) {
+  const int total = g.t.nranges * g.t.n, nvl = ((g.t.row_bytes >> 4) + 31) >> 5;
+  gemv_stages(body, mode, g);
+  g.ns = 0; g.W = 1; g.NG = ETXB_NSTAGE; g.R = 1; g.S = 1; g.rw = 1; g.one = 0; g.rspr = 0.f;
+  if (total > 0 && g.rps > 0) {
+    if (g.spr) { g.rspr = __frcp_rn((float)g.spr); g.ns = g.t.nranges * g.spr; }
+    else g.ns = total < (1 << 21) ? udiv_small(total + g.rps - 1, g.rps) : (total + g.rps - 1) / g.rps;
+    const int m = min(g.rps, g.spr ? g.t.n : total);
+    g.R = g.few ? 1 : nvl <= 7 ? 4 : nvl == 8 ? 3 : m == 3 || m == 5 ? 3 : m == 4 ? 4 : 1;
+    g.one = g.R == 1 && nvl > 8;
+    int rw = g.R == 4 ? (m + 3) >> 2 : g.R == 3 ? (m + 2) * 171 >> 9 : m;       // (m + 2 < 512: rows of more than 1792 values)
+    rw = rw <= 4 ? rw : rw <= 6 ? 6 : rw <= 8 ? 8 : rw <= 12 ? 12 : 16;
+    if (mode & ETXB_MODE_SUM_SLOTS) {                              // (its epilogue adds slots, not parts of rows)
+    } else if (g.few) {
+#pragma unroll 1
+      while (g.S < 4 && total * g.S <= 8 && 2 * g.S <= nvl && g.ns <= gemv_groups(2 * g.S * rw)) g.S *= 2;
+    } else if (nvl > 8 && total <= ETXB_XF_FLOATS / 4) g.S = rw == 1 && g.ns > ETXB_NSTAGE ? 4 : 2;    // (rw: 1 or 2 there)
+    g.rw = rw; g.W = rw * g.S;
+    g.NG = gemv_groups(g.W);
+  }
+  g.wmul = g.W <= 4 ? (g.W == 3 ? 86 : 256 >> (g.W >> 1)) : g.W == 6 ? 43 : g.W == 8 ? 32 : g.W == 12 ? 22 : 16;   // ceil(256 / W): exact for 16 warps and for ETXB_EMPTY_COUNT / W
+  g.cnt = ETXB_EMPTY_COUNT * g.wmul >> 8;                           // 48 / W
+  g.shared = g.NG == 4 || g.NG == 5;                                // (the groups that do not divide ETXB_NSTAGE)
 }
 
 // Expert ids (and routing weights, unless lwts is null) of the task's slots into `lids` / `lwts` (indexed by global slot).  One warp, all
@@ -280,16 +369,17 @@ __device__ __forceinline__ void gemv_geom(int body, GemvGeom& g) {
 template <bool LEAN, bool SH = !LEAN>
 __device__ __forceinline__ void gemv_routing(const etxb_gemv_args& d, int32_t* lids, float* lwts) {
   const int fold = d.mode & 0xff, lane = tidx() & 31;
+  const uint32_t fl = (d.mode & ETXB_MODE_WORDS_IN) ? s_vars.flag : 0u;
   if (fold >= 2) {
     if constexpr (SH) {
       const int ns = (d.mode >> 24) & 0xf;
-      warp_topk<LEAN>(d.logits, d.E, d.R - ns, fold == 3, (d.mode & ETXB_MODE_BF16_WTS) != 0, lids, lwts, nullptr);
+      warp_topk<LEAN>(d.logits, fl, d.E, d.R - ns, fold == 3, (d.mode & ETXB_MODE_BF16_WTS) != 0, lids, lwts, nullptr);
       if (ns > 0) {
         if (lane < ns) { lids[d.R - ns + lane] = d.E + lane; if (lwts != nullptr) lwts[d.R - ns + lane] = 1.f; }
         __syncwarp();
       }
     } else {
-      warp_topk<LEAN>(d.logits, d.E, d.R, fold == 3, (d.mode & ETXB_MODE_BF16_WTS) != 0, lids, lwts, nullptr);
+      warp_topk<LEAN>(d.logits, fl, d.E, d.R, fold == 3, (d.mode & ETXB_MODE_BF16_WTS) != 0, lids, lwts, nullptr);
     }
   } else {
     if (lane < 16) {
@@ -313,9 +403,9 @@ __device__ __forceinline__ const unsigned char* gemv_range_base(int body, const 
 
 // ---------------------------------------------------------------------------------------------- producer side
 // Issue the bulk copies of one task.  One warp; lane 0 issues.  n = running stage counter of this CTA.
-// ptr: the task's trace row when tracing (slot 7 <- time the first stage was issued, slot 6 <- the last), else null.
+// ranges: a stage ends with its range.  ptr: the task's trace row when tracing (slot 7 <- time the first stage was issued, slot 6 <- the last), else null.
 template <bool SH = true>
-__device__ __forceinline__ bool produce_task(int body, const etxb_gemv_args& d, const GemvTask& t, int rps, const int32_t* lids, uint32_t& n,
+__device__ __forceinline__ bool produce_task(int body, const etxb_gemv_args& d, const GemvTask& t, int rps, bool ranges, const int32_t* lids, uint32_t& n,
                                              const Smem& sm, int where, uint64_t* ptr = nullptr) {
   const int total = t.nranges * t.n;
   if (total <= 0) return true;
@@ -327,7 +417,7 @@ __device__ __forceinline__ bool produce_task(int body, const etxb_gemv_args& d, 
   if ((tidx() & 31) == 0) {
     const uint64_t pol = l2_policy_evict_first();
     int rg = 0, r = 0;                                             // the range and the row in it that come next
-    for (int q0 = 0; q0 < total && ok; q0 += rps) {
+    for (int q0 = 0, i = 0; q0 < total && ok; ++i) {
       const uint32_t st = n % ETXB_NSTAGE, par = (n / ETXB_NSTAGE) & 1;
       ok = mbar_wait(sm.empty + st, par ^ 1, sm, where);           // a fresh barrier passes the first round
       if (!ok) break;
@@ -338,10 +428,10 @@ __device__ __forceinline__ bool produce_task(int body, const etxb_gemv_args& d, 
       // costs more than it gives (gate+up 12.5 -> 13.6 us).  (Not unrolled: the compiler's four copies of the wait are 4 KB of
       // code in this loop, and a step pays for them in instruction fetch whether it waits or not: 12 layers of a dense 4096-wide
       // model 1270 -> 1252 us without them, 9 of a latent-attention one 719 -> 709, 12 of a 128-expert one 700 -> 695.)
-      if (body == 3 && q0 < ETXB_NSTAGE * rps)
+      if (body == 3 && i < ETXB_NSTAGE)
 #pragma unroll 1
         for (int spin = 0; spin < 64 && *(volatile const int*)&sm.vars->hold != 0; ++spin) __nanosleep(40);
-      const int nr = min(rps, total - q0);
+      const int nr = min(rps, ranges ? t.n - r : total - q0);
       unsigned char* dst = sm.ring + (size_t)st * ETXB_STAGE_BYTES;
       *((volatile uint32_t*)(sm.full + 2 * ETXB_NSTAGE) + st) = n;  // (see wait_use)
       mbar_expect_tx(sm.full + st, (uint32_t)(nr * t.row_bytes));
@@ -353,8 +443,9 @@ __device__ __forceinline__ bool produce_task(int body, const etxb_gemv_args& d, 
         r += cnt;
         if (r == t.n) { r = 0; ++rg; }
       }
-      if (ptr != nullptr) { if (q0 == 0) ptr[7] = globaltimer(); ptr[6] = globaltimer(); }
+      if (ptr != nullptr) { if (i == 0) ptr[7] = globaltimer(); ptr[6] = globaltimer(); }
       ++n;
+      q0 += nr;
     }
   }
   ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -371,66 +462,38 @@ __device__ __forceinline__ float dot8(const uint4 w, const uint4 x, float a) {
   return a;
 }
 
-// What happens to a row's result: the epilogue of the three tiles (held in registers: a pointer to a struct would put it
-// on the stack, and beside 227 KB of shared memory the L1 that backs the stack is small).
+// Where a row's result goes: fp32 to `g` (S partial sums a row), from which the tile's epilogue takes all of them behind a barrier (in order, so
+// that its stores are coalesced, and one copy of it serves every form of the multiplication); g null (GemvGeom::direct, a plain task of more rows than
+// `g` holds): bf16(v + bias) to `out` at once.
 struct GemvEpi {
-  int body;                  // 3, 4, 5
-  int M;                     // down: rows of an expert's output
-  __nv_bfloat16* out;        // gemv: row 0 of the task;  down, not summed: slot 0, row 0 of the task
-  const void* aux;           // gemv: bias of row 0 of the task (bf16);  down: routing weight per slot of the task (fp32);  or null
-  float* g;                  // up: bf16-rounded results per row;  down: weighted results per row when they are summed, else null
+  float* g;
+  __nv_bfloat16* out;        // row 0 of the task
+  const void* bias;          // bf16, row 0 of the task, or null
 };
-__device__ __forceinline__ void gemv_epi(const GemvEpi& e, int q, int rg, int rows, float v) {
-  if (e.body == 3) {
-    e.out[q] = __float2bfloat16_rn(e.aux ? __fadd_rn(v, __bfloat162float(((const __nv_bfloat16*)e.aux)[q])) : v);
-  } else {
-    float y = bfr(v);
-    if (e.aux) y = bfr(__fmul_rn(y, ((const float*)e.aux)[rg]));
-    if (e.g) e.g[q] = y;
-    else e.out[(size_t)rg * e.M + (q - rg * rows)] = __float2bfloat16_rn(y);
-  }
+__device__ __forceinline__ void gemv_epi(const GemvEpi& e, int q, int S, int h, float v) {
+  if (e.g) e.g[q * S + h] = v;
+  else e.out[q] = __float2bfloat16_rn(e.bias ? __fadd_rn(v, __bfloat162float(((const __nv_bfloat16*)e.bias)[q])) : v);
 }
 
-// Rows j, j + W, .. (R of them, those past the stage's nr repeat the last one and are dropped) of one stage by one warp.
-// XS: a row's activation vector is its range's (xb + range * xstride), else one vector serves all.  rg, rgend: the range
-// of the warp's current row and the row where it ends.
-template <int R, bool XS>
-__device__ __forceinline__ void gemv_rows(const unsigned char* stage, int row_bytes, int j, int W, int nr, int q0, int rows, int& rg, int& rgend,
-                                          const __nv_bfloat16* xb, int xstride, const GemvEpi& e) {
-  const int lane = tidx() & 31, nvec = row_bytes >> 4;
-  const uint4* wv[R];
-  const uint4* xv[XS ? R : 1];
-  int rgu[R];
-#pragma unroll
-  for (int u = 0; u < R; ++u) {
-    const int jj = min(j + u * W, nr - 1);
-    wv[u] = (const uint4*)(stage + (size_t)jj * row_bytes);
-    rgu[u] = 0;
-    if (XS) {
-      while (q0 + jj >= rgend) { ++rg; rgend += rows; }
-      rgu[u] = rg;
-      xv[u] = (const uint4*)(xb + (size_t)rg * xstride);
-    }
-  }
-  if (!XS) xv[0] = (const uint4*)xb;
+// Rows j, j + rw, .. (R of them, those past the stage's nr repeat the last one and are dropped) of one stage by one warp, vectors h * 32 + lane,
+// (h + S) * 32 + lane, .. of each, U at a time.  stage, x: shared-memory addresses of the stage and of the activation vector; q0: the stage's
+// first row.  (One copy for 1 to 4 rows, told apart inside the loop: 35 rows of 2048 in 3250 clocks against 2500.)
+template <int R, int U>
+__device__ __forceinline__ void gemv_rows(uint32_t stage, int row_bytes, int j, int rw, int nr, int h, int S, int q0, uint32_t x, const GemvEpi& e) {
+  const int lane = tidx() & 31;
+  uint32_t w[R];
   float a[R];
 #pragma unroll
-  for (int u = 0; u < R; ++u) a[u] = 0.f;
-  constexpr int U = R == 1 ? 4 : 1;
+  for (int u = 0; u < R; ++u) { w[u] = stage + (uint32_t)(min(j + u * rw, nr - 1) * row_bytes); a[u] = 0.f; }
 #pragma unroll U
-  for (int v = lane; v < nvec; v += 32) {
-    if (XS) {
+  for (int o = (h * 32 + lane) * 16; o < row_bytes; o += S * 512) {
+    const uint4 xv = lds128(x + o);
 #pragma unroll
-      for (int u = 0; u < R; ++u) a[u] = dot8(wv[u][v], xv[u][v], a[u]);
-    } else {
-      const uint4 x = xv[0][v];
-#pragma unroll
-      for (int u = 0; u < R; ++u) a[u] = dot8(wv[u][v], x, a[u]);
-    }
+    for (int u = 0; u < R; ++u) a[u] = dot8(lds128(w[u] + o), xv, a[u]);
   }
   if constexpr (R == 1) {
     const float s = warp_sum(a[0]);
-    if (lane == 0) gemv_epi(e, q0 + j, rgu[0], rows, s);
+    if (lane == 0) gemv_epi(e, q0 + j, S, h, s);
   } else {
     // the butterfly of warp_sum on R values at once: the lanes split the values between them at distances 16 and 8, then
     // 4, 2, 1 as usual -- the same sums in the same order, 6 shuffles instead of 5 R
@@ -444,18 +507,13 @@ __device__ __forceinline__ void gemv_rows(const unsigned char* stage, int row_by
     k += __shfl_xor_sync(0xffffffffu, h8 ? k0 : k1, 8);
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-    const int u = (h16 ? 2 : 0) + (h8 ? 1 : 0), jj = j + u * W;
-    if ((lane & 7) == 0 && u < R && jj < nr) {
-      int r = rgu[0];
-#pragma unroll
-      for (int i = 1; i < R; ++i) r = u == i ? rgu[i] : r;
-      gemv_epi(e, q0 + jj, r, rows, k);
-    }
+    const int u = (h16 ? 2 : 0) + (h8 ? 1 : 0), jj = j + u * rw;
+    if ((lane & 7) == 0 && u < R && jj < nr) gemv_epi(e, q0 + jj, S, h, k);
   }
 }
 
 // Consume the stages of one task: row q (0 .. total-1, range q / rows) . its activation vector -> gemv_epi.
-// Range i uses the vector at xb + i * xstride (xstride = 0: one vector for all).  A stage is waited for, read and given
+// Where a stage ends with its range, range i uses the vector i * K further on.  A stage is waited for, read and given
 // back by its group's W warps only (each arrives ETXB_EMPTY_COUNT / W times); the stage counter runs on by the task's
 // stages in every warp.
 // (Measured and not kept: the packed fma.rn.f32x2 form of the inner loop, +1.3 % step time; the mixed fma.rn.f32.bf16,
@@ -464,41 +522,39 @@ __device__ __forceinline__ void gemv_rows(const unsigned char* stage, int row_by
 // +0.6 %; mma.sync m16n8k16 with conflict-free unpadded rows (row r reads the 16-byte chunks in the order c ^ r and column r
 // of B holds the activations in that order): 3800 clocks for 35 rows of 2048, with an error 1.2 times as large; this function as a
 // call, one copy for all tiles: its arguments and saved registers on the stack cost 2 us per phase.)
-__device__ __forceinline__ void consume_task(uint32_t& n, const Smem& sm, const __nv_bfloat16* xb, int xstride, int where, const GemvEpi& e) {
+__device__ __forceinline__ void consume_task(uint32_t& n, const Smem& sm, const __nv_bfloat16* xb, int where, const GemvEpi& e) {
+  static_assert(ETXB_NSTAGE == 6, "which numbers of groups divide the ring (GemvGeom::shared)");
   const int lane = tidx() & 31, cw = tidx() >> 5;
-  const GemvGeom& geo = *sm.geo;
-  const int W = geo.W, NG = geo.NG, g = (cw * geo.wmul) >> 8, wi = cw - g * W;
-  const int rows = geo.t.n, total = geo.t.nranges * rows, rps = geo.rps, row_bytes = geo.t.row_bytes, R = geo.R;
-  const uint32_t n0 = n;
+  const GemvGeom geo = *sm.geo;
+  const int g = (cw * geo.wmul) >> 8, wi = cw - g * geo.W, h = wi & (geo.S - 1), j0 = geo.S == 1 ? wi : wi >> (geo.S == 2 ? 1 : 2);
+  const int rows = geo.t.n, total = geo.t.nranges * rows, row_bytes = geo.t.row_bytes;
+  const uint32_t ring = smem_u32(sm.ring), xa = smem_u32(xb);
+  uint32_t k = n + (uint32_t)g;
   n += (uint32_t)geo.ns;
-  if (g >= NG) return;
-  const uint32_t cnt = (uint32_t)ETXB_EMPTY_COUNT * (uint32_t)geo.wmul >> 8;   // 48 / W
-  uint32_t st = n0 % ETXB_NSTAGE, par = (n0 / ETXB_NSTAGE) & 1, k = n0 + g;
-  st += g;
-  while (st >= ETXB_NSTAGE) { st -= ETXB_NSTAGE; par ^= 1; }
+  if (g >= geo.NG) return;
   volatile const uint32_t* use = (volatile const uint32_t*)(sm.full + 2 * ETXB_NSTAGE);
-  int rg = 0, rgend = rows;
-  for (int q0 = g * rps; q0 < total; q0 += NG * rps) {
+#pragma unroll 1
+  for (int i = g; i < geo.ns; i += geo.NG, k += (uint32_t)geo.NG) {
+    const uint32_t rd = k / ETXB_NSTAGE, st = k - rd * ETXB_NSTAGE;
     // A parity wait tells use k of a stage from use k - 1 only, and with a number of groups that does not divide the ring
     // the use before this one may be another group's that is still being filled: the wait would be answered by use k - 2.
     // So the producer's note of the use it fills is looked at first (when it names k, k - 1 is over).
-    if (ETXB_NSTAGE % NG != 0 && !wait_use(use + st, k, sm, where)) return;
-    if (!mbar_wait(sm.full + st, par, sm, where)) return;          // step abandoned: touch nothing
-    if (q0 == 0) mark(sm, 1);
-    const int nr = min(rps, total - q0);
-    const unsigned char* stage = sm.ring + (size_t)st * ETXB_STAGE_BYTES;
-    for (int j = wi; j < nr; j += R * W) {
-      if (xstride != 0) {
-        if (R == 4) gemv_rows<4, true>(stage, row_bytes, j, W, nr, q0, rows, rg, rgend, xb, xstride, e);
-        else gemv_rows<1, true>(stage, row_bytes, j, W, nr, q0, rows, rg, rgend, xb, xstride, e);
-      } else if (R == 4) gemv_rows<4, false>(stage, row_bytes, j, W, nr, q0, rows, rg, rgend, xb, 0, e);
-      else if (R == 3) gemv_rows<3, false>(stage, row_bytes, j, W, nr, q0, rows, rg, rgend, xb, 0, e);
-      else gemv_rows<1, false>(stage, row_bytes, j, W, nr, q0, rows, rg, rgend, xb, 0, e);
+    if (geo.shared && !wait_use(use + st, k, sm, where)) return;
+    if (!mbar_wait(sm.full + st, rd & 1, sm, where)) return;       // step abandoned: touch nothing
+    if (i == 0) mark(sm, 1);
+    const int rg = __float2int_rz(((float)i + 0.5f) * geo.rspr), r0 = (i - rg * geo.spr) * geo.rps;   // (spr = 0: range 0, row i * rps of all)
+    const int nr = min(geo.rps, (geo.spr != 0 ? rows : total) - r0), q0 = rg * rows + r0;
+    const uint32_t stage = ring + st * ETXB_STAGE_BYTES, x = xa + (uint32_t)(rg * row_bytes);
+#pragma unroll 1
+    for (int j = j0; j < nr; j += geo.R * geo.rw) {
+      // (one row at a time: long rows four vectors deep; a few short ones in a loop that is short to fetch)
+      if (geo.R == 4) gemv_rows<4, 1>(stage, row_bytes, j, geo.rw, nr, h, geo.S, q0, x, e);
+      else if (geo.R == 3) gemv_rows<3, 1>(stage, row_bytes, j, geo.rw, nr, h, geo.S, q0, x, e);
+      else if (geo.one) gemv_rows<1, 4>(stage, row_bytes, j, geo.rw, nr, h, geo.S, q0, x, e);
+      else gemv_rows<1, 1>(stage, row_bytes, j, geo.rw, nr, h, geo.S, q0, x, e);
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive_n(sm.empty + st, cnt);
-    st += NG; k += NG;
-    while (st >= ETXB_NSTAGE) { st -= ETXB_NSTAGE; par ^= 1; }
+    if (lane == 0) mbar_arrive_n(sm.empty + st, (uint32_t)geo.cnt);
   }
 }
 
@@ -507,6 +563,117 @@ __device__ __forceinline__ void consume_task(uint32_t& n, const Smem& sm, const 
 __device__ __forceinline__ void stage_xb(const void* x, int K, __nv_bfloat16* xb) {
   const int nv = K >> 3;
   for (int i = tidx(); i < nv; i += ETXB_CONSUMERS) ((uint4*)xb)[i] = ld_act16((const __nv_bfloat16*)x + 8 * i);
+  csync();
+}
+
+// K words -> bf16 values in shared memory, K % 4 == 0.
+__device__ __forceinline__ void stage_words(const uint32_t* w, int K, uint32_t fl, __nv_bfloat16* xb) {
+  const int nv = K >> 2;
+#pragma unroll 1
+  for (int i = tidx(); i < nv; i += 4 * ETXB_CONSUMERS) {
+    uint4 v[4];
+    uint32_t spins = 0;
+    for (;;) {
+      uint32_t miss = 0u;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = i + u * ETXB_CONSUMERS < nv ? ld_words4(w + 4 * (i + u * ETXB_CONSUMERS)) : make_uint4(fl, fl, fl, fl);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) miss |= words_miss(v[u], fl);
+      if (miss == 0u || !words_again(spins, fl)) break;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * ETXB_CONSUMERS < nv) ((uint2*)xb)[i + u * ETXB_CONSUMERS] = words_pack(v[u]);
+  }
+  csync();
+}
+
+// Norm fold (below) for the hand-off as words: z = bf16(resid_in + row) or resid_in, x = bf16(ln * bf16(z * r)) -> xb; `store`: z and x
+// also to memory, as bf16 and as words.  in: rows / resid_in name words.  K % 4 == 0, K <= 8192.
+// A chain of latencies in front of every phase that folds a norm, so a warp's vectors are the blocks of 128 values that numpy's order
+// sums up (sumsq_numpy_order): squares are added without a barrier, and the blocks' sums meet behind the only one.
+__device__ __forceinline__ void stage_norm_words(const etxb_gemv_args& d, const etxb_gemv_words& wd, uint32_t fl, bool in, bool store,
+                                                 float* xf, __nv_bfloat16* xb, float* scr) {
+  const int K = d.K, nv = K >> 2, nblk = (K + 127) >> 7, lane = tidx() & 31, warp = tidx() >> 5;
+  const float inv = __int_as_float((127 - (31 - __clz(K))) << 23);  // 1 / K where K is a power of two: the same as dividing
+  const int LD = nblk <= ETXB_XF_FLOATS / 136 ? 136 : 128;         // floats from block to block (136: the accumulators of four blocks in 32 banks)
+#pragma unroll 1
+  for (int i = tidx(); i < 32 * nblk; i += ETXB_CONSUMERS) {       // vector i: block i / 32
+    float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < nv) {
+      const uint2 ln = __ldg((const uint2*)d.ln + i);
+      uint4 r, a;                                                  // values in the upper halves
+      if (in) {
+        uint32_t spins = 0;
+        do {
+          r = ld_words4((const uint32_t*)d.resid_in + 4 * i);
+          a = ld_words4((const uint32_t*)d.rows + 4 * i);
+        } while ((words_miss(r, fl) | words_miss(a, fl)) != 0u && words_again(spins, fl));
+        r = make_uint4(r.x << 16, r.y << 16, r.z << 16, r.w << 16);
+        a = make_uint4(a.x << 16, a.y << 16, a.z << 16, a.w << 16);
+      } else {
+        const uint2 q = __ldcg((const uint2*)d.resid_in + i);
+        r = make_uint4(q.x << 16, q.x & 0xffff0000u, q.y << 16, q.y & 0xffff0000u);
+        if (d.rows != nullptr) {
+          const uint2 p = __ldcg((const uint2*)d.rows + i);
+          a = make_uint4(p.x << 16, p.x & 0xffff0000u, p.y << 16, p.y & 0xffff0000u);
+        }
+      }
+      z = make_float4(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z), __uint_as_float(r.w));
+      if (d.rows != nullptr) {
+        z.x = bfr(__fadd_rn(z.x, __uint_as_float(a.x))); z.y = bfr(__fadd_rn(z.y, __uint_as_float(a.y)));
+        z.z = bfr(__fadd_rn(z.z, __uint_as_float(a.z))); z.w = bfr(__fadd_rn(z.w, __uint_as_float(a.w)));
+      }
+      ((uint2*)xb)[i] = ln;                                        // (where this thread's x goes)
+      if (store) {
+        const uint32_t u0 = __float_as_uint(z.x), u1 = __float_as_uint(z.y), u2 = __float_as_uint(z.z), u3 = __float_as_uint(z.w);
+        if (wd.z != nullptr) st_words4(wd.z + 4 * i, make_uint4((u0 >> 16) | fl, (u1 >> 16) | fl, (u2 >> 16) | fl, (u3 >> 16) | fl));
+        if (d.resid_out != nullptr) ((uint2*)d.resid_out)[i] = make_uint2((u0 >> 16) | (u1 & 0xffff0000u), (u2 >> 16) | (u3 & 0xffff0000u));
+      }
+    }
+    *(float4*)(xf + (i >> 5) * LD + 4 * lane) = z;
+  }
+  __syncwarp();
+  {
+    const int blk = warp + 16 * (lane >> 3);                       // this lane: accumulator lane % 8 of one of the warp's (up to four) blocks
+    float s = 0.f;
+    if (blk < nblk) {
+      const float* x = xf + blk * LD + (lane & 7);
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = x[8 * i];
+      s = __fmul_rn(v[0], v[0]);
+#pragma unroll
+      for (int i = 1; i < 16; ++i) s = __fadd_rn(s, __fmul_rn(v[i], v[i]));
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+    if ((lane & 7) == 0) scr[blk] = s;                             // (64 of them: blocks past the last one are 0)
+  }
+  csync();
+  float ss = scr[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, o));
+  if (nblk > 32) {
+    float s1 = scr[32 + lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) s1 = __fadd_rn(s1, __shfl_xor_sync(0xffffffffu, s1, o));
+    ss = __fadd_rn(ss, s1);
+  }
+  const float mean = (K & (K - 1)) == 0 ? __fmul_rn(ss, inv) : __fdiv_rn(ss, (float)K);
+  const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, d.eps)));
+#pragma unroll 1
+  for (int i = tidx(); i < nv; i += ETXB_CONSUMERS) {
+    const float4 z = *(const float4*)(xf + (i >> 5) * LD + 4 * lane);
+    const uint2 w = ((const uint2*)xb)[i];
+    const uint2 o = make_uint2(pack_bf(__fmul_rn(bf_lo(w.x), bfr(__fmul_rn(z.x, r))), __fmul_rn(bf_hi(w.x), bfr(__fmul_rn(z.y, r)))),
+                               pack_bf(__fmul_rn(bf_lo(w.y), bfr(__fmul_rn(z.z, r))), __fmul_rn(bf_hi(w.y), bfr(__fmul_rn(z.w, r)))));
+    ((uint2*)xb)[i] = o;
+    if (store) {
+      if (wd.x != nullptr) st_words4(wd.x + 4 * i, make_uint4((o.x & 0xffffu) | fl, (o.x >> 16) | fl, (o.y & 0xffffu) | fl, (o.y >> 16) | fl));
+      if (d.x != nullptr) ((uint2*)d.x)[i] = o;
+    }
+  }
   csync();
 }
 
@@ -655,89 +822,163 @@ __device__ __forceinline__ void stage_norm_col(const void* rows, const void* rin
 //   (examples/llm/ref_numpy.py:142-148), which the reference leaves to the next layer's norm fold.
 // One function with one copy of the multiplication: the phases of a step share its code, so it stays in the instruction
 // cache from one to the next.
+// A down task whose routing comes as words, which the gate+up grid publishes when it begins: nothing the task waits for is needed to read
+// it, so that is done while its event is being waited for (at the head of the body it took 4000 clocks of the phase).
+__device__ __forceinline__ bool gemv_routed_early(int body, const etxb_gemv_args& d) {
+  return body == 5 && (d.mode & 0xff) >= 2 && (d.mode & (ETXB_MODE_WORDS_IN | ETXB_MODE_ROUTE_READY)) == (ETXB_MODE_WORDS_IN | ETXB_MODE_ROUTE_READY);
+}
+// For the summed form of down: the slots in ascending expert id (where their results begin) at scr + 64, with their weights at 80; ids and
+// weights of all slots are at 96 and 112.  One warp.
+__device__ __forceinline__ void gemv_slot_order(const GemvTask& t, float* scr) {
+  const int32_t* lids = (const int32_t*)(scr + 96) + t.group * t.spt;
+  const int lane = tidx() & 31;
+  if (lane < t.spt) {
+    const int mine = lids[lane];
+    int rank = 0;
+#pragma unroll 1
+    for (int j = 0; j < t.spt; ++j) { const int o = lids[j]; rank += (o < mine) || (o == mine && j < lane); }
+    ((int*)(scr + 64))[rank] = lane * t.n;
+    (scr + 80)[rank] = (scr + 112)[t.group * t.spt + lane];
+  }
+}
+__device__ __forceinline__ void gemv_route_words(const etxb_gemv_args& d, const etxb_gemv_words& wd, const GemvTask& t, float* scr) {
+  const int lane = tidx() & 31;
+  if (lane < 16) {
+    uint32_t u = 0u, spins = 0;
+    uint2 v = make_uint2(__float_as_uint(1.f), 0u);
+    if (lane < d.R) {
+      const uint32_t fl = s_vars.flag;
+      const uint2* pw = (const uint2*)(wd.route + 16) + lane;
+      do { u = ld_word(wd.route + lane); v = ld_volatile8(pw); } while ((((u ^ fl) >> 16) != 0u || v.y != fl) && words_again(spins, fl));
+      u &= 0xffffu;
+    }
+    ((int32_t*)(scr + 96))[lane] = u == 0xffffu ? 0x7fffffff : (int32_t)u;
+    (scr + 112)[lane] = __uint_as_float(v.x);
+  }
+  __syncwarp();
+  if (d.mode & ETXB_MODE_SUM_SLOTS) gemv_slot_order(t, scr);
+}
+// Routing of a task's slots otherwise.  One warp.  A gate+up group's first chunk also publishes its slots' routing.
+template <bool LEAN, bool SH, bool WD>
+__device__ __forceinline__ void gemv_route_task(int body, const etxb_gemv_args& d, const etxb_gemv_words& wd, int blk, const GemvTask& t, float* scr) {
+  int32_t* lids = (int32_t*)(scr + 96); float* lwts = scr + 112;
+  const int fold = d.mode & 0xff, lane = tidx() & 31;
+  if (body == 4 && !(fold >= 2 && blk - t.group * d.tpe == 0)) return;    // (gate+up needs the routing only to publish it)
+  if (body == 5 && fold >= 2 && (d.mode & ETXB_MODE_ROUTE_READY) && d.ids != nullptr && d.wts != nullptr) {
+    if (lane < 16) {
+      lids[lane] = lane < d.R ? __ldcg(d.ids + lane) : 0;
+      lwts[lane] = lane < d.R ? __ldcg(d.wts + lane) : 1.f;
+    }
+    __syncwarp();
+  } else gemv_routing<LEAN, SH>(d, lids, lwts);
+  if (body == 4 && lane < t.spt) {
+    const int sl = t.group * t.spt + lane;
+    if (WD && (d.mode & ETXB_MODE_WORDS_OUT) && wd.route != nullptr) {
+      const uint32_t fl = s_vars.flag;
+      st_word(wd.route + sl, ((uint32_t)lids[sl] < 0xffffu ? (uint32_t)lids[sl] : 0xffffu) | fl);
+      st_relaxed8((uint2*)(wd.route + 16) + sl, __float_as_uint(lwts[sl]), fl);
+    }
+    if (d.ids) ((int32_t*)d.ids)[sl] = lids[sl];
+    if (d.wts) ((float*)d.wts)[sl] = lwts[sl];
+  }
+  // (known as soon as the routing is: worked out here, under the weight stream, and not after it)
+  if (body == 5 && (d.mode & ETXB_MODE_SUM_SLOTS)) gemv_slot_order(t, scr);
+}
 template <bool LEAN, bool XCH = false, bool SH = !LEAN>
 __device__ __forceinline__ void tile_gemv_family(int body, const unsigned char* a, int blk, const Smem& sm, uint32_t& n, int where) {
   const etxb_gemv_args& d = *(const etxb_gemv_args*)a;
   const GemvTask& t = sm.geo->t;
   if (t.n <= 0) return;
-  int32_t* lids = (int32_t*)(sm.scr + 96); float* lwts = sm.scr + 112;
-  const int fold = d.mode & 0xff, rows = t.n, K = d.K, spt = t.spt;
-  __nv_bfloat16* xb = smem_xb(sm);
-  float* g = smem_g(sm);                                           // up: per slot, rows gate results, then rows up results;  down: rows per slot
-  GemvEpi e;
-  e.body = body; e.M = d.M; e.out = (__nv_bfloat16*)d.out; e.aux = nullptr; e.g = nullptr;
-  const bool sum = body == 5 && (d.mode & ETXB_MODE_SUM_SLOTS) != 0;
-  if (body != 3 && tidx() < 32) {
-    if (body == 5 && fold >= 2 && (d.mode & ETXB_MODE_ROUTE_READY) && d.ids != nullptr && d.wts != nullptr) {
-      if (tidx() < 16) {
-        lids[tidx()] = tidx() < d.R ? __ldcg(d.ids + tidx()) : 0;
-        lwts[tidx()] = tidx() < d.R ? __ldcg(d.wts + tidx()) : 1.f;
-      }
-      __syncwarp();
-    } else if (body == 5 || (fold >= 2 && blk - t.group * d.tpe == 0)) {    // (gate+up needs the routing only to publish it)
-      gemv_routing<LEAN, SH>(d, lids, lwts);
-    }
-    if (body == 4 && fold >= 2 && blk - t.group * d.tpe == 0 && tidx() < spt) {   // the group's first chunk publishes its slots' routing
-      const int sl = t.group * spt + tidx();
-      if (d.ids) ((int32_t*)d.ids)[sl] = lids[sl];
-      if (d.wts) ((float*)d.wts)[sl] = lwts[sl];
-    }
-    // the slots in ascending expert id, for the summed form (as the row of g where the slot's results begin): known as soon
-    // as the routing is, so it is worked out here, under the weight stream, and not after it
-    if (sum && tidx() < spt) {
-      const int mine = lids[t.group * spt + tidx()];
-      int rank = 0;
-      for (int j = 0; j < spt; ++j) {
-        const int o = lids[t.group * spt + j];
-        rank += (o < mine) || (o == mine && j < tidx());
-      }
-      ((int*)(sm.scr + 64))[rank] = tidx() * rows;
-    }
-  }
-  if (body == 5) {
-    for (int i = tidx(); i < spt * (K >> 3); i += ETXB_CONSUMERS)             // the task's slots' activation vectors, one behind the other
-      ((uint4*)xb)[i] = ld_act16((const __nv_bfloat16*)d.x + (size_t)t.group * spt * K + 8 * i);
+  constexpr bool WD = !XCH;                                        // (a sharded session has no words of this kind)
+  const int mode = d.mode, fold = mode & 0xff, K = d.K;
+  const bool win = WD && (mode & ETXB_MODE_WORDS_IN), wout = WD && (mode & ETXB_MODE_WORDS_OUT);
+  const bool sum = body == 5 && (mode & ETXB_MODE_SUM_SLOTS) != 0;
+  const etxb_gemv_words& wd = *(const etxb_gemv_words*)(a + sizeof(etxb_gemv_args));
+  __nv_bfloat16* const xb = smem_xb(sm);
+  if (body == 3 && !win && fold == 0) stage_xb(d.x, K, xb);        // (a stand-alone launch waits for its activations and for this code: the short way)
+  else {
+  if (body != 3 && !(WD && gemv_routed_early(body, d)) && tidx() < 32) gemv_route_task<LEAN, SH, WD>(body, d, wd, blk, t, sm.scr);
+  // the activations
+  if (fold == ETXB_MODE_NORM && (win || wout)) stage_norm_words(d, wd, s_vars.flag, win, blk == 0, sm.xs, xb, sm.scr);
+  else if (win) {                                                  // (down: the task's slots' vectors, one behind the other)
+    const bool dn = body == 5;
+    stage_words((const uint32_t*)d.x + (dn ? t.group * t.spt * K : 0), dn ? t.spt * K : K, s_vars.flag, xb);
+  } else if (body == 5) {
+    for (int i = tidx(); i < t.spt * (K >> 3); i += ETXB_CONSUMERS) ((uint4*)xb)[i] = ld_act16((const __nv_bfloat16*)d.x + (size_t)t.group * t.spt * K + 8 * i);
     csync();
-    e.out += (size_t)t.group * spt * d.M + t.r0;
-    e.g = sum ? g : nullptr;
-    e.aux = fold >= 2 || d.wts != nullptr ? lwts + t.group * spt : nullptr;
-    if (sum) e.out -= (size_t)t.group * spt * d.M;                 // (the summed form writes one row)
-  } else {
-    if (fold == ETXB_MODE_NORM)                                    // (a dense MLP's gate+up: the post-attention norm folded in)
-      stage_norm_col<LEAN, XCH>(d.rows, d.resid_in, d.resid_out, (void*)d.x, d.ln, body == 3 ? d.ids : nullptr, d.R, K, d.eps, sm.xs, xb, sm.scr, blk == 0,
-                                (XCH && (d.mode & ETXB_MODE_FLAGGED)) ? row_flag(sm.epoch()) : 0u, &sm);
-    else
-      stage_xb(d.x, K, xb);
-    if (body == 3) {
-      e.out += t.r0;
-      e.aux = (d.mode & ETXB_MODE_BIAS) ? (const __nv_bfloat16*)d.wts + t.r0 : nullptr;
-    } else {
-      e.g = g;
-    }
+  } else if (fold == ETXB_MODE_NORM)                               // (a dense MLP's gate+up: the post-attention norm folded in)
+    stage_norm_col<LEAN, XCH>(d.rows, d.resid_in, d.resid_out, (void*)d.x, d.ln, body == 3 ? d.ids : nullptr, d.R, K, d.eps, sm.xs, xb, sm.scr, blk == 0,
+                              (XCH && (mode & ETXB_MODE_FLAGGED)) ? row_flag(sm.epoch()) : 0u, &sm);
+  else stage_xb(d.x, K, xb);
   }
+  const int rows = t.n, spt = t.spt, S = sm.geo->S;
+  float* const g = sm.xs;                                          // results (S partial sums each): up: per slot, rows gate results, then rows up results;  down: rows per slot
+  const float* const lwts = sm.scr + 112;
+  GemvEpi e;
+  e.g = sm.geo->direct ? nullptr : g;
+  e.out = (__nv_bfloat16*)d.out + t.r0;
+  e.bias = body == 3 && (mode & ETXB_MODE_BIAS) ? (const __nv_bfloat16*)d.wts + t.r0 : nullptr;
   mark(sm, 0);
-  consume_task(n, sm, xb, body == 5 && t.nranges > 1 ? K : 0, where, e);
-  if (body == 3 || (body == 5 && !sum)) return;
+  consume_task(n, sm, xb, where, e);
+  if (e.g == nullptr) return;
   csync();
-  if (body == 5 && tidx() == 0) *(volatile int*)&sm.vars->hold = 1;
+  if (sum && tidx() == 0) *(volatile int*)&sm.vars->hold = 1;
   mark(sm, 2);
-  if (body == 4) {
-    __nv_bfloat16* act = e.out + (size_t)t.group * spt * e.M + t.r0;
-    for (int s = 0, r = tidx(); s < spt; ++s, r -= rows, act += e.M, g += 2 * rows)
-      for (; r < rows; r += ETXB_CONSUMERS) act[r] = __float2bfloat16_rn(__fmul_rn(bfr(silu_f(g[r])), g[rows + r]));
-  } else {
+  const uint32_t fl = s_vars.flag;
+  uint32_t* const words = wout ? wd.out : nullptr;
+  __nv_bfloat16* const out = (__nv_bfloat16*)d.out;
+  auto val = [&](int q) {                                          // (partial sums pairwise)
+    float v = g[q * S];
+    if (S > 1) {
+      v = __fadd_rn(v, g[q * S + 1]);
+      if (S > 2) v = __fadd_rn(v, __fadd_rn(g[q * S + 2], g[q * S + 3]));
+    }
+    return v;
+  };
+  auto put = [&](uint32_t at, float y) {
+    const uint32_t u = bf_bits(y);
+    if (WD && words != nullptr) st_word(words + at, u | fl);
+    ((unsigned short*)out)[at] = (unsigned short)u;
+  };
+  if (body == 3) {
+#pragma unroll 1
+    for (int r = tidx(); r < rows; r += ETXB_CONSUMERS) {
+      float y = val(r);
+      if (e.bias) y = __fadd_rn(y, __bfloat162float(((const __nv_bfloat16*)e.bias)[r]));
+      put((uint32_t)(t.r0 + r), y);
+    }
+  } else if (sum) {
     const int* order = (const int*)(sm.scr + 64);
+    const bool weighted = fold >= 2 || d.wts != nullptr;
+#pragma unroll 1
     for (int r = tidx(); r < rows; r += ETXB_CONSUMERS) {
       float acc = 0.f;
+#pragma unroll 1
       for (int k0 = 0; k0 < spt; k0 += 8) {
         float v[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = g[order[min(k0 + k, spt - 1)] + r];
+        for (int k = 0; k < 8; ++k) {
+          const int i = min(k0 + k, spt - 1);
+          v[k] = bfr(g[order[i] + r]);                             // (S = 1 there)
+          if (weighted) v[k] = bfr(__fmul_rn(v[k], (sm.scr + 80)[i]));
+        }
 #pragma unroll
         for (int k = 0; k < 8; ++k) if (k0 + k < spt) acc = bfr(__fadd_rn(acc, v[k]));
       }
-      e.out[r] = __float2bfloat16_rn(acc);
+      put((uint32_t)(t.r0 + r), acc);
     }
+  } else {
+    uint32_t at = (uint32_t)(t.group * spt * d.M + t.r0);
+    const float* const wt = body == 5 && (fold >= 2 || d.wts != nullptr) ? lwts + t.group * spt : nullptr;
+#pragma unroll 1
+    for (int s = 0, r = tidx(), q = 0; s < spt; ++s, r -= rows, at += (uint32_t)d.M, q += body == 4 ? 2 * rows : rows)
+#pragma unroll 1
+      for (; r < rows; r += ETXB_CONSUMERS) {
+        float y = val(q + r);
+        if (body == 4) y = __fmul_rn(bfr(silu_f(bfr(y))), bfr(val(q + rows + r)));
+        else if (wt) y = __fmul_rn(bfr(y), wt[s]);
+        put(at + (uint32_t)r, y);
+      }
   }
 }
 

@@ -35,11 +35,6 @@ __device__ __forceinline__ void tile_prologue(const etxb_stepv& S) {
 __device__ __forceinline__ void st_volatile8(void* p, uint32_t a, uint32_t b) {
   asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(a), "r"(b) : "memory");
 }
-__device__ __forceinline__ uint2 ld_volatile8(const void* p) {
-  uint2 v;
-  asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ void argmax_exchange(const etxb_params& p, const Smem& sm, float& bv, int& bi) {
   const uint32_t fl = row_flag(p.epoch);
   bi += p.rank * p.step.V;
@@ -177,12 +172,6 @@ __device__ __forceinline__ void fetch_ctx(const etxb_params& p, TaskCtx* ctx, in
   }
 }
 
-// The persistent kernel's shared memory beside the dynamic part.  At namespace scope so that the tiles that are calls find
-// it at known addresses too: passed by reference, Smem would live on the stack; passed by value, in registers.
-__shared__ int s_stop;
-__shared__ unsigned long long s_deadline;
-__shared__ GemvGeom s_geo;
-__shared__ CtaVars s_vars;
 __shared__ __align__(8) TcShared s_tc;                             // (used by the kernels of a batched plan only)
 __device__ __forceinline__ Smem smem_view() {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -219,8 +208,9 @@ __device__ __noinline__ void argmax_col_call(const etxb_params& p, const unsigne
 }
 // Attention out of a kernel that holds all its forms, a call each: the grouped form (gq > 0 in the argument block; head_dim 128,
 // cache blocks of 16) and, in the full kernel, the general tile and latent attention.  They return the running stage count of the ring.
+template <bool WD>
 __device__ __noinline__ uint32_t attn_call(const etxb_attnf_args& d, int blk, const etxb_stepv& S, uint32_t n, uint32_t mg) {
-  attn_gq_tile(d, blk, smem_view(), S, n, mg);
+  attn_gq_tile<WD>(d, blk, smem_view(), S, n, mg);
   return n;
 }
 __device__ __noinline__ uint32_t narrow_call(const unsigned char* args, int blk, uint32_t n) {
@@ -231,6 +221,12 @@ __device__ __noinline__ uint32_t mla_call(const unsigned char* args, int blk, co
   tile_mla_attn(args, blk, smem_view(), S, n);
   return n;
 }
+// (in the full kernel: inlined there, its code spilled into the other tiles' paths)
+template <bool XCH>
+__device__ __noinline__ uint32_t gemv_call(int body, const unsigned char* args, int blk, uint32_t n, int cur) {
+  tile_gemv_family<false, XCH, true>(body, args, blk, smem_view(), n, cur);
+  return n;
+}
 template <bool GENERAL>
 __device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, int cur, const etxb_stepv& S, uint32_t& n, uint32_t mg) {
   const etxb_attnf_args& d = *(const etxb_attnf_args*)a;
@@ -239,7 +235,7 @@ __device__ __forceinline__ void tile_attn_any(const unsigned char* a, int blk, i
     if constexpr (GENERAL) { if (attn_fused_128(d)) batch_call<12 + 128>(a, blk, cur, S); else batch_call<12>(a, blk, cur, S); }
     return;
   }
-  n = attn_call(d, blk, S, n, mg);
+  n = attn_call<GENERAL>(d, blk, S, n, mg);
 }
 
 // Run the body of the task whose context is `c` on the consumer warps.
@@ -266,16 +262,19 @@ __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c,
   constexpr bool FULL = KV == 0, BATCHED = KV == ETXB_VARIANT_BATCH;
   // (a body this variant does not hold: the host picks the variant from the plan's bodies, so this is a corrupted record)
 #define ETXB_TILE(cond, call) if constexpr (cond) { call; } else { if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK); } break
+  if constexpr (LEAN && !BATCHED) {                                // (four of five phases; a jump table first is a trip for its entry)
+    if ((unsigned)(c->r.body - 3) < 3u) { tile_gemv_family<LEAN, XCH, SH>(c->r.body, args, c0, sm, n, cur); return; }
+  }
   switch (c->r.body) {
     case 0: break;
     case 1: ETXB_TILE(!BATCHED, tile_prologue(p.step));
     case 2: ETXB_TILE(!BATCHED, tile_argmax<XCH>(p, sm));
-    case 3: case 4: case 5: ETXB_TILE(!BATCHED, (tile_gemv_family<LEAN, XCH, SH>(c->r.body, args, c0, sm, n, cur)));
+    case 3: case 4: case 5: ETXB_TILE(FULL, n = gemv_call<XCH>(c->r.body, args, c0, n, cur));
     case 12:
       if constexpr (KV == ETXB_VARIANT_MLA) { if (tidx() == 0) atomicOr(p.ctrl, ETXB_CTRL_BADTASK); }      // (the latent-attention variant has no GQA tile)
       else if constexpr (KV == ETXB_VARIANT_LEAN) {
         const etxb_attnf_args& d = *(const etxb_attnf_args*)args;
-        if (c0 < (int)d.nblocks && d.gq > 0) attn_gq_tile(d, c0, sm, p.step, n, c->r.mirror);
+        if (c0 < (int)d.nblocks && d.gq > 0) attn_gq_tile<!XCH>(d, c0, sm, p.step, n, c->r.mirror);
       } else tile_attn_any<FULL>(args, c0, cur, p.step, n, c->r.mirror);
       break;
     case 6: ETXB_TILE(!LEAN, tile_topk(args, c0, sm));
@@ -316,12 +315,12 @@ __device__ __forceinline__ void run_body(const etxb_params& p, const TaskCtx* c,
 // Producer warp: waits for what the addresses of a task's stream depend on; false when the step is being abandoned.
 __device__ __forceinline__ bool producer_wait(const etxb_params& p, const Smem& sm, const etxb_rec* t, int cur) {
   const int sw = t->stream_word;
-  if (sw == -1) return ld_relaxed(p.ctrl) == 0;
+  if (sw == -1) return true;                                       // (an abandoned step ends at a stage that nobody gives back; a look at the word here is a trip to L2 per task)
   int good = 1;
   if ((tidx() & 31) == 0) {
     if (sw >= 0) good = wait_event(p, sw, (int32_t)(p.epoch * (uint32_t)p.evcount[sw]), cur, *sm.deadline) ? 1 : 0;
     else
-      for (int i = 0; good && i < t->in_n; ++i) {
+      for (int i = 0; good && i < (t->in_n & (ETXB_IN_ROUTED - 1)); ++i) {
         const int word = i < 4 ? t->in_word[i] : p.inwords[t->in_off + i];
         good = wait_event(p, word, (int32_t)(p.epoch * (uint32_t)p.evcount[word]), cur, *sm.deadline) ? 1 : 0;
       }
@@ -380,12 +379,16 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
     __syncwarp();
     GemvGeom gg;                                                   // (nor does the task's geometry)
     gg.t = gemv_task(body, *pa, t->c0);
-    gemv_geom(body, gg);
+    gemv_stages(body, pa->mode, gg);
     const GemvTask gt = gg.t;
     if constexpr (TC) { if (p.tc_on != 0u && !queue_done(sm, cur)) break; }
+    // (a down grid behind its gate+up grid: the ids are there.  With the event waited for and the top-k done again, 2 us, its stream began
+    // when the gate+up rows in the ring were used up)
+    if (!(t->in_n & ETXB_IN_ROUTED)) {
     if (!producer_wait(p, sm, t, cur)) break;
     if (gt.n > 0 && body != 3) gemv_routing<LEAN, SH>(*pa, sm.prod, nullptr);    // (the ids alone: the stream waits for them)
-    ok = produce_task<SH>(body, *pa, gt, gg.rps, sm.prod, n, sm, cur, p.trace ? p.trace + 8 * (size_t)t->id : nullptr);
+    }
+    ok = produce_task<SH>(body, *pa, gt, gg.rps, gg.spr != 0, sm.prod, n, sm, cur, p.trace ? p.trace + 8 * (size_t)t->id : nullptr);
   }
   // Nothing is left in flight on a normal exit (the consumers waited for every stage).  When the step was abandoned,
   // wait (bounded) for the copies already issued before the CTA's shared memory goes away.
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
   const Smem sm = smem_view();
   if (threadIdx.x == 0) {
     s_stop = 0;
-    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.cur = 0; s_vars.halt = 0; s_vars.hold = 0; s_vars.done = -1;
+    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.flag = row_flag(p.epoch + p.salt); s_vars.cur = 0; s_vars.halt = 0; s_vars.hold = 0; s_vars.done = -1;
     s_deadline = globaltimer() + p.timeout_ns;
     for (int i = 0; i < ETXB_NSTAGE; ++i) { mbar_init(sm.full + i, 1); mbar_init(sm.empty + i, ETXB_EMPTY_COUNT); ((uint32_t*)(sm.empty + ETXB_NSTAGE))[i] = 0xffffffffu; }
     if constexpr (TC) {
@@ -450,7 +453,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
   for (int cur = vars->q0; cur < vars->q1; ++cur) {
     const TaskCtx* c = ctx + ((cur - vars->q0) & (ETXB_CTX_SLOTS - 1));
     if (tidx() == 0) {
-      const int in_n = c->r.in_n;
+      const int in_n = c->r.in_n & (ETXB_IN_ROUTED - 1);
       if (p.trace) p.trace[8 * (size_t)c->r.id] = globaltimer();
       // Everybody must leave the loop at the same task, or a barrier waits for warps that have left.  s_stop may be set at any
       // time (by the producer warp, by a warp whose wait in a body gives up), so only this thread looks at it, before the barrier.
@@ -472,16 +475,23 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
       if (body >= 3 && body <= 5) {
         GemvGeom g;
         g.t = gemv_task(body, *(const etxb_gemv_args*)c->args, c->r.c0);
-        gemv_geom(body, g);
+        gemv_geom(body, ((const etxb_gemv_args*)c->args)->mode, g);
         s_geo = g;
       }
     }
-    csync();
-    if (vars->halt) break;
-    if (tidx() >= ETXB_CONSUMERS - 32) {                            // the last consumer warp keeps the contexts coming (asynchronously)
+    else if (KV != ETXB_VARIANT_BATCH && !XCH && (tidx() >> 5) == 2) {   // .. and the routing of a down task, where it is known already
+      const etxb_gemv_args& d = *(const etxb_gemv_args*)c->args;
+      const int body = c->r.body;
+      if (body == 5 && gemv_routed_early(body, d)) {
+        const GemvTask t = gemv_task(body, d, c->r.c0);
+        if (t.n > 0) gemv_route_words(d, *(const etxb_gemv_words*)(c->args + sizeof d), t, smem_view().scr);
+      }
+    } else if (tidx() >= ETXB_CONSUMERS - 32) {                    // the last consumer warp keeps the contexts coming (asynchronously)
       const int q1 = vars->q1;
       fetch_ctx(p, ctx, vars->q0, cur + 2 < q1 ? cur + 2 : -1, cur + 1 < q1 ? cur + 1 : -1);
     }
+    csync();
+    if (vars->halt) break;
     run_body<KV, XCH>(p, c, cur, smem_view(), n);
     cur = vars->cur;                                               // (before the barrier: thread 0 moves it on behind it)
     c = ctx + ((cur - vars->q0) & (ETXB_CTX_SLOTS - 1));
@@ -504,11 +514,14 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
       }
     }
     if (tidx() == 0) {
-      const int out_n = c->r.out_n, id = c->r.id;
+      const int out_n = c->r.out_n & (ETXB_OUT_RELAXED - 1), id = c->r.id;
+      const bool relaxed = (c->r.out_n & ETXB_OUT_RELAXED) != 0;   // (the readers look at the words themselves)
       if (s_stop == 0)                                             // (set when a stage wait gave up inside the body: no arrivals then)
+#pragma unroll 1
         for (int i = 0; i < out_n; ++i) {                          // release: orders the CTA's stores (seen through the barrier) before the count
           const int word = i < 4 ? c->r.out_word[i] : p.outwords[c->r.out_off + i];
-          red_release_add(p.events + (size_t)word * ETXB_EV_STRIDE, 1);
+          if (relaxed) red_relaxed_add(p.events + (size_t)word * ETXB_EV_STRIDE, 1);
+          else red_release_add(p.events + (size_t)word * ETXB_EV_STRIDE, 1);
         }
       vars->hold = 0;
       if constexpr (TC) vars->done = cur + 1;

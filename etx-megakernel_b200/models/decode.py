@@ -75,7 +75,8 @@ class DecodeProgram:
                 t = self.w[name]
             return t.data_ptr()
         self.graph, self.pool, self.sizing = Q.build_graph(dims, ptr, maxlen, self.machine, fold_topk=fold_topk, fused_attn=fused_attn,
-                                                              ranks=ranks, rank=rank, flagged=flagged)
+                                                              ranks=ranks, rank=rank, flagged=flagged,
+                                                              words=ranks == 1 and not flagged and fold_topk)
         pool = self.pool.bytes()
         self.plan = compile_graph(self.graph, self.machine, {"POOL": len(pool)}, options=PassOptions(workers=workers))
         self.session = Session(self.plan, {"vl": self.vl}, pool, device)

@@ -260,13 +260,26 @@ def buffer_shapes(d: Dims, maxlen: int, steps: int, parts: int) -> dict:
          "token_time": ((2 * (steps + 1),), "i64"),
          "exp_sums": ((d.NH, parts), "f32"), "max_logits": ((d.NH, parts), "f32"), "tmp_out": ((d.NH, parts, max(d.HD, op_attn.GQ_PARTIAL_FLOATS)), "f32"),
          "kc": ((d.L, nblk, d.NKV, d.HD // X, BS, X), "bf16"), "vc": ((d.L, nblk, d.NKV, d.HD, BS), "bf16"),
-         "attn_counters": ((d.L, d.NH), "i32"), "moe_out": ((d.H,), "bf16")}
+         "attn_counters": ((d.L, d.NH), "i32"), "moe_out": ((d.H,), "bf16"), "words": ((d.L, words_layout(d)[1]), "i32")}
     if d.moe:
         s.update({"rlog": ((d.E,), "bf16"), "tw": ((d.TOPK,), "f32"), "ti": ((d.TOPK,), "i32"), "tei": ((d.TOPK,), "i32"),
                   "mc2": ((d.TOPK, d.MI), "bf16"), "mc3": ((d.TOPK, d.H), "bf16")})
     else:
         s.update({"mc2": ((1, d.INTER), "bf16"), "mc3": ((1, d.H), "bf16")})
     return s
+
+
+def words_layout(d: Dims) -> tuple[dict, int]:
+    """Hand-off as words: name -> first word of a layer's vectors in its part of the buffer "words", and that part's length (each vector on a
+    16-byte boundary).  qkv rows, attention outputs, o_proj rows, the two residual sums, the normed vector and the logits of the
+    router, the routing, the MLP activations, the layer's output."""
+    slots, mi = (d.TOPK, d.MI) if d.moe else (1, d.INTER)
+    at, out = 0, {}
+    for name, n in (("qkv", d.NQKV), ("attn", d.NH * d.HD), ("o", d.H), ("z1", d.H), ("z2", d.H), ("x2", d.H), ("rlog", d.E if d.moe else 0),
+                    ("route", op_gemv.ROUTE_WORDS if d.moe else 0), ("act", slots * mi), ("out", d.H)):
+        out[name] = at
+        at += -(-n // 4) * 4
+    return out, at
 
 
 def weight_shapes(d: Dims, maxlen: int) -> dict:
@@ -370,12 +383,17 @@ class ArgPool:
 
 
 def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = "b200", *, fold_topk: bool = True,
-                fused_attn: bool | str = True, ranks: int = 1, rank: int = 0, flagged: bool = False):
+                fused_attn: bool | str = True, ranks: int = 1, rank: int = 0, flagged: bool = False, words: bool = False):
     """The decode step of `d` as a Graph plus its argument pool.
 
     flagged (one rank): hand the row-parallel grids' outputs (o_proj, down) to the norm folds that follow as flagged words
     in an exchange region of one row per block -- the single-GPU form of the sharded hand-off below: the fold polls the
     data itself instead of waiting for the producing grid's event and then loading.
+
+    words (one rank, folded top-k): the vectors a grid hands to the next one of the step also travel as words -- a bf16 value
+    and a flag of the step in 4 bytes -- through ptr("words") (words_layout), every layer through its own.  A word says itself
+    whether it has arrived, so a grid announces itself without waiting for its stores.  Same graph, same arithmetic, the bf16 vectors are
+    written as before.
 
     ranks > 1: the step of ONE rank of a model sharded `ranks` ways (`d` = shard_dims(full, ranks): its share of the
     heads and of the MLP / expert rows).  ptr("xrows") then names the rank's exchange region: 2 * L blocks of
@@ -408,6 +426,21 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
     if not (1 <= ranks <= 8 and 0 <= rank < ranks):
         raise ValueError("1 <= ranks <= 8 and 0 <= rank < ranks")
     exch = ranks > 1 or flagged
+    if words and (exch or not fold_topk):
+        raise ValueError("hand-off as words: one rank, folded top-k")
+    awords = words and fused_attn is True and sz.attn[0] > 0           # (the other attention tiles read and write bf16 vectors only)
+    wat, wlen = words_layout(d)
+    WI, WO = (op_gemv.MODE_WORDS_IN, op_gemv.MODE_WORDS_OUT) if words else (0, 0)
+
+    def wptr(layer, name):
+        return ptr("words") + 4 * (layer * wlen + wat[name])
+
+    def source(plain, layer, name, on=words):
+        """Where a grid reads a vector: the layer's words or the bf16 buffer."""
+        return wptr(layer, name) if on else ptr(plain)
+
+    def with_words(blob, **w):
+        return op_gemv.words_block(blob, **{k: wptr(*v) for k, v in w.items()}) if words else blob
     xmode = op_gemv.MODE_FLAGGED if exch else 0
 
     def xblock(layer, kind):
@@ -440,10 +473,11 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
         t, rpt = sz.qkv
         first = L == 0
         blob = gemv_block("dsl_gemv_fold", t, W=W("wqkv"), x=ptr("hn"), out=ptr("qkv"), M=d.NQKV, K=d.H, rpt=rpt, tpe=1,
-                          rows=0 if first else (xblock(L - 1, 1) or ptr("moe_out")), resid_in=ptr("resid") if first else ptr("resid2"),
+                          rows=0 if first else (xblock(L - 1, 1) or source("moe_out", L - 1, "out")), resid_in=ptr("resid") if first else source("resid2", L - 1, "z2"),
                           resid_out=0 if first else ptr("resid"), ln=W("ln1"), R=0 if first else ranks, eps=d.eps,
                           ids=0, wts=W("bqkv") if d.bias else 0,
-                          mode=op_gemv.MODE_NORM | (op_gemv.MODE_BIAS if d.bias else 0) | (0 if first else xmode), nb=1)
+                          mode=op_gemv.MODE_NORM | (op_gemv.MODE_BIAS if d.bias else 0) | (0 if first else xmode | WI) | WO, nb=1)
+        blob = with_words(blob, z=(L, "z1"), **({"out": (L, "qkv")} if awords else {}))
         # (sharded: the fold polls the step flags of the rows the ranks publish, which says more than the exchanged grid's
         # event -- that only counts this rank's tasks -- so it waits for the event BEFORE that grid and starts polling at once)
         prev = add(f"qkv_{L}", "dsl_gemv_fold", "qkv", L, blob, t, (t,), (before_x if exch and not first else prev), "i->(0)", f"E_qkv_{L}", "i->(0)", (1,), t, d.NQKV, d.H, after="")
@@ -452,13 +486,13 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
             gq, plen, gparts = (0, 0, 0) if fused_attn == "general" else sz.attn
             nparts, ntask = (gparts, gparts * (d.NH // gq)) if gq else (sz.parts, sz.parts * d.NKV)
             op_attn.check_fused(d.NH, d.NKV, d.HD, BS, X, nparts, gq, plen)
-            blob = argblock.pack_named(ent["attn_fused"], (ntask, 1, 1), qkv=ptr("qkv"), qw=W("qn") if d.qk_norm else 0,
+            blob = argblock.pack_named(ent["attn_fused"], (ntask, 1, 1), qkv=source("qkv", L, "qkv", awords), qw=W("qn") if d.qk_norm else 0,
                                        kw=W("kn") if d.qk_norm else 0, cos_sin=ptr("cos_sin"), kc=ptr("kc") + L * kv_layer_bytes,
                                        vc=ptr("vc") + L * kv_layer_bytes, block_tables=ptr("block_tables"), seq_lens=ptr("seq_lens"),
-                                       positions=ptr("positions"), slot_mapping=ptr("slot_mapping"), exp_sums=ptr("exp_sums"),
+                                       positions=ptr("positions"), slot_mapping=ptr("slot_mapping"), exp_sums=source("exp_sums", L, "attn", awords),
                                        max_logits=ptr("max_logits"), tmp_out=ptr("tmp_out"), out=ptr("attn_out"),
                                        counters=ptr("attn_counters") + 4 * L * d.NH, scale=scale, eps=d.eps, NH=d.NH, NKV=d.NKV, HD=d.HD,
-                                       BS=BS, X=X, max_parts=nparts, gq=gq, part_len=op_attn.tagged_part_len(L) if gq else plen)
+                                       BS=BS, X=X, max_parts=nparts, gq=gq, part_len=op_attn.tagged_part_len(L, words=awords, lim=op_attn.GQ_LIM) if gq else plen)
             prev = add(f"attn_{L}", "attn_fused", "attn_fused", L, blob, ntask, (ntask,), prev, "i->(0)",
                        f"E_red_{L}", "i->(0)", (1,), ntask, after="E_pro")    # (cached rows depend on the step's position alone)
         else:
@@ -480,16 +514,18 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
 
         # ---- o_proj
         t, rpt = sz.o
-        blob = gemv_block("dsl_gemv", t, W=W("wo"), x=ptr("attn_out"), out=ptr("o"), M=d.H, K=d.NH * d.HD, rpt=rpt, tpe=1, eps=d.eps, nb=1,
-                          rows=xblock(L, 0), mode=xmode)
+        blob = gemv_block("dsl_gemv", t, W=W("wo"), x=source("attn_out", L, "attn", awords), out=ptr("o"), M=d.H, K=d.NH * d.HD, rpt=rpt, tpe=1, eps=d.eps, nb=1,
+                          rows=xblock(L, 0), mode=xmode | (WI if awords else 0) | WO)
+        blob = with_words(blob, out=(L, "o"))
         before_x = prev
         prev = add(f"o_proj_{L}", "dsl_gemv", "o_proj", L, blob, t, (t,), prev, "i->(0)", f"E_o_{L}", "i->(0)", (1,), t, d.H, d.NH * d.HD, after="", exchange=True)
         fold_in = before_x if exch else prev
         if d.moe:
             # ---- router with the post-attention norm fold: task 0 stores resid2 and the normed vector
             t, rpt = sz.router
-            blob = gemv_block("dsl_gemv_fold", t, W=W("wr"), x=ptr("o_norm"), out=ptr("rlog"), M=d.E, K=d.H, rpt=rpt, tpe=1, rows=xblock(L, 0) or ptr("o"),
-                              resid_in=ptr("resid"), resid_out=ptr("resid2"), ln=W("ln2"), R=ranks, eps=d.eps, mode=op_gemv.MODE_NORM | xmode, nb=1)
+            blob = gemv_block("dsl_gemv_fold", t, W=W("wr"), x=ptr("o_norm"), out=ptr("rlog"), M=d.E, K=d.H, rpt=rpt, tpe=1, rows=xblock(L, 0) or source("o", L, "o"),
+                              resid_in=source("resid", L, "z1"), resid_out=ptr("resid2"), ln=W("ln2"), R=ranks, eps=d.eps, mode=op_gemv.MODE_NORM | xmode | WI | WO, nb=1)
+            blob = with_words(blob, out=(L, "rlog"), z=(L, "z2"), x=(L, "x2"))
             prev = add(f"router_{L}", "dsl_gemv_fold", "router", L, blob, t, (t,), fold_in, "i->(0)", f"E_rt_{L}", "i->(0)", (1,), t, d.E, d.H, after="")
             topk_mode = (op_gemv.MODE_TOPK_RENORM if d.norm_topk else op_gemv.MODE_TOPK) | hf_mode
             if not fold_topk:
@@ -502,16 +538,18 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
             spt, tpe, rpt = sz.up
             groups = slots // spt
             up_export = "dsl_moe_up_fold" if fold_topk else "dsl_moe_up"
-            blob = gemv_block(up_export, groups * tpe, W=W("w13"), x=ptr("o_norm"), out=ptr("mc2"),
+            blob = gemv_block(up_export, groups * tpe, W=W("w13"), x=source("o_norm", L, "x2"), out=ptr("mc2"),
                               ids=ptr("ti"), wts=ptr("tw"), estride=2 * d.MI * d.H, M=d.MI, K=d.H, rpt=rpt, tpe=tpe, R=d.TOPK, eps=d.eps,
-                              mode=(topk_mode if fold_topk else 0) | op_gemv.mode_spt(spt), E=d.E, logits=ptr("rlog"), nb=1)
+                              mode=(topk_mode if fold_topk else 0) | op_gemv.mode_spt(spt) | WI | WO, E=d.E, logits=source("rlog", L, "rlog"), nb=1)
+            blob = with_words(blob, out=(L, "act"), route=(L, "route"))
             prev = add(f"moe_up_{L}", up_export, "moe_up", L, blob, groups * tpe, (groups * tpe,),
                        prev, "i->(0)", f"E_up_{L}", "i->(0)", (1,), groups * tpe, d.MI, d.H)
             tpe, rpt = sz.down
             dn_export = "dsl_moe_down_fold" if fold_topk else "dsl_moe_down"
-            blob = gemv_block(dn_export, tpe, W=W("w2"), x=ptr("mc2"), out=ptr("moe_out"), ids=ptr("ti"), wts=ptr("tw"), rows=xblock(L, 1),
+            blob = gemv_block(dn_export, tpe, W=W("w2"), x=source("mc2", L, "act"), out=ptr("moe_out"), ids=ptr("ti"), wts=ptr("tw"), rows=xblock(L, 1),
                               estride=d.H * d.MI, M=d.H, K=d.MI, rpt=rpt, tpe=tpe, R=d.TOPK, eps=d.eps,
-                              mode=(topk_mode | op_gemv.MODE_ROUTE_READY if fold_topk else 0) | op_gemv.mode_spt(slots) | op_gemv.MODE_SUM_SLOTS | xmode, E=d.E, logits=ptr("rlog"), nb=1)
+                              mode=(topk_mode | op_gemv.MODE_ROUTE_READY if fold_topk else 0) | op_gemv.mode_spt(slots) | op_gemv.MODE_SUM_SLOTS | xmode | WI | WO, E=d.E, logits=source("rlog", L, "rlog"), nb=1)
+            blob = with_words(blob, out=(L, "out"), route=(L, "route"))
             # expert weights depend on the routing only: with the top-k folded in, the stream may start once the router is done
             before_x = prev
             prev = add(f"moe_down_{L}", dn_export, "moe_down", L, blob, tpe, (tpe,), prev, "i->(0)",
@@ -520,12 +558,14 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
             # ---- dense SwiGLU: gate+up with the post-attention norm fold, then down
             spt, tpe, rpt = sz.up
             blob = gemv_block("dsl_moe_up", tpe, W=W("wgu"), x=ptr("o_norm"), out=ptr("mc2"), estride=0, M=d.INTER, K=d.H, rpt=rpt, tpe=tpe,
-                              rows=xblock(L, 0) or ptr("o"), resid_in=ptr("resid"), resid_out=ptr("resid2"), ln=W("ln2"), R=ranks, eps=d.eps,
-                              mode=op_gemv.MODE_NORM | xmode, nb=1)
+                              rows=xblock(L, 0) or source("o", L, "o"), resid_in=source("resid", L, "z1"), resid_out=ptr("resid2"), ln=W("ln2"), R=ranks, eps=d.eps,
+                              mode=op_gemv.MODE_NORM | xmode | WI | WO, nb=1)
+            blob = with_words(blob, out=(L, "act"), z=(L, "z2"))
             prev = add(f"gate_up_{L}", "dsl_moe_up", "gate_up", L, blob, tpe, (tpe,), fold_in, "i->(0)", f"E_up_{L}", "i->(0)", (1,), tpe, d.INTER, d.H, after="")
             tpe, rpt = sz.down
-            blob = gemv_block("dsl_moe_down", tpe, W=W("wd"), x=ptr("mc2"), out=ptr("moe_out"), estride=0, M=d.H, K=d.INTER, rpt=rpt, tpe=tpe,
-                              eps=d.eps, nb=1, rows=xblock(L, 1), mode=xmode)
+            blob = gemv_block("dsl_moe_down", tpe, W=W("wd"), x=source("mc2", L, "act"), out=ptr("moe_out"), estride=0, M=d.H, K=d.INTER, rpt=rpt, tpe=tpe,
+                              eps=d.eps, nb=1, rows=xblock(L, 1), mode=xmode | WI | WO)
+            blob = with_words(blob, out=(L, "out"))
             before_x = prev
             prev = add(f"down_{L}", "dsl_moe_down", "down", L, blob, tpe, (tpe,), prev, "i->(0)", f"E_dn_{L}", "i->(0)", (1,), tpe, d.H, d.INTER, after="", exchange=True)
     # ---- lm_head with the final-norm fold, then greedy sampling
@@ -533,8 +573,9 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
     # (a sharded lm_head: this rank's d.VL rows -- of the whole embedding when the weights are tied -- and its logits only)
     blob = gemv_block("dsl_gemv_fold", t, W=ptr("embed") + (rank * d.VL * d.H * 2 if d.VL else 0) if d.tie else ptr("lm_head"), x=ptr("hn"),
                       out=ptr("logits"), M=d.lm_rows, K=d.H, rpt=rpt,
-                      tpe=1, rows=xblock(d.L - 1, 1) or ptr("moe_out"), resid_in=ptr("resid2"), resid_out=ptr("resid"), ln=ptr("final_norm"), R=ranks, eps=d.eps,
-                      ids=0, mode=op_gemv.MODE_NORM | xmode, nb=1)
+                      tpe=1, rows=xblock(d.L - 1, 1) or source("moe_out", d.L - 1, "out"), resid_in=source("resid2", d.L - 1, "z2"), resid_out=ptr("resid"), ln=ptr("final_norm"), R=ranks, eps=d.eps,
+                      ids=0, mode=op_gemv.MODE_NORM | xmode | WI, nb=1)
+    blob = op_gemv.words_block(blob) if words else blob
     prev = add("lm_head", "dsl_gemv_fold", "lm_head", -1, blob, t, (t,), (before_x if exch else prev), "i->(0)", "E_lm", "i->(0)", (1,), t, d.lm_rows, d.H, after="")
     g.etensor("E_argmax", (1,), wait_count=1)
     g.call_device("argmax", (1,), tile("vl_argmax"), resource=res, args=["vl"], consts=(0,), in_edges={prev: "i->(0)"},

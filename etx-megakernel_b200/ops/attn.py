@@ -34,15 +34,17 @@ F_PARAMS = [("qkv", "ptr addrspace(1)", 0, 8), ("qw", "ptr addrspace(1)", 8, 8),
             # part * (NH / gq) + group, one counter per group; gq = 0: the general form (32 positions x one kv head)
             ("gq", "i32", 152, 4), ("part_len", "i32", 156, 4)]
 GQ_PART = 128
-GQ_WHOLE = 1 << 24
+GQ_WHOLE, GQ_WORDS = 1 << 24, 1 << 25
 GQ_WHOLE_MAX = 157         # partitions x q heads per task that a whole-sequence task takes
 
 
-def tagged_part_len(tag: int, whole: bool = False) -> int:
+def tagged_part_len(tag: int, whole: bool = False, words: bool = False, lim: int = 0) -> int:
     """part_len word of a grouped attention block: 128 positions per task, and in bits 16..23 a tag that differs between the
     grids of a step that share the partial buffers (the layer index): a merger only accepts partials carrying its own.
-    whole: bit 24, the form with one task per (sequence, q group) that takes all partitions itself (the batched step)."""
-    return GQ_PART | ((tag & 0xff) << 16) | (GQ_WHOLE if whole else 0)
+    whole: bit 24, the form with one task per (sequence, q group) that takes all partitions itself (the batched step).
+    words: bit 25, qkv names words (bf16 value | step flag << 16) and the outputs are also written as words, at exp_sums.
+    lim: bits 26..30, a context of up to so many partitions is taken whole by the tasks of the first one (no partials, no merge)."""
+    return GQ_PART | (min(lim, 31) << 26) | ((tag & 0xff) << 16) | (GQ_WHOLE if whole else 0) | (GQ_WORDS if words else 0)
 
 
 def whole_sequence_fits(gq: int, max_parts: int) -> bool:
@@ -52,6 +54,10 @@ def whole_sequence_fits(gq: int, max_parts: int) -> bool:
     return max_parts * gq <= GQ_WHOLE_MAX
 
 
+# Contexts of up to this many partitions are taken whole by one task per group.  16 warps have two partitions' units at once, and nothing is published
+# or merged.  Us of a step with the limit 0 / 2 / 4: 4 layers of a 128-expert model at 200 positions 270.2 / 266.5 / 266.7, at 330 270.3 / 270.0 / 274.2, at
+# 500 270.4 / 271.2 / 284.0; 6 of a small dense model at 200 294.6 / 288.9 / 288.7; 4 sequences at 200 598 / 585 / 585.
+GQ_LIM = 2
 GQ_PARTIAL_FLOATS = 272   # grouped form: floats of `tmp_out` per (q head, partition) -- 136 (value, flag) pairs: 128 outputs, max, sum, padding
 
 
@@ -68,7 +74,7 @@ def check_fused(NH: int, NKV: int, HD: int, BS: int, X: int, max_parts: int, gq:
     check_shape(NH, NKV, HD, BS, X, max_parts)
     G = NH // NKV
     if gq:
-        if gq not in (1, 2, 4, 8) or G % gq or HD != 128 or BS != 16 or (part_len & 0xffff) != GQ_PART or part_len >> 25:
+        if gq not in (1, 2, 4, 8) or G % gq or HD != 128 or BS != 16 or (part_len & 0xffff) != GQ_PART or part_len >> 31 or ((part_len >> 24) & 1 and part_len >> 25):
             raise ValueError(f"attn_fused grouped form: needs gq in (1, 2, 4, 8) dividing G={G}, head_dim 128, block size 16 and "
                              f"part_len {GQ_PART} (gq={gq}, HD={HD}, BS={BS}, part_len={part_len})")
         if gq * max_parts > 4096:

@@ -17,6 +17,8 @@ publishes the rows it wrote into row `rank` of it on every rank, a norm fold rea
 """
 from __future__ import annotations
 
+import numpy as np
+
 from ._layout import entry
 
 ARG_BYTES, GRID_OFF = 160, 144
@@ -32,6 +34,15 @@ FORMS = {"dsl_gemv": "plain", "dsl_moe_up": "silu_mul", "dsl_moe_down": "scale",
          "dsl_gemv_fold": "plain", "dsl_moe_up_fold": "silu_mul", "dsl_moe_down_fold": "scale"}
 MODE_NORM, MODE_TOPK, MODE_TOPK_RENORM, MODE_BF16_WTS, MODE_BIAS, MODE_SUM_SLOTS, MODE_ROUTE_READY = 1, 2, 3, 0x100, 0x200, 0x400, 0x800
 MODE_FLAGGED = 0x1000      # sharded model: `rows` is a [ranks][M or K] block of flagged words (see build_graph(ranks=...))
+# one GPU, one token: vectors handed from grid to grid as words (bf16 value | step flag << 16); four pointers follow the block
+MODE_WORDS_IN, MODE_WORDS_OUT = 0x2000, 0x4000
+WORDS_BYTES, ROUTE_WORDS = 32, 48          # routing of a token: 16 expert ids, then 16 (weight, flag) pairs
+
+
+def words_block(block: bytes, out: int = 0, z: int = 0, x: int = 0, route: int = 0) -> bytes:
+    """`block` (MODE_WORDS_IN / _OUT set) with the addresses of the words behind it: results; a norm fold's sum and normed vector;
+    the routing (gate+up writes it, down reads it)."""
+    return block + np.asarray([out, z, x, route], "<u8").tobytes()
 
 
 def mode_shared(ns: int) -> int:

@@ -210,6 +210,7 @@ static int32_t check_mla_block(const unsigned char* blk, size_t bytes) {
     why = "C <= 512 and DR <= 64 (multiples of 8), DN + DR <= 256";
   else if (a.maxlen < 1 || a.maxlen > ETXB_MLA_MAXCTX) why = "1 <= maxlen <= 8192";
   else if (!a.qkv || !a.kvln || !a.cos_sin || !a.wkvb || !a.cache || !a.positions || !a.out || !a.tmp) why = "null pointer";
+  else if (a.words && (((uintptr_t)a.words & 3) || ((uintptr_t)a.qkv & 3) || (a.C & 1))) why = "hand-off as words: qkv and words name 4-byte words";
   else if (a.max_parts < 1 || a.max_parts > 64 || (long long)a.max_parts * ETXB_MLA_PART < a.maxlen) why = "max_parts partitions of 128 positions cover maxlen (at most 64)";
   else if (a.nblocks != (uint32_t)(a.NH * (a.max_parts + ETXB_MLA_FIN))) why = "the grid is (max_parts + 4) * NH tasks: the partitions, then four finishing tasks per head";
   if (!why) return ETXB_OK;
@@ -823,6 +824,10 @@ static int32_t upload_type_args(etxb_session* s) {
       etxb_attnf_args a;
       memcpy(&a, s->h_pool.data() + off, sizeof a);
       words = a.gq > 0 && (a.part_len & ETXB_GQ_WORDS) != 0;
+    } else if (ty.args[0] == 0 && off >= 0 && ty.body == ETXB_BODY_MLA_ATTN && (uint64_t)off + sizeof(etxb::etxb_mla_args) <= s->h_pool.size()) {
+      etxb::etxb_mla_args a;
+      memcpy(&a, s->h_pool.data() + off, sizeof a);
+      words = a.words != nullptr;
     }
     if (words && s->xbase != nullptr) return fail(ETXB_E_UNSUPPORTED, "a sharded session hands rows over as flagged words of its exchange region only");
     if (words && t.out_n < ETXB_OUT_RELAXED) r.out_n |= ETXB_OUT_RELAXED;
@@ -1077,6 +1082,7 @@ extern "C" int32_t etxb_op_launch(int device, int32_t body, const void* argblock
     bool words = false;
     if (body == ETXB_BODY_GEMV || body == ETXB_BODY_MOE_UP || body == ETXB_BODY_MOE_DOWN) words = (((const etxb_gemv_args*)argblock)->mode & (ETXB_MODE_WORDS_IN | ETXB_MODE_WORDS_OUT)) != 0;
     else if (body == ETXB_BODY_ATTN_FUSED) words = ((const etxb_attnf_args*)argblock)->gq > 0 && (((const etxb_attnf_args*)argblock)->part_len & ETXB_GQ_WORDS) != 0;
+    else if (body == ETXB_BODY_MLA_ATTN) words = ((const etxb::etxb_mla_args*)argblock)->words != nullptr;
     if (words) return fail(ETXB_E_UNSUPPORTED, "hand-off as words: the flags are a session's step, a single tile has none");
   }
   cudaStream_t st = (cudaStream_t)cuda_stream;

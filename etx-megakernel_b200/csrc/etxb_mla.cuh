@@ -43,10 +43,14 @@ struct etxb_mla_args {
   float scale, eps;            // 80..87
   void* tmp;                   // 88  (value, flag) pairs [NH][max_parts][C + 8]: weighted latent, then max logit and exp sum
   int32_t max_parts, tag;      // 96, 100: partitions the grid covers (tasks = (max_parts + 4) * NH: partitions, then finishing tasks); tag tells the layers that share tmp apart
-  int32_t pad[2];              // 104..111
+  uint32_t* words;             // 104  hand-off as words: qkv names words, the outputs are also written as words here; null: bf16 vectors
   uint32_t grid[3], nblocks;   // 112..127
 };
 
+__device__ __forceinline__ void mla_out(const etxb_mla_args& d, int i, float v) {
+  if (d.words != nullptr) st_word(d.words + i, bf_bits(v) | s_vars.flag);
+  ((__nv_bfloat16*)d.out)[i] = __float2bfloat16_rn(v);
+}
 // A finishing task of head h: waits (bounded) for the head's np partials, merges them -- weights exp(m_p - max m),
 // partitions in ascending order -- and applies rows [f * DV / FIN, ..) of W_UV.  The finishing tasks come after the
 // partition tasks in the grid, so whatever they wait for runs on another worker or ran before them on their own; the
@@ -57,69 +61,71 @@ __device__ __forceinline__ void mla_finish(const etxb_mla_args& d, const Smem& s
   const int tid = tidx(), lane = tid & 31, warp = tid >> 5;
   const uint32_t fl = pair_flag(sm.epoch(), d.tag << 16);
   float* oc = sm.xs;                                               // [C] merged, normalised latent
-  float* wl = oc + 512;                                            // [np <= 64] max logits, then weights
-  float* es = wl + 64;                                             // [np] exp sums
-  float* red = es + 64;
   const __nv_bfloat16* wuv = (const __nv_bfloat16*)d.wkvb + ((size_t)h * (DN + DV) + DN) * C;
   const int v_lo = f * ((DV + ETXB_MLA_FIN - 1) / ETXB_MLA_FIN), v_hi = min(DV, v_lo + (DV + ETXB_MLA_FIN - 1) / ETXB_MLA_FIN);
-  // this task's rows of W_UV travel while it waits for the partials
-  uint4 w[2][2];
+  // this task's rows of W_UV (the first 32 of them) travel to shared memory while it waits for the partials
+  unsigned char* const wsm = (unsigned char*)sm.xs + 16384;        // [32][C] bf16
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int v = v_lo + warp + r * ETXB_CONSUMER_WARPS, j = 8 * lane + 256 * k;
-      w[r][k] = (v < v_hi && j < C) ? __ldg((const uint4*)(wuv + (size_t)v * C + j)) : make_uint4(0u, 0u, 0u, 0u);
-    }
+  for (int r = 0; r < 2; ++r) {
+    const int v = v_lo + warp + r * ETXB_CONSUMER_WARPS;
+    if (v < v_hi)
+      for (int j = 8 * lane; j < C; j += 256) cp_async16(wsm + ((warp + r * ETXB_CONSUMER_WARPS) * C + j) * 2, wuv + (size_t)v * C + j, true);
+  }
+  cp_async_commit();
   const uint2* ph = (const uint2*)d.tmp + (size_t)h * d.max_parts * PW;
-  for (int q = tid; q < np; q += ETXB_CONSUMERS) {
-    wl[q] = poll_pair(ph + (size_t)q * PW + C, fl, sm);
-    es[q] = poll_pair(ph + (size_t)q * PW + C + 1, fl, sm);
-  }
-  csync();
-  if (warp == 0) {
-    float mm = -INFINITY;
-    for (int q = lane; q < np; q += 32) mm = fmaxf(mm, wl[q]);
-    mm = warp_max(mm);
-    float L = 0.f;
-    for (int q = lane; q < np; q += 32) {
-      const float wq = expf(__fsub_rn(wl[q], mm));
-      wl[q] = wq;
-      L = __fmaf_rn(wq, es[q], L);
-    }
-    L = warp_sum(L);
-    if (lane == 0) red[0] = L;
-  }
-  csync();
-  for (int j = tid; j < C; j += ETXB_CONSUMERS) {
-    float o = 0.f;
-    for (int q0 = 0; q0 < np; q0 += 8) {                             // eight partitions' pairs requested at once
-      uint2 first[8];
+  // A round: up to NF partitions' statistics (a lane each, every warp for itself) and this thread's values of them, requested together: behind the
+  // slowest partition comes one trip to L2.  Between rounds (contexts of more than 1280 positions) the sums are rescaled to the larger maximum.
+  // (Statistics, then weights by one warp, then values, a barrier between any two: 1.3 us more.)
+  constexpr int NF = 10;
+  const uint2* vp = ph + min(tid, C - 1);
+  float o = 0.f, L = 0.f, M = -INFINITY;
+#pragma unroll 1
+  for (int p0 = 0; p0 < np; p0 += NF) {
+    const int pe = min(np - p0, NF);
+    const uint2* sp = ph + (size_t)p0 * PW + C;
+    uint2 first[NF];
+    uint4 v;
+    uint32_t spins = 0;
+    for (;;) {
+      v = ld_volatile16(sp + (size_t)min(lane, pe - 1) * PW);      // (maximum, flag, sum, flag)
 #pragma unroll
-      for (int u = 0; u < 8; ++u) first[u] = ld_pair(ph + (size_t)min(q0 + u, np - 1) * PW + j);
+      for (int u = 0; u < NF; ++u) first[u] = ld_pair(vp + (size_t)(p0 + min(u, pe - 1)) * PW);
+      bool ok = v.y == fl && v.w == fl;
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (q0 + u < np) o = __fmaf_rn(wl[q0 + u], first[u].y == fl ? __uint_as_float(first[u].x) : poll_pair(ph + (size_t)(q0 + u) * PW + j, fl, sm), o);
+      for (int u = 0; u < NF; ++u) ok = ok && first[u].y == fl;
+      if (ok || !poll_again(spins, sp, pe, PW, fl, sm)) break;
     }
-    oc[j] = __fdiv_rn(o, red[0]);
+    __syncwarp();
+    const float m = lane < pe ? __uint_as_float(v.x) : -INFINITY;
+    const float Mn = fmaxf(M, warp_max(m)), Mz = Mn == -INFINITY ? 0.f : Mn;
+    const float f = expf(__fsub_rn(M, Mz)), wq = expf(__fsub_rn(m, Mz));       // (lanes past the round: 0)
+    M = Mn;
+    o = __fmul_rn(o, f);
+    L = __fmaf_rn(L, f, lane < pe ? __fmul_rn(wq, __uint_as_float(v.z)) : 0.f);
+#pragma unroll
+    for (int u = 0; u < NF; ++u) {
+      const float wu = __shfl_sync(0xffffffffu, wq, u);
+      if (u < pe) o = __fmaf_rn(wu, __uint_as_float(first[u].x), o);
+    }
   }
+  L = warp_sum(L);
+  if (tid < C) oc[tid] = __fdiv_rn(o, L);
+  cp_async_wait0();
   csync();
   // ---- out[v] = W_UV[h][v] . o_c: a warp per output row, lanes over the columns
   for (int r = 0; r < 2; ++r) {
     const int v = v_lo + warp + r * ETXB_CONSUMER_WARPS;
     float acc = 0.f;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int j = 8 * lane + 256 * k;
-      if (j < C) {
-        const uint4 x = w[r][k];
+    if (v < v_hi)
+#pragma unroll 2
+      for (int j = 8 * lane; j < C; j += 256) {
+        const uint4 x = *(const uint4*)(wsm + ((warp + r * ETXB_CONSUMER_WARPS) * C + j) * 2);
         const float wf[8] = {bf_lo(x.x), bf_hi(x.x), bf_lo(x.y), bf_hi(x.y), bf_lo(x.z), bf_hi(x.z), bf_lo(x.w), bf_hi(x.w)};
 #pragma unroll
         for (int u = 0; u < 8; ++u) acc = __fmaf_rn(wf[u], oc[j + u], acc);
       }
-    }
     acc = warp_sum(acc);
-    if (lane == 0 && v < v_hi) ((__nv_bfloat16*)d.out)[(size_t)h * DV + v] = __float2bfloat16_rn(acc);
+    if (lane == 0 && v < v_hi) mla_out(d, h * DV + v, acc);
   }
   for (int v0 = v_lo + 2 * ETXB_CONSUMER_WARPS; v0 < v_hi; v0 += ETXB_CONSUMER_WARPS) {   // (more than 32 rows per finishing task: DV > 128)
     const int v = v0 + warp;
@@ -132,7 +138,7 @@ __device__ __forceinline__ void mla_finish(const etxb_mla_args& d, const Smem& s
         for (int u = 0; u < 8; ++u) acc = __fmaf_rn(wf[u], oc[j + u], acc);
       }
     acc = warp_sum(acc);
-    if (lane == 0 && v < v_hi) ((__nv_bfloat16*)d.out)[(size_t)h * DV + v] = __float2bfloat16_rn(acc);
+    if (lane == 0 && v < v_hi) mla_out(d, h * DV + v, acc);
   }
   csync();
 }
@@ -208,11 +214,11 @@ __device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, c
   float* part = qc + 512;       // [16][512] the warps' partial sums (q_c, then o_c)
   float* red = part + 16 * 512; // [64]
   float* st = red + 64;         // [16][2] the warps' maximum and sum
-  const __nv_bfloat16* qkv = (const __nv_bfloat16*)d.qkv;
+  auto ldq = [&](int i) { return d.words != nullptr ? bf_lo(poll_word((const uint32_t*)d.qkv + i, s_vars.flag)) : ld_bf(d.qkv, i); };
   for (int i = tid; i < QH + 2 * DR + (owner ? ROW : 0); i += ETXB_CONSUMERS) {
-    if (i < QH) qf[i] = ld_bf(qkv, (size_t)h * QH + i);
+    if (i < QH) qf[i] = ldq(h * QH + i);
     else if (i < QH + 2 * DR) cs[i - QH] = __ldg((const float*)d.cos_sin + (size_t)tk.pos * 2 * DR + (i - QH));
-    else kvf[i - QH - 2 * DR] = ld_bf(qkv, (size_t)d.NH * QH + (i - QH - 2 * DR));
+    else kvf[i - QH - 2 * DR] = ldq(d.NH * QH + (i - QH - 2 * DR));
   }
   csync();
   mark(sm, 0);
@@ -336,20 +342,22 @@ __device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, c
   mark(sm, 2);
   // ---- publish the partition's partial as flagged pairs: weighted latent [C], then max and sum (the warps' in warp order)
   uint2* pw = (uint2*)d.tmp + ((size_t)h * d.max_parts + tk.part) * PW;
-  if (tid < C) {
-    float M = st[0];
+  {
+    // lane w works out warp w's factor (one exponential instead of sixteen), the sums take them by shuffle
+    const float2 ml = *(const float2*)(st + 2 * (lane & 15));
+    float M = ml.x;
 #pragma unroll
-    for (int w = 1; w < 16; ++w) M = fmaxf(M, st[2 * w]);
-    const float Mz = M == -INFINITY ? 0.f : M;                     // (a warp without a position: maximum -inf, weight 0)
-    float L = 0.f, v = 0.f;
-#pragma unroll 4
-    for (int w = 0; w < 16; ++w) {
-      const float g = expf(__fsub_rn(st[2 * w], Mz));
-      L = __fmaf_rn(g, st[2 * w + 1], L);
-      v = __fmaf_rn(g, part[w * 512 + tid], v);
+    for (int x = 1; x < 16; x <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, x));
+    const float g = expf(__fsub_rn(ml.x, M == -INFINITY ? 0.f : M));           // (a warp without a position: maximum -inf, weight 0)
+    float L = __fmul_rn(g, ml.y), v = 0.f;
+#pragma unroll
+    for (int x = 1; x < 16; x <<= 1) L = __fadd_rn(L, __shfl_xor_sync(0xffffffffu, L, x));
+#pragma unroll
+    for (int w = 0; w < 16; ++w) v = __fmaf_rn(__shfl_sync(0xffffffffu, g, w), part[w * 512 + min(tid, C - 1)], v);
+    if (tid < C) {
+      st_pair(pw + tid, v, fl);
+      if (tid == 0) { st_pair(pw + C, M, fl); st_pair(pw + C + 1, L, fl); }
     }
-    st_pair(pw + tid, v, fl);
-    if (tid == 0) { st_pair(pw + C, M, fl); st_pair(pw + C + 1, L, fl); }
   }
   mark(sm, 3);
 }

@@ -230,8 +230,18 @@ def buffer_shapes(d: MlaDims, maxlen: int, steps: int) -> dict:
          "token_in": ((steps + 2,), "i32"), "token_out": ((steps + 1,), "i32"), "token_time": ((2 * (steps + 1),), "i64"),
          "ckv": ((d.L, maxlen, d.ROW), "bf16"), "moe_out": ((d.H,), "bf16"), "mla_tmp": ((op_mla.tmp_pairs(d.NH, d.C, maxlen), 2), "f32"),
          "rlog": ((max(d.E, 1),), "bf16"), "tw": ((max(d.SLOTS, 1),), "f32"), "ti": ((max(d.SLOTS, 1),), "i32"),
-         "mc2": ((max(d.SLOTS * mi, d.DENSE_INTER, 1),), "bf16")}
+         "mc2": ((max(d.SLOTS * mi, d.DENSE_INTER, 1),), "bf16"), "words": ((d.L, words_layout(d)[1]), "i32")}
     return s
+
+
+def words_layout(d: MlaDims) -> tuple[dict, int]:
+    """Hand-off as words (models.qwen.words_layout): name -> first word in a layer's part of the buffer "words", and the part's length."""
+    at, out = 0, {}
+    for name, n in (("qkv", d.NQKV), ("attn", d.NH * d.DV), ("o", d.H), ("z1", d.H), ("z2", d.H), ("x2", d.H), ("rlog", max(d.E, 1)),
+                    ("route", op_gemv.ROUTE_WORDS), ("act", max(d.SLOTS * max(d.MI, 1), d.DENSE_INTER, 1)), ("out", d.H)):
+        out[name] = at
+        at += -(-n // 4) * 4
+    return out, at
 
 
 def step_bytes(d: MlaDims, ctx: int) -> dict:
@@ -244,9 +254,10 @@ def step_bytes(d: MlaDims, ctx: int) -> dict:
 
 
 # ------------------------------------------------------------------------------------------------ the graph
-def build_graph(d: MlaDims, ptr, maxlen: int = 1072, machine: MachineModel | str = "b200"):
+def build_graph(d: MlaDims, ptr, maxlen: int = 1072, machine: MachineModel | str = "b200", *, words: bool = False):
     """The decode step of `d` as a Graph plus its argument pool.  ptr(name) -> device address of a buffer (buffer_shapes) or
-    packed weight (weight_shapes).  Returns (graph, pool: ArgPool, info)."""
+    packed weight (weight_shapes).  words: the vectors of a step are handed over as words, as in models.qwen.build_graph.  Returns
+    (graph, pool: ArgPool, info)."""
     m = load_machine(machine) if isinstance(machine, str) else machine
     op_mla.check_shape(d.NH, d.C, d.DN, d.DR, d.DV, maxlen)
     ent = {}
@@ -276,6 +287,18 @@ def build_graph(d: MlaDims, ptr, maxlen: int = 1072, machine: MachineModel | str
     def gb(export, tasks, **f):
         return argblock.pack_named(ent[export], (tasks, 1, 1), **f)
 
+    wat, wlen = words_layout(d)
+    WI, WO = (op_gemv.MODE_WORDS_IN, op_gemv.MODE_WORDS_OUT) if words else (0, 0)
+
+    def wptr(layer, name):
+        return ptr("words") + 4 * (layer * wlen + wat[name])
+
+    def source(plain, layer, name):
+        return wptr(layer, name) if words else ptr(plain)
+
+    def with_words(blob, **w):
+        return op_gemv.words_block(blob, **{k: wptr(*v) for k, v in w.items()}) if words else blob
+
     g.etensor("E_pro", (1,), wait_count=1)
     g.call_device("prologue", (1,), cuda_link(SRC, "vl_prologue"), resource=res, args=["vl"], consts=(0,), out_edges={"E_pro": "i->i"}, duration_us=3.8)
     prev = "E_pro"
@@ -285,45 +308,53 @@ def build_graph(d: MlaDims, ptr, maxlen: int = 1072, machine: MachineModel | str
         Wl = lambda n, L=L: ptr(f"{L}.{n}")                                  # noqa: E731
         first = L == 0
         t, rpt = m.gemv_tasks(d.NQKV)
-        blob = gb("dsl_gemv_fold", t, W=Wl("wqa"), x=ptr("hn"), out=ptr("qkv"), M=d.NQKV, K=d.H, rpt=rpt, tpe=1, rows=0 if first else ptr("moe_out"),
-                  resid_in=ptr("resid") if first else ptr("resid2"), resid_out=0 if first else ptr("resid"), ln=Wl("ln1"), R=0 if first else 1, eps=d.eps,
-                  mode=op_gemv.MODE_NORM, nb=1)
+        blob = gb("dsl_gemv_fold", t, W=Wl("wqa"), x=ptr("hn"), out=ptr("qkv"), M=d.NQKV, K=d.H, rpt=rpt, tpe=1, rows=0 if first else source("moe_out", L - 1, "out"),
+                  resid_in=ptr("resid") if first else source("resid2", L - 1, "z2"), resid_out=0 if first else ptr("resid"), ln=Wl("ln1"), R=0 if first else 1, eps=d.eps,
+                  mode=op_gemv.MODE_NORM | (0 if first else WI) | WO, nb=1)
+        blob = with_words(blob, out=(L, "qkv"), z=(L, "z1"))
         prev = add(f"qkv_{L}", "dsl_gemv_fold", "qkv", L, blob, t, prev, f"E_qkv_{L}", d.NQKV, d.H, after="")
-        blob = argblock.pack_named(ent["mla_attn"], (d.NH * (nparts + op_mla.FINISHERS), 1, 1), qkv=ptr("qkv"), kvln=Wl("kvln"), cos_sin=ptr("cos_sin"), wkvb=Wl("wkvb"),
+        blob = argblock.pack_named(ent["mla_attn"], (d.NH * (nparts + op_mla.FINISHERS), 1, 1), qkv=source("qkv", L, "qkv"), kvln=Wl("kvln"), cos_sin=ptr("cos_sin"), wkvb=Wl("wkvb"),
                                    cache=ptr("ckv") + L * cache_layer_bytes, positions=ptr("positions"), out=ptr("attn_out"), NH=d.NH, C=d.C, DN=d.DN, DR=d.DR,
-                                   DV=d.DV, maxlen=maxlen, scale=d.scale, eps=d.eps, tmp=ptr("mla_tmp"), max_parts=nparts, tag=L & 0xff)
+                                   DV=d.DV, maxlen=maxlen, scale=d.scale, eps=d.eps, tmp=ptr("mla_tmp"), max_parts=nparts, tag=L & 0xff, words=wptr(L, "attn") if words else 0)
         prev = add(f"attn_{L}", "mla_attn", "attn_fused", L, blob, d.NH * (nparts + op_mla.FINISHERS), prev, f"E_attn_{L}",
                    after="E_pro")                                      # (W_UK depends on nothing, the cached rows on the step's position alone)
         t, rpt = m.gemv_tasks(d.H)
-        blob = gb("dsl_gemv", t, W=Wl("wo"), x=ptr("attn_out"), out=ptr("o"), M=d.H, K=d.NH * d.DV, rpt=rpt, tpe=1, eps=d.eps, nb=1)
+        blob = gb("dsl_gemv", t, W=Wl("wo"), x=source("attn_out", L, "attn"), out=ptr("o"), M=d.H, K=d.NH * d.DV, rpt=rpt, tpe=1, eps=d.eps, nb=1, mode=WI | WO)
+        blob = with_words(blob, out=(L, "o"))
         prev = add(f"o_proj_{L}", "dsl_gemv", "o_proj", L, blob, t, prev, f"E_o_{L}", d.H, d.NH * d.DV, after="")
         if d.dense(L):
             spt, tpe, rpt = dense_sz.up
-            blob = gb("dsl_moe_up", tpe, W=Wl("wgu"), x=ptr("o_norm"), out=ptr("mc2"), estride=0, M=d.DENSE_INTER, K=d.H, rpt=rpt, tpe=tpe, rows=ptr("o"),
-                      resid_in=ptr("resid"), resid_out=ptr("resid2"), ln=Wl("ln2"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM, nb=1)
+            blob = gb("dsl_moe_up", tpe, W=Wl("wgu"), x=ptr("o_norm"), out=ptr("mc2"), estride=0, M=d.DENSE_INTER, K=d.H, rpt=rpt, tpe=tpe, rows=source("o", L, "o"),
+                      resid_in=source("resid", L, "z1"), resid_out=ptr("resid2"), ln=Wl("ln2"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM | WI | WO, nb=1)
+            blob = with_words(blob, out=(L, "act"), z=(L, "z2"))
             prev = add(f"gate_up_{L}", "dsl_moe_up", "gate_up", L, blob, tpe, prev, f"E_up_{L}", d.DENSE_INTER, d.H, after="", slots=2)
             tpe, rpt = dense_sz.down
-            blob = gb("dsl_moe_down", tpe, W=Wl("wd"), x=ptr("mc2"), out=ptr("moe_out"), estride=0, M=d.H, K=d.DENSE_INTER, rpt=rpt, tpe=tpe, eps=d.eps, nb=1)
+            blob = gb("dsl_moe_down", tpe, W=Wl("wd"), x=source("mc2", L, "act"), out=ptr("moe_out"), estride=0, M=d.H, K=d.DENSE_INTER, rpt=rpt, tpe=tpe, eps=d.eps, nb=1, mode=WI | WO)
+            blob = with_words(blob, out=(L, "out"))
             prev = add(f"down_{L}", "dsl_moe_down", "down", L, blob, tpe, prev, f"E_dn_{L}", d.H, d.DENSE_INTER, after="")
             continue
         t, rpt = moe_sz.router
-        blob = gb("dsl_gemv_fold", t, W=Wl("wr"), x=ptr("o_norm"), out=ptr("rlog"), M=d.E, K=d.H, rpt=rpt, tpe=1, rows=ptr("o"), resid_in=ptr("resid"),
-                  resid_out=ptr("resid2"), ln=Wl("ln2"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM, nb=1)
+        blob = gb("dsl_gemv_fold", t, W=Wl("wr"), x=ptr("o_norm"), out=ptr("rlog"), M=d.E, K=d.H, rpt=rpt, tpe=1, rows=source("o", L, "o"), resid_in=source("resid", L, "z1"),
+                  resid_out=ptr("resid2"), ln=Wl("ln2"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM | WI | WO, nb=1)
+        blob = with_words(blob, out=(L, "rlog"), z=(L, "z2"), x=(L, "x2"))
         prev = add(f"router_{L}", "dsl_gemv_fold", "router", L, blob, t, prev, f"E_rt_{L}", d.E, d.H, after="")
         topk_mode = (op_gemv.MODE_TOPK_RENORM if d.norm_topk else op_gemv.MODE_TOPK) | op_gemv.mode_shared(d.NS)
         spt, tpe, rpt = moe_sz.up
         groups = d.SLOTS // spt
-        blob = gb("dsl_moe_up_fold", groups * tpe, W=Wl("w13"), x=ptr("o_norm"), out=ptr("mc2"), ids=ptr("ti"), wts=ptr("tw"), estride=2 * d.MI * d.H, M=d.MI,
-                  K=d.H, rpt=rpt, tpe=tpe, R=d.SLOTS, eps=d.eps, mode=topk_mode | op_gemv.mode_spt(spt), E=d.E, logits=ptr("rlog"), nb=1)
+        blob = gb("dsl_moe_up_fold", groups * tpe, W=Wl("w13"), x=source("o_norm", L, "x2"), out=ptr("mc2"), ids=ptr("ti"), wts=ptr("tw"), estride=2 * d.MI * d.H, M=d.MI,
+                  K=d.H, rpt=rpt, tpe=tpe, R=d.SLOTS, eps=d.eps, mode=topk_mode | op_gemv.mode_spt(spt) | WI | WO, E=d.E, logits=source("rlog", L, "rlog"), nb=1)
+        blob = with_words(blob, out=(L, "act"), route=(L, "route"))
         prev = add(f"moe_up_{L}", "dsl_moe_up_fold", "moe_up", L, blob, groups * tpe, prev, f"E_up_{L}", d.MI, d.H, slots=2 * d.SLOTS)
         tpe, rpt = moe_sz.down
-        blob = gb("dsl_moe_down_fold", tpe, W=Wl("w2"), x=ptr("mc2"), out=ptr("moe_out"), ids=ptr("ti"), wts=ptr("tw"), estride=d.H * d.MI, M=d.H, K=d.MI,
-                  rpt=rpt, tpe=tpe, R=d.SLOTS, eps=d.eps, mode=topk_mode | op_gemv.MODE_ROUTE_READY | op_gemv.mode_spt(d.SLOTS) | op_gemv.MODE_SUM_SLOTS,
-                  E=d.E, logits=ptr("rlog"), nb=1)
+        blob = gb("dsl_moe_down_fold", tpe, W=Wl("w2"), x=source("mc2", L, "act"), out=ptr("moe_out"), ids=ptr("ti"), wts=ptr("tw"), estride=d.H * d.MI, M=d.H, K=d.MI,
+                  rpt=rpt, tpe=tpe, R=d.SLOTS, eps=d.eps, mode=topk_mode | op_gemv.MODE_ROUTE_READY | op_gemv.mode_spt(d.SLOTS) | op_gemv.MODE_SUM_SLOTS | WI | WO,
+                  E=d.E, logits=source("rlog", L, "rlog"), nb=1)
+        blob = with_words(blob, out=(L, "out"), route=(L, "route"))
         prev = add(f"moe_down_{L}", "dsl_moe_down_fold", "moe_down", L, blob, tpe, prev, f"E_dn_{L}", d.H, d.MI, after=f"E_rt_{L}", slots=d.SLOTS)
     t, rpt = m.gemv_tasks(d.V, waves=1)
-    blob = gb("dsl_gemv_fold", t, W=ptr("lm_head"), x=ptr("hn"), out=ptr("logits"), M=d.V, K=d.H, rpt=rpt, tpe=1, rows=ptr("moe_out"), resid_in=ptr("resid2"),
-              resid_out=ptr("resid"), ln=ptr("final_norm"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM, nb=1)
+    blob = gb("dsl_gemv_fold", t, W=ptr("lm_head"), x=ptr("hn"), out=ptr("logits"), M=d.V, K=d.H, rpt=rpt, tpe=1, rows=source("moe_out", d.L - 1, "out"), resid_in=source("resid2", d.L - 1, "z2"),
+              resid_out=ptr("resid"), ln=ptr("final_norm"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM | WI, nb=1)
+    blob = op_gemv.words_block(blob) if words else blob
     prev = add("lm_head", "dsl_gemv_fold", "lm_head", -1, blob, t, prev, "E_lm", d.V, d.H, after="")
     g.etensor("E_argmax", (1,), wait_count=1)
     g.call_device("argmax", (1,), cuda_link(SRC, "vl_argmax"), resource=res, args=["vl"], consts=(0,), in_edges={prev: "i->(0)"},
@@ -351,7 +382,7 @@ class MlaProgram:
             if t is None:
                 t = self.w[name]
             return t.data_ptr()
-        self.graph, self.pool, self.info = build_graph(dims, ptr, maxlen, self.machine)
+        self.graph, self.pool, self.info = build_graph(dims, ptr, maxlen, self.machine, words=True)
         pool = self.pool.bytes()
         self.plan = compile_graph(self.graph, self.machine, {"POOL": len(pool)}, options=PassOptions())
         self.session = Session(self.plan, {"vl": self.vl}, pool, device)

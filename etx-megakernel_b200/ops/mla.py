@@ -12,6 +12,7 @@ It stands where the reference's DeepSeek-V2-Lite graph runs q_absorb, the chunke
   tmp       (value, flag) pairs [NH][max_parts][C + 8] (8 bytes each): the partitions' partial results; the four
             finishing tasks per head merge them and apply a quarter of W_UV each.  max_parts * 128 >= maxlen; grid =
             (max_parts + 4) * NH tasks (task = partition * NH + head, then the finishing tasks); tag = a number that differs between the grids sharing tmp (the layer)
+  words     0, or the hand-off as words (bf16 value | step flag << 16): qkv names words, the outputs are also written as words here
 """
 from __future__ import annotations
 
@@ -25,7 +26,7 @@ PARAMS = [("qkv", "ptr addrspace(1)", 0, 8), ("kvln", "ptr addrspace(1)", 8, 8),
           ("wkvb", "ptr addrspace(1)", 24, 8), ("cache", "ptr addrspace(1)", 32, 8), ("positions", "ptr addrspace(1)", 40, 8),
           ("out", "ptr addrspace(1)", 48, 8), ("NH", "i32", 56, 4), ("C", "i32", 60, 4), ("DN", "i32", 64, 4), ("DR", "i32", 68, 4),
           ("DV", "i32", 72, 4), ("maxlen", "i32", 76, 4), ("scale", "float", 80, 4), ("eps", "float", 84, 4),
-          ("tmp", "ptr addrspace(1)", 88, 8), ("max_parts", "i32", 96, 4), ("tag", "i32", 100, 4)]
+          ("tmp", "ptr addrspace(1)", 88, 8), ("max_parts", "i32", 96, 4), ("tag", "i32", 100, 4), ("words", "ptr addrspace(1)", 104, 8)]
 
 
 def import_entries(threads: int = 544) -> dict:

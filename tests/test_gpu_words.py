@@ -129,3 +129,28 @@ def test_words_are_refused_where_nobody_flags_them():
                                mode=gemv.MODE_WORDS_IN | gemv.MODE_WORDS_OUT)
     with pytest.raises(EtxbError, match="words"):
         op_launch("gemv", gemv.words_block(blob, out=t.data_ptr()), 1)
+
+
+def test_latent_attention_words_give_the_bits_of_the_vectors(monkeypatch):
+    """Two layers (dense, experts) of the latent-attention model; 11 partitions are two rounds of the finishing tasks."""
+    from etx_megakernel_b200.models import dsv2 as M
+    d = M.load_dims("deepseek-v2-lite", layers=2)
+    w = M.random_weights(d, 1400, torch.device(DEV), seed=2)
+
+    def run():
+        prog = M.MlaProgram(d, w, device=0, maxlen=1400)
+        gen = torch.Generator(device=DEV)
+        gen.manual_seed(7)
+        prog.buf["ckv"].normal_(0, 1, generator=gen)
+        out = []
+        for i, pos in enumerate([0, 127, 300, 1279, 1290]):
+            prog.buf["token_in"][0] = 11 + i
+            prog.step(0, pos, write_next=False)
+            out += [prog.read(n).copy() for n in ("logits", "attn_out", "resid", "moe_out")]
+        out.append(prog.read("ckv"))
+        prog.close()
+        return out
+    got = run()
+    monkeypatch.setattr(M, "build_graph", functools.partial(lambda build, *a, **k: build(*a, **{**k, "words": False}), M.build_graph))
+    for g, e in zip(got, run()):
+        assert np.array_equal(g, e)

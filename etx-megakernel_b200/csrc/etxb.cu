@@ -1042,22 +1042,79 @@ extern "C" int32_t etxb_decode_host(etxb_session* s, const int32_t* tokens_in, i
   CU(cudaSetDevice(s->device));
   cudaStream_t st = s->own_stream;
   int32_t next = tokens_in[0];
+  bool prologue = false, argmax = false, columns = false;
+  for (const etxb_type& ty : s->types) {
+    prologue = prologue || ty.body == ETXB_BODY_PROLOGUE; argmax = argmax || ty.body == ETXB_BODY_ARGMAX;
+    columns = columns || ty.body == ETXB_BODY_PROLOGUE_NB || ty.body == ETXB_BODY_ARGMAX_NB;
+  }
+  if (!prologue || !argmax || columns) {
+    for (int t = 0; t < n_total; ++t) {
+      const int32_t tok = t < n_in ? tokens_in[t] : next;
+      s->h_tok[0] = tok;
+      // slot 0 of token_in / token_out is reused every step: the host owns the sequence
+      CU(cudaMemcpyAsync(s->step.token_in, s->h_tok, 4, cudaMemcpyHostToDevice, st));
+      s->step.tok = 0; s->step.pos = start_pos + t; s->step.write_next = 0;
+      int32_t rc = etxb_launch(s, st);
+      if (rc) return rc;
+      CU(cudaMemcpyAsync(s->h_tok + 8, s->step.token_out, 4, cudaMemcpyDeviceToHost, st));
+      rc = etxb_wait(s, 60.0);
+      if (rc) return rc;
+      CU(cudaStreamSynchronize(st));
+      next = s->h_tok[8];
+      tokens_out[t] = next;
+      if (step_ms) step_ms[t] = s->last_ms;
+    }
+    return ETXB_OK;
+  }
+  // One sequence: the prologue reads its token from a pinned word and the argmax writes its own to another, over PCIe inside the step, and the
+  // host launches the next step when it sees that one.  The control words are looked at when the token does not come and behind the last
+  // step: an abandoned step leaves them set, so that none of the following ones gets far.  (Copies in front of and behind every launch, the control
+  // words in another and two waits per token: 12 tokens of a tiny model 1134 us, so 907.)
+  struct Restore {                                                 // the session's own slots and events again, whatever happens
+    etxb_session* s; int32_t *in, *out; cudaEvent_t e0, e1, x0 = nullptr, x1 = nullptr;
+    ~Restore() {
+      s->step.token_in = in; s->step.token_out = out;
+      if (s->launched) cudaStreamSynchronize(s->own_stream);       // (an early return: the step still uses these)
+      s->ev0 = e0; s->ev1 = e1;
+      if (x0) cudaEventDestroy(x0);
+      if (x1) cudaEventDestroy(x1);
+    }
+  } own{s, s->step.token_in, s->step.token_out, s->ev0, s->ev1};
+  CU(cudaEventCreate(&own.x0)); CU(cudaEventCreate(&own.x1));
+  cudaEvent_t y0 = own.x0, y1 = own.x1;                            // the pair of the step before
+  volatile int32_t* const tok_in = s->h_tok; volatile int32_t* const tok_out = s->h_tok + 8;
+  s->step.token_in = s->h_tok; s->step.token_out = s->h_tok + 8;
   for (int t = 0; t < n_total; ++t) {
-    const int32_t tok = t < n_in ? tokens_in[t] : next;
-    s->h_tok[0] = tok;
-    // slot 0 of token_in / token_out is reused every step: the host owns the sequence
-    CU(cudaMemcpyAsync(s->step.token_in, s->h_tok, 4, cudaMemcpyHostToDevice, st));
+    *tok_in = t < n_in ? tokens_in[t] : next;
+    *tok_out = INT32_MIN;
+    std::atomic_thread_fence(std::memory_order_seq_cst);
     s->step.tok = 0; s->step.pos = start_pos + t; s->step.write_next = 0;
     int32_t rc = etxb_launch(s, st);
     if (rc) return rc;
-    CU(cudaMemcpyAsync(s->h_tok + 8, s->step.token_out, 4, cudaMemcpyDeviceToHost, st));
-    rc = etxb_wait(s, 60.0);
-    if (rc) return rc;
-    CU(cudaStreamSynchronize(st));
-    next = s->h_tok[8];
+    if (t > 0 && step_ms) { CU(cudaEventSynchronize(y1)); CU(cudaEventElapsedTime(step_ms + t - 1, y0, y1)); }
+    const auto t0 = std::chrono::steady_clock::now();
+    for (uint32_t n = 1; *tok_out == INT32_MIN; ++n) {
+      if ((n & 4095u) != 0) continue;
+      const cudaError_t q = cudaStreamQuery(st);
+      if (q != cudaSuccess && q != cudaErrorNotReady) return fail(ETXB_E_CUDA, std::string("kernel failed: ") + cudaGetErrorString(q));
+      const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+      if ((q == cudaSuccess && *tok_out == INT32_MIN) || el > 60.0) {          // over without a token, or the host's watchdog
+        rc = etxb_wait(s, 1e-3);
+        return rc ? rc : fail(ETXB_E_ABORTED, "a step ended without a token");
+      }
+    }
+    next = *tok_out;
     tokens_out[t] = next;
-    if (step_ms) step_ms[t] = s->last_ms;
+    y0 = s->ev0; y1 = s->ev1;
+    if (t + 1 < n_total) { s->ev0 = y0 == own.e0 ? own.x0 : own.e0; s->ev1 = y1 == own.e1 ? own.x1 : own.e1; }
   }
+  int32_t rc = etxb_wait(s, 60.0);
+  if (rc) return rc;
+  if (step_ms) step_ms[n_total - 1] = s->last_ms;
+  // (the device's slots hold the last step's tokens, as after any step)
+  CU(cudaMemcpyAsync(own.in, s->h_tok, 4, cudaMemcpyHostToDevice, st));
+  CU(cudaMemcpyAsync(own.out, s->h_tok + 8, 4, cudaMemcpyHostToDevice, st));
+  CU(cudaStreamSynchronize(st));
   return ETXB_OK;
 }
 

@@ -165,6 +165,50 @@ __device__ __forceinline__ uint4 poll_words4(const uint32_t* p, uint32_t fl) {
 // softmax over E bf16 logits (fp32), K rounds of argmax with the lower index winning ties, optional renormalisation
 // over the selected weights (numpy's summation order for <= 16 values), optional bf16 rounding of the weights.
 // One warp (all 32 lanes call); E <= 256, K <= 16.  fl: 0, or the flag of the words that `logits` names.  ids / wts / tei may point to shared or global memory.
+// The ids alone, as a stream of expert rows waits for them: ordered by the logits themselves, value and index in one 24-bit key, a reduction per round.
+// The probabilities order alike unless two distinct logits among the K best and the next one become one probability: closer than 2^-14 (l - max is
+// rounded to 2^-18 at most within the range asked for), or so far below the maximum that they underflow.  Then, and where a logit is NaN or the maximum
+// infinite, nothing is written and false is returned.  One warp.  (Softmax, 64-bit candidates and two or three exchanges a round: the first expert rows
+// of a 128-expert layer were asked for 2.9 us after the router's event, so after 2.3.)
+template <int NK>
+__device__ __forceinline__ bool topk_ids_by_logit(const float (&p)[NK], int E, int K, int32_t* ids) {
+  const int lane = tidx() & 31;
+  uint32_t c[NK];
+  bool nan = false;
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+    const int e = lane + 32 * k;
+    const uint32_t u = __float_as_uint(__fadd_rn(p[k], 0.f)) >> 16;  // (-0 and +0 are one logit)
+    nan = nan || (e < E && p[k] != p[k]);
+    c[k] = e < E ? ((u & 0x8000u ? ~u & 0xffffu : u | 0x8000u) << 8) | (uint32_t)(255 - e) : 0u;
+  }
+  if (__any_sync(0xffffffffu, nan)) return false;
+#pragma unroll
+  for (int i = 1; i < NK; ++i)                                      // c[0] >= c[1] >= ...
+#pragma unroll
+    for (int j = i; j > 0; --j) { const uint32_t hi = max(c[j - 1], c[j]), lo = min(c[j - 1], c[j]); c[j - 1] = hi; c[j] = lo; }
+  const int n = min(K + 1, E);
+  uint32_t mine = 0u;
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) {
+    const uint32_t top = __reduce_max_sync(0xffffffffu, c[0]);
+    if (c[0] == top) {                                              // (keys are unique: one lane pops its head)
+#pragma unroll
+      for (int k = 0; k + 1 < NK; ++k) c[k] = c[k + 1];
+      c[NK - 1] = 0u;
+    }
+    if (lane == t) mine = top;
+  }
+  const uint32_t u = mine >> 8;
+  const float l = __uint_as_float((u & 0x8000u ? u & 0x7fffu : ~u & 0xffffu) << 16);
+  const float m = __shfl_sync(0xffffffffu, l, 0), d = __fsub_rn(l, __shfl_down_sync(0xffffffffu, l, 1));
+  const bool bad = lane < n && (!(m < INFINITY) || !(__fsub_rn(l, m) >= -80.f) || (lane + 1 < n && !(d == 0.f || d >= 6.103515625e-5f)));
+  if (__any_sync(0xffffffffu, bad)) return false;
+  if (lane < K) ids[lane] = 255 - (int)(mine & 0xffu);
+  __syncwarp();
+  return true;
+}
+
 template <int NK>
 __device__ __forceinline__ void warp_topk_n(const void* logits, uint32_t fl, int E, int K, bool renorm, bool bf16w,
                                             int32_t* ids, float* wts, int32_t* tei) {
@@ -186,6 +230,7 @@ __device__ __forceinline__ void warp_topk_n(const void* logits, uint32_t fl, int
 #pragma unroll
     for (int k = 0; k < NK; ++k) p[k] = ld_bf(logits, min(lane + 32 * k, E - 1));
   }
+  if (wts == nullptr && topk_ids_by_logit<NK>(p, E, K, ids)) return;
 #pragma unroll
   for (int k = 0; k < NK; ++k) {
     if (lane + 32 * k >= E) p[k] = -INFINITY;
@@ -897,7 +942,7 @@ __device__ __forceinline__ void tile_gemv_family(int body, const unsigned char* 
   __nv_bfloat16* const xb = smem_xb(sm);
   if (body == 3 && !win && fold == 0) stage_xb(d.x, K, xb);        // (a stand-alone launch waits for its activations and for this code: the short way)
   else {
-  if (body != 3 && !(WD && gemv_routed_early(body, d)) && tidx() < 32) gemv_route_task<LEAN, SH, WD>(body, d, wd, blk, t, sm.scr);
+  if (body == 5 && !(WD && gemv_routed_early(body, d)) && tidx() < 32) gemv_route_task<LEAN, SH, WD>(body, d, wd, blk, t, sm.scr);
   // the activations
   if (fold == ETXB_MODE_NORM && (win || wout)) stage_norm_words(d, wd, s_vars.flag, win, blk == 0, sm.xs, xb, sm.scr);
   else if (win) {                                                  // (down: the task's slots' vectors, one behind the other)
@@ -919,6 +964,8 @@ __device__ __forceinline__ void tile_gemv_family(int body, const unsigned char* 
   e.out = (__nv_bfloat16*)d.out + t.r0;
   e.bias = body == 3 && (mode & ETXB_MODE_BIAS) ? (const __nv_bfloat16*)d.wts + t.r0 : nullptr;
   mark(sm, 0);
+  // (the top-k that a gate+up group's first chunk publishes: nothing in this task waits for it, and the last warp mostly has no rows)
+  if (body == 4 && tidx() >= ETXB_CONSUMERS - 32) gemv_route_task<LEAN, SH, WD>(body, d, wd, blk, t, sm.scr);
   consume_task(n, sm, xb, where, e);
   if (e.g == nullptr) return;
   csync();

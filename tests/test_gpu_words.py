@@ -154,3 +154,25 @@ def test_latent_attention_words_give_the_bits_of_the_vectors(monkeypatch):
     monkeypatch.setattr(M, "build_graph", functools.partial(lambda build, *a, **k: build(*a, **{**k, "words": False}), M.build_graph))
     for g, e in zip(got, run()):
         assert np.array_equal(g, e)
+
+
+@pytest.mark.parametrize("E", [16, 128, 200])
+@pytest.mark.parametrize("logits", ["spread", "equal", "tiny", "far"])
+def test_expert_ids_by_logit_are_those_by_probability(E, logits):
+    """Router rows that make logits equal, closer than the probabilities tell apart, or so far below the largest that their probabilities are 0: the
+    program whose streams take the ids from the logits against the one whose top-k is a grid of its own (softmax, then ids from memory)."""
+    d = Q.Dims(name="ids", H=512, NH=4, NKV=2, HD=128, INTER=0, L=2, V=1000, qk_norm=True, moe=True, E=E, TOPK=8, MI=64, norm_topk=True)
+    w = D.random_packed_weights(d, 32, DEV, seed=9)
+    for L in range(d.L):
+        wr = w[f"{L}.wr"]
+        if logits == "equal":
+            wr[1::3] = wr[0]
+            wr[2::3] = 0
+        elif logits == "tiny":
+            wr.mul_(1e-5)
+        elif logits == "far":
+            wr.mul_(2000.0)
+    got, want = steps(d, w, 32, [0, 1, 2, 3, 20]), steps(d, w, 32, [0, 1, 2, 3, 20], fold_topk=False)
+    for g, e in zip(got, want):
+        for n in e:
+            assert np.array_equal(g[n], e[n]), n

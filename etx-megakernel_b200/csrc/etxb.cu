@@ -142,7 +142,7 @@ static int32_t check_attnf_block(const etxb_attnf_args& a) {
     if (!(a.gq == 1 || a.gq == 2 || a.gq == 4 || a.gq == 8) || G % a.gq) why = "gq is 1, 2, 4 or 8 and divides NH / NKV";
     else if (a.HD != 128 || a.BS != 16 || (a.part_len & 0xffff) != 128) why = "the grouped form is head_dim 128, cache blocks of 16, partitions of 128";
     else if (a.gq * a.max_parts > 4096) why = "gq * max_parts <= 4096";
-    else if (a.part_len < 0 || ((a.part_len & ETXB_GQ_WHOLE) && (a.part_len >> ETXB_GQ_LIM_SHIFT))) why = "part_len bit 31 is zero, bits 26..30 with partitions only";
+    else if (a.part_len < 0 || ((a.part_len & ETXB_GQ_WHOLE) && (a.part_len >> ETXB_GQ_LIM_SHIFT) > 1)) why = "part_len bit 31 is zero, bits 27..30 with partitions only";
     else if ((a.part_len & ETXB_GQ_WORDS) && ((a.part_len & ETXB_GQ_WHOLE) || !a.exp_sums || ((uintptr_t)a.exp_sums & 3) || ((uintptr_t)a.qkv & 15)))
       why = "hand-off as words: partitions, qkv 16-byte aligned, exp_sums names the words of the outputs";
     else if ((a.part_len & ETXB_GQ_WHOLE) && (a.nblocks > (uint32_t)(a.NH / a.gq) || a.max_parts * a.gq > ETXB_GQ_WHOLE_MAX))

@@ -25,7 +25,7 @@
 #define ETXB_EMPTY_COUNT 48          // arrivals that give a stage back: its W consumer warps arrive 48 / W times each
 #define ETXB_RING_BYTES (ETXB_STAGE_BYTES * ETXB_NSTAGE)
 #ifndef ETXB_GEN_BYTES
-#define ETXB_GEN_BYTES 65536         // activations: fp32 scratch [0,32K), bf16 x [32K,56K), row results [56K,64K); attention tiles use all of it
+#define ETXB_GEN_BYTES 65536         // activations: fp32 scratch of a fold, then row results [0,32K), bf16 x [32K,56K); attention tiles use all of it
 #endif
 #ifndef ETXB_XF_FLOATS
 #define ETXB_XF_FLOATS 8192          // norm fold works on K <= 8192 floats
@@ -35,9 +35,6 @@
 #endif
 #ifndef ETXB_XB_ELEMS
 #define ETXB_XB_ELEMS 12288          // streamed GEMV rows are at most 12288 elements long
-#endif
-#ifndef ETXB_G_OFF
-#define ETXB_G_OFF 57344
 #endif
 #ifndef ETXB_G_FLOATS
 #define ETXB_G_FLOATS 2048
@@ -221,7 +218,8 @@ struct etxb_attnf_args {
   int32_t gq, part_len;   // 152..159: gq > 0 selects the grouped form (gq q heads x 128 positions per task, task = part * (NH / gq) + group);
                           // part_len: bits 0..15 = 128, bits 16..23 = a tag that tells the grids sharing the partial buffers apart (the layer),
                           // bit 24 = whole-sequence form: task = q group, takes every partition (the batched step)
-                          // bits 26..30: contexts of up to so many partitions are taken whole, by the tasks of the first partition
+                          // bits 26..30: contexts of up to so many partitions are taken whole, by the tasks of the first partition;
+                          // in the whole-sequence form bit 26 = probabilities of cached positions with all 24 bits (else 17)
                           // bit 25 = hand-off as words (partitions): qkv names words, the outputs are also written as words at exp_sums
   uint32_t grid[3], nblocks;                                                                                    // 160..175
 };

@@ -9,8 +9,8 @@
 //     ldmatrix), its own running maximum and sum, the probabilities transposed by movmatrix into the second product's operand, 128
 //     output sums per head in its registers.  No barrier between units; the warps' results meet once, at the end.
 //   * the probabilities go into the product as a bf16 value, the bf16 of what that rounding lost and that of what the second one lost: the
-//     24 bits of their fp32 value, as they were multiplied before.  Whole contexts: the first two (2^-17 of the value), as before too, but
-//     all three for the unit of the new position, whose probability was multiplied in fp32.
+//     24 bits of their fp32 value, as they were multiplied before.  Plans with a task per whole context: the first two (2^-17 of the value), as before
+//     too, but all three for the unit of the new position, whose probability was multiplied in fp32, and where the block asks for it (ETXB_GQ_PRECISE).
 //     Sums meet in fp32, so that the partials are no further from 64-bit ones than plain fp32 chains of 32 terms leave them: 1.3e-7 at 1038
 //     and 8151 positions against 1.6e-7 (summed up inside the products 1.8e-7).
 // Bound by the stream of K / V at long contexts, by the chain q rows -> norm -> scores -> publish -> merge at short ones.
@@ -32,6 +32,7 @@ namespace etxb {
 #define ETXB_GQ_WHOLE (1 << 24)   // part_len bit: one task per (sequence, q group) takes all partitions
 #define ETXB_GQ_WORDS (1 << 25)   // part_len bit: qkv names words, the outputs are also written as words (at exp_sums)
 #define ETXB_GQ_LIM_SHIFT 26      // part_len bits 26..31: contexts of up to so many partitions are taken whole, by the tasks of the first one
+#define ETXB_GQ_PRECISE (1 << 26) // .. in the whole-context form: cached units with all 24 bits of their probabilities, too
 #define ETXB_GQ_WHOLE_MAX 157     // .. of partitions x q heads at most (the builder's rule: ops/attn.py)
 #define ETXB_GQ_PW 136     // 8-byte (value, flag) pairs a task publishes per q head and partition: 128 outputs, max, sum, padding
 #define ETXB_GQ_SHARE 64   // partials (gq x partitions) from which the merge is shared out.  Shared / by one task, us of a phase: 72 partials (8 sequences)
@@ -444,7 +445,7 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
         const uint32_t h0 = movmatrix(pack_bf(c[0], c[1])), h1 = movmatrix(pack_bf(c[2], c[3]));
         const uint32_t w0 = movmatrix(pack_bf(r[0], r[1])), w1 = movmatrix(pack_bf(r[2], r[3]));
         uint32_t x0 = 0u, x1 = 0u;
-        const bool third = !(d.part_len & ETXB_GQ_WHOLE) || ragged;
+        const bool third = ragged || (d.part_len & (ETXB_GQ_WHOLE | ETXB_GQ_PRECISE)) != ETXB_GQ_WHOLE;
         if (third) {                                               // what the second rounding lost
 #pragma unroll
           for (int j = 0; j < 4; ++j) r[j] = __fsub_rn(r[j], bfr(r[j]));
@@ -524,20 +525,21 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
     mark(sm, 1);
     for (int idx = tid; idx < gq * HD; idx += ETXB_CONSUMERS) {
       // a warp's 32 outputs are one head's: lane w works out slot w's factor (one exponential instead of eight), the sums take them by shuffle.
-      // (Every thread for itself: 1900 clocks of the phase with one q head to 1100 outputs.)
+      // (Eight exponentials in every thread: 0.76 us from the barrier to the stores, so 0.51.)
       const int g = idx >> 7, dd = idx & (HD - 1), w0 = lane & 7;
       const float2 ml = w0 < nslot ? *(const float2*)(s.st + (w0 * 8 + g) * 2) : make_float2(-INFINITY, 0.f);
       float M = ml.x;
 #pragma unroll
       for (int o = 1; o < 8; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
       const float f = expf(__fsub_rn(ml.x, M == -INFINITY ? 0.f : M));
-      float o = 0.f, L = __fmul_rn(f, ml.y);
-#pragma unroll
-      for (int x = 1; x < 8; x <<= 1) L = __fadd_rn(L, __shfl_xor_sync(0xffffffffu, L, x));
+      float o = 0.f, L = 0.f;
 #pragma unroll
       for (int w = 0; w < 8; ++w) {
-        const float fw = __shfl_sync(0xffffffffu, f, w);
-        if (w < nslot) o = __fmaf_rn(fw, s.po[w * 1152 + g * 132 + dd], o);
+        const float fw = __shfl_sync(0xffffffffu, f, w), lw = __shfl_sync(0xffffffffu, ml.y, w);
+        if (w < nslot) {
+          L = __fmaf_rn(fw, lw, L);
+          o = __fmaf_rn(fw, s.po[w * 1152 + g * 132 + dd], o);
+        }
       }
       if (t.whole || np == 1) {
         gq_out<WD>(d, sm, t.hq0 * HD + idx, __fdiv_rn(o, L));

@@ -16,7 +16,7 @@
 // on an mbarrier per stage).  Weights depend on no event (expert weights: only on the routing), so the stream keeps
 // running while the consumers wait for their activations: HBM stays busy across phase boundaries.  A stage
 // belongs to a group of 1 .. 16 consumer warps (GemvGeom), consecutive stages to different groups; a warp of the group
-// multiplies 1, 3 or 4 of the stage's rows at once: 16-byte weight and activation vectors from shared memory, fp32
+// multiplies 1, 3 or 4 of the stage's rows at once, or a part of them: 16-byte weight and activation vectors from shared memory, fp32
 // accumulators in a fixed order (lane-strided, then xor butterfly), and hands the row results to the tile's epilogue.
 #pragma once
 #include "etxb_prims.cuh"
@@ -61,7 +61,7 @@ struct CtaVars {
   int hold;                  // the running task's results are on their way out: the producer starts no further stage (see produce_task)
 };
 struct Smem {
-  float* xs;                 // general region (ETXB_GEN_BYTES): fp32 scratch, bf16 activations, row results
+  float* xs;                 // general region (ETXB_GEN_BYTES): fp32 scratch, then the rows' results; bf16 activations behind it
   float* scr;                // ETXB_SCR_FLOATS of reduction / routing scratch
   unsigned char* ring;       // ETXB_NSTAGE stages
   uint64_t* full;            // [ETXB_NSTAGE] stage filled (transaction bytes landed)
@@ -85,7 +85,6 @@ __shared__ CtaVars s_vars;
 // in-body time stamp k (0..3) of the running task; thread 0 only, no-op unless tracing
 __device__ __forceinline__ void mark(const Smem& sm, int k) { if (tidx() == 0 && sm.tr() != nullptr) sm.tr()[4 + k] = globaltimer(); }
 __device__ __forceinline__ __nv_bfloat16* smem_xb(const Smem& sm) { return (__nv_bfloat16*)((unsigned char*)sm.xs + ETXB_XB_OFF); }
-__device__ __forceinline__ float* smem_g(const Smem& sm) { return (float*)((unsigned char*)sm.xs + ETXB_G_OFF); }
 
 // Bounded mbarrier wait: true when the phase completed; false when the step is being abandoned (another thread gave
 // up, the host aborted, or the deadline passed -- then this thread records it).

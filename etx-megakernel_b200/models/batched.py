@@ -85,6 +85,7 @@ def build_graph(d: Q.Dims, ptr, B: int, maxlen: int = 1072, machine: MachineMode
     # (Whole contexts / partitions, us of 3 layers: 13 sequences at 333 positions 794 / 818, 16 at 700 834 / 869, 16 at 1400 865 / 927, 8 at 600 702 / 714,
     # 8 at 1033 718 / 718; but 5 at 1400 655 / 637, 2 at 1033 572 / 539.)
     whole = B * (d.NH // gq) >= 3 * W // 10 and op_attn.whole_sequence_fits(gq, gparts)
+    precise = B * (d.NH // gq) < W // 2                                      # (fewer sequences than this had partitions: all bits of their probabilities, still)
     ntask = (d.NH // gq) if whole else gparts * (d.NH // gq)
     op_attn.check_fused(d.NH, d.NKV, d.HD, BS, X, gparts, gq, plen)
     scale = float(np.float32(1.0 / np.sqrt(d.HD)))
@@ -144,7 +145,7 @@ def build_graph(d: Q.Dims, ptr, B: int, maxlen: int = 1072, machine: MachineMode
                 slot_mapping=ptr("slot_mapping") + 8 * b, exp_sums=ptr("exp_sums") + b * d.NH * gparts * 4, max_logits=ptr("max_logits") + b * d.NH * gparts * 4,
                 tmp_out=ptr("tmp_out") + b * d.NH * gparts * op_attn.GQ_PARTIAL_FLOATS * 4, out=ptr("attn_out") + b * d.NH * d.HD * 2,
                 counters=ptr("attn_counters") + 4 * (L * B + b) * d.NH, scale=scale, eps=d.eps, NH=d.NH, NKV=d.NKV, HD=d.HD, BS=BS, X=X,
-                max_parts=gparts, gq=gq, part_len=op_attn.tagged_part_len(L, whole, lim=0 if whole else op_attn.GQ_LIM))
+                max_parts=gparts, gq=gq, part_len=op_attn.tagged_part_len(L, whole, lim=int(precise) if whole else op_attn.GQ_LIM))
         add(f"attn_{L}", "etx_tile_attn_fused", blobs, (ntask, B), ntask * B, two_d=True, stride=op_attn.F_ARG_BYTES,
             after="E_prologue")                                        # (the cached rows a task reads depend on its sequence's position alone)
         dense(f"o_proj_{L}", Wl("wo"), "attn_out", "o", d.H, d.NH * d.HD)

@@ -43,7 +43,8 @@ def tagged_part_len(tag: int, whole: bool = False, words: bool = False, lim: int
     grids of a step that share the partial buffers (the layer index): a merger only accepts partials carrying its own.
     whole: bit 24, the form with one task per (sequence, q group) that takes all partitions itself (the batched step).
     words: bit 25, qkv names words (bf16 value | step flag << 16) and the outputs are also written as words, at exp_sums.
-    lim: bits 26..30, a context of up to so many partitions is taken whole by the tasks of the first one (no partials, no merge)."""
+    lim: bits 26..30, a context of up to so many partitions is taken whole by the tasks of the first one (no partials, no merge); with `whole`: 1 = the
+    probabilities of cached positions go into the product with all 24 bits, 0 = with 17."""
     return GQ_PART | (min(lim, 31) << 26) | ((tag & 0xff) << 16) | (GQ_WHOLE if whole else 0) | (GQ_WORDS if words else 0)
 
 
@@ -74,7 +75,7 @@ def check_fused(NH: int, NKV: int, HD: int, BS: int, X: int, max_parts: int, gq:
     check_shape(NH, NKV, HD, BS, X, max_parts)
     G = NH // NKV
     if gq:
-        if gq not in (1, 2, 4, 8) or G % gq or HD != 128 or BS != 16 or (part_len & 0xffff) != GQ_PART or part_len >> 31 or ((part_len >> 24) & 1 and part_len >> 25):
+        if gq not in (1, 2, 4, 8) or G % gq or HD != 128 or BS != 16 or (part_len & 0xffff) != GQ_PART or part_len >> 31 or ((part_len >> 24) & 1 and part_len >> 25 not in (0, 2)):
             raise ValueError(f"attn_fused grouped form: needs gq in (1, 2, 4, 8) dividing G={G}, head_dim 128, block size 16 and "
                              f"part_len {GQ_PART} (gq={gq}, HD={HD}, BS={BS}, part_len={part_len})")
         if gq * max_parts > 4096:

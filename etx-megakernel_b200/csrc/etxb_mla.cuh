@@ -75,7 +75,7 @@ __device__ __forceinline__ void mla_finish(const etxb_mla_args& d, const Smem& s
   const uint2* ph = (const uint2*)d.tmp + (size_t)h * d.max_parts * PW;
   // A round: up to NF partitions' statistics (a lane each, every warp for itself) and this thread's values of them, requested together: behind the
   // slowest partition comes one trip to L2.  Between rounds (contexts of more than 1280 positions) the sums are rescaled to the larger maximum.
-  // (Statistics, then weights by one warp, then values, a barrier between any two: 1.3 us more.)
+  // (Statistics, then weights by one warp, then values, a barrier between any two, and bf16 vectors instead of words: 18.1 us a phase at 1043 positions, so 15.6.)
   constexpr int NF = 10;
   const uint2* vp = ph + min(tid, C - 1);
   float o = 0.f, L = 0.f, M = -INFINITY;

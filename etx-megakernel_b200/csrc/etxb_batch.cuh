@@ -151,7 +151,7 @@ __device__ __forceinline__ void tile_route(const unsigned char* a, int blk, cons
   const int warp = tidx() >> 5, lane = tidx() & 31;
   if (d.elist == nullptr) {
     if (blk < d.nb && warp == 0)
-      warp_topk<false>((const __nv_bfloat16*)d.logits + (size_t)blk * d.E, 0u, d.E, d.K, (d.mode & 0xff) == 1, (d.mode & ETXB_MODE_BF16_WTS) != 0,
+      warp_topk<false, false>((const __nv_bfloat16*)d.logits + (size_t)blk * d.E, 0u, d.E, d.K, (d.mode & 0xff) == 1, (d.mode & ETXB_MODE_BF16_WTS) != 0,
                        d.ids + (size_t)blk * d.K, d.wts + (size_t)blk * d.K, nullptr);
     return;
   }
@@ -159,7 +159,7 @@ __device__ __forceinline__ void tile_route(const unsigned char* a, int blk, cons
   int32_t* sids = (int32_t*)sm.xs;                                 // [nb][K]
   float* swts = sm.xs + 2048;
   for (int b = warp; b < d.nb; b += ETXB_CONSUMER_WARPS) {
-    warp_topk<false>((const __nv_bfloat16*)d.logits + (size_t)b * d.E, 0u, d.E, d.K, (d.mode & 0xff) == 1, (d.mode & ETXB_MODE_BF16_WTS) != 0,
+    warp_topk<false, false>((const __nv_bfloat16*)d.logits + (size_t)b * d.E, 0u, d.E, d.K, (d.mode & 0xff) == 1, (d.mode & ETXB_MODE_BF16_WTS) != 0,
                      sids + b * d.K, swts + b * d.K, nullptr);
     if (lane < d.K) { d.ids[b * d.K + lane] = sids[b * d.K + lane]; d.wts[b * d.K + lane] = swts[b * d.K + lane]; }
   }

@@ -145,6 +145,18 @@ def test_topk_against_reference_rows(golden_dir):
         np.testing.assert_allclose(host(w)[:K], wts[:K], rtol=4e-6, atol=1e-30)
 
 
+@pytest.mark.parametrize("E,K", [(16, 4), (128, 8), (200, 16)])
+def test_topk_without_weights_still_gives_ids_and_positions(E, K):
+    """wts = 0: the ids and the slots' positions alone."""
+    bits = TW.bf16_bits(np.random.default_rng(E).normal(0, 1, E).astype(np.float32))
+    lg = torch.from_numpy(bits.view(np.int16)).to(DEV).view(torch.bfloat16)
+    i = torch.full((16,), -1, dtype=torch.int32, device=DEV); te = torch.full((16,), -1, dtype=torch.int32, device=DEV)
+    blob = argblock.pack_named(ENT["dsl_topk"], (1, 1, 1), logits=lg.data_ptr(), wts=0, ids=i.data_ptr(), tei=te.data_ptr(), E=E, K=K, mode=0, nbsv=0)
+    op_launch("topk", blob, 1)
+    assert host(i)[:K].tolist() == O.softmax_topk(TW.bf16_to_f32(bits), K, False)[0].tolist()
+    assert host(te)[:K].tolist() == list(range(K))
+
+
 def test_topk_matches_decode_oracle_with_bf16_weights():
     rng = np.random.default_rng(2)
     for _ in range(20):

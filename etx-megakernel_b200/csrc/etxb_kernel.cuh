@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
     }
     if (tidx() == 0) {
       const int out_n = c->r.out_n & (ETXB_OUT_RELAXED - 1), id = c->r.id;
-      const bool relaxed = (c->r.out_n & ETXB_OUT_RELAXED) != 0;   // (the readers look at the words themselves)
+      const bool relaxed = KV != ETXB_VARIANT_BATCH && (c->r.out_n & ETXB_OUT_RELAXED) != 0;   // (the readers look at the words themselves; batched plans have none)
       if (s_stop == 0)                                             // (set when a stage wait gave up inside the body: no arrivals then)
 #pragma unroll 1
         for (int i = 0; i < out_n; ++i) {                          // release: orders the CTA's stores (seen through the barrier) before the count

@@ -430,30 +430,39 @@ static void share_merges(etxb_session* s) {
 // the same parameters, and waited for the event that this one waits for before it reads them (whoever rewrites the logits in between
 // would have to know that this task is done).
 static void share_routing(const etxb_session* s, std::vector<etxb_rec>& recs) {
-  auto block = [&](int32_t i, etxb_gemv_args& a) {
-    const etxb_task& t = s->tasks[i];
+  auto block = [&](const etxb_task& t, etxb_gemv_args& a) {
     const etxb_type& ty = s->types[t.type];
     const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
     if (ty.args[0] != 0 || off < 0 || (uint64_t)off + sizeof a > s->h_pool.size()) return false;
     memcpy(&a, s->h_pool.data() + off, sizeof a);
-    const int j = t.coord[0];
-    return (a.mode & 0xff) >= 2 && a.tpe > 0 && a.rpt > 0 && j >= 0 && j < (int)a.nblocks && (long long)(j % a.tpe) * a.rpt < a.M;   // (a task with rows: its producer looks)
+    return (a.mode & 0xff) >= 2 && a.tpe > 0 && a.rpt > 0;
   };
+  auto rows = [](const etxb_gemv_args& a, int j) { return j >= 0 && j < (int)a.nblocks && (long long)(j % a.tpe) * a.rpt < a.M; };   // (a task with rows: its producer looks)
+  // what two grids' blocks say about each other does not depend on the task: kept by the later grid, for the earlier one and the columns it was asked with
+  struct Pair { int32_t ptype = -1, pcol = 0, col = 0; bool same = false; etxb_gemv_args p, a; };
+  std::vector<Pair> pairs(s->types.size());
   for (uint32_t w = 0; w < s->h.n_workers; ++w) {
     int32_t prev = -1;                                             // the streaming task before
     for (int32_t i = s->qbegin[w]; i < s->qbegin[w + 1]; ++i) {
-      const int body = s->types[s->tasks[i].type].body;
-      if (body < ETXB_BODY_GEMV || body > ETXB_BODY_MOE_DOWN) continue;
-      etxb_gemv_args a, b;
-      if (body != ETXB_BODY_GEMV && prev >= 0 && s->types[s->tasks[prev].type].body != ETXB_BODY_GEMV && block(prev, b) && block(i, a)) {
-        const uint32_t same = 0x0f0000ffu | ETXB_MODE_WORDS_IN;    // fold, always-on experts, where the logits come from
-        const int32_t ev = s->types[s->tasks[i].type].stream_word, pev = s->types[s->tasks[prev].type].stream_word;
-        bool waited = pev == ev;
-        if (pev == -2)
-          for (int k = 0; k < s->tasks[prev].in_n; ++k) waited = waited || s->inwords[s->tasks[prev].in_off + k] == ev;
-        if (ev >= 0 && waited && a.logits == b.logits && a.E == b.E && a.R == b.R && ((a.mode ^ b.mode) & same) == 0 && recs[i].in_n < ETXB_IN_ROUTED) recs[i].in_n |= ETXB_IN_ROUTED;
-      }
+      const etxb_task& t = s->tasks[i];
+      const etxb_type& ty = s->types[t.type];
+      if (ty.body < ETXB_BODY_GEMV || ty.body > ETXB_BODY_MOE_DOWN) continue;
+      const int32_t before = prev, ev = ty.stream_word;
       prev = i;
+      if (ty.body == ETXB_BODY_GEMV || ev < 0 || before < 0 || recs[i].in_n >= ETXB_IN_ROUTED) continue;
+      const etxb_task& b = s->tasks[before];
+      const etxb_type& bt = s->types[b.type];
+      bool waited = bt.stream_word == ev;
+      if (bt.stream_word == -2)
+        for (int k = 0; k < b.in_n; ++k) waited = waited || s->inwords[b.in_off + k] == ev;
+      if (bt.body == ETXB_BODY_GEMV || !waited) continue;
+      Pair& q = pairs[t.type];
+      if (q.ptype != b.type || q.pcol != b.coord[1] || q.col != t.coord[1]) {
+        q.ptype = b.type; q.pcol = b.coord[1]; q.col = t.coord[1];
+        const uint32_t bits = 0x0f0000ffu | ETXB_MODE_WORDS_IN;    // fold, always-on experts, where the logits come from
+        q.same = block(b, q.p) && block(t, q.a) && q.p.logits == q.a.logits && q.p.E == q.a.E && q.p.R == q.a.R && ((q.p.mode ^ q.a.mode) & bits) == 0;
+      }
+      if (q.same && rows(q.p, b.coord[0]) && rows(q.a, t.coord[0])) recs[i].in_n |= ETXB_IN_ROUTED;
     }
   }
 }
@@ -770,6 +779,31 @@ static int32_t build_tensor_maps(etxb_session* s) {
   return ETXB_OK;
 }
 
+// Whether the tasks of column `c` of a grid hand their results over as words (a few bytes of the block: this is asked for every task).
+static bool hands_over_words(const etxb_session* s, const etxb_type& ty, int32_t c) {
+  const int64_t off = (int64_t)ty.cst[0] + (int64_t)c * ty.cst[1], room = (int64_t)s->h_pool.size() - off;
+  if (ty.args[0] != 0 || off < 0) return false;
+  const unsigned char* blk = s->h_pool.data() + off;
+  const void* at = nullptr;
+  if (ty.body >= ETXB_BODY_GEMV && ty.body <= ETXB_BODY_MOE_DOWN) {
+    int32_t mode = 0;
+    if (room < (int64_t)(sizeof(etxb_gemv_args) + sizeof(etxb_gemv_words))) return false;
+    memcpy(&mode, blk + offsetof(etxb_gemv_args, mode), sizeof mode);
+    memcpy(&at, blk + sizeof(etxb_gemv_args) + offsetof(etxb_gemv_words, out), sizeof at);
+    return (mode & ETXB_MODE_WORDS_OUT) && at != nullptr;          // (null: its readers take the bf16 vector)
+  }
+  if (ty.body == ETXB_BODY_ATTN_FUSED) {
+    int32_t gq = 0, part_len = 0;
+    if (room < (int64_t)sizeof(etxb_attnf_args)) return false;
+    memcpy(&gq, blk + offsetof(etxb_attnf_args, gq), sizeof gq);
+    memcpy(&part_len, blk + offsetof(etxb_attnf_args, part_len), sizeof part_len);
+    return gq > 0 && (part_len & ETXB_GQ_WORDS) != 0;
+  }
+  if (ty.body != ETXB_BODY_MLA_ATTN || room < (int64_t)sizeof(etxb::etxb_mla_args)) return false;
+  memcpy(&at, blk + offsetof(etxb::etxb_mla_args, words), sizeof at);
+  return at != nullptr;
+}
+
 static int32_t upload_type_args(etxb_session* s) {
   std::vector<void*> ta((size_t)s->h.n_types * ETXB_MAX_ARGS, nullptr);
   for (size_t t = 0; t < s->types.size(); ++t)
@@ -810,25 +844,7 @@ static int32_t upload_type_args(etxb_session* s) {
     r.args = has_block ? (uint64_t)(uintptr_t)ta[(size_t)t.type * ETXB_MAX_ARGS] + (uint64_t)ty.cst[0] + (uint64_t)t.coord[1] * (uint64_t)ty.cst[1]
                        : (uint64_t)(uintptr_t)s->d_pool;
     // a grid whose readers look at words announces itself without waiting for its stores
-    const int64_t off = (int64_t)ty.cst[0] + (int64_t)t.coord[1] * ty.cst[1];
-    bool words = false;
-    if (ty.args[0] == 0 && off >= 0 && (ty.body == ETXB_BODY_GEMV || ty.body == ETXB_BODY_MOE_UP || ty.body == ETXB_BODY_MOE_DOWN) && (uint64_t)off + sizeof(etxb_gemv_args) <= s->h_pool.size()) {
-      etxb_gemv_args a;
-      memcpy(&a, s->h_pool.data() + off, sizeof a);
-      etxb_gemv_words w;
-      if ((a.mode & ETXB_MODE_WORDS_OUT) && (uint64_t)off + sizeof a + sizeof w <= s->h_pool.size()) {
-        memcpy(&w, s->h_pool.data() + off + sizeof a, sizeof w);
-        words = w.out != nullptr;                                  // (null: its readers take the bf16 vector)
-      }
-    } else if (ty.args[0] == 0 && off >= 0 && ty.body == ETXB_BODY_ATTN_FUSED && (uint64_t)off + sizeof(etxb_attnf_args) <= s->h_pool.size()) {
-      etxb_attnf_args a;
-      memcpy(&a, s->h_pool.data() + off, sizeof a);
-      words = a.gq > 0 && (a.part_len & ETXB_GQ_WORDS) != 0;
-    } else if (ty.args[0] == 0 && off >= 0 && ty.body == ETXB_BODY_MLA_ATTN && (uint64_t)off + sizeof(etxb::etxb_mla_args) <= s->h_pool.size()) {
-      etxb::etxb_mla_args a;
-      memcpy(&a, s->h_pool.data() + off, sizeof a);
-      words = a.words != nullptr;
-    }
+    const bool words = hands_over_words(s, ty, t.coord[1]);
     if (words && s->xbase != nullptr) return fail(ETXB_E_UNSUPPORTED, "a sharded session hands rows over as flagged words of its exchange region only");
     if (words && t.out_n < ETXB_OUT_RELAXED) r.out_n |= ETXB_OUT_RELAXED;
     r.stream_word = ty.stream_word;
@@ -838,11 +854,7 @@ static int32_t upload_type_args(etxb_session* s) {
       if (rc) return rc;
     }
   }
-  std::vector<etxb_rec> routed = recs;
-  share_routing(s, routed);
-  if (!s->d_recs) CU(cudaMalloc((void**)&s->d_recs, recs.size() * sizeof(etxb_rec) + 96));
-  CU(cudaMemcpy(s->d_recs, routed.data(), routed.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
-  // the same records (every launch finds its own expert ids) grouped by grid (type), worker by worker, for the one-launch-per-grid baseline
+  // the records (every launch finds its own expert ids) grouped by grid (type), worker by worker, for the one-launch-per-grid baseline
   const uint32_t W = s->h.n_workers, NT = s->h.n_types;
   std::vector<etxb_rec> ug; ug.reserve(recs.size());
   std::vector<int32_t> uq((size_t)NT * (W + 1), 0);
@@ -865,6 +877,9 @@ static int32_t upload_type_args(etxb_session* s) {
   if (!s->d_urecs) { CU(cudaMalloc((void**)&s->d_urecs, ug.size() * sizeof(etxb_rec) + 96)); CU(cudaMalloc((void**)&s->d_uqbegin, uq.size() * 4)); }
   CU(cudaMemcpy(s->d_urecs, ug.data(), ug.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
   CU(cudaMemcpy(s->d_uqbegin, uq.data(), uq.size() * 4, cudaMemcpyHostToDevice));
+  share_routing(s, recs);
+  if (!s->d_recs) CU(cudaMalloc((void**)&s->d_recs, recs.size() * sizeof(etxb_rec) + 96));
+  CU(cudaMemcpy(s->d_recs, recs.data(), recs.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
   s->args_dirty = false;
   return ETXB_OK;
 }

@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -60,8 +61,12 @@ struct etxb_session {
   int32_t* h_ctrl = nullptr;           // pinned mirror
   int32_t* h_tok = nullptr;            // pinned staging of the host decode loop
   bool args_dirty = true, trace = false, launched = false;
-  uint32_t epoch = 0;
-  uint32_t salt = 0;                   // added to the epoch in the flags of words: sessions that share buffers do not take each other's
+  uint32_t epoch = 0, serial = 0;      // steps launched; number of the last launch among all of the process (g_launches)
+  // The words its grids hand over (address ranges), whether they may hold anything but its own last step's, and the sessions whose
+  // words overlap them (see claim_words)
+  std::vector<std::pair<uintptr_t, uintptr_t>> words;
+  bool words_stale = true;
+  std::vector<etxb_session*> sharers;
   unsigned long long timeout_ns = 2000000000ull;
   etxb_stepv step{};
   cudaStream_t stream = nullptr, own_stream = nullptr;
@@ -79,6 +84,10 @@ struct etxb_session {
   bool tc_on = false;                  // the plan has tensor-core tiles (tcgen05): the kernel allocates tensor memory
   void* d_maps = nullptr;              // their TMA tensor maps, one per grid (128 bytes each)
 };
+
+// Launches of this process: the flags of attention partials carry the number, so that no launch takes another's, whatever sessions and
+// single-tile launches share the buffers (23 bits: eight million launches until a number comes back).
+static std::atomic<uint32_t> g_launches{0};
 
 static int g_kernel_ready[64];
 
@@ -560,13 +569,12 @@ static int32_t parse_plan(etxb_session* s, const unsigned char* b, size_t n) {
   return ETXB_OK;
 }
 
+static void forget_words(etxb_session* s);
 extern "C" int32_t etxb_create(const void* plan_blob, size_t bytes, int device, etxb_session** out) {
   if (!plan_blob || !out) return fail(ETXB_E_ARG, "null argument");
   *out = nullptr;
   etxb_session* s = new etxb_session();
   s->device = device;
-  static std::atomic<uint32_t> sessions{0};
-  s->salt = sessions.fetch_add(1u) * 2749u;
   int32_t rc = prepare_kernel(device, &s->workers);
   if (rc == ETXB_OK) rc = parse_plan(s, (const unsigned char*)plan_blob, bytes);
   if (rc == ETXB_OK && (int)s->h.n_workers > s->workers) rc = fail(ETXB_E_RESIDENCY, "plan wants more workers than the device has SMs");
@@ -583,6 +591,7 @@ extern "C" int32_t etxb_create(const void* plan_blob, size_t bytes, int device, 
 
 extern "C" int32_t etxb_destroy(etxb_session* s) {
   if (!s) return ETXB_OK;
+  forget_words(s);
   cudaSetDevice(s->device);
   if (s->launched) cudaDeviceSynchronize();
   void* ptrs[] = {s->d_tasks, s->d_recs, s->d_urecs, s->d_uqbegin, s->d_qbegin, s->d_types, s->d_type_args, s->d_events, s->d_evcount, s->d_inwords, s->d_outwords,
@@ -804,6 +813,91 @@ static bool hands_over_words(const etxb_session* s, const etxb_type& ty, int32_t
   return at != nullptr;
 }
 
+// Flags of words have 15 bits of the session's own step number: in memory that nobody else writes a word is one step old until it is written again.  So
+// the words must hold nothing else when a step begins: they are zeroed before the first step behind a binding (the memory may have been another,
+// closed session's), and before a step that follows one of another session whose words overlap.
+static std::mutex g_words_mutex;
+static std::vector<etxb_session*> g_words_sessions;                // bound sessions that hand words over
+
+static void forget_words(etxb_session* s) {
+  std::lock_guard<std::mutex> lock(g_words_mutex);
+  auto drop = [&](std::vector<etxb_session*>& v) { v.erase(std::remove(v.begin(), v.end(), s), v.end()); };
+  for (etxb_session* o : s->sharers) drop(o->sharers);
+  drop(g_words_sessions);
+  s->sharers.clear();
+  s->words.clear();
+  s->words_stale = true;
+}
+static void find_words(etxb_session* s) {
+  forget_words(s);
+  std::vector<std::pair<uintptr_t, uintptr_t>> all;
+  auto add = [&](const void* p, int64_t n) { if (p != nullptr && n > 0) all.emplace_back((uintptr_t)p, (uintptr_t)p + 4 * (uintptr_t)n); };
+  std::vector<int32_t> cols(s->types.size(), 0);                   // a grid's last column with a block of its own
+  for (const etxb_task& t : s->tasks)
+    if (s->types[t.type].cst[1] != 0) cols[t.type] = std::max(cols[t.type], t.coord[1]);
+  for (size_t i = 0; i < s->types.size(); ++i) {
+    const etxb_type& ty = s->types[i];
+    const bool family = ty.body >= ETXB_BODY_GEMV && ty.body <= ETXB_BODY_MOE_DOWN;
+    for (int32_t c = 0; c <= cols[i]; ++c) {
+      const int64_t off = (int64_t)ty.cst[0] + (int64_t)c * ty.cst[1], room = (int64_t)s->h_pool.size() - off;
+      if (ty.args[0] != 0 || off < 0 || (!family && !hands_over_words(s, ty, c))) continue;
+      const unsigned char* blk = s->h_pool.data() + off;
+      if (ty.body == ETXB_BODY_ATTN_FUSED) {
+        etxb_attnf_args a;
+        memcpy(&a, blk, sizeof a);
+        add(a.exp_sums, (int64_t)a.NH * a.HD);
+      } else if (ty.body == ETXB_BODY_MLA_ATTN) {
+        etxb::etxb_mla_args a;
+        memcpy(&a, blk, sizeof a);
+        add(a.words, (int64_t)a.NH * a.DV);
+      } else {
+        etxb_gemv_args a;
+        etxb_gemv_words w;
+        if (room < (int64_t)(sizeof a + sizeof w)) continue;
+        memcpy(&a, blk, sizeof a);
+        if (!(a.mode & ETXB_MODE_WORDS_OUT)) continue;
+        memcpy(&w, blk + sizeof a, sizeof w);
+        const int spt = ((a.mode >> 16) & 0xff) ? ((a.mode >> 16) & 0xff) : 1;
+        const bool one = ty.body == ETXB_BODY_GEMV || (a.mode & ETXB_MODE_SUM_SLOTS) || a.tpe < 1;
+        add(w.out, (int64_t)a.M * (one ? 1 : (((int64_t)a.nblocks + a.tpe - 1) / a.tpe) * spt));
+        if ((a.mode & 0xff) == ETXB_MODE_NORM) { add(w.z, a.K); add(w.x, a.K); }
+        if (ty.body == ETXB_BODY_MOE_UP && (a.mode & 0xff) >= 2) add(w.route, 48);
+      }
+    }
+  }
+  if (all.empty()) return;
+  std::sort(all.begin(), all.end());
+  for (const auto& r : all)
+    if (!s->words.empty() && r.first <= s->words.back().second) s->words.back().second = std::max(s->words.back().second, r.second);
+    else s->words.push_back(r);
+  std::lock_guard<std::mutex> lock(g_words_mutex);
+  for (etxb_session* o : g_words_sessions) {
+    bool overlap = false;
+    size_t i = 0, j = 0;
+    while (!overlap && i < s->words.size() && j < o->words.size()) {
+      overlap = s->words[i].first < o->words[j].second && o->words[j].first < s->words[i].second;
+      if (s->words[i].second < o->words[j].second) ++i; else ++j;
+    }
+    if (overlap) { s->sharers.push_back(o); o->sharers.push_back(s); }
+  }
+  g_words_sessions.push_back(s);
+}
+// In front of a step on s->stream.
+static int32_t claim_words(etxb_session* s) {
+  if (s->words.empty()) return ETXB_OK;
+  bool stale;
+  {
+    std::lock_guard<std::mutex> lock(g_words_mutex);
+    for (etxb_session* o : s->sharers) o->words_stale = true;
+    stale = s->words_stale;
+  }
+  if (!stale) return ETXB_OK;
+  for (const auto& r : s->words) CU(cudaMemsetAsync((void*)r.first, 0, r.second - r.first, s->stream));
+  std::lock_guard<std::mutex> lock(g_words_mutex);
+  s->words_stale = false;
+  return ETXB_OK;
+}
+
 static int32_t upload_type_args(etxb_session* s) {
   std::vector<void*> ta((size_t)s->h.n_types * ETXB_MAX_ARGS, nullptr);
   for (size_t t = 0; t < s->types.size(); ++t)
@@ -880,6 +974,7 @@ static int32_t upload_type_args(etxb_session* s) {
   share_routing(s, recs);
   if (!s->d_recs) CU(cudaMalloc((void**)&s->d_recs, recs.size() * sizeof(etxb_rec) + 96));
   CU(cudaMemcpy(s->d_recs, recs.data(), recs.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
+  find_words(s);
   s->args_dirty = false;
   return ETXB_OK;
 }
@@ -889,7 +984,7 @@ static void fill_params(etxb_session* s, etxb_params& p) {
   p.events = s->d_events; p.evcount = s->d_evcount; p.inwords = s->d_inwords; p.outwords = s->d_outwords;
   p.ctrl = s->d_ctrl; p.trace = s->trace ? s->d_trace : nullptr; p.exec_count = s->trace ? s->d_exec : nullptr;
   p.step_dev = nullptr; p.timeout_ns = s->timeout_ns; p.epoch = s->epoch; p.n_workers = (int32_t)s->h.n_workers;
-  p.step = s->step; p.salt = s->salt;
+  p.step = s->step; p.serial = s->serial = g_launches.fetch_add(1u) + 1u;
   p.n_peers = s->n_ranks - 1; p.rank = s->rank; p.xargmax = s->xargmax; p.tc_on = s->tc_on ? 1u : 0u; p.xbase = s->xbase;
   for (int q = 0; q < ETXB_MAX_PEERS; ++q) p.xpeer[q] = s->xpeer[q];
 }
@@ -907,6 +1002,7 @@ extern "C" int32_t etxb_launch(etxb_session* s, void* cuda_stream) {
   if (s->args_dirty) { int32_t rc = upload_type_args(s); if (rc) return rc; }
   s->stream = cuda_stream ? (cudaStream_t)cuda_stream : s->own_stream;
   if (s->trace && s->d_exec) CU(cudaMemsetAsync(s->d_exec, 0, (size_t)s->h.n_tasks * 4, s->stream));
+  { int32_t rc = claim_words(s); if (rc) return rc; }
   ++s->epoch;
   etxb_params p;
   fill_params(s, p);
@@ -930,6 +1026,7 @@ extern "C" int32_t etxb_launch_unfused(etxb_session* s, void* cuda_stream) {
   if (s->n_ranks > 1) return fail(ETXB_E_UNSUPPORTED, "a sharded session runs as the single launch only");   // (its grids wait for peers: launches of two ranks could not be ordered)
   s->stream = cuda_stream ? (cudaStream_t)cuda_stream : s->own_stream;
   if (s->trace && s->d_exec) CU(cudaMemsetAsync(s->d_exec, 0, (size_t)s->h.n_tasks * 4, s->stream));
+  { int32_t rc = claim_words(s); if (rc) return rc; }
   ++s->epoch;
   etxb_params p;
   fill_params(s, p);
@@ -948,6 +1045,9 @@ extern "C" int32_t etxb_launch_unfused(etxb_session* s, void* cuda_stream) {
 static int32_t read_ctrl(etxb_session* s) {
   CU(cudaMemcpyAsync(s->h_ctrl, s->d_ctrl, 32, cudaMemcpyDeviceToHost, s->stream));
   CU(cudaStreamSynchronize(s->stream));
+  if (s->h_ctrl[0] != 0 && s->h_ctrl[2] == -3)                     // a partial that never came: its flag by the session's steps, as all else is reported
+    for (int i = 3; i <= 4; ++i)
+      if (s->h_ctrl[i] != 0) s->h_ctrl[i] = (int32_t)(((uint32_t)s->h_ctrl[i] - ((s->serial - s->epoch) << 8)) | 0x80000000u);
   return ETXB_OK;
 }
 
@@ -961,7 +1061,7 @@ static int32_t recover(etxb_session* s) {
   // per kv head, max_parts arrivals per step, elected when the count reaches a multiple of max_parts): a step abandoned
   // in the middle of an attention phase leaves them off a multiple, and every later step would then elect its merging
   // task too early.  Zero is a multiple: clear the counters of every fused attention grid of the pool.  (The grouped
-  // form has no counters: its partials carry the step number, which only grows.)
+  // form has no counters: its partials carry the launch's number, which only grows.)
   for (const etxb_type& ty : s->types) {
     if (ty.body != ETXB_BODY_ATTN_FUSED || ty.args[0] != 0 || ty.cst[0] < 0 || (size_t)ty.cst[0] + sizeof(etxb_attnf_args) > s->h_pool.size()) continue;
     etxb_attnf_args a;
@@ -1225,8 +1325,7 @@ extern "C" int32_t etxb_op_launch(int device, int32_t body, const void* argblock
   etxb_params p; memset(&p, 0, sizeof p);
   p.tasks = c.d_tasks; p.recs = c.d_recs; p.qbegin = c.d_qbegin; p.types = c.d_type; p.type_args = c.d_targs; p.events = c.d_events;
   p.evcount = c.d_zero; p.inwords = c.d_zero; p.outwords = c.d_zero; p.ctrl = c.d_ctrl; p.timeout_ns = 2000000000ull;
-  static uint32_t op_epoch[64];                                    // a new step number per launch: flags a tile derives from it never repeat
-  p.epoch = ++op_epoch[device];
+  p.serial = p.epoch = g_launches.fetch_add(1u) + 1u;
   p.n_workers = W;
   if (step) memcpy(&p.step, step, sizeof(p.step));
   return launch_kernel(p, W, st);

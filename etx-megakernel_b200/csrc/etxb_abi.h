@@ -131,7 +131,7 @@ struct etxb_params {
                                                    // argmax (lm_head split by vocabulary); 0 = every rank holds all logits
   unsigned char* xbase;
   unsigned char* xpeer[ETXB_MAX_PEERS];
-  uint32_t salt, pad;                              // added to the epoch in the flags of words on this GPU: sessions that share buffers differ
+  uint32_t serial, pad;                            // number of the launch among all of the process: the flags of attention partials (words: the epoch)
 };
 
 // ctrl[0] bits

@@ -48,11 +48,11 @@ namespace etxb {
 // polls while the others work) -- which re-reads a pair until its flag is this step's.  No counter, no election, no
 // fence: the producers only store, the merger's loads are its wait.  Nothing has to be reset between steps or after an
 // abandoned step; a buffer that was zeroed once never shows a current flag by accident (flags are never 0, differ
-// from grid to grid within a step and grow with the step).  Bounded like every wait: on a give-up the step is abandoned with the timeout status.
-// The flag names the step AND the grid: the layers of a step share the partial buffers, and a merger must not take the
+// from grid to grid within a step and grow with every launch of the process, so sessions may share the buffers, one after the other).  Bounded like every wait: on a give-up the step is abandoned with the timeout status.
+// The flag names the launch AND the grid: the layers of a step share the partial buffers, and a merger must not take the
 // previous layer's partials of the same step for its own.  The grid's tag travels in the upper half of the block's
 // part_len word (the builder puts the layer index there).
-__device__ __forceinline__ uint32_t pair_flag(uint32_t epoch, int part_len) { return ((epoch << 8) | (((uint32_t)part_len >> 16) & 0xffu)) | 0x80000000u; }
+__device__ __forceinline__ uint32_t pair_flag(uint32_t serial, int part_len) { return ((serial << 8) | (((uint32_t)part_len >> 16) & 0xffu)) | 0x80000000u; }
 __device__ __forceinline__ void st_pair(uint2* p, float v, uint32_t fl) {
   asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(__float_as_uint(v)), "r"(fl) : "memory");
 }
@@ -309,7 +309,7 @@ __device__ __forceinline__ void attn_gq_tile(const etxb_attnf_args& d, int blk, 
   constexpr int HD = 128, BS = 16;
   const GqTask t = gq_task(d, blk, S);
   const int NKV = d.NKV, gq = d.gq, tid = tidx(), lane = tid & 31, warp = tid >> 5;
-  const uint32_t fl = pair_flag(sm.epoch(), d.part_len);
+  const uint32_t fl = pair_flag(sm.serial(), d.part_len);
   const int np = min((t.seq + ETXB_GQ_PART - 1) / ETXB_GQ_PART, d.max_parts);
   const GqSmem s(sm.xs);
   const uint32_t n0 = n;

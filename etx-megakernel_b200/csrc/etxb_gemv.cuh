@@ -52,8 +52,8 @@ struct __align__(16) GemvGeom {
 struct CtaVars {
   int32_t* ctrl;
   uint64_t* tr;              // 8 stamps of the running task when tracing, else null (slots 4..7 are in-body marks)
-  uint32_t epoch;            // the step (sharded sessions: the flag of this step's exchanged words derives from it)
-  uint32_t flag;             // flag of this step's words on this GPU (of the step and the session)
+  uint32_t serial;           // number of the launch in the process (flags of attention partials)
+  uint32_t flag;             // flag of this step's words: of the hand-off on this GPU, and of the rows a sharded session exchanges
   int cur;                   // the running task's index in the queue order (reported when a wait gives up)
   int q0, q1;                // the CTA's queue
   int done;                  // tasks of the queue before this one are over (kernels whose other tiles use the ring's memory too)
@@ -73,7 +73,7 @@ struct Smem {
   CtaVars* vars;       // null outside the persistent kernel
   __device__ __forceinline__ int32_t* ctrl() const { return vars->ctrl; }
   __device__ __forceinline__ uint64_t* tr() const { return vars ? vars->tr : nullptr; }
-  __device__ __forceinline__ uint32_t epoch() const { return vars ? vars->epoch : 0u; }
+  __device__ __forceinline__ uint32_t serial() const { return vars ? vars->serial : 0u; }
   __device__ __forceinline__ int cur() const { return vars->cur; }
 };
 // The persistent kernel's shared memory beside the dynamic part.  At namespace scope so that the tiles that are calls find
@@ -955,7 +955,7 @@ __device__ __forceinline__ void tile_gemv_family(int body, const unsigned char* 
     csync();
   } else if (fold == ETXB_MODE_NORM)                               // (a dense MLP's gate+up: the post-attention norm folded in)
     stage_norm_col<LEAN, XCH>(d.rows, d.resid_in, d.resid_out, (void*)d.x, d.ln, body == 3 ? d.ids : nullptr, d.R, K, d.eps, sm.xs, xb, sm.scr, blk == 0,
-                              (XCH && (mode & ETXB_MODE_FLAGGED)) ? row_flag(sm.epoch()) : 0u, &sm);
+                              (XCH && (mode & ETXB_MODE_FLAGGED)) ? s_vars.flag : 0u, &sm);
   else stage_xb(d.x, K, xb);
   }
   const int rows = t.n, spt = t.spt, S = sm.geo->S;

@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
   const Smem sm = smem_view();
   if (threadIdx.x == 0) {
     s_stop = 0;
-    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.epoch = p.epoch; s_vars.flag = row_flag(p.epoch + p.salt); s_vars.cur = 0; s_vars.halt = 0; s_vars.hold = 0; s_vars.done = -1;
+    s_vars.ctrl = p.ctrl; s_vars.tr = nullptr; s_vars.serial = p.serial; s_vars.flag = row_flag(p.epoch); s_vars.cur = 0; s_vars.halt = 0; s_vars.hold = 0; s_vars.done = -1;
     s_deadline = globaltimer() + p.timeout_ns;
     for (int i = 0; i < ETXB_NSTAGE; ++i) { mbar_init(sm.full + i, 1); mbar_init(sm.empty + i, ETXB_EMPTY_COUNT); ((uint32_t*)(sm.empty + ETXB_NSTAGE))[i] = 0xffffffffu; }
     if constexpr (TC) {

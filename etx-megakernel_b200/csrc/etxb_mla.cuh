@@ -59,7 +59,7 @@ __device__ __forceinline__ void mla_out(const etxb_mla_args& d, int i, float v) 
 __device__ __forceinline__ void mla_finish(const etxb_mla_args& d, const Smem& sm, int h, int f, int np) {
   const int C = d.C, DN = d.DN, DV = d.DV, PW = C + 8;
   const int tid = tidx(), lane = tid & 31, warp = tid >> 5;
-  const uint32_t fl = pair_flag(sm.epoch(), d.tag << 16);
+  const uint32_t fl = pair_flag(sm.serial(), d.tag << 16);
   float* oc = sm.xs;                                               // [C] merged, normalised latent
   const __nv_bfloat16* wuv = (const __nv_bfloat16*)d.wkvb + ((size_t)h * (DN + DV) + DN) * C;
   const int v_lo = f * ((DV + ETXB_MLA_FIN - 1) / ETXB_MLA_FIN), v_hi = min(DV, v_lo + (DV + ETXB_MLA_FIN - 1) / ETXB_MLA_FIN);
@@ -202,7 +202,7 @@ __device__ __forceinline__ void tile_mla_attn(const unsigned char* a, int blk, c
   if (tk.part >= tk.np) return;
   const int h = tk.h, C = d.C, DN = d.DN, DR = d.DR, QH = DN + DR, ROW = C + DR, PW = C + 8;
   const bool owner = tk.owner;
-  const uint32_t fl = pair_flag(sm.epoch(), d.tag << 16);
+  const uint32_t fl = pair_flag(sm.serial(), d.tag << 16);
   const int tid = tidx(), lane = tid & 31, warp = tid >> 5, where = sm.cur();
   float* qf = sm.xs;            // [QH <= 256] this head's q row
   float* kvf = qf + 256;        // [ROW <= 640] the raw kv_a row

@@ -130,6 +130,8 @@ int32_t etxb_set_step(etxb_session* s, const etxb_step_params* p);
 /* Options: "timeout_ms" (device wait deadline), "trace" (0/1: per-task stamps + execution counts), "full_kernel" (0/1: run
  * the kernel that holds every tile even when the plan qualifies for a smaller one; see etxb_status_t.kernel_variant). */
 int32_t etxb_set_option(etxb_session* s, const char* key, int64_t value);
+/* Sessions may share device buffers when their steps follow one another (one stream, or synchronised in between): what a step leaves in scratch
+ * memory -- words, partial results -- is never taken for another step's. */
 int32_t etxb_launch(etxb_session* s, void* cuda_stream);
 /* The unfused baseline: the same step as one kernel launch PER GRID, in plan order on one stream (what the reference
  * builds with kernel.py:645-681 and runs with host.h:440-457 to state the gain of the single launch).  Same results;

@@ -218,7 +218,7 @@ static int32_t check_mla_block(const unsigned char* blk, size_t bytes) {
   if (a.NH < 1 || a.C < 8 || a.C > 512 || (a.C & 7) || a.DR < 8 || a.DR > 64 || (a.DR & 7) || a.DN < 1 || a.DN + a.DR > 256 || a.C + a.DR > 640 || a.DV < 1)
     why = "C <= 512 and DR <= 64 (multiples of 8), DN + DR <= 256";
   else if (a.maxlen < 1 || a.maxlen > ETXB_MLA_MAXCTX) why = "1 <= maxlen <= 8192";
-  else if (!a.qkv || !a.kvln || !a.cos_sin || !a.wkvb || !a.cache || !a.positions || !a.out || !a.tmp) why = "null pointer";
+  else if (!a.qkv || !a.kvln || !a.cos_sin || !a.wkvb || !a.cache || !a.positions || (!a.out && !a.words) || !a.tmp) why = "null pointer";
   else if (a.words && (((uintptr_t)a.words & 3) || ((uintptr_t)a.qkv & 3) || (a.C & 1))) why = "hand-off as words: qkv and words name 4-byte words";
   else if (a.max_parts < 1 || a.max_parts > 64 || (long long)a.max_parts * ETXB_MLA_PART < a.maxlen) why = "max_parts partitions of 128 positions cover maxlen (at most 64)";
   else if (a.nblocks != (uint32_t)(a.NH * (a.max_parts + ETXB_MLA_FIN))) why = "the grid is (max_parts + 4) * NH tasks: the partitions, then four finishing tasks per head";
@@ -813,6 +813,58 @@ static bool hands_over_words(const etxb_session* s, const etxb_type& ty, int32_t
   return at != nullptr;
 }
 
+// Refuses plans in which a tile reads a bf16 vector that a grid with relaxed arrivals writes (ETXB_OUT_RELAXED), as far as the blocks in the pool show it.
+static int32_t check_words_readers(const etxb_session* s) {
+  std::vector<std::pair<uintptr_t, uintptr_t>> written;
+  std::vector<std::pair<const void*, size_t>> read;                // (address, the grid)
+  auto wrote = [&](const void* p, int64_t bytes) { if (p != nullptr && bytes > 0) written.emplace_back((uintptr_t)p, (uintptr_t)p + (uintptr_t)bytes); };
+  for (size_t i = 0; i < s->types.size(); ++i) {
+    const etxb_type& ty = s->types[i];
+    const int64_t off = ty.cst[0], room = (int64_t)s->h_pool.size() - off;
+    if (ty.body == ETXB_BODY_ARGMAX) read.emplace_back(s->step.logits, i);
+    if (ty.args[0] != 0 || off < 0 || room <= 0) continue;
+    const unsigned char* blk = s->h_pool.data() + off;
+    const bool words = hands_over_words(s, ty, 0);
+    if (ty.body >= ETXB_BODY_GEMV && ty.body <= ETXB_BODY_MOE_DOWN && room >= (int64_t)sizeof(etxb_gemv_args)) {
+      etxb_gemv_args a;
+      memcpy(&a, blk, sizeof a);
+      const int fold = a.mode & 0xff;
+      if (!(a.mode & ETXB_MODE_WORDS_IN)) {
+        if (fold == ETXB_MODE_NORM) { read.emplace_back(a.rows, i); read.emplace_back(a.resid_in, i); }
+        else read.emplace_back(a.x, i);
+        if (fold >= 2) read.emplace_back(a.logits, i);
+        else if (ty.body != ETXB_BODY_GEMV) { read.emplace_back(a.ids, i); read.emplace_back(a.wts, i); }
+      }
+      if (!words) continue;
+      const int spt = ((a.mode >> 16) & 0xff) ? ((a.mode >> 16) & 0xff) : 1;
+      wrote(a.out, 2 * (int64_t)a.M * (ty.body == ETXB_BODY_GEMV || (a.mode & ETXB_MODE_SUM_SLOTS) || a.tpe < 1 ? 1 : (((int64_t)a.nblocks + a.tpe - 1) / a.tpe) * spt));
+      if (fold == ETXB_MODE_NORM) { wrote(a.resid_out, 2 * (int64_t)a.K); wrote(a.x, 2 * (int64_t)a.K); }
+      if (ty.body == ETXB_BODY_MOE_UP && fold >= 2) { wrote(a.ids, 4 * (int64_t)a.R); wrote(a.wts, 4 * (int64_t)a.R); }
+    } else if (ty.body == ETXB_BODY_ATTN_FUSED && room >= (int64_t)sizeof(etxb_attnf_args)) {
+      etxb_attnf_args a;
+      memcpy(&a, blk, sizeof a);
+      if (words) wrote(a.out, 2 * (int64_t)a.NH * a.HD); else read.emplace_back(a.qkv, i);
+    } else if (ty.body == ETXB_BODY_MLA_ATTN && room >= (int64_t)sizeof(etxb::etxb_mla_args)) {
+      etxb::etxb_mla_args a;
+      memcpy(&a, blk, sizeof a);
+      if (words) wrote(a.out, 2 * (int64_t)a.NH * a.DV); else read.emplace_back(a.qkv, i);
+    } else if (ty.body == ETXB_BODY_TOPK && room >= (int64_t)sizeof(etxb_topk_args)) {
+      etxb_topk_args a;
+      memcpy(&a, blk, sizeof a);
+      read.emplace_back(a.logits, i);
+    }
+  }
+  std::sort(written.begin(), written.end());
+  for (const auto& r : read) {
+    const uintptr_t p = (uintptr_t)r.first;
+    auto it = std::upper_bound(written.begin(), written.end(), std::make_pair(p, UINTPTR_MAX));
+    if (p != 0 && it != written.begin() && p < std::prev(it)->second)
+      return fail(ETXB_E_UNSUPPORTED, "hand-off as words: grid " + std::to_string(r.second) + " (body " + std::to_string(s->types[r.second].body) +
+                                          ") reads a bf16 vector of a grid whose arrivals do not wait for its stores; it has to read the words");
+  }
+  return ETXB_OK;
+}
+
 // Flags of words have 15 bits of the session's own step number: in memory that nobody else writes a word is one step old until it is written again.  So
 // the words must hold nothing else when a step begins: they are zeroed before the first step behind a binding (the memory may have been another,
 // closed session's), and before a step that follows one of another session whose words overlap.
@@ -974,6 +1026,10 @@ static int32_t upload_type_args(etxb_session* s) {
   share_routing(s, recs);
   if (!s->d_recs) CU(cudaMalloc((void**)&s->d_recs, recs.size() * sizeof(etxb_rec) + 96));
   CU(cudaMemcpy(s->d_recs, recs.data(), recs.size() * sizeof(etxb_rec), cudaMemcpyHostToDevice));
+  {
+    int32_t rc = check_words_readers(s);
+    if (rc) return rc;
+  }
   find_words(s);
   s->args_dirty = false;
   return ETXB_OK;

@@ -43,7 +43,12 @@
 #define ETXB_CTX_BYTES 288           // one prefetched task context: 96-byte record + 192 bytes of argument block
 #define ETXB_CTX_SLOTS 4
 #define ETXB_SMEM_BYTES (ETXB_RING_BYTES + ETXB_GEN_BYTES + ETXB_SCR_FLOATS * 4 + 512 + ETXB_CTX_SLOTS * ETXB_CTX_BYTES)
-#define ETXB_OUT_RELAXED 0x10000     // etxb_rec.out_n: the arrivals need not wait for the task's stores (its readers look at words)
+// etxb_rec.out_n: the arrivals need not wait for the task's stores, its readers look at words.  Behind such an arrival the words alone are ordered:
+// a task that waits for it does not see the grid's bf16 vectors, nor what the grid itself had acquired.  So whoever waits for it reads words, step
+// parameters or what it waits for by a releasing grid's event of its own; a plan whose tasks read a bf16 vector of such a grid is refused
+// (check_words_readers), and of the layers' bf16 vectors only those of the last writer hold anything to rely on when the step is over (a null
+// address leaves one out).
+#define ETXB_OUT_RELAXED 0x10000
 #define ETXB_IN_ROUTED 0x10000        // etxb_rec.in_n: the streaming task before this one in the queue waited for the same event and found the same expert ids
 #define ETXB_ATTN_PART 32            // KV positions per attention task
 #define ETXB_MAX_PEERS 7           // ranks of a sharded model besides this one

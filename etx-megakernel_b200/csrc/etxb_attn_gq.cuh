@@ -220,7 +220,7 @@ __device__ __forceinline__ void head_norm_rope_r(uint2 x, float* xh, bool norm, 
 template <bool WD>
 __device__ __forceinline__ void gq_out(const etxb_attnf_args& d, const Smem& sm, int i, float v) {
   if (WD && (d.part_len & ETXB_GQ_WORDS)) st_word((uint32_t*)d.exp_sums + i, bf_bits(v) | s_vars.flag);
-  ((__nv_bfloat16*)d.out)[i] = __float2bfloat16_rn(v);
+  if (!WD || d.out != nullptr) ((__nv_bfloat16*)d.out)[i] = __float2bfloat16_rn(v);
 }
 // one row of 128 values of this step's qkv, four per lane
 template <bool WD>

@@ -987,7 +987,7 @@ __device__ __forceinline__ void tile_gemv_family(int body, const unsigned char* 
   auto put = [&](uint32_t at, float y) {
     const uint32_t u = bf_bits(y);
     if (WD && words != nullptr) st_word(words + at, u | fl);
-    ((unsigned short*)out)[at] = (unsigned short)u;
+    if (out != nullptr) ((unsigned short*)out)[at] = (unsigned short)u;
   };
   if (body == 3) {
 #pragma unroll 1

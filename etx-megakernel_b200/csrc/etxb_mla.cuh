@@ -49,7 +49,7 @@ struct etxb_mla_args {
 
 __device__ __forceinline__ void mla_out(const etxb_mla_args& d, int i, float v) {
   if (d.words != nullptr) st_word(d.words + i, bf_bits(v) | s_vars.flag);
-  ((__nv_bfloat16*)d.out)[i] = __float2bfloat16_rn(v);
+  if (d.out != nullptr) ((__nv_bfloat16*)d.out)[i] = __float2bfloat16_rn(v);
 }
 // A finishing task of head h: waits (bounded) for the head's np partials, merges them -- weights exp(m_p - max m),
 // partitions in ascending order -- and applies rows [f * DV / FIN, ..) of W_UV.  The finishing tasks come after the

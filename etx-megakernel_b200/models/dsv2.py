@@ -293,6 +293,9 @@ def build_graph(d: MlaDims, ptr, maxlen: int = 1072, machine: MachineModel | str
     def wptr(layer, name):
         return ptr("words") + 4 * (layer * wlen + wat[name])
 
+    def kept(plain, layer):                                            # (models.qwen.build_graph)
+        return ptr(plain) if not words or layer == d.L - 1 else 0
+
     def source(plain, layer, name):
         return wptr(layer, name) if words else ptr(plain)
 
@@ -308,45 +311,45 @@ def build_graph(d: MlaDims, ptr, maxlen: int = 1072, machine: MachineModel | str
         Wl = lambda n, L=L: ptr(f"{L}.{n}")                                  # noqa: E731
         first = L == 0
         t, rpt = m.gemv_tasks(d.NQKV)
-        blob = gb("dsl_gemv_fold", t, W=Wl("wqa"), x=ptr("hn"), out=ptr("qkv"), M=d.NQKV, K=d.H, rpt=rpt, tpe=1, rows=0 if first else source("moe_out", L - 1, "out"),
-                  resid_in=ptr("resid") if first else source("resid2", L - 1, "z2"), resid_out=0 if first else ptr("resid"), ln=Wl("ln1"), R=0 if first else 1, eps=d.eps,
+        blob = gb("dsl_gemv_fold", t, W=Wl("wqa"), x=0 if words else ptr("hn"), out=kept("qkv", L), M=d.NQKV, K=d.H, rpt=rpt, tpe=1, rows=0 if first else source("moe_out", L - 1, "out"),
+                  resid_in=ptr("resid") if first else source("resid2", L - 1, "z2"), resid_out=0 if first or words else ptr("resid"), ln=Wl("ln1"), R=0 if first else 1, eps=d.eps,
                   mode=op_gemv.MODE_NORM | (0 if first else WI) | WO, nb=1)
         blob = with_words(blob, out=(L, "qkv"), z=(L, "z1"))
         prev = add(f"qkv_{L}", "dsl_gemv_fold", "qkv", L, blob, t, prev, f"E_qkv_{L}", d.NQKV, d.H, after="")
         blob = argblock.pack_named(ent["mla_attn"], (d.NH * (nparts + op_mla.FINISHERS), 1, 1), qkv=source("qkv", L, "qkv"), kvln=Wl("kvln"), cos_sin=ptr("cos_sin"), wkvb=Wl("wkvb"),
-                                   cache=ptr("ckv") + L * cache_layer_bytes, positions=ptr("positions"), out=ptr("attn_out"), NH=d.NH, C=d.C, DN=d.DN, DR=d.DR,
+                                   cache=ptr("ckv") + L * cache_layer_bytes, positions=ptr("positions"), out=kept("attn_out", L), NH=d.NH, C=d.C, DN=d.DN, DR=d.DR,
                                    DV=d.DV, maxlen=maxlen, scale=d.scale, eps=d.eps, tmp=ptr("mla_tmp"), max_parts=nparts, tag=L & 0xff, words=wptr(L, "attn") if words else 0)
         prev = add(f"attn_{L}", "mla_attn", "attn_fused", L, blob, d.NH * (nparts + op_mla.FINISHERS), prev, f"E_attn_{L}",
                    after="E_pro")                                      # (W_UK depends on nothing, the cached rows on the step's position alone)
         t, rpt = m.gemv_tasks(d.H)
-        blob = gb("dsl_gemv", t, W=Wl("wo"), x=source("attn_out", L, "attn"), out=ptr("o"), M=d.H, K=d.NH * d.DV, rpt=rpt, tpe=1, eps=d.eps, nb=1, mode=WI | WO)
+        blob = gb("dsl_gemv", t, W=Wl("wo"), x=source("attn_out", L, "attn"), out=kept("o", L), M=d.H, K=d.NH * d.DV, rpt=rpt, tpe=1, eps=d.eps, nb=1, mode=WI | WO)
         blob = with_words(blob, out=(L, "o"))
         prev = add(f"o_proj_{L}", "dsl_gemv", "o_proj", L, blob, t, prev, f"E_o_{L}", d.H, d.NH * d.DV, after="")
         if d.dense(L):
             spt, tpe, rpt = dense_sz.up
-            blob = gb("dsl_moe_up", tpe, W=Wl("wgu"), x=ptr("o_norm"), out=ptr("mc2"), estride=0, M=d.DENSE_INTER, K=d.H, rpt=rpt, tpe=tpe, rows=source("o", L, "o"),
-                      resid_in=source("resid", L, "z1"), resid_out=ptr("resid2"), ln=Wl("ln2"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM | WI | WO, nb=1)
+            blob = gb("dsl_moe_up", tpe, W=Wl("wgu"), x=kept("o_norm", L), out=kept("mc2", L), estride=0, M=d.DENSE_INTER, K=d.H, rpt=rpt, tpe=tpe, rows=source("o", L, "o"),
+                      resid_in=source("resid", L, "z1"), resid_out=kept("resid2", L), ln=Wl("ln2"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM | WI | WO, nb=1)
             blob = with_words(blob, out=(L, "act"), z=(L, "z2"))
             prev = add(f"gate_up_{L}", "dsl_moe_up", "gate_up", L, blob, tpe, prev, f"E_up_{L}", d.DENSE_INTER, d.H, after="", slots=2)
             tpe, rpt = dense_sz.down
-            blob = gb("dsl_moe_down", tpe, W=Wl("wd"), x=source("mc2", L, "act"), out=ptr("moe_out"), estride=0, M=d.H, K=d.DENSE_INTER, rpt=rpt, tpe=tpe, eps=d.eps, nb=1, mode=WI | WO)
+            blob = gb("dsl_moe_down", tpe, W=Wl("wd"), x=source("mc2", L, "act"), out=kept("moe_out", L), estride=0, M=d.H, K=d.DENSE_INTER, rpt=rpt, tpe=tpe, eps=d.eps, nb=1, mode=WI | WO)
             blob = with_words(blob, out=(L, "out"))
             prev = add(f"down_{L}", "dsl_moe_down", "down", L, blob, tpe, prev, f"E_dn_{L}", d.H, d.DENSE_INTER, after="")
             continue
         t, rpt = moe_sz.router
-        blob = gb("dsl_gemv_fold", t, W=Wl("wr"), x=ptr("o_norm"), out=ptr("rlog"), M=d.E, K=d.H, rpt=rpt, tpe=1, rows=source("o", L, "o"), resid_in=source("resid", L, "z1"),
-                  resid_out=ptr("resid2"), ln=Wl("ln2"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM | WI | WO, nb=1)
+        blob = gb("dsl_gemv_fold", t, W=Wl("wr"), x=kept("o_norm", L), out=kept("rlog", L), M=d.E, K=d.H, rpt=rpt, tpe=1, rows=source("o", L, "o"), resid_in=source("resid", L, "z1"),
+                  resid_out=kept("resid2", L), ln=Wl("ln2"), R=1, eps=d.eps, mode=op_gemv.MODE_NORM | WI | WO, nb=1)
         blob = with_words(blob, out=(L, "rlog"), z=(L, "z2"), x=(L, "x2"))
         prev = add(f"router_{L}", "dsl_gemv_fold", "router", L, blob, t, prev, f"E_rt_{L}", d.E, d.H, after="")
         topk_mode = (op_gemv.MODE_TOPK_RENORM if d.norm_topk else op_gemv.MODE_TOPK) | op_gemv.mode_shared(d.NS)
         spt, tpe, rpt = moe_sz.up
         groups = d.SLOTS // spt
-        blob = gb("dsl_moe_up_fold", groups * tpe, W=Wl("w13"), x=source("o_norm", L, "x2"), out=ptr("mc2"), ids=ptr("ti"), wts=ptr("tw"), estride=2 * d.MI * d.H, M=d.MI,
+        blob = gb("dsl_moe_up_fold", groups * tpe, W=Wl("w13"), x=source("o_norm", L, "x2"), out=kept("mc2", L), ids=kept("ti", L), wts=kept("tw", L), estride=2 * d.MI * d.H, M=d.MI,
                   K=d.H, rpt=rpt, tpe=tpe, R=d.SLOTS, eps=d.eps, mode=topk_mode | op_gemv.mode_spt(spt) | WI | WO, E=d.E, logits=source("rlog", L, "rlog"), nb=1)
         blob = with_words(blob, out=(L, "act"), route=(L, "route"))
         prev = add(f"moe_up_{L}", "dsl_moe_up_fold", "moe_up", L, blob, groups * tpe, prev, f"E_up_{L}", d.MI, d.H, slots=2 * d.SLOTS)
         tpe, rpt = moe_sz.down
-        blob = gb("dsl_moe_down_fold", tpe, W=Wl("w2"), x=source("mc2", L, "act"), out=ptr("moe_out"), ids=ptr("ti"), wts=ptr("tw"), estride=d.H * d.MI, M=d.H, K=d.MI,
+        blob = gb("dsl_moe_down_fold", tpe, W=Wl("w2"), x=source("mc2", L, "act"), out=kept("moe_out", L), ids=ptr("ti"), wts=ptr("tw"), estride=d.H * d.MI, M=d.H, K=d.MI,
                   rpt=rpt, tpe=tpe, R=d.SLOTS, eps=d.eps, mode=topk_mode | op_gemv.MODE_ROUTE_READY | op_gemv.mode_spt(d.SLOTS) | op_gemv.MODE_SUM_SLOTS | WI | WO,
                   E=d.E, logits=source("rlog", L, "rlog"), nb=1)
         blob = with_words(blob, out=(L, "out"), route=(L, "route"))

@@ -435,6 +435,11 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
     def wptr(layer, name):
         return ptr("words") + 4 * (layer * wlen + wat[name])
 
+    def kept(plain, layer, on=words):
+        """Where a grid leaves its bf16 vector: with words only the last layer's, which the caller may look at when the step is over (the layers write
+        one buffer each in turn, and nothing orders their stores behind relaxed arrivals)."""
+        return ptr(plain) if not on or layer == d.L - 1 else 0
+
     def source(plain, layer, name, on=words):
         """Where a grid reads a vector: the layer's words or the bf16 buffer."""
         return wptr(layer, name) if on else ptr(plain)
@@ -472,9 +477,9 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
         # ---- qkv with the input-norm fold
         t, rpt = sz.qkv
         first = L == 0
-        blob = gemv_block("dsl_gemv_fold", t, W=W("wqkv"), x=ptr("hn"), out=ptr("qkv"), M=d.NQKV, K=d.H, rpt=rpt, tpe=1,
+        blob = gemv_block("dsl_gemv_fold", t, W=W("wqkv"), x=0 if words else ptr("hn"), out=kept("qkv", L, awords), M=d.NQKV, K=d.H, rpt=rpt, tpe=1,
                           rows=0 if first else (xblock(L - 1, 1) or source("moe_out", L - 1, "out")), resid_in=ptr("resid") if first else source("resid2", L - 1, "z2"),
-                          resid_out=0 if first else ptr("resid"), ln=W("ln1"), R=0 if first else ranks, eps=d.eps,
+                          resid_out=0 if first or words else ptr("resid"), ln=W("ln1"), R=0 if first else ranks, eps=d.eps,
                           ids=0, wts=W("bqkv") if d.bias else 0,
                           mode=op_gemv.MODE_NORM | (op_gemv.MODE_BIAS if d.bias else 0) | (0 if first else xmode | WI) | WO, nb=1)
         blob = with_words(blob, z=(L, "z1"), **({"out": (L, "qkv")} if awords else {}))
@@ -490,7 +495,7 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
                                        kw=W("kn") if d.qk_norm else 0, cos_sin=ptr("cos_sin"), kc=ptr("kc") + L * kv_layer_bytes,
                                        vc=ptr("vc") + L * kv_layer_bytes, block_tables=ptr("block_tables"), seq_lens=ptr("seq_lens"),
                                        positions=ptr("positions"), slot_mapping=ptr("slot_mapping"), exp_sums=source("exp_sums", L, "attn", awords),
-                                       max_logits=ptr("max_logits"), tmp_out=ptr("tmp_out"), out=ptr("attn_out"),
+                                       max_logits=ptr("max_logits"), tmp_out=ptr("tmp_out"), out=kept("attn_out", L, awords),
                                        counters=ptr("attn_counters") + 4 * L * d.NH, scale=scale, eps=d.eps, NH=d.NH, NKV=d.NKV, HD=d.HD,
                                        BS=BS, X=X, max_parts=nparts, gq=gq, part_len=op_attn.tagged_part_len(L, words=awords, lim=op_attn.GQ_LIM) if gq else plen)
             prev = add(f"attn_{L}", "attn_fused", "attn_fused", L, blob, ntask, (ntask,), prev, "i->(0)",
@@ -514,7 +519,7 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
 
         # ---- o_proj
         t, rpt = sz.o
-        blob = gemv_block("dsl_gemv", t, W=W("wo"), x=source("attn_out", L, "attn", awords), out=ptr("o"), M=d.H, K=d.NH * d.HD, rpt=rpt, tpe=1, eps=d.eps, nb=1,
+        blob = gemv_block("dsl_gemv", t, W=W("wo"), x=source("attn_out", L, "attn", awords), out=kept("o", L), M=d.H, K=d.NH * d.HD, rpt=rpt, tpe=1, eps=d.eps, nb=1,
                           rows=xblock(L, 0), mode=xmode | (WI if awords else 0) | WO)
         blob = with_words(blob, out=(L, "o"))
         before_x = prev
@@ -523,8 +528,8 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
         if d.moe:
             # ---- router with the post-attention norm fold: task 0 stores resid2 and the normed vector
             t, rpt = sz.router
-            blob = gemv_block("dsl_gemv_fold", t, W=W("wr"), x=ptr("o_norm"), out=ptr("rlog"), M=d.E, K=d.H, rpt=rpt, tpe=1, rows=xblock(L, 0) or source("o", L, "o"),
-                              resid_in=source("resid", L, "z1"), resid_out=ptr("resid2"), ln=W("ln2"), R=ranks, eps=d.eps, mode=op_gemv.MODE_NORM | xmode | WI | WO, nb=1)
+            blob = gemv_block("dsl_gemv_fold", t, W=W("wr"), x=kept("o_norm", L), out=kept("rlog", L), M=d.E, K=d.H, rpt=rpt, tpe=1, rows=xblock(L, 0) or source("o", L, "o"),
+                              resid_in=source("resid", L, "z1"), resid_out=kept("resid2", L), ln=W("ln2"), R=ranks, eps=d.eps, mode=op_gemv.MODE_NORM | xmode | WI | WO, nb=1)
             blob = with_words(blob, out=(L, "rlog"), z=(L, "z2"), x=(L, "x2"))
             prev = add(f"router_{L}", "dsl_gemv_fold", "router", L, blob, t, (t,), fold_in, "i->(0)", f"E_rt_{L}", "i->(0)", (1,), t, d.E, d.H, after="")
             topk_mode = (op_gemv.MODE_TOPK_RENORM if d.norm_topk else op_gemv.MODE_TOPK) | hf_mode
@@ -538,15 +543,15 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
             spt, tpe, rpt = sz.up
             groups = slots // spt
             up_export = "dsl_moe_up_fold" if fold_topk else "dsl_moe_up"
-            blob = gemv_block(up_export, groups * tpe, W=W("w13"), x=source("o_norm", L, "x2"), out=ptr("mc2"),
-                              ids=ptr("ti"), wts=ptr("tw"), estride=2 * d.MI * d.H, M=d.MI, K=d.H, rpt=rpt, tpe=tpe, R=d.TOPK, eps=d.eps,
+            blob = gemv_block(up_export, groups * tpe, W=W("w13"), x=source("o_norm", L, "x2"), out=kept("mc2", L),
+                              ids=kept("ti", L), wts=kept("tw", L), estride=2 * d.MI * d.H, M=d.MI, K=d.H, rpt=rpt, tpe=tpe, R=d.TOPK, eps=d.eps,
                               mode=(topk_mode if fold_topk else 0) | op_gemv.mode_spt(spt) | WI | WO, E=d.E, logits=source("rlog", L, "rlog"), nb=1)
             blob = with_words(blob, out=(L, "act"), route=(L, "route"))
             prev = add(f"moe_up_{L}", up_export, "moe_up", L, blob, groups * tpe, (groups * tpe,),
                        prev, "i->(0)", f"E_up_{L}", "i->(0)", (1,), groups * tpe, d.MI, d.H)
             tpe, rpt = sz.down
             dn_export = "dsl_moe_down_fold" if fold_topk else "dsl_moe_down"
-            blob = gemv_block(dn_export, tpe, W=W("w2"), x=source("mc2", L, "act"), out=ptr("moe_out"), ids=ptr("ti"), wts=ptr("tw"), rows=xblock(L, 1),
+            blob = gemv_block(dn_export, tpe, W=W("w2"), x=source("mc2", L, "act"), out=kept("moe_out", L), ids=ptr("ti"), wts=ptr("tw"), rows=xblock(L, 1),
                               estride=d.H * d.MI, M=d.H, K=d.MI, rpt=rpt, tpe=tpe, R=d.TOPK, eps=d.eps,
                               mode=(topk_mode | op_gemv.MODE_ROUTE_READY if fold_topk else 0) | op_gemv.mode_spt(slots) | op_gemv.MODE_SUM_SLOTS | xmode | WI | WO, E=d.E, logits=source("rlog", L, "rlog"), nb=1)
             blob = with_words(blob, out=(L, "out"), route=(L, "route"))
@@ -557,13 +562,13 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
         else:
             # ---- dense SwiGLU: gate+up with the post-attention norm fold, then down
             spt, tpe, rpt = sz.up
-            blob = gemv_block("dsl_moe_up", tpe, W=W("wgu"), x=ptr("o_norm"), out=ptr("mc2"), estride=0, M=d.INTER, K=d.H, rpt=rpt, tpe=tpe,
-                              rows=xblock(L, 0) or source("o", L, "o"), resid_in=source("resid", L, "z1"), resid_out=ptr("resid2"), ln=W("ln2"), R=ranks, eps=d.eps,
+            blob = gemv_block("dsl_moe_up", tpe, W=W("wgu"), x=kept("o_norm", L), out=kept("mc2", L), estride=0, M=d.INTER, K=d.H, rpt=rpt, tpe=tpe,
+                              rows=xblock(L, 0) or source("o", L, "o"), resid_in=source("resid", L, "z1"), resid_out=kept("resid2", L), ln=W("ln2"), R=ranks, eps=d.eps,
                               mode=op_gemv.MODE_NORM | xmode | WI | WO, nb=1)
             blob = with_words(blob, out=(L, "act"), z=(L, "z2"))
             prev = add(f"gate_up_{L}", "dsl_moe_up", "gate_up", L, blob, tpe, (tpe,), fold_in, "i->(0)", f"E_up_{L}", "i->(0)", (1,), tpe, d.INTER, d.H, after="")
             tpe, rpt = sz.down
-            blob = gemv_block("dsl_moe_down", tpe, W=W("wd"), x=source("mc2", L, "act"), out=ptr("moe_out"), estride=0, M=d.H, K=d.INTER, rpt=rpt, tpe=tpe,
+            blob = gemv_block("dsl_moe_down", tpe, W=W("wd"), x=source("mc2", L, "act"), out=kept("moe_out", L), estride=0, M=d.H, K=d.INTER, rpt=rpt, tpe=tpe,
                               eps=d.eps, nb=1, rows=xblock(L, 1), mode=xmode | WI | WO)
             blob = with_words(blob, out=(L, "out"))
             before_x = prev

@@ -131,6 +131,44 @@ def test_words_are_refused_where_nobody_flags_them():
         op_launch("gemv", gemv.words_block(blob, out=t.data_ptr()), 1)
 
 
+def test_a_reader_of_vectors_behind_words_is_refused():
+    """A grid that hands words over does not wait for its bf16 stores: a plan whose next grid reads the bf16 vector does not run."""
+    from etx_megakernel_b200 import ops
+    from etx_megakernel_b200.frontends import cuda_link
+    from etx_megakernel_b200.importer import argblock
+    from etx_megakernel_b200.ir import Graph
+    from etx_megakernel_b200.ops import gemv
+    from etx_megakernel_b200.passes import compile_graph
+    from etx_megakernel_b200.runtime import Session
+    from etx_megakernel_b200.runtime.lib import EtxbError
+    W = torch.zeros((64, 64), dtype=torch.bfloat16, device=DEV)
+    x, y, z = (torch.zeros(64, dtype=torch.bfloat16, device=DEV) for _ in range(3))
+    words = torch.zeros(64, dtype=torch.int32, device=DEV)
+    f = dict(W=W.data_ptr(), M=64, K=64, rpt=64, tpe=1, nb=1)
+    first = gemv.words_block(argblock.pack_named(ops.all_entries()["dsl_gemv"], (1, 1, 1), x=x.data_ptr(), out=y.data_ptr(), mode=gemv.MODE_WORDS_OUT, **f), out=words.data_ptr())
+
+    def session(second):
+        g = Graph("readers")
+        g.tensor("impargs", (len(first) + len(second),), role="weight", bytes_per_elem=1)
+        g.etensor("E_a", (1,), wait_count=1)
+        g.etensor("E_b", (1,), wait_count=1)
+        g.call_device("a", (1,), cuda_link("", "etx_tile_dsl_gemv", stream_after=""), args=["impargs"], consts=(0,), out_edges={"E_a": "i->(0)"})
+        g.call_device("b", (1,), cuda_link("", "etx_tile_dsl_gemv", stream_after=""), args=["impargs"], consts=(len(first),), in_edges={"E_a": "i->(0)"}, out_edges={"E_b": "i->(0)"})
+        return Session(compile_graph(g, "b200", {}), {}, first + second, 0)
+    ent = ops.all_entries()["dsl_gemv"]
+    for at in (y, y[8:]):                                           # the vector, and a part of it
+        s = session(argblock.pack_named(ent, (1, 1, 1), x=at.data_ptr(), out=z.data_ptr(), **{**f, "K": at.numel()}))
+        with pytest.raises(EtxbError, match="words"):
+            s.run(5.0)
+        s.close()
+    s = session(gemv.words_block(argblock.pack_named(ent, (1, 1, 1), x=words.data_ptr(), out=z.data_ptr(), mode=gemv.MODE_WORDS_IN, **f)))
+    s.run(5.0)
+    s.close()
+    s = session(argblock.pack_named(ent, (1, 1, 1), x=x.data_ptr(), out=z.data_ptr(), **f))       # (another vector)
+    s.run(5.0)
+    s.close()
+
+
 def test_latent_attention_words_give_the_bits_of_the_vectors(monkeypatch):
     """Two layers (dense, experts) of the latent-attention model; 11 partitions are two rounds of the finishing tasks."""
     from etx_megakernel_b200.models import dsv2 as M

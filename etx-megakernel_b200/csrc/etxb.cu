@@ -1264,11 +1264,14 @@ extern "C" int32_t etxb_decode_host(etxb_session* s, const int32_t* tokens_in, i
     if (rc) return rc;
     if (t > 0 && step_ms) { CU(cudaEventSynchronize(y1)); CU(cudaEventElapsedTime(step_ms + t - 1, y0, y1)); }
     const auto t0 = std::chrono::steady_clock::now();
+    bool patient = false;                                          // a step of more than 0.2 ms: the core is other threads', too, while it runs
     for (uint32_t n = 1; *tok_out == INT32_MIN; ++n) {
-      if ((n & 4095u) != 0) continue;
+      if (patient) std::this_thread::yield();
+      if ((n & (patient ? 255u : 4095u)) != 0) continue;
       const cudaError_t q = cudaStreamQuery(st);
       if (q != cudaSuccess && q != cudaErrorNotReady) return fail(ETXB_E_CUDA, std::string("kernel failed: ") + cudaGetErrorString(q));
       const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+      patient = el > 200e-6;
       if ((q == cudaSuccess && *tok_out == INT32_MIN) || el > 60.0) {          // over without a token, or the host's watchdog
         rc = etxb_wait(s, 1e-3);
         return rc ? rc : fail(ETXB_E_ABORTED, "a step ended without a token");

@@ -178,8 +178,10 @@ int32_t etxb_trace(etxb_session* s, void* host_buf, size_t bytes);
 int32_t etxb_exec_counts(etxb_session* s, int32_t* host_buf, size_t count);
 int32_t etxb_destroy(etxb_session* s);
 
-/* Greedy decode with HOST buffers: token ids come from and go back to host memory every step (one 8-byte H2D of
- * {token, position} through pinned memory and one 4-byte D2H per step, both inside the call).  tokens_in[n_in] are
+/* Greedy decode with HOST buffers: token ids come from and go back to host memory every step.  One sequence: the step's prologue
+ * reads its 4-byte token from pinned host memory and its argmax writes the next one there, and the host launches the following step when
+ * it sees that one (a step that fails ends the call with its error; the tokens of the steps before it are in tokens_out, and the
+ * session can be used again).  Plans of several columns: a 4-byte copy each way around every step.  tokens_in[n_in] are
  * fed first (teacher-forced); generation continues greedily until n_total steps ran.  tokens_out[n_total] receives
  * the argmax of every step.  start_pos is the position of tokens_in[0]. */
 int32_t etxb_decode_host(etxb_session* s, const int32_t* tokens_in, int32_t n_in, int32_t n_total,

@@ -385,8 +385,8 @@ __device__ __forceinline__ void producer_loop(const etxb_params& p, const Smem& 
     // (a down grid behind its gate+up grid: the ids are there.  With the event waited for and the top-k done again, 2 us, its stream began
     // when the gate+up rows in the ring were used up)
     if (!(t->in_n & ETXB_IN_ROUTED)) {
-    if (!producer_wait(p, sm, t, cur)) break;
-    if (gt.n > 0 && body != 3) gemv_routing<LEAN, SH>(*pa, sm.prod, nullptr);    // (the ids alone: the stream waits for them)
+      if (!producer_wait(p, sm, t, cur)) break;
+      if (gt.n > 0 && body != 3) gemv_routing<LEAN, SH>(*pa, sm.prod, nullptr);  // (the ids alone: the stream waits for them)
     }
     ok = produce_task<SH>(body, *pa, gt, gg.rps, gg.spr != 0, sm.prod, n, sm, cur, p.trace ? p.trace + 8 * (size_t)t->id : nullptr);
   }
@@ -491,7 +491,10 @@ __global__ void __launch_bounds__(ETXB_THREADS, 1) etxb_megakernel(const __grid_
       fetch_ctx(p, ctx, vars->q0, cur + 2 < q1 ? cur + 2 : -1, cur + 1 < q1 ? cur + 1 : -1);
     }
     csync();
-    if (vars->halt) break;
+    if (vars->halt) {                                              // the context copies of this task are waited for at its end otherwise
+      if (tidx() >= ETXB_CONSUMERS - 32) cp_async_wait_all();
+      break;
+    }
     run_body<KV, XCH>(p, c, cur, smem_view(), n);
     cur = vars->cur;                                               // (before the barrier: thread 0 moves it on behind it)
     c = ctx + ((cur - vars->q0) & (ETXB_CTX_SLOTS - 1));

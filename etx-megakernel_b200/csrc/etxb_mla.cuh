@@ -74,7 +74,9 @@ __device__ __forceinline__ void mla_finish(const etxb_mla_args& d, const Smem& s
   cp_async_commit();
   const uint2* ph = (const uint2*)d.tmp + (size_t)h * d.max_parts * PW;
   // A round: up to NF partitions' statistics (a lane each, every warp for itself) and this thread's values of them, requested together: behind the
-  // slowest partition comes one trip to L2.  Between rounds (contexts of more than 1280 positions) the sums are rescaled to the larger maximum.
+  // slowest partition comes one trip to L2.  Between rounds (contexts of more than 1280 positions) the sums are rescaled to the larger maximum:
+  // rms error of the weighted means at 4080 / 8150 positions 1.39e-7 / 1.72e-7, with all maxima waited for first 1.35e-7 / 1.70e-7, and 4 layers at 4080 in 440 us
+  // instead of 428; the same scheme over the former sums of the warps 1.36e-7 / 1.69e-7 (and 6.3e-8 for the sum of the weights, so 4.1e-8).
   // (Statistics, then weights by one warp, then values, a barrier between any two, and bf16 vectors instead of words: 18.1 us a phase at 1043 positions, so 15.6.)
   constexpr int NF = 10;
   const uint2* vp = ph + min(tid, C - 1);

@@ -74,3 +74,40 @@ def test_rows_whose_score_is_minus_infinity_take_no_part():
         else:
             assert np.isnan(want).all() and np.isnan(got).all()
     assert finite == 1
+
+
+@pytest.mark.parametrize("ctx", [5, 1043, 1290, 4095, 8150])
+def test_long_contexts_to_fp32(ctx):
+    """Weighted means to 32 bits, through the bf16 output: latent columns that hold one constant c_j at every position have c_j as their mean whatever the
+    weights are, and an output row c_k o_j - c_j o_k leaves the errors of the sums alone.  The roundings in a mean: 8 positions a warp, 16 warps,
+    the partitions, once more for the sum of the weights, the division and the product."""
+    NH, C, DN, DR, DV, maxlen = 2, 512, 128, 64, 128, ctx + 9
+    d = M.MlaDims(name="t", H=NH * DV, NH=NH, C=C, DN=DN, DR=DR, DV=DV, MI=128, E=4, TOPK=2, NS=0, DENSE_LAYERS=0, DENSE_INTER=0, L=1, V=256)
+    rng = np.random.default_rng(ctx)
+    const = rng.integers(4, 16, 480).astype(np.float32) / 8                            # (short mantissas: c_k o_j rounds once)
+    cache = np.zeros((maxlen, d.ROW), np.float32)
+    cache[:ctx, :480] = const
+    cache[:ctx, 480:] = bfr(rng.standard_normal((ctx, d.ROW - 480), dtype=np.float32))
+    cache[:ctx, 480] = bfr(8 * np.arange(ctx, dtype=np.float32) / ctx)                 # the partitions' maxima differ, most grow
+    wkvb = np.zeros((NH, DN + DV, C), np.float32)
+    wkvb[:, :DN, 480:] = bfr(0.3 * rng.standard_normal((NH, DN, 32), dtype=np.float32))
+    pair = rng.permuted(np.tile(np.arange(480), (NH * DV, 1)), axis=1)[:, :2].reshape(NH, DV, 2)
+    for h in range(NH):
+        for v in range(DV):
+            j, k = pair[h, v]
+            wkvb[h, DN + v, j], wkvb[h, DN + v, k] = const[k], -const[j]
+    qkv = np.concatenate([bfr(rng.standard_normal(NH * (DN + DR), dtype=np.float32)), np.ones(C, np.float32), bfr(rng.standard_normal(DR, dtype=np.float32))])
+    ln = np.concatenate([const, np.ones(32, np.float32)])                              # the new position's normed latent: the constants again
+    nparts = op_mla.partitions(maxlen)
+    tasks = NH * (nparts + op_mla.FINISHERS)
+    t = {"qkv": dev_bf16(qkv), "kvln": dev_bf16(ln), "wkvb": dev_bf16(wkvb.reshape(-1, C)), "cos_sin": torch.from_numpy(M.yarn_table(d, maxlen)).to(DEV),
+         "cache": dev_bf16(cache), "positions": torch.tensor([ctx], dtype=torch.int64, device=DEV), "out": torch.zeros(NH * DV, dtype=torch.bfloat16, device=DEV),
+         "tmp": torch.zeros((op_mla.tmp_pairs(NH, C, maxlen), 2), dtype=torch.float32, device=DEV)}
+    op_launch("mla_attn", argblock.pack_named(ops.all_entries()["mla_attn"], (tasks, 1, 1), **{n: v.data_ptr() for n, v in t.items()}, NH=NH, C=C, DN=DN, DR=DR, DV=DV,
+                                              maxlen=maxlen, scale=d.scale, eps=d.eps, max_parts=nparts, tag=3), tasks)
+    got = host(t["out"]).reshape(NH, DV)
+    assert np.array_equal(host(t["cache"])[ctx, :480], const)
+    size = const[pair[..., 0]] * const[pair[..., 1]]
+    roundings = 2 * (8 + 16 + -(-(ctx + 1) // 128)) + 2
+    assert np.isfinite(got).all() and np.abs(got).max() > 0 or ctx < 10
+    assert (np.abs(got) <= 2 * roundings * 2.0 ** -24 * size).all(), np.abs(got / size).max()

@@ -20,7 +20,7 @@ from tests.test_gpu_ops import dev_bf16, host  # noqa: E402
 DEV, HD, SCALE = "cuda:0", 128, float(np.float32(1.0 / np.sqrt(128)))
 
 
-def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True, behind=None, norm=None, seqs=None, pos=None):
+def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True, behind=None, norm=None, seqs=None, pos=None, lim=0):
     """One attention grid over B sequences.  K, V: per sequence [seq][NKV][HD], the last position being the new one (its cache row holds NaN and comes from qkv
     [B][NH + 2 NKV][HD] instead).  Returns (out [B][NH][HD] bf16 values, the cached k rows at the new positions [B][NKV][HD], the partials
     [B][NH][partitions][128 sums, maximum, sum of the probabilities]).  behind: a second grid of one empty task that waits for the first attention task
@@ -52,7 +52,7 @@ def run(NH, NKV, K, V, qkv, maxlen, gq, whole=False, scale=SCALE, rotary=True, b
             "tmp_out": NH * parts * ops.attn.GQ_PARTIAL_FLOATS * 4, "out": NH * HD * 2}
     ntask = NH // gq * (1 if whole else parts)
     blobs = b"".join(argblock.pack_named(ops.all_entries()["attn_fused"], (ntask, 1, 1), **{n: x.data_ptr() + b * step.get(n, 0) for n, x in t.items()}, scale=scale,
-                                         eps=1e-6, NH=NH, NKV=NKV, HD=HD, BS=16, X=8, max_parts=parts, gq=gq, part_len=ops.attn.tagged_part_len(3, whole)) for b in range(B))
+                                         eps=1e-6, NH=NH, NKV=NKV, HD=HD, BS=16, X=8, max_parts=parts, gq=gq, part_len=ops.attn.tagged_part_len(3, whole, lim=lim)) for b in range(B))
     g = Graph("attn")
     g.tensor("impargs", (len(blobs),), role="weight", bytes_per_elem=1)
     if behind is None:
@@ -156,11 +156,8 @@ def test_partials_are_as_exact_as_fp32_chains(seq, NH, NKV, gq):
     assert got <= plain
 
 
-@pytest.mark.parametrize("whole", [True, False])
-def test_the_new_position_keeps_all_bits_of_its_probability(whole):
-    """Two cached positions of probability 1 take away the first two bf16 parts of the new position's, so what is left of the sum is its third part (2^-18
-    of it and less): 0 if that part were not multiplied.  A difference of two units in the last place of exp() is 2^-5 of what is left."""
-    NH, gq = 8, 8
+def third_parts(NH):
+    """NH differences of scores whose probability has a third bf16 part of 2^-19 of it and more, and the probability with its parts."""
     d = np.arange(1, 4096, dtype=np.float32) / np.float32(1024)                          # bf16-exact differences of the scores, the third parts largest
     d = d[O.bfr(d) == d]
     p = np.exp(-d.astype(np.float64)).astype(np.float32)
@@ -170,6 +167,15 @@ def test_the_new_position_keeps_all_bits_of_its_probability(whole):
     best = np.argsort(-np.abs(third) / p)[:NH]
     d, first, second, third, p = (x[best].astype(np.float64) for x in (d, first, second, third, p))
     assert np.all(np.abs(third) / p > 2.0 ** -19)
+    return d, first, second, third, p
+
+
+@pytest.mark.parametrize("whole", [True, False])
+def test_the_new_position_keeps_all_bits_of_its_probability(whole):
+    """Two cached positions of probability 1 take away the first two bf16 parts of the new position's, so what is left of the sum is its third part (2^-18
+    of it and less): 0 if that part were not multiplied.  A difference of two units in the last place of exp() is 2^-5 of what is left."""
+    NH, gq = 8, 8
+    d, first, second, third, p = third_parts(NH)
     K, V, qkv = np.zeros((3, 1, HD), np.float32), np.zeros((3, 1, HD), np.float32), np.zeros((NH + 2, HD), np.float32)
     K[:2, 0, 0], qkv[:NH, 0] = 1.0, d                                                    # score of a cached position: d of the head, of the new one: 0
     V[0, 0, :NH], V[1, 0, :NH], qkv[NH + 1, :NH] = -first, -second, 1.0
@@ -177,6 +183,22 @@ def test_the_new_position_keeps_all_bits_of_its_probability(whole):
     want = third / (2.0 + p)
     got = out[0, np.arange(NH), np.arange(NH)]
     assert np.all(np.abs(got - want) <= 2.0 ** -4 * np.abs(want)), (got, want)
+
+
+@pytest.mark.parametrize("whole,lim,all_bits", [(False, 0, True), (False, 2, True), (True, 1, True), (True, 0, False)])
+def test_a_cached_position_keeps_all_bits_of_its_probability(whole, lim, all_bits):
+    """The same with the third of the three in the cache, in a unit of 16 positions that the new one is not in (its probability and those of the others are
+    below 2^-100): partitions and contexts up to the limit keep 24 bits, whole contexts where the block asks for them, else 17."""
+    NH, gq, seq = 8, 8, 40
+    d, first, second, third, p = third_parts(NH)
+    K, V, qkv = np.zeros((seq, 1, HD), np.float32), np.zeros((seq, 1, HD), np.float32), np.zeros((NH + 2, HD), np.float32)
+    K[:2, 0, 0], K[3:, 0, 1], qkv[NH, 1] = 1.0, -128.0, -128.0
+    qkv[:NH, 0], qkv[:NH, 1] = d, 1.0                                                    # scores: d, d, 0, then -128
+    V[0, 0, :NH], V[1, 0, :NH], V[2, 0, :NH] = -first, -second, 1.0
+    out, _, _ = run(NH, 1, [K], [V], qkv[None], 128, gq, whole=whole, scale=1.0, rotary=False, lim=lim)
+    want = third / (2.0 + p)
+    got = out[0, np.arange(NH), np.arange(NH)]
+    assert np.all(np.abs(got - want) <= 2.0 ** -4 * np.abs(want)) == all_bits, (got, want)
 
 
 @pytest.mark.parametrize("seq,NH,NKV,gq,whole", [(300, 8, 2, 4, False), (40, 8, 1, 8, False), (300, 8, 2, 4, True)])

@@ -12,6 +12,7 @@ import etx_megakernel_b200  # noqa: E402,F401
 from etx_megakernel_b200.models import batched as BT  # noqa: E402
 from etx_megakernel_b200.models import decode as D  # noqa: E402
 from etx_megakernel_b200.models import qwen as Q  # noqa: E402
+from etx_megakernel_b200.ops import attn as op_attn  # noqa: E402
 from oracle import ref_decode as O  # noqa: E402
 from tests.golden.cases import SMALL_MOE  # noqa: E402
 
@@ -60,7 +61,7 @@ def check_columns(name, got, od, W, prompts, n_gen, ctx):
     return identical
 
 
-@pytest.mark.parametrize("od,B,engine", [(SMALL_MOE, 4, "tc"), (MID, 8, "tc"), (MID, 32, "tc"), (MID, 40, "tc"), (SMALL_MOE, 4, "mma"), (MID, 32, "mma")])
+@pytest.mark.parametrize("od,B,engine", [(SMALL_MOE, 4, "tc"), (MID, 8, "tc"), (MID, 13, "tc"), (MID, 32, "tc"), (MID, 40, "tc"), (SMALL_MOE, 4, "mma"), (MID, 32, "mma")])
 def test_batched_greedy_tokens_per_column(od, B, engine):
     """Both engines of the batched grids: tcgen05.mma (TMA tensor copies, accumulators in tensor memory; 40 columns = two
     passes of the dense grids) and the mma.sync tiles."""
@@ -91,11 +92,12 @@ def test_columns_do_not_depend_on_their_neighbours():
     prog.close()
 
 
-def test_whole_sequence_attention_agrees_with_the_partitioned_form():
+def test_whole_sequence_attention_agrees_with_the_partitioned_form(monkeypatch):
     """20 sequences of a 150-token prompt (two partitions of 128 positions) through ONE layer, so that nothing but the
     attention phase separates the two forms: at B = 20 the attention grid has one task per (sequence, kv head) that
     takes the whole context (the probabilities of cached positions as a bf16 value plus the bf16 of its rounding error);
-    at B = 10 it has one task per partition (a third bf16 part) and a merge through flagged partials.  Sums in another order: the KV
+    at B = 10 it has one task per partition (a third bf16 part) and a merge through flagged partials, where contexts of two
+    partitions are not taken whole (limit 0).  Sums in another order: the KV
     caches are bit-identical, the attention output agrees within 2 bf16 ulps per element with >= 90 % of the elements
     identical.  (Through several MoE layers a one-ulp difference can flip a near-tie routing decision, which is why the
     multi-layer comparisons are made against the oracle with its tie rule, not between the two forms.)"""
@@ -108,10 +110,13 @@ def test_whole_sequence_attention_agrees_with_the_partitioned_form():
     whole.generate(prompts, 1)
     att, kc, vc = whole.read("attn_out"), whole.read("kc"), whole.read("vc")
     whole.close()
+    monkeypatch.setattr(op_attn, "GQ_LIM", 0)
     for half in range(2):
         part = program(od, W, 10, 192)
         assert not part.info["attn_whole"]
         part.generate(prompts[10 * half: 10 * half + 10], 1)
+        flags = part.buf["tmp_out"].view(torch.int32).reshape(-1, 2)[:, 1]
+        assert int((flags != 0).sum()) == 10 * od.NH * 2 * 130       # both partitions' partials were published: 128 sums, maximum, sum
         patt, pkc, pvc = part.read("attn_out"), part.read("kc"), part.read("vc")
         part.close()
         nblk = pkc.shape[1] // 10
@@ -189,7 +194,7 @@ def test_an_expert_with_more_tokens_than_one_pass(engine):
         assert top2[1] - top2[0] <= 4 * abs(top2[1]) * 2.0 ** -7
 
 
-@pytest.mark.parametrize("B,whole", [(5, False), (20, True), (40, True)])
+@pytest.mark.parametrize("B,whole", [(5, False), (10, False), (11, True), (18, True), (20, True), (40, True)])
 def test_the_batched_plan_gets_its_own_kernel_and_matches_the_full_one(B, whole):
     """A batched step on the tensor cores (one attention argument block per sequence, either attention form, one or two
     passes of the dense grids) runs on the kernel that holds only its tiles; the full kernel gives the same bits."""

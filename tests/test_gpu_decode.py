@@ -10,6 +10,7 @@ pytestmark = pytest.mark.gpu
 import etx_megakernel_b200  # noqa: E402,F401
 from etx_megakernel_b200.models import decode as D  # noqa: E402
 from etx_megakernel_b200.models import qwen as Q  # noqa: E402
+from etx_megakernel_b200.ops import attn as op_attn  # noqa: E402
 from etx_megakernel_b200.runtime import EtxbError  # noqa: E402
 from oracle import ref_decode as O  # noqa: E402
 from tests.golden.cases import SMALL_DENSE, SMALL_MOE  # noqa: E402
@@ -169,13 +170,16 @@ def test_lean_kernel_is_picked_for_decode_plans_and_matches_the_full_kernel():
     dense.close()
 
 
-def test_decode_across_partition_and_block_boundaries_up_to_the_last_cache_position():
-    """A context that grows through the 128-position partition boundary of the grouped attention tile, through 16-position
-    cache block boundaries, and ends on the very last position the cache has: tokens against the oracle (tie rule)."""
+@pytest.mark.parametrize("n_prompt,n_gen,maxlen,limit", [(118, 27, 144, 2), (118, 27, 144, 0), (246, 27, 272, 2)])
+def test_decode_across_partition_and_block_boundaries_up_to_the_last_cache_position(monkeypatch, n_prompt, n_gen, maxlen, limit):
+    """A context that grows through the 128-position partition boundary of the grouped attention tile (taken whole, and merged), through the
+    256 positions up to which it is taken whole, through 16-position cache block boundaries, and ends on the very last position the cache has: tokens
+    against the oracle (tie rule)."""
+    monkeypatch.setattr(op_attn, "GQ_LIM", limit)
     od = O.Dims(name="edge", H=256, NH=4, NKV=2, HD=128, INTER=0, L=2, V=512, qk_norm=True, moe=True, E=8, TOPK=2, MI=64, norm_topk=True)
     W = O.SyntheticWeights(od, seed=21, gamma="ones")
-    prompt = np.random.default_rng(22).integers(0, od.V, 118)
-    check_greedy(od, W, prompt, 27, 144)                                    # positions 0 .. 143 = maxlen - 1
+    prompt = np.random.default_rng(22).integers(0, od.V, n_prompt)
+    check_greedy(od, W, prompt, n_gen, maxlen)                              # positions 0 .. maxlen - 1
 
 
 def test_launch_per_grid_baseline_gives_the_same_tokens():

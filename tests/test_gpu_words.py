@@ -66,6 +66,42 @@ def test_words_of_a_width_that_is_no_power_of_two(monkeypatch):
             assert np.linalg.norm(g[n] - e[n]) <= 2.0 ** -8 * np.linalg.norm(e[n]), n
 
 
+@pytest.mark.parametrize("K", [64, 1024, 1096, 1536, 2880, 8184, 8192])
+def test_the_norms_mean_to_fp32(K):
+    """The norm fold of a grid that writes words, against 64-bit sums: a value of the normed vector may differ from the one rounded from 64 bits only where it
+    lies within the fp32 roundings of the boundary between two.  Those of 1 / sqrt(mean + eps): a square, 15 + 3 + 6 sums, the mean and its eps, all
+    halved by the root, then root, division and product: 17, so 20 units of 2^-24."""
+    from etx_megakernel_b200 import ops
+    from etx_megakernel_b200.frontends import cuda_link
+    from etx_megakernel_b200.importer import argblock
+    from etx_megakernel_b200.ir import Graph
+    from etx_megakernel_b200.ops import gemv
+    from etx_megakernel_b200.passes import compile_graph
+    from etx_megakernel_b200.runtime import Session
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(K)
+    z = torch.empty(K, dtype=torch.bfloat16, device=DEV).normal_(0, 1.5, generator=gen)
+    ln, W = torch.ones(K, dtype=torch.bfloat16, device=DEV), torch.zeros((8, K), dtype=torch.bfloat16, device=DEV)
+    x, out = torch.zeros_like(z), torch.zeros(8, dtype=torch.bfloat16, device=DEV)
+    words = torch.zeros(K + 8, dtype=torch.int32, device=DEV)
+    blob = gemv.words_block(argblock.pack_named(ops.all_entries()["dsl_gemv_fold"], (1, 1, 1), W=W.data_ptr(), x=x.data_ptr(), out=out.data_ptr(), M=8, K=K, rpt=8, tpe=1,
+                                                rows=0, resid_in=z.data_ptr(), resid_out=0, ln=ln.data_ptr(), R=0, eps=1e-6, mode=gemv.MODE_NORM | gemv.MODE_WORDS_OUT, nb=1),
+                            out=words.data_ptr() + 4 * K, x=words.data_ptr())
+    g = Graph("norm")
+    g.tensor("impargs", (len(blob),), role="weight", bytes_per_elem=1)
+    g.etensor("E_done", (1,), wait_count=1)
+    g.call_device("norm", (1,), cuda_link("", "etx_tile_dsl_gemv_fold", stream_after=""), args=["impargs"], consts=(0,), out_edges={"E_done": "i->(0)"})
+    s = Session(compile_graph(g, "b200", {}), {}, blob, 0)
+    s.run(5.0)
+    s.close()
+    v = z.double() / torch.sqrt((z.double() ** 2).mean() + float(np.float32(1e-6)))
+    d = 20 * 2.0 ** -24
+    lo, hi = ((v * (1 + t * torch.sign(v))).float().bfloat16().float() for t in (-d, d))
+    lo, hi = torch.minimum(lo, hi), torch.maximum(lo, hi)
+    assert bool(((x.float() >= lo) & (x.float() <= hi)).all())
+    assert torch.equal(x.view(torch.int16).int() & 0xffff, words[:K] & 0xffff)
+
+
 @pytest.mark.parametrize("K,N", [(8, 5), (264, 37), (1792, 900), (2048, 1), (2048, 2000), (2056, 300), (3072, 700), (4096, 1500), (6152, 777), (8960, 100), (12288, 640), (64, 310000)])
 def test_rows_shared_by_the_warps(K, N):
     """One-grid plans: a few rows and many, rows of a lane's one vector to 48, several warps a row, more rows per task than the results' place holds.

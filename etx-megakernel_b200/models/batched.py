@@ -82,8 +82,9 @@ def build_graph(d: Q.Dims, ptr, B: int, maxlen: int = 1072, machine: MachineMode
     W = m.workers()
     gq, plen, gparts = d.G, op_attn.GQ_PART, -(-maxlen // op_attn.GQ_PART)      # one task per (128 positions, kv head): K / V read once
     # enough sequences to fill three tenths of the workers: one task per (sequence, kv head) walks the whole context; else one per partition.
-    # (Whole contexts / partitions, us of 3 layers: 13 sequences at 333 positions 794 / 818, 16 at 700 834 / 869, 16 at 1400 865 / 927, 8 at 600 702 / 714,
-    # 8 at 1033 718 / 718; but 5 at 1400 655 / 637, 2 at 1033 572 / 539.)
+    # (Whole contexts / partitions, us of 3 layers: 11 sequences at 300 positions 766 / 770, at 600 778 / 793, at 1000 791 / 816, at 2400 847 / 905, 12 at 700 789 / 802,
+    # at 1400 816 / 852, at 2400 846 / 937, 13 at 333 794 / 818, 16 at 700 834 / 869, at 1400 865 / 927, at 2400 905 / 1066, 18 at 2400 978 / 1157, 8 at 600 702 / 714,
+    # 8 at 1033 718 / 718; but 5 at 1400 655 / 637, 2 at 1033 572 / 539.  At most 2432 positions: a longer context's partitions do not fit one task.)
     whole = B * (d.NH // gq) >= 3 * W // 10 and op_attn.whole_sequence_fits(gq, gparts)
     precise = B * (d.NH // gq) < W // 2                                      # (fewer sequences than this had partitions: all bits of their probabilities, still)
     ntask = (d.NH // gq) if whole else gparts * (d.NH // gq)

@@ -59,7 +59,9 @@ class DecodeProgram:
             if k not in weights or tuple(weights[k].shape) != tuple(shp):
                 raise ValueError(f"weight {k}: expected shape {shp}, got {tuple(weights[k].shape) if k in weights else None}")
         sz = Q.size_for(dims, self.machine, maxlen)
-        self.buf = {n: torch.zeros(shape, dtype=_DT[dt], device=self.dev) for n, (shape, dt) in Q.buffer_shapes(dims, maxlen, self.steps, sz.parts).items()}
+        words = ranks == 1 and not flagged and fold_topk
+        self.buf = {n: torch.zeros(shape, dtype=_DT[dt], device=self.dev) for n, (shape, dt) in Q.buffer_shapes(dims, maxlen, self.steps, sz.parts).items()
+                    if n != "words" or words}
         self.buf["block_tables"].copy_(torch.arange(self.buf["block_tables"].numel(), dtype=torch.int32))
         self.vl = torch.zeros(1, dtype=torch.int64, device=self.dev)
 
@@ -76,7 +78,7 @@ class DecodeProgram:
             return t.data_ptr()
         self.graph, self.pool, self.sizing = Q.build_graph(dims, ptr, maxlen, self.machine, fold_topk=fold_topk, fused_attn=fused_attn,
                                                               ranks=ranks, rank=rank, flagged=flagged,
-                                                              words=ranks == 1 and not flagged and fold_topk)
+                                                              words=words)
         pool = self.pool.bytes()
         self.plan = compile_graph(self.graph, self.machine, {"POOL": len(pool)}, options=PassOptions(workers=workers))
         self.session = Session(self.plan, {"vl": self.vl}, pool, device)

@@ -390,10 +390,11 @@ def build_graph(d: Dims, ptr, maxlen: int = 1072, machine: MachineModel | str = 
     in an exchange region of one row per block -- the single-GPU form of the sharded hand-off below: the fold polls the
     data itself instead of waiting for the producing grid's event and then loading.
 
-    words (one rank, folded top-k): the vectors a grid hands to the next one of the step also travel as words -- a bf16 value
+    words (one rank, folded top-k): the vectors a grid hands to the next one of the step travel as words -- a bf16 value
     and a flag of the step in 4 bytes -- through ptr("words") (words_layout), every layer through its own.  A word says itself
-    whether it has arrived, so a grid announces itself without waiting for its stores.  Same graph, same arithmetic, the bf16 vectors are
-    written as before.
+    whether it has arrived, so a grid announces itself without waiting for its stores.  Same graph; the bf16 vectors are written by the last layer
+    only.  The arithmetic is the same where the hidden size is a power of two; else a norm's squares are summed by blocks of 128 here and
+    in strided chains there (both in fp32).
 
     ranks > 1: the step of ONE rank of a model sharded `ranks` ways (`d` = shard_dims(full, ranks): its share of the
     heads and of the MLP / expert rows).  ptr("xrows") then names the rank's exchange region: 2 * L blocks of
